@@ -88,6 +88,40 @@ def test_rounding_boundaries_and_many_rows(dt, bits, gs):
     assert np.array_equal(data[0].cpu().numpy(), ref_d)
 
 
+@pytest.mark.parametrize("mode,T,H", [("k3v2", 1, 1), ("k3v2", 15, 3), ("k4v4", 17, 2), ("k3v2", 4097, 1), ("k4v4", 20001, 3)])
+def test_kv_kernel_at_its_edges(mode, T, H):
+    """Token counts around a batch and several batches per block; values the quick arithmetic does not
+    cover (past 2^125, infinite, NaN) in single rows, whose neighbours must not notice."""
+    ops = _ops()
+    kb, vb, gs = {"k3v2": (3, 2, 64), "k4v4": (4, 4, 128)}[mode]
+    g = torch.Generator().manual_seed(T)
+    k = torch.randn(T, H, 128, generator=g).to(torch.bfloat16)
+    v = (torch.randn(T, H, 128, generator=g) * 1e-9).to(torch.bfloat16)   # the clamp of the scale
+    special = [T // 3, T // 2] if T > 8 else []
+    if special:
+        k[special[0], 0, ::3] = 3.0e38          # finite, still exact
+        k[special[1], 0, 5] = float("inf")
+        v[special[1], 0, 7] = float("nan")
+    slots = torch.arange(T, dtype=torch.int64)
+    slots[-1] = -1 if T > 1 else 0
+    num_slots = (T + 15) // 16 * 16
+    kd = torch.full((H, num_slots, 16 * kb), 0xA5, dtype=torch.uint8, device="cuda")
+    vd = torch.full((H, num_slots, 16 * vb), 0xA5, dtype=torch.uint8, device="cuda")
+    ks = torch.zeros(H, num_slots, 128 // gs, dtype=torch.bfloat16, device="cuda")
+    vs = torch.zeros_like(ks)
+    ops.fused_quant_write_kv(k.cuda(), v.cuda(), slots.cuda(), kd, ks, vd, vs, gs, kb, vb)
+    torch.cuda.synchronize()
+    with np.errstate(invalid="ignore"):
+        rk, rks = O.quantize_and_pack(f32_values(k), gs, kb)
+        rv, rvs = O.quantize_and_pack(f32_values(v), gs, vb)
+    keep = np.array([t for t in range(T) if int(slots[t]) >= 0 and t not in special[1:]])
+    for data, scale, rd, rs in ((kd, ks, rk, rks), (vd, vs, rv, rvs)):
+        assert np.array_equal(data.cpu().numpy()[:, keep].transpose(1, 0, 2), rd[keep])
+        assert np.array_equal(to_bits(scale)[:, keep].transpose(1, 0, 2), rs[keep])
+    if T > 1:
+        assert bool((kd[:, T - 1:] == 0xA5).all()) and bool((vd[:, T - 1:] == 0xA5).all())
+
+
 def test_kv_pair_and_out_of_range_slot():
     ops = _ops()
     g = torch.Generator().manual_seed(7)
