@@ -3,8 +3,9 @@
     python -m jetfire_b200.build [--force]
 
 The library is plain C ABI (``include/jetfire_b200.h``); Python loads it with ctypes
-(``jetfire_b200._lib``).  The build is skipped when the library is newer than every
-source file.
+(``jetfire_b200._lib``).  Beside it ``_host.so`` is built from ``csrc/torch_host.cpp``: the
+tensor-taking half of ``ops.py``, a CPython extension against the installed torch and this
+library.  The build is skipped when both are newer than every source file.
 """
 from __future__ import annotations
 
@@ -17,6 +18,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libjetfire_b200.so"
+HOST = PKG / "_host.so"
 SOURCES = ["pack_append.cu", "decode_scan.cu", "decode_scan_k4v4.cu", "topk_select.cu", "decode_finish.cu", "decode_static.cu",
            "jf_misc.cu", "mirror_append.cu", "mirror_correct.cu", "cpu_correction.cpp", "numa_place.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -31,12 +33,26 @@ def nvcc_path() -> str:
 
 
 def up_to_date() -> bool:
-    if not LIB.exists():
+    if not LIB.exists() or not HOST.exists():
         return False
-    t = LIB.stat().st_mtime
+    t = min(LIB.stat().st_mtime, HOST.stat().st_mtime)
     deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.h")) + \
         [PKG.parent / "include" / "jetfire_b200.h"]
     return all(d.stat().st_mtime <= t for d in deps)
+
+
+def host_command(nvcc: str) -> list[str]:
+    """The compile-and-link command of ``_host.so``; its libraries are found next to it at run time."""
+    import sysconfig
+
+    import torch
+    base = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc).resolve().parents[1]
+    inc = [base / "include", base / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in inc),
+            str(CSRC / "torch_host.cpp"), "-o", str(HOST), f"-L{base / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
+            "-ltorch", "-lc10_cuda", "-lc10", f"-L{PKG}", "-ljetfire_b200", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -65,6 +81,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}")
+    r = subprocess.run(host_command(nvcc), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {HOST.name} failed:\n{r.stdout}")
     return LIB
 
 

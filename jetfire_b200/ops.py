@@ -3,7 +3,8 @@
 Names, argument order and meaning follow the reference's torch-extension ops and Triton
 writers so that its adapter can call these unchanged; torch is used only for device
 memory and streams.  Each op validates like the reference's ``TORCH_CHECK``s (raising
-``RuntimeError``) and runs on ``torch.cuda.current_stream()``.
+``RuntimeError``) and runs on ``torch.cuda.current_stream()``.  The ops of the append and decode
+path do their checks, allocations and launches in native code (``jetfire_b200._host``).
 
 Reference interfaces mirrored here (paths inside the JetFire project):
   * ``fused_quant_write_int{2,3,4}_sym`` -- jetfire_vllm/kernels/fused_quant_write.py:242, :337, :746
@@ -22,6 +23,7 @@ import torch
 
 from . import _lib
 from ._lib import DecodeArgs, JetFireError, check, lib
+from . import _host   # after the library it is linked to
 
 MODE_IDS = {"k3v2": _lib.JF_MODE_K3V2, "k4v4": _lib.JF_MODE_K4V4,
             "SymInt3K_SymInt2V": _lib.JF_MODE_K3V2, "SymInt4K_SymInt4V": _lib.JF_MODE_K4V4}
@@ -53,31 +55,8 @@ def _packed_dim(nbits: int) -> int:
     return 128 * nbits // 8
 
 
-def _check_side(x_tok, out_data, out_scale, nbits, group_size, name):
-    _require(x_tok.is_cuda and out_data.is_cuda and out_scale.is_cuda, f"{name}: tensors must be CUDA")
-    _require(x_tok.dim() == 3 and x_tok.shape[2] == 128, f"{name}: x_tok must be (T, H_kv, 128)")
-    _require(x_tok.stride(2) == 1, f"{name}: x_tok innermost dim must be contiguous")
-    _require(out_data.dtype == torch.uint8 and out_data.is_contiguous(), f"{name}: out_data must be contiguous uint8")
-    _require(out_scale.dtype == torch.bfloat16 and out_scale.is_contiguous(), f"{name}: out_scale must be contiguous bf16")
-    _require(group_size in (64, 128), f"{name}: group_size must be 64 or 128")
-    h = x_tok.shape[1]
-    _require(out_data.dim() == 3 and out_data.shape[0] == h and out_data.shape[2] == _packed_dim(nbits),
-             f"{name}: out_data must be (H_kv, num_slots, {_packed_dim(nbits)})")
-    _require(out_scale.shape[0] == h and out_scale.shape[1] == out_data.shape[1]
-             and out_scale.numel() == h * out_data.shape[1] * (128 // group_size),
-             f"{name}: out_scale must be (H_kv, num_slots, {128 // group_size})")
-
-
 def _quant_write(x_tok, slot_idx, out_data, out_scale, group_size, nbits, name):
-    _check_side(x_tok, out_data, out_scale, nbits, group_size, name)
-    _require(slot_idx.is_cuda and slot_idx.dtype == torch.int64 and slot_idx.dim() == 1
-             and slot_idx.shape[0] == x_tok.shape[0], f"{name}: slot_idx must be (T,) int64 CUDA")
-    slot_idx = slot_idx.contiguous()
-    st = lib.jf_pack_append(x_tok.data_ptr(), _dtype_id(x_tok), x_tok.shape[0], x_tok.shape[1],
-                            x_tok.stride(0), x_tok.stride(1), slot_idx.data_ptr(),
-                            out_data.data_ptr(), out_scale.data_ptr(), out_data.shape[1],
-                            nbits, group_size, _stream())
-    check(name, st)
+    check(name, _host.quant_write(name, x_tok, slot_idx, out_data, out_scale, group_size, nbits))
 
 
 def fused_quant_write_int2_sym(x_tok, slot_idx, out_data, out_scale, group_size=128):
@@ -96,33 +75,14 @@ def fused_quant_write_int4_sym(x_tok, slot_idx, out_data, out_scale, group_size=
 def fused_quant_write_kv(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
                          group_size, k_bits, v_bits):
     """K and V of the same tokens in one launch, any bit pair."""
-    name = "fused_quant_write_kv"
-    _check_side(key_tok, k_data, k_scales, k_bits, group_size, name)
-    _check_side(value_tok, v_data, v_scales, v_bits, group_size, name)
-    _require(key_tok.shape == value_tok.shape and key_tok.dtype == value_tok.dtype,
-             f"{name}: key/value shape or dtype mismatch")
-    _require(k_data.shape[1] == v_data.shape[1], f"{name}: K and V caches differ in num_slots")
-    _require(slot_idx.is_cuda and slot_idx.dtype == torch.int64 and slot_idx.dim() == 1
-             and slot_idx.shape[0] == key_tok.shape[0], f"{name}: slot_idx must be (T,) int64 CUDA")
-    slot_idx = slot_idx.contiguous()
-    st = lib.jf_pack_append_kv(key_tok.data_ptr(), value_tok.data_ptr(), _dtype_id(key_tok),
-                               key_tok.shape[0], key_tok.shape[1],
-                               key_tok.stride(0), key_tok.stride(1), value_tok.stride(0), value_tok.stride(1),
-                               slot_idx.data_ptr(), k_data.data_ptr(), k_scales.data_ptr(),
-                               v_data.data_ptr(), v_scales.data_ptr(), k_data.shape[1],
-                               k_bits, v_bits, group_size, _stream())
-    check(name, st)
+    check("fused_quant_write_kv",
+          _host.quant_write_kv("fused_quant_write_kv", key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
+                               group_size, k_bits, v_bits, None, None))
 
 
 def fused_quant_write_int4_sym_kv(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
                                   group_size=128):
     fused_quant_write_kv(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales, group_size, 4, 4)
-
-
-def _check_mirror(t, key_tok, k_data, name):
-    _require(t.is_cuda and t.is_contiguous() and t.dtype == key_tok.dtype and t.dim() == 3
-             and t.shape[0] == k_data.shape[0] and t.shape[1] == k_data.shape[1] and t.shape[2] == 128,
-             f"{name}: mirror must be a contiguous device-visible (H_kv, num_slots, 128) tensor of the tokens' dtype")
 
 
 def fused_quant_write_kv_mirror(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
@@ -133,24 +93,8 @@ def fused_quant_write_kv_mirror(key_tok, value_tok, slot_idx, k_data, k_scales, 
     append is one launch with no host step, in place of the reference's copy + sync +
     index_copy_ (jetfire_vllm/adapter/cache_store.py:746-756)."""
     name = "fused_quant_write_kv_mirror"
-    _check_side(key_tok, k_data, k_scales, k_bits, group_size, name)
-    _check_side(value_tok, v_data, v_scales, v_bits, group_size, name)
-    _require(key_tok.shape == value_tok.shape and key_tok.dtype == value_tok.dtype,
-             f"{name}: key/value shape or dtype mismatch")
-    _require(k_data.shape[1] == v_data.shape[1], f"{name}: K and V caches differ in num_slots")
-    _require(slot_idx.is_cuda and slot_idx.dtype == torch.int64 and slot_idx.dim() == 1
-             and slot_idx.shape[0] == key_tok.shape[0], f"{name}: slot_idx must be (T,) int64 CUDA")
-    _check_mirror(k_mirror_dev, key_tok, k_data, name)
-    _check_mirror(v_mirror_dev, key_tok, k_data, name)
-    slot_idx = slot_idx.contiguous()
-    st = lib.jf_pack_append_kv_mirror(key_tok.data_ptr(), value_tok.data_ptr(), _dtype_id(key_tok),
-                                      key_tok.shape[0], key_tok.shape[1],
-                                      key_tok.stride(0), key_tok.stride(1), value_tok.stride(0), value_tok.stride(1),
-                                      slot_idx.data_ptr(), k_data.data_ptr(), k_scales.data_ptr(),
-                                      v_data.data_ptr(), v_scales.data_ptr(), k_data.shape[1],
-                                      k_bits, v_bits, group_size, k_mirror_dev.data_ptr(), v_mirror_dev.data_ptr(),
-                                      _stream())
-    check(name, st)
+    check(name, _host.quant_write_kv(name, key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales, group_size, k_bits,
+                                     v_bits, k_mirror_dev, v_mirror_dev))
 
 
 def map_host_tensor(host: torch.Tensor) -> torch.Tensor:
@@ -236,7 +180,6 @@ class FusedAttnOut(NamedTuple):
     scores: torch.Tensor | None  # (B, H_q, max_S) f32 when requested
 
 
-_WORKSPACES: dict[tuple[int, int], torch.Tensor] = {}
 _PARTS = {"all": _lib.JF_SCAN_ALL, "k": _lib.JF_SCAN_K_ONLY, "v": _lib.JF_SCAN_V_ONLY}
 _STAGE_B = {"fp32": _lib.JF_STAGE_B_FP32, "int8p": _lib.JF_STAGE_B_INT8P}
 
@@ -247,16 +190,10 @@ def decode_workspace_bytes(mode, B, H_q, H_kv, max_S, top_k) -> int:
 
 
 def get_workspace(nbytes: int, device) -> torch.Tensor:
-    """Cached scratch (grows monotonically per device); one per current stream is the
+    """Cached scratch (grows monotonically per device and stream); one per current stream is the
     caller's business when streams overlap."""
     dev = torch.device(device)
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream().cuda_stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=dev)
-        _WORKSPACES[key] = ws
-    return ws
+    return _host.get_workspace(nbytes, dev.index if dev.index is not None else torch.cuda.current_device())
 
 
 class DecodeCall:
@@ -366,23 +303,23 @@ class DecodeCall:
         a.workspace, a.workspace_bytes = ws_ptr, ws_bytes
         a.topk_slots_i32 = ptr(s32)
         self.args = a
-        self._ref = C.byref(a)
+        self._addr = C.addressof(a)
 
     def scan(self):
-        check("jf_decode_scan", lib.jf_decode_scan(self._ref, _stream()))
+        check("jf_decode_scan", _host.decode(1, self._addr))
 
     def select(self):
-        check("jf_topk_select", lib.jf_topk_select(self._ref, _stream()))
+        check("jf_topk_select", _host.decode(2, self._addr))
 
     def finish(self):
-        check("jf_decode_finish", lib.jf_decode_finish(self._ref, _stream()))
+        check("jf_decode_finish", _host.decode(3, self._addr))
 
     def fused(self):
-        check("jf_decode_fused", lib.jf_decode_fused(self._ref, _stream()))
+        check("jf_decode_fused", _host.decode(0, self._addr))
 
     def select_finish(self):
         """Select and finish in one kernel, after ``scan()`` (together: ``fused()``)."""
-        check("jf_select_finish", lib.jf_select_finish(self._ref, _stream()))
+        check("jf_select_finish", _host.decode(4, self._addr))
 
     def exact_stats(self):
         """Exact row maximum and 1 / sum exp(s - max) of the stored scores into ``softmax_m`` /
@@ -393,7 +330,7 @@ class DecodeCall:
 
     def status(self):
         """Synchronises the stream and raises if a kernel recorded a bounded-wait timeout."""
-        check("jf_decode_status", lib.jf_decode_status(self._ref, _stream()))
+        check("jf_decode_status", lib.jf_decode_status(C.byref(self.args), _stream()))
 
     def status_record(self) -> torch.Tensor:
         """The status record's bytes in the workspace (a CUDA uint8 view): copy them to pinned host
@@ -427,11 +364,12 @@ def fused_attn_topk(mode, q, k_data, k_scales, v_data, v_scales, block_table, se
     """One call: approximate attention over the packed cache, exact top-k, and the
     selected set's approximate contribution.  Returns ``(o_hat, topk_slots, o_old_unnorm,
     W, ...)`` -- the first four as the reference's ``int2_fused_attn_topk``."""
-    call = DecodeCall(mode, q, k_data, k_scales, v_data, v_scales, block_table, seq_lens,
-                      max_S, H_q, H_kv, block_size, top_k, attn_scale, workspace=workspace,
-                      want_scores=want_scores, stage_b=stage_b)
-    call.fused()
-    return call.result()
+    _require(stage_b in _STAGE_B, "fused_attn_topk: bad stage_b")
+    st, *out = _host.fused_attn("fused_attn_topk", MODE_IDS[mode] if isinstance(mode, str) else mode, q, k_data, k_scales, v_data,
+                                v_scales, block_table, seq_lens, max_S, H_q, H_kv, block_size, top_k, attn_scale, workspace,
+                                want_scores, _STAGE_B[stage_b])
+    check("jf_decode_fused", st)
+    return FusedAttnOut(*out)
 
 
 def int2_fused_attn_topk(q, k_data, k_scales, k_zp, v_data, v_scales, block_table, seq_lens,
@@ -443,10 +381,11 @@ def int2_fused_attn_topk(q, k_data, k_scales, k_zp, v_data, v_scales, block_tabl
     _require(k_zp is None, "int2_fused_attn_topk: asymmetric keys (k_zp) are not supported")
     widths = (int(k_data.shape[-1]), int(v_data.shape[-1]))
     _require(widths in ((48, 32), (64, 64)), f"int2_fused_attn_topk: unsupported packed widths {widths}")
-    mode = "k3v2" if widths == (48, 32) else "k4v4"
-    r = fused_attn_topk(mode, q, k_data, k_scales, v_data, v_scales, block_table, seq_lens,
-                        max_S, H_q, H_kv, block_size, top_k, attn_scale)
-    return r.o_hat, r.topk_slots, r.o_old_unnorm, r.W
+    st, o_hat, slots, o_old, W, *_ = _host.fused_attn(
+        "int2_fused_attn_topk", _lib.JF_MODE_K3V2 if widths == (48, 32) else _lib.JF_MODE_K4V4, q, k_data, k_scales, v_data,
+        v_scales, block_table, seq_lens, max_S, H_q, H_kv, block_size, top_k, attn_scale, None, False, _lib.JF_STAGE_B_FP32)
+    check("jf_decode_fused", st)
+    return o_hat, slots, o_old, W
 
 
 # -- the reference's Stage A / Stage B ops under their own names, argument order and return lists,
@@ -456,15 +395,9 @@ def int2_fused_attn_topk(q, k_data, k_scales, k_zp, v_data, v_scales, block_tabl
 
 def _stage_a(mode, name, q, k_data, k_scales, block_table, seq_lens, max_S, H_q, H_kv, block_size,
              attn_scale, top_k, stats):
-    _require(int(block_size) == 16, f"{name}: block_size must be 16")
-    call = DecodeCall(mode, q, k_data, k_scales, None, None, block_table, seq_lens, int(max_S), int(H_q), int(H_kv),
-                      int(block_size), int(top_k), float(attn_scale), want_scores=True, parts="k")
-    call.scan()
-    call.select()
-    out = [call.scores, call.out["topk_idx"], call.out["topk_slots"]]
-    if stats:
-        call.exact_stats()
-        out += [call.out["softmax_m"], call.out["softmax_inv_z"]]
+    st, *out = _host.stage_a(name, MODE_IDS[mode], q, k_data, k_scales, block_table, seq_lens, max_S, H_q, H_kv, block_size,
+                             attn_scale, top_k, stats)
+    check(name, st)
     return out
 
 
@@ -486,25 +419,10 @@ def int8tc_qk_scores_topk_stats(q, k_data, k_scales, block_table, seq_lens, max_
 
 def _stage_b(mode, name, stage_b, scores, v_data, v_scales, block_table, seq_lens, topk_idx, max_S, H_q, H_kv,
              block_size, top_k, out=None):
-    _require(int(block_size) == 16, f"{name}: block_size must be 16")
-    _require(scores.is_cuda and scores.dtype == torch.float32 and scores.dim() == 3, f"{name}: scores must be f32 (B,H_q,max_S)")
-    _require(topk_idx.is_cuda and topk_idx.dtype == torch.int64 and topk_idx.dim() == 3
-             and topk_idx.shape[2] == int(top_k), f"{name}: topk_idx must be int64 (B,H_q,top_k)")
-    B = scores.shape[0]
-    if out is not None:
-        for t, shape in zip(out, ((B, int(H_q), 128), (B, int(H_q), 128), (B, int(H_q)))):
-            _require(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and tuple(t.shape) == shape,
-                     f"{name}: outputs must be contiguous f32 of shapes (B,H_q,128), (B,H_q,128), (B,H_q)")
-        f32 = dict(dtype=torch.float32, device=scores.device)
-        out = dict(o_hat=out[0], o_old_unnorm=out[1], W=out[2], softmax_m=torch.empty(B, int(H_q), **f32),
-                   softmax_inv_z=torch.empty(B, int(H_q), **f32), topk_idx=topk_idx.contiguous(),
-                   topk_slots=torch.empty_like(topk_idx))
-    call = DecodeCall(mode, None, None, None, v_data, v_scales, block_table, seq_lens, int(max_S), int(H_q), int(H_kv),
-                      int(block_size), int(top_k), 1.0, parts="v", stage_b=stage_b, scores=scores.contiguous(),
-                      topk_idx=topk_idx.contiguous(), out=out)
-    call.scan()
-    call.finish()
-    return [call.out["o_hat"], call.out["o_old_unnorm"], call.out["W"]]
+    st, *res = _host.stage_b(name, MODE_IDS[mode], _STAGE_B[stage_b], scores, v_data, v_scales, block_table, seq_lens, topk_idx,
+                             max_S, H_q, H_kv, block_size, top_k, out)
+    check(name, st)
+    return res
 
 
 def int2_softmax_v_with_pre_corr_wvs2(scores, v_data, v_scales, block_table, seq_lens, topk_idx, max_S, H_q, H_kv,
@@ -546,21 +464,7 @@ def int8tc_softmax_v_with_pre_corr_reg_stats(scores, softmax_m, softmax_inv_z, v
 
 def blend_unnorm_into(o_hat, o_old_unnorm, W, o_new, out) -> None:
     """``out = dtype(o_hat + W * o_new - o_old_unnorm)``; ``out`` contiguous bf16/fp16."""
-    name = "blend_unnorm_into"
-    _require(o_hat.is_cuda and o_old_unnorm.is_cuda and W.is_cuda and o_new.is_cuda and out.is_cuda,
-             f"{name}: all tensors must be CUDA")
-    _require(o_hat.dtype == torch.float32 and o_old_unnorm.dtype == torch.float32 and W.dtype == torch.float32,
-             f"{name}: o_hat, o_old_unnorm, W must be float32")
-    _require(o_new.dtype == out.dtype, f"{name}: o_new and out dtypes differ")
-    _require(o_hat.dim() == 3 and o_old_unnorm.dim() == 3 and o_new.dim() == 3 and out.dim() == 3 and W.dim() == 2,
-             f"{name}: tensors must be 3D (W 2D)")
-    _require(out.is_contiguous(), f"{name}: out must be contiguous")
-    _require(o_old_unnorm.shape == o_hat.shape and o_new.shape == o_hat.shape and out.shape == o_hat.shape
-             and W.shape == o_hat.shape[:2] and o_hat.shape[2] == 128, f"{name}: shape mismatch")
-    o_hat, o_old_unnorm, W, o_new = o_hat.contiguous(), o_old_unnorm.contiguous(), W.contiguous(), o_new.contiguous()
-    st = lib.jf_merge_correct(o_hat.data_ptr(), o_old_unnorm.data_ptr(), W.data_ptr(), o_new.data_ptr(),
-                              out.data_ptr(), _dtype_id(out), o_hat.shape[0], o_hat.shape[1], _stream())
-    check(name, st)
+    check("blend_unnorm_into", _host.blend("blend_unnorm_into", o_hat, o_old_unnorm, W, o_new, out))
 
 
 # ---------------------------------------------------------------------------------------

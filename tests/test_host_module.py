@@ -1,0 +1,19 @@
+"""The native half of ``ops``: argument errors are RuntimeErrors that name the op, before any launch."""
+import pytest
+import torch
+
+from jetfire_b200 import ops
+
+
+@pytest.mark.parametrize("call", [
+    lambda t: ops.fused_quant_write_int3_sym(t, t, t, t, 64),
+    lambda t: ops.fused_quant_write_kv(t, t, t, t, t, t, t, 64, 3, 2),
+    lambda t: ops.fused_attn_topk("k3v2", t, t, t, t, t, t, t, 16, 8, 2, 16, 32, 1.0),
+    lambda t: ops.int3_qk_scores_topk(t, t, t, t, t, 16, 8, 2, 16, 1.0, 32),
+    lambda t: ops.int2_softmax_v_with_pre_corr_wvs2(t, t, t, t, t, t, 16, 8, 2, 16, 32),
+    lambda t: ops.blend_unnorm_into(t, t, t, t, t),
+    lambda t: ops.blend_unnorm_into(None, t, t, t, t),
+])
+def test_host_tensors_are_refused_by_name(call):
+    with pytest.raises(RuntimeError, match=r"^[a-z0-9_]+: "):
+        call(torch.zeros(1, 8, 128))
