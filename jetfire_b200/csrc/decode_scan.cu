@@ -11,13 +11,17 @@
 // which materialise scores and weights in HBM and read V once per *query* head.
 //
 // Data movement: a 16-token page of the cache is contiguous per tensor (768 B of INT3 K,
-// 512 B of INT2 V, 64 + 64 B of bf16 scales for K3V2), so a page is fetched with four
-// bulk-async copies (TMA, non-tensor form) into a per-warp ring of two-page slots in shared
-// memory, completion counted on the slot's mbarrier; two pages in neighbouring cache blocks
-// share their copies.  A page is exactly one MMA M tile.  Block-table entries are fetched
-// sixteen at a time, a chunk ahead of their use, and parked in shared memory together with
-// what the copies need, so that the loop never waits for a global load and the warp-uniform
-// work per page stays small.
+// 512 B of INT2 V, 64 + 64 B of bf16 scales for K3V2); a warp fetches two pages at a time with
+// asynchronous 16-byte copies, half a warp per page, into its own ring of four two-page slots in
+// shared memory, and reads them back with ldmatrix.  A page is exactly one MMA M tile.
+// Block-table entries are fetched sixteen at a time, a chunk ahead of their use, and parked in
+// shared memory together with what the copies need, so that the loop never waits for a global
+// load and the warp-uniform work per page stays small.
+//
+// What bounds it: instruction issue and the half-rate logic pipe (a field mask is two issue
+// cycles), not memory.  Measured per pipe: LOP3 2 cycles, HFMA2.BF16 2, HMMA 16816 8; the 72 + 32 +
+// 18 of a page alone are 255 cycles of a scheduler.  On a layer of 4 sequences x 8 KV heads x 65536
+// positions: 352 -> 277 warp instructions per page, 74.4 -> 62.4 us (0.46 of the copy peak).
 //
 // Compute: tokens sit on the MMA M axis and the (<= 8) query heads on N = 8.  Packed codes
 // are expanded in registers straight into the A fragments of mma.sync.m16n8k16 (the
@@ -44,28 +48,6 @@ __device__ __forceinline__ constexpr int v2_pos(int f) { return f <= 4 ? 2 * f :
 // 16-bit load, codes MSB-first inside a byte
 __device__ __forceinline__ constexpr int v2_dlocal(int f) { return 4 * (f >> 2) + 3 - (f & 3); }
 
-
-// Shared-memory loads with a 32-bit address and an immediate offset: one instruction each,
-// no 64-bit pointer arithmetic in the loop.
-template <int OFF>
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
-  return v;
-}
-template <int OFF>
-__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
-  uint32_t v;  // a 32-bit destination is zero-extended by the 16-bit load
-  asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF));
-  return v;
-}
-// lo | (hi << 16) for two 16-bit values, as an integer multiply-add (runs on the FMA pipe,
-// which has twice the throughput of the logic pipe that PRMT/SHL/LOP3 share)
-__device__ __forceinline__ uint32_t join16(uint32_t lo, uint32_t hi) {
-  uint32_t d;
-  asm("mad.lo.u32 %0, %1, 65536, %2;" : "=r"(d) : "r"(hi), "r"(lo));
-  return d;
-}
 
 // Dequantised K in the reference's rounding, times a power of two, in ONE bf16x2 fma per two
 // codes.  The masked 3-bit field, read as bf16, is the subnormal f * 2^POS * 2^-133 (exponent
@@ -117,9 +99,16 @@ __device__ __forceinline__ void k3_unpack_row(uint32_t P0, uint32_t P1, uint32_t
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the fp16 form without ordering against other asm statements (the compiler interleaves the pages)
+__device__ __forceinline__ void mma_f16_nv(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                           uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -140,119 +129,255 @@ __device__ __forceinline__ uint32_t v2_field(uint32_t v) {
 }
 constexpr uint32_t kOnesF16x2 = 0x3C003C00u;
 
+// Shared-memory matrix loads: four 8 x 8 matrices of 16-bit elements, one row of 16 bytes per lane.
+__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <int OFF>
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(OFF) : "memory");
+  return v;
+}
+// Pairs of floats for the packed fp32 instructions (two results per issue slot).
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpair_f32(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// base + index * SIZE in one multiply-add
+template <int SIZE>
+__device__ __forceinline__ const uint8_t* page_ptr(const void* base, uint32_t index) {
+  uint64_t d;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(index), "n"(SIZE), "l"(base));
+  return reinterpret_cast<const uint8_t*>(d);
+}
+// largest magnitudes of two packed bf16 pairs (NaN wins, sign bits are left over)
+__device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+
 // Per-warp state that lives across pages.
 template <int QT>
 struct K3State {
   uint32_t qf[QT][8][2];   // query fragments (B operand of the K MMA)
   float oacc[10][4];       // output accumulators, O^T fragments; tiles 8, 9: sum of the P operand per V group
-  float m_ref0, m_ref1, l0, l1;
-  float pm_a, pm_b;        // largest score of this lane's tokens in the current round, heads 2tig and 2tig+1
-  uint32_t smax_bits;      // largest K group scale seen (bf16 bits; positive floats order as integers)
+  float m_ref0, m_ref1;    // softmax reference points of heads 2tig, 2tig+1
+  uint64_t l2;             // softmax sums of the two heads
+  uint32_t smax2;          // largest K group scales seen (bf16 pair: group 0, group 1; sign bits are noise)
   uint32_t ks_sel;         // PRMT selector: this lane's K group scale into both halves
 };
 
-// One 16-token page.  `sb` = shared-memory address of the ring slot; the offsets select the
-// page's half of it.  kPartial: the last page of
-// a sequence (or a page whose block id was invalid) -- rows at or past `valid` are neutralised;
-// the common full-page instance carries none of that logic.
+// Scores of one page: token g of the lane in acc[0..1] (heads 2tig, 2tig+1), token g + 8 in acc[2..3].
+template <int QT>
+__device__ __forceinline__ void k3_scores(const K3State<QT>& st, float (&acc)[4], uint32_t p0a, uint32_t p0b, uint32_t p1a,
+                                          uint32_t p1b, uint32_t p2a, uint32_t p2b, uint32_t ksa, uint32_t ksb) {
+  uint32_t R0[2][8], R1[2][8];
+  k3_unpack_row(p0a, p1a, p2a, k3_scale(prmt(ksa, ksa, st.ks_sel)), R0);
+  k3_unpack_row(p0b, p1b, p2b, k3_scale(prmt(ksb, ksb, st.ks_sel)), R1);
+  acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+#pragma unroll
+  for (int t = 0; t < QT; ++t)
+#pragma unroll
+    for (int x = 0; x < 8; ++x)
+      mma_bf16_16816(acc, R0[0][x], R1[0][x], R0[1][x], R1[1][x], st.qf[t][x][0], st.qf[t][x][1]);
+}
+
+// The P operand of one page: weights p[0..1] of token g, p[2..3] of token g + 8 (heads 2tig, 2tig+1) times
+// the V scales, as {tokens 2tig, 2tig+1 | 2tig+8, 2tig+9} of head g, for channel half 0 then 1.
+__device__ __forceinline__ void k3_weights(uint32_t (&B)[4], const float (&p)[4], uint32_t vsa, uint32_t vsb) {
+#pragma unroll
+  for (int qh = 0; qh < 2; ++qh) {
+    const float va = __uint_as_float(qh ? (vsa & 0xFFFF0000u) : (vsa << 16)), vb = __uint_as_float(qh ? (vsb & 0xFFFF0000u) : (vsb << 16));
+    B[2 * qh] = movmatrix_trans(pack_f16x2_sat(p[0] * va, p[1] * va));
+    B[2 * qh + 1] = movmatrix_trans(pack_f16x2_sat(p[2] * vb, p[3] * vb));
+  }
+}
+// One page's (P * vscale).V into the output accumulators.  X = the page's V words, transposed so that a
+// register holds two tokens' halves: {tokens 0-7, tokens 8-15} of channel half 0, then of half 1.
+__device__ __forceinline__ void k3_values(float (&oacc)[10][4], const uint32_t (&B)[4], const uint32_t (&X)[4]) {
+#pragma unroll
+  for (int qh = 0; qh < 2; ++qh) {
+    const uint32_t B0 = B[2 * qh], B1 = B[2 * qh + 1], XA = X[2 * qh], XB = X[2 * qh + 1];
+    const uint32_t XA2 = XA >> 10, XB2 = XB >> 10;
+    // fields 2ml -> output row g, 2ml+1 -> output row g+8
+    mma_f16_nv(oacc[qh * 4 + 0], v2_field<0>(XA), v2_field<2>(XA), v2_field<0>(XB), v2_field<2>(XB), B0, B1);
+    mma_f16_nv(oacc[qh * 4 + 1], v2_field<4>(XA), v2_field<6>(XA), v2_field<4>(XB), v2_field<6>(XB), B0, B1);
+    mma_f16_nv(oacc[qh * 4 + 2], v2_field<8>(XA), v2_field<0>(XA2), v2_field<8>(XB), v2_field<0>(XB2), B0, B1);
+    mma_f16_nv(oacc[qh * 4 + 3], v2_field<2>(XA2), v2_field<4>(XA2), v2_field<2>(XB2), v2_field<4>(XB2), B0, B1);
+    mma_f16_nv(oacc[8 + qh], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
+  }
+}
+
+// One round: two 16-token pages (A and B, one ring slot at shared-memory address `sb`).  Rows of the
+// pages are MMA rows in order; a lane holds tokens g and g + 8 of both.  ldmatrix does what used to be
+// fourteen scalar loads and four joins per page: untransposed it hands each lane its word of a K byte
+// plane, transposed it pairs two tokens' V halves in one register.
+// kMasked: only the first `live_a` / `live_b` tokens count (the last page of a sequence, a page whose block
+// id was invalid, an absent second page: -1); the common instance carries none of that logic.
 // kParts: 0 = scores and output partials; 1 = scores and softmax sums only (no V);
 // 2 = output partials from scores read back from memory (no K).
-template <int QT, bool kPartial, int kParts>
-__device__ __forceinline__ void k3v2_page(K3State<QT>& st, uint32_t sb, uint32_t k_addr_off, uint32_t v_addr_off,
-                                          uint32_t s_addr_off, int t0, int valid, float attn, float* sp0,
-                                          float* sp1, bool st0, bool st1) {
+template <int QT, bool kMasked, int kParts>
+__device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const uint32_t (&off)[4], int g, int live_a, int live_b,
+                                           float attn, float* row0, float* row1, uint32_t at, bool st0, bool st1,
+                                           float* pm_row, uint32_t pm_at, bool pm_store, int lane) {
   using T = Tile<JF_MODE_K3V2>;
   constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
-  // ---------------- K: unpack + Q.K^T ----------------
-  const uint32_t sa = sb + s_addr_off;
-  uint32_t ksw0 = 0u, ksw1 = 0u, vsw0 = 0u, vsw1 = 0u;
-  if (kDoK) { ksw0 = lds32<0>(sa); ksw1 = lds32<32>(sa); }
-  if (kDoV) { vsw0 = lds32<T::kVsRel>(sa); vsw1 = lds32<T::kVsRel + 32>(sa); }
-  float vs00 = __uint_as_float(vsw0 << 16), vs01 = __uint_as_float(vsw0 & 0xFFFF0000u);
-  float vs10 = __uint_as_float(vsw1 << 16), vs11 = __uint_as_float(vsw1 & 0xFFFF0000u);
-  if (kPartial) {
-    if (t0 >= valid) { ksw0 = 0u; vs00 = vs01 = 0.f; }
-    if (t0 + 8 >= valid) { ksw1 = 0u; vs10 = vs11 = 0.f; }
-  }
-  // all shared-memory reads of the page are issued up front (the loads keep their source order)
-  const uint32_t ka = sb + k_addr_off;
-  uint32_t kw0 = 0u, kw1 = 0u, kw2 = 0u, kw3 = 0u, kw4 = 0u, kw5 = 0u;
+  // the lane's scores: two rows of the warp's, at the same byte offset (32 bits: one register for both)
+  float* const sp0 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(row0) + at);
+  float* const sp1 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(row1) + at);
+  // the K side's shared-memory reads are issued up front
+  uint32_t ka[4], kb[4], kc[4];   // planes 0, 1 of page A; of page B; plane 2 of both: {tokens 0-7, 8-15} each
+  uint32_t ksa0 = 0u, ksa1 = 0u, ksb0 = 0u, ksb1 = 0u, vsa0 = 0u, vsa1 = 0u, vsb0 = 0u, vsb1 = 0u;
+  uint32_t xa[4], xb[4];
+  const uint32_t sc = sb + off[3];
   if (kDoK) {
-    kw0 = lds32<0>(ka); kw1 = lds32<16>(ka); kw2 = lds32<32>(ka);
-    kw3 = lds32<8 * T::kKRow>(ka); kw4 = lds32<8 * T::kKRow + 16>(ka); kw5 = lds32<8 * T::kKRow + 32>(ka);
+    ldsm_x4(ka, sb + off[0]);
+    ldsm_x4(kc, sb + off[1]);
+    ldsm_x4(kb, sb + off[0] + T::kPageTx);
+    ksa0 = lds32<0>(sc); ksa1 = lds32<32>(sc); ksb0 = lds32<T::kPageTx>(sc); ksb1 = lds32<T::kPageTx + 32>(sc);
   }
-  const uint32_t va_addr = sb + v_addr_off;
-  uint32_t vh[2][4] = {{0u, 0u, 0u, 0u}, {0u, 0u, 0u, 0u}};
-  if (kDoV) {
-    vh[0][0] = lds16<0>(va_addr); vh[0][1] = lds16<4 * T::kVRow>(va_addr);
-    vh[0][2] = lds16<8 * T::kVRow>(va_addr); vh[0][3] = lds16<12 * T::kVRow>(va_addr);
-    vh[1][0] = lds16<16>(va_addr); vh[1][1] = lds16<4 * T::kVRow + 16>(va_addr);
-    vh[1][2] = lds16<8 * T::kVRow + 16>(va_addr); vh[1][3] = lds16<12 * T::kVRow + 16>(va_addr);
-  }
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  if (kDoK) {
-    const uint32_t sc0 = prmt(ksw0, ksw0, st.ks_sel), sc1 = prmt(ksw1, ksw1, st.ks_sel);
-    st.smax_bits = max(st.smax_bits, max(sc0 & 0x7FFFu, sc1 & 0x7FFFu));
-    uint32_t R0[2][8], R1[2][8];
-    k3_unpack_row(kw0, kw1, kw2, k3_scale(sc0), R0);
-    k3_unpack_row(kw3, kw4, kw5, k3_scale(sc1), R1);
-#pragma unroll
-    for (int t = 0; t < QT; ++t)
-#pragma unroll
-      for (int x = 0; x < 8; ++x)
-        mma_bf16_16816(acc, R0[0][x], R1[0][x], R0[1][x], R1[1][x], st.qf[t][x][0], st.qf[t][x][1]);
+  const bool la = !kMasked || g < live_a, ha = !kMasked || g + 8 < live_a;
+  const bool lb = !kMasked || g < live_b, hb = !kMasked || g + 8 < live_b;
+  if (kMasked) {   // what an absent page's half of the slot holds need not even be finite
+    if (!la) ksa0 = 0u;
+    if (!ha) ksa1 = 0u;
+    if (!lb) ksb0 = 0u;
+    if (!hb) ksb1 = 0u;
   }
 
   // ---------------- scores ----------------
-  float s0 = acc[0] * attn;  // row g,   head 2tig
-  float s1 = acc[1] * attn;  // row g,   head 2tig+1
-  float s2 = acc[2] * attn;  // row g+8, head 2tig
-  float s3 = acc[3] * attn;  // row g+8, head 2tig+1
-  const bool lo = !kPartial || t0 < valid, hi = !kPartial || t0 + 8 < valid;
-  if (!kDoK) {
+  float sA[4] = {0.f, 0.f, 0.f, 0.f}, sB[4] = {0.f, 0.f, 0.f, 0.f};
+  if (kDoK) {
+    st.smax2 = absmax_bf16x2(st.smax2, absmax_bf16x2(absmax_bf16x2(ksa0, ksa1), absmax_bf16x2(ksb0, ksb1)));
+    k3_scores<QT>(st, sA, ka[0], ka[1], ka[2], ka[3], kc[0], kc[1], ksa0, ksa1);
+    k3_scores<QT>(st, sB, kb[0], kb[1], kb[2], kb[3], kc[2], kc[3], ksb0, ksb1);
+    const uint64_t attn2 = pair_f32(attn, attn);
+    unpair_f32(mul2(pair_f32(sA[0], sA[1]), attn2), sA[0], sA[1]);
+    unpair_f32(mul2(pair_f32(sA[2], sA[3]), attn2), sA[2], sA[3]);
+    unpair_f32(mul2(pair_f32(sB[0], sB[1]), attn2), sB[0], sB[1]);
+    unpair_f32(mul2(pair_f32(sB[2], sB[3]), attn2), sB[2], sB[3]);
+  } else {
     // the scores an earlier scan stored (heads past the group stay at 0: their columns are dropped)
-    if (st0 && lo) s0 = sp0[0];
-    if (st0 && hi) s2 = sp0[8];
-    if (st1 && lo) s1 = sp1[0];
-    if (st1 && hi) s3 = sp1[8];
+    if (st0) {
+      if (la) sA[0] = sp0[0];
+      if (ha) sA[2] = sp0[8];
+      if (lb) sB[0] = sp0[16];
+      if (hb) sB[2] = sp0[24];
+    }
+    if (st1) {
+      if (la) sA[1] = sp1[0];
+      if (ha) sA[3] = sp1[8];
+      if (lb) sB[1] = sp1[16];
+      if (hb) sB[3] = sp1[24];
+    }
   }
-  if (kPartial) {
-    if (!lo) { s0 = s1 = -INFINITY; }
-    if (!hi) { s2 = s3 = -INFINITY; }
+  if (kMasked) {
+    if (!la) sA[0] = sA[1] = -INFINITY;
+    if (!ha) sA[2] = sA[3] = -INFINITY;
+    if (!lb) sB[0] = sB[1] = -INFINITY;
+    if (!hb) sB[2] = sB[3] = -INFINITY;
   }
   if (kDoK) {
-    if (kPartial) {
-      if (st0 && lo) sp0[0] = s0;
-      if (st0 && hi) sp0[8] = s2;
-      if (st1 && lo) sp1[0] = s1;
-      if (st1 && hi) sp1[8] = s3;
-    } else {
-      if (st0) { sp0[0] = s0; sp0[8] = s2; }
-      if (st1) { sp1[0] = s1; sp1[8] = s3; }
+    if (st0) {
+      if (la) sp0[0] = sA[0];
+      if (ha) sp0[8] = sA[2];
+      if (lb) sp0[16] = sB[0];
+      if (hb) sp0[24] = sB[2];
     }
-    // running maxima of this lane's tokens, for the page-pair maxima the select kernel reads
-    st.pm_a = fmaxf(st.pm_a, fmaxf(s0, s2));
-    st.pm_b = fmaxf(st.pm_b, fmaxf(s1, s3));
+    if (st1) {
+      if (la) sp1[0] = sA[1];
+      if (ha) sp1[8] = sA[3];
+      if (lb) sp1[16] = sB[1];
+      if (hb) sp1[24] = sB[3];
+    }
   }
 
-  // ---------------- online softmax ----------------
-  float p0, p1, p2, p3;
-  softmax_step(s0, s1, s2, s3, st.m_ref0, st.m_ref1, st.l0, st.l1, st.oacc, p0, p1, p2, p3);
-  // ---------------- V: unpack + (P * vscale).V ----------------
+  // the V side, requested ahead of the softmax (with the K side it would not fit the registers)
+  if (kDoV) {
+    ldsm_x4_trans(xa, sb + off[2]);
+    ldsm_x4_trans(xb, sb + off[2] + T::kPageTx);
+    vsa0 = lds32<T::kVsRel>(sc); vsa1 = lds32<T::kVsRel + 32>(sc);
+    vsb0 = lds32<T::kVsRel + T::kPageTx>(sc); vsb1 = lds32<T::kVsRel + T::kPageTx + 32>(sc);
+    if (kMasked) {
+      if (!la) vsa0 = 0u;
+      if (!ha) vsa1 = 0u;
+      if (!lb) vsb0 = 0u;
+      if (!hb) vsb1 = 0u;
+    }
+  }
+
+  // ---------------- online softmax over both pages ----------------
+  // The reference point may lag the true maximum by less than 4 (exp stays below e^4, the fp16 P
+  // operand cannot overflow); the exact maximum is only taken when a score runs ahead of it.
+  float mx0 = fmaxf(fmaxf(sA[0], sA[2]), fmaxf(sB[0], sB[2])), mx1 = fmaxf(fmaxf(sA[1], sA[3]), fmaxf(sB[1], sB[3]));
+  if (kDoK) {
+    // largest score of the round's pages per head, for the select kernel's threshold: the halves of the
+    // warp trade one head for the other (each lane sends one value and keeps one), then reduce over lane
+    // bits 3 and 2
+    const bool up = (lane & 16) != 0;
+    float v = fmaxf(up ? mx1 : mx0, __shfl_xor_sync(0xFFFFFFFFu, up ? mx0 : mx1, 16));
+    v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
+    v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 4));
+    if (pm_store) *reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(pm_row) + pm_at) = v;
+  }
+  if (__any_sync(0xFFFFFFFFu, mx0 > st.m_ref0 + 4.0f || mx1 > st.m_ref1 + 4.0f)) {
 #pragma unroll
-  for (int qh = 0; kDoV && qh < 2; ++qh) {
-    const float va = qh ? vs01 : vs00, vb = qh ? vs11 : vs10;
-    const uint32_t B0 = movmatrix_trans(pack_f16x2_sat(p0 * va, p1 * va));  // tokens tig, tig+4
-    const uint32_t B1 = movmatrix_trans(pack_f16x2_sat(p2 * vb, p3 * vb));  // tokens tig+8, tig+12
-    const uint32_t Ha = vh[qh][0], Hb = vh[qh][1], Hc = vh[qh][2], Hd = vh[qh][3];
-    const uint32_t XA = join16(Ha, Hb), XB = join16(Hc, Hd);
-    const uint32_t XA2 = XA >> 10, XB2 = XB >> 10;
-    // fields 2ml -> output row g, 2ml+1 -> output row g+8
-    mma_f16_16816(st.oacc[qh * 4 + 0], v2_field<0>(XA), v2_field<2>(XA), v2_field<0>(XB), v2_field<2>(XB), B0, B1);
-    mma_f16_16816(st.oacc[qh * 4 + 1], v2_field<4>(XA), v2_field<6>(XA), v2_field<4>(XB), v2_field<6>(XB), B0, B1);
-    mma_f16_16816(st.oacc[qh * 4 + 2], v2_field<8>(XA), v2_field<0>(XA2), v2_field<8>(XB), v2_field<0>(XB2), B0, B1);
-    mma_f16_16816(st.oacc[qh * 4 + 3], v2_field<2>(XA2), v2_field<4>(XA2), v2_field<2>(XB2), v2_field<4>(XB2), B0, B1);
-    mma_f16_16816(st.oacc[8 + qh], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
+    for (int o = 4; o < 32; o <<= 1) {
+      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, o));
+      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, o));
+    }
+    const float n0 = fmaxf(st.m_ref0, mx0), n1 = fmaxf(st.m_ref1, mx1);
+    const float f0 = ex2((st.m_ref0 - n0) * kLog2e), f1 = ex2((st.m_ref1 - n1) * kLog2e);
+    st.l2 = mul2(st.l2, pair_f32(f0, f1));
+    if (kDoV) {
+#pragma unroll
+      for (int i = 0; i < 10; ++i) { st.oacc[i][0] *= f0; st.oacc[i][1] *= f1; st.oacc[i][2] *= f0; st.oacc[i][3] *= f1; }
+    }
+    st.m_ref0 = n0; st.m_ref1 = n1;
+  }
+  const uint64_t c2 = pair_f32(kLog2e, kLog2e), mb2 = pair_f32(-st.m_ref0 * kLog2e, -st.m_ref1 * kLog2e);
+  float pA[4], pB[4];
+  unpair_f32(fma2(pair_f32(sA[0], sA[1]), c2, mb2), pA[0], pA[1]);
+  unpair_f32(fma2(pair_f32(sA[2], sA[3]), c2, mb2), pA[2], pA[3]);
+  unpair_f32(fma2(pair_f32(sB[0], sB[1]), c2, mb2), pB[0], pB[1]);
+  unpair_f32(fma2(pair_f32(sB[2], sB[3]), c2, mb2), pB[2], pB[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { pA[i] = ex2(pA[i]); pB[i] = ex2(pB[i]); }
+  st.l2 = add2(st.l2, add2(add2(pair_f32(pA[0], pA[1]), pair_f32(pA[2], pA[3])), add2(pair_f32(pB[0], pB[1]), pair_f32(pB[2], pB[3]))));
+
+  // ---------------- (P * vscale).V ----------------
+  if (kDoV) {
+    uint32_t BA[4], BB[4];
+    k3_weights(BA, pA, vsa0, vsa1);
+    k3_weights(BB, pB, vsb0, vsb1);
+    k3_values(st.oacc, BA, xa);
+    k3_values(st.oacc, BB, xb);
   }
 }
 
@@ -267,10 +392,9 @@ scan_k3v2_kernel(const ScanParams p) {
   using T = Tile<JF_MODE_K3V2>;
   constexpr int kQTerms = (DT == JF_DTYPE_FP16) ? 2 : 1;
   constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
-  constexpr uint32_t kTxPage = (kDoK ? T::kKPage + T::kSPage : 0) + (kDoV ? T::kVPage + T::kSPage : 0);
   extern __shared__ __align__(128) uint8_t smem[];
   // the warp index is the same for all lanes; routing it through a shuffle tells the
-  // compiler so, and lets stage / barrier addresses live in uniform registers
+  // compiler so, and lets slot addresses live in uniform registers
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
   const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
@@ -279,15 +403,9 @@ scan_k3v2_kernel(const ScanParams p) {
   constexpr int kRingBytes = kScanWarps * T::kSlots * T::kSlotBytes;
   constexpr int kPagesInFlight = 2 * T::kSlots;
   const uint32_t slots0 = smem_base + warp * (T::kSlots * T::kSlotBytes);
-  const uint32_t bars0 = smem_base + kRingBytes + warp * (T::kSlots * 8);   // one barrier per slot
-  // parked per page: the first cache row of its block and how many of its 16 tokens are live
-  int2* bt_s = reinterpret_cast<int2*>(smem + kRingBytes + kScanWarps * T::kSlots * 8) + warp * (2 * kBtChunk);
+  // parked per page: its index in the cache (over all KV heads) and how many of its 16 tokens are live
+  int2* bt_s = reinterpret_cast<int2*>(smem + kRingBytes) + warp * (2 * kBtChunk);
 
-  if (lane == 0) {
-    for (int s = 0; s < T::kSlots; ++s) mbar_init(reinterpret_cast<uint64_t*>(smem + (bars0 - smem_base)) + s, 1);
-  }
-  fence_barrier_init();
-  __syncwarp();
   pdl_wait();  // nothing above reads global memory
 
   const int len = min(p.seq_lens[b], p.max_S);
@@ -308,62 +426,57 @@ scan_k3v2_kernel(const ScanParams p) {
   int64_t bt_pend = bt_load(0);
   const int64_t n_blocks_phys = p.num_slots >> 4;
 
-  // One elected lane issues the four bulk copies of a page (K data, V data, K scales, V scales).
-  // The packed cache is read once per call: fetched as first-to-evict, it leaves the scores
-  // this kernel writes (and the next kernel reads) in L2.
-  const uint64_t stream_policy = l2_policy_evict_first();
-  const int64_t head_rows = static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots;
-  const uint8_t* ks_b = reinterpret_cast<const uint8_t*>(p.k_scales);
-  const uint8_t* vs_b = reinterpret_cast<const uint8_t*>(p.v_scales);
+  const uint32_t head_page0 = static_cast<uint32_t>(hkv >> p.kv_shift) * static_cast<uint32_t>(n_blocks_phys);
   const int last_pg = (len & 15) ? (n_pages - 1) : -1;   // the only page that can be partial
   // entry e of this warp (page pg_first + e) from its block id, worked out by sixteen lanes at
   // once when a chunk arrives: an invalid block id reads block 0 and counts no live token; the
-  // sequence's last page may be partial
+  // sequence's last page may be partial; entries past the warp's range count -1
   auto bt_entry = [&](int64_t blk64, int e) -> int2 {
     const int pg = pg_first + e;
     const bool bad = blk64 < 0 || blk64 >= n_blocks_phys;
-    const int valid = bad ? 0 : (pg == last_pg ? len - pg * 16 : 16);
-    return make_int2(static_cast<int>(head_rows + (bad ? 0 : blk64) * 16), valid);
+    const int valid = e >= my_n ? -1 : bad ? 0 : (pg == last_pg ? len - pg * 16 : 16);
+    return make_int2(static_cast<int>(head_page0 + (bad ? 0u : static_cast<uint32_t>(blk64))), valid);
   };
-  // By one elected lane: the copies of one or two pages into slot `sl`.  Two pages whose blocks
-  // are neighbours in the cache take one copy per array; otherwise each page takes its own four.
-  // Either way everything lands on the slot's barrier.
-  auto refill = [&](int sl, int2 ent_a, int2 ent_b, bool two) {
-    if (elect_one()) {
-      const uint32_t bar = bars0 + sl * 8;
-      const uint32_t dst = slots0 + sl * T::kSlotBytes;
-      const int64_t ra = ent_a.x, rb = ent_b.x;
-      const bool joined = two && rb == ra + 16;
-      const uint32_t n = joined ? 2u : 1u;
-      mbar_expect_tx_u32(bar, two ? 2 * kTxPage : kTxPage);
+  // The copies of a slot's one or two pages, 16 bytes a lane: each half of the warp fetches a page
+  // (lanes of an absent one stay out), seven instructions and four address multiply-adds per round.
+  // (Bulk copies issued by one elected lane cost the warp 30 instructions more per page.)  Completion
+  // is counted per thread and round (commit groups); a round without copies commits an empty group, so
+  // that the count stays right.
+  const int half = lane >> 4, l16 = lane & 15;
+  const uint32_t dst = slots0 + half * T::kPageTx + 16 * l16;
+  const uint32_t lane16 = 16 * l16;
+  auto refill = [&](uint32_t slot_off, int e0) {   // pages e0, e0 + 1 of the warp; uniform
+    const int2 ent = bt_s[(e0 + half) & (2 * kBtChunk - 1)];
+    if (ent.y >= 0) {
+      const uint32_t page = static_cast<uint32_t>(ent.x), d = dst + slot_off;
       if (kDoK) {
-        bulk_g2s_u32_hint(dst, p.k_data + ra * T::kKRow, n * T::kKPage, bar, stream_policy);
-        bulk_g2s_u32(dst + T::kKsOff, ks_b + ra * (2 * T::kNG), n * T::kSPage, bar);
+        const uint8_t* src = page_ptr<T::kKPage>(p.k_data, page) + lane16;
+        cp_async_16_off<0>(d, src);
+        cp_async_16_off<256>(d, src);
+        cp_async_16_off<512>(d, src);
       }
       if (kDoV) {
-        bulk_g2s_u32_hint(dst + T::kVOff, p.v_data + ra * T::kVRow, n * T::kVPage, bar, stream_policy);
-        bulk_g2s_u32(dst + T::kKsOff + T::kVsRel, vs_b + ra * (2 * T::kNG), n * T::kSPage, bar);
+        const uint8_t* src = page_ptr<T::kVPage>(p.v_data, page) + lane16;
+        cp_async_16_off<0>(d + T::kVOff, src);
+        cp_async_16_off<256>(d + T::kVOff, src);
       }
-      if (two && !joined) {
-        if (kDoK) {
-          bulk_g2s_u32_hint(dst + T::kKPage, p.k_data + rb * T::kKRow, T::kKPage, bar, stream_policy);
-          bulk_g2s_u32(dst + T::kKsOff + T::kSPage, ks_b + rb * (2 * T::kNG), T::kSPage, bar);
-        }
-        if (kDoV) {
-          bulk_g2s_u32_hint(dst + T::kVOff + T::kVPage, p.v_data + rb * T::kVRow, T::kVPage, bar, stream_policy);
-          bulk_g2s_u32(dst + T::kKsOff + T::kVsRel + T::kSPage, vs_b + rb * (2 * T::kNG), T::kSPage, bar);
-        }
-      }
+      // lanes 0-3 of a half: the K scales, 4-7: the V scales (next to them in the slot)
+      if (kDoK && l16 < 4) cp_async_16_off<0>(d + T::kKsOff, page_ptr<T::kSPage>(p.k_scales, page) + lane16);
+      if (kDoV && (l16 & 12) == 4) cp_async_16_off<0>(d + T::kKsOff, page_ptr<T::kSPage>(p.v_scales, page) + (lane16 - 64));
     }
   };
+  const int4* ent_s = reinterpret_cast<const int4*>(bt_s);   // entries of a round's two pages (16 rounds resident)
 
   // prologue: chunk 0 to shared memory, chunk 1 requested, the ring filled
   if (lane < kBtChunk) bt_s[lane] = bt_entry(bt_pend, lane);
   int bt_stored = 0;   // chunks 0..bt_stored are in shared memory; chunk bt_stored + 1 is in bt_pend
   bt_pend = bt_load(1);
   __syncwarp();
-  for (int sl = 0; sl < T::kSlots; ++sl)
-    if (2 * sl < my_n) refill(sl, bt_s[2 * sl], bt_s[2 * sl + 1], 2 * sl + 1 < my_n);
+#pragma unroll
+  for (int sl = 0; sl < T::kSlots; ++sl) {
+    if (2 * sl < my_n) refill(sl * T::kSlotBytes, 2 * sl);
+    cp_async_commit();
+  }
 
   // ---- query fragments: B operand of the K MMA, scaled by 2^(33 - pos) of the code it meets.
   //      Lane (head n = g, tig) covers channels 32 tig + 8 j + x (group j, code x); k-step x
@@ -405,66 +518,45 @@ scan_k3v2_kernel(const ScanParams p) {
   st.ks_sel = (tig >> 1) ? 0x3232u : 0x1010u;
 #pragma unroll
   for (int i = 0; i < 10; ++i) { st.oacc[i][0] = st.oacc[i][1] = st.oacc[i][2] = st.oacc[i][3] = 0.f; }
-  st.m_ref0 = kMinusBig; st.m_ref1 = kMinusBig; st.l0 = 0.f; st.l1 = 0.f;
-  st.smax_bits = 0u;
-  st.pm_a = st.pm_b = -INFINITY;
-  bool failed = false;
+  st.m_ref0 = kMinusBig; st.m_ref1 = kMinusBig; st.l2 = 0ull;
+  st.smax2 = 0u;
 
-  const int t0 = (g >> 1) | ((g & 1) << 2);  // token of MMA row g (rows g + 8 -> t0 + 8)
-  const uint32_t k_addr_off = t0 * T::kKRow + tig * 4;               // in the slot's first half
-  const uint32_t v_addr_off = T::kVOff + tig * T::kVRow + 2 * g;
-  const uint32_t s_addr_off = T::kKsOff + t0 * 4;
-  const int h0 = hkv * p.G + 2 * tig;
-  float* sp0 = p.scores + (static_cast<int64_t>(b) * p.H_q + h0) * p.max_S + t0 +
-               static_cast<int64_t>(pg_first) * 16;
-  float* sp1 = sp0 + p.max_S;
+  // this lane's offsets in a slot: the matrix rows it names (row r of matrix m = lane >> 3) and its scales
+  const int mr = (lane & 7) + 8 * ((lane >> 3) & 1), mh = lane >> 4;
+  const uint32_t off[4] = {
+      static_cast<uint32_t>(mr * T::kKRow + 16 * mh),                      // K planes 0 and 1 of page A (B: + kPageTx)
+      static_cast<uint32_t>(mr * T::kKRow + 32 + T::kPageTx * mh),         // K plane 2 of pages A and B
+      static_cast<uint32_t>(T::kVOff + mr * T::kVRow + 16 * mh),           // V halves of page A (B: + kPageTx)
+      static_cast<uint32_t>(T::kKsOff + g * 4)};                           // scales of token g
+  // scores: byte offsets from the rows of the KV head's first two query heads (eight rows of at most
+  // 2^18 positions: 32 bits reach)
+  float* const row0 = p.scores + (static_cast<int64_t>(b) * p.H_q + hkv * p.G) * p.max_S;
+  float* const row1 = row0 + p.max_S;
+  uint32_t at = 4u * (2u * tig * static_cast<uint32_t>(p.max_S) + g + 16u * pg_first);
   const bool st0 = (2 * tig) < p.G, st1 = (2 * tig + 1) < p.G;
   // Page-pair maxima (pages 2m, 2m+1; a warp's range starts at an even page): after the round's
   // butterfly the lanes with bits 2 and 3 clear hold them -- lane bit 4 clear: head 2tig, set: 2tig+1.
   const int pm_head = 2 * tig + (lane >> 4);
   const bool want_pm = kDoK && p.pmax != nullptr;   // the same for the whole grid
-  float* pmw = (want_pm && (lane & 12) == 0 && pm_head < p.G)
-                   ? p.pmax + (static_cast<int64_t>(b) * p.H_q + hkv * p.G + pm_head) * p.np_stride + (pg_first >> 1)
-                   : nullptr;
+  const bool pm_store = want_pm && (lane & 12) == 0 && pm_head < p.G;
+  float* const pm_row = p.pmax + (static_cast<int64_t>(b) * p.H_q + hkv * p.G) * p.np_stride;
+  uint32_t pm_at = 4u * (pm_head * static_cast<uint32_t>(p.np_stride) + (pg_first >> 1));
   const float attn = p.attn_scale;
 
-  // A round takes one slot: two pages (one at the end of the range), processed one after the
-  // other; the ring bookkeeping and the election of the copying lane are paid once per round.
-  int sl = 0;
-  uint32_t parity = 0u;
+  // A round takes one slot: two pages (one at the end of the range).
+  uint32_t slot_off = 0u;
   for (int it = 0; it < my_n; it += 2) {
-    const int n_here = (it + 1 < my_n) ? 2 : 1;
-    if (!mbar_wait(reinterpret_cast<uint64_t*>(smem + (bars0 - smem_base)) + sl, parity)) {
-      // give the copies that were already issued a short, bounded chance to land
-      for (int j = 1; j < T::kSlots && it + 2 * j < my_n; ++j) {
-        const int o = (sl + j) % T::kSlots;
-        mbar_wait(reinterpret_cast<uint64_t*>(smem + (bars0 - smem_base)) + o, o > sl ? parity : parity ^ 1u, 1000000ull);
-      }
-      failed = true;
-      break;
-    }
-    const uint32_t sb = slots0 + sl * T::kSlotBytes;
-#pragma unroll 1
-    for (int k = 0; k < n_here; ++k) {
-      const int live = bt_s[(it + k) & (2 * kBtChunk - 1)].y;   // the page's parked entry is still resident
-      const uint32_t ko = k_addr_off + k * T::kKPage, vo = v_addr_off + k * T::kVPage, so = s_addr_off + k * T::kSPage;
-      if (live != 16)
-        k3v2_page<kQTerms, true, kParts>(st, sb, ko, vo, so, t0, live, attn, sp0, sp1, st0, st1);
-      else
-        k3v2_page<kQTerms, false, kParts>(st, sb, ko, vo, so, t0, 16, attn, sp0, sp1, st0, st1);
-      sp0 += 16;
-      sp1 += 16;
-    }
-    if (want_pm) {
-      // largest score of the round's pages per head: the halves of the warp trade one head for the
-      // other (each lane sends one value and keeps one), then reduce over lane bits 3 and 2
-      const bool up = (lane & 16) != 0;
-      float v = fmaxf(up ? st.pm_b : st.pm_a, __shfl_xor_sync(0xFFFFFFFFu, up ? st.pm_a : st.pm_b, 16));
-      v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
-      v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 4));
-      if (pmw) *pmw++ = v;
-      st.pm_a = st.pm_b = -INFINITY;
-    }
+    cp_async_wait_group<T::kSlots - 1>();   // this lane's copies of the round have landed ...
+    __syncwarp();                           // ... and every other lane's
+    const uint32_t sb = slots0 + slot_off;
+    const int4 ent = ent_s[(it >> 1) & (kBtChunk - 1)];   // the round's parked entries are still resident
+    if (ent.y + ent.w == 32)
+      k3v2_round<kQTerms, false, kParts>(st, sb, off, g, 16, 16, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store, lane);
+    else
+      k3v2_round<kQTerms, true, kParts>(st, sb, off, g, ent.y, ent.w, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store,
+                                        lane);
+    at += 128u;
+    pm_at += 4u;
     __syncwarp();
     if (((it + kPagesInFlight + 1) >> 4) > bt_stored) {   // the refill below reads entries up to it + kPagesInFlight + 1
       ++bt_stored;
@@ -473,16 +565,16 @@ scan_k3v2_kernel(const ScanParams p) {
       __syncwarp();
     }
     const int e0 = it + kPagesInFlight;   // first page to fetch into the slot just freed
-    if (e0 < my_n) refill(sl, bt_s[e0 & (2 * kBtChunk - 1)], bt_s[(e0 + 1) & (2 * kBtChunk - 1)], e0 + 1 < my_n);
-    if (++sl == T::kSlots) { sl = 0; parity ^= 1u; }
+    if (e0 < my_n) refill(slot_off, e0);
+    cp_async_commit();
+    slot_off = (slot_off == (T::kSlots - 1) * T::kSlotBytes) ? 0u : slot_off + T::kSlotBytes;
   }
 
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
-  if (failed && lane == 0) report_status(p.status, JF_ERR_TIMEOUT);
   if (kDoK && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) p.status[4] = want_pm ? kPageMaxTag : 0;
 
   // ---------------- CTA merge: 4 warps -> one partial ----------------
-  __syncthreads();  // every warp is done with its stages (or gave up); smem is reused below
+  __syncthreads();  // every warp is done with its slots; smem is reused below
   {
     float* wo = reinterpret_cast<float*>(smem) + warp * (kHeadsPad * JF_HEAD_DIM);
 #pragma unroll
@@ -498,9 +590,10 @@ scan_k3v2_kernel(const ScanParams p) {
       wo[(2 * tig + 1) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][3], ub, -2.0f * st.oacc[8 + qh][3]);
     }
   }
-  const float smax = __uint_as_float(st.smax_bits << 16);
-  cta_merge_store(p, smem, st.l0, st.l1, st.m_ref0, st.m_ref1, (tig >> 1) ? 0.f : smax, (tig >> 1) ? smax : 0.f,
-                  split, hkv, b);
+  float l0, l1;
+  unpair_f32(st.l2, l0, l1);
+  cta_merge_store(p, smem, l0, l1, st.m_ref0, st.m_ref1, __uint_as_float((st.smax2 & 0x7FFFu) << 16),
+                  __uint_as_float(st.smax2 & 0x7FFF0000u), split, hkv, b);
 }
 
 // ------------------------------------------------------------------------------------
@@ -540,7 +633,7 @@ jf_status_t validate_decode_args(const jf_decode_args* a) {
 template <int DT, int kParts>
 jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
   using T = Tile<JF_MODE_K3V2>;
-  const size_t smem = kScanWarps * T::kSlots * (T::kSlotBytes + 8) + kScanWarps * 2 * kBtChunk * 8;  // ring, barriers, block-table chunks
+  const size_t smem = kScanWarps * T::kSlots * T::kSlotBytes + kScanWarps * 2 * kBtChunk * 8;  // ring, block-table chunks
   static_assert(kScanWarps * T::kSlots * T::kSlotBytes >= kMergeBytes, "merge buffer");
   JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts>), smem);
   JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts>, grid, dim3(kScanWarps * 32), smem, stream, sp));

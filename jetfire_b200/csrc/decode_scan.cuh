@@ -8,14 +8,12 @@ namespace jf {
 
 template <int MODE> struct Tile;
 template <> struct Tile<JF_MODE_K3V2> {
-  // A warp's ring is made of two-page slots: [K page A | K page B | V page A | V page B |
-  // K scales A, B | V scales A, B]; two pages whose blocks are neighbours in the cache are
-  // fetched with one bulk copy per array.
+  // A warp's ring is made of slots of two pages; a page is [K | V | K scales | V scales].
   static constexpr int kKRow = 48, kVRow = 32, kNG = 2;
   static constexpr int kKPage = 768, kVPage = 512, kSPage = 64;   // bytes per page and array
-  static constexpr int kVOff = 1536, kKsOff = 2560, kVsRel = 128; // slot-relative; V scales from the K scales
-  static constexpr int kSlotBytes = 2816;
-  static constexpr int kPageTx = 1408;    // bytes that land per page
+  static constexpr int kVOff = 768, kKsOff = 1280, kVsRel = 64;   // page-relative; V scales from the K scales
+  static constexpr int kPageTx = 1408;    // bytes per page
+  static constexpr int kSlotBytes = 2 * kPageTx;
   static constexpr int kSlots = 4;        // two-page slots per warp: eight pages in flight
 };
 template <> struct Tile<JF_MODE_K4V4> {
@@ -60,14 +58,7 @@ struct ScanParams {
   int tile_base[9];
 };
 
-constexpr uint32_t kMagic = 0x64006400u;  // fp16 1024.0 in both halves
 constexpr int kBtChunk = 16;              // block-table entries fetched per load (one per lane of a half-warp)
-
-template <int DT>
-__device__ __forceinline__ float load_q(const void* q, int64_t idx) {
-  return Elem<DT>::to_f32(reinterpret_cast<const uint16_t*>(q)[idx]);
-}
-
 
 // Bytes of shared memory the merge needs (per-warp output tiles + statistics).
 constexpr int kMergeBytes = (kScanWarps * kHeadsPad * JF_HEAD_DIM + 3 * kScanWarps * kHeadsPad) * 4;
@@ -128,35 +119,6 @@ __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* sm
     for (int w = 0; w < kScanWarps; ++w) s = fmaxf(s, sm_s[w * 2 + threadIdx.x]);
     p.part_smax[pidx * 2 + threadIdx.x] = s;
   }
-}
-
-// Online-softmax step shared by the modes: the reference point may lag the true maximum
-// by less than 4 (so exp stays below e^4 and the fp16 P operand cannot overflow); the
-// exact warp-wide maximum is only taken when a score runs ahead of it.
-template <int NT>
-__device__ __forceinline__ void softmax_step(float s0, float s1, float s2, float s3, float& m_ref0, float& m_ref1,
-                                             float& l0, float& l1, float (&oacc)[NT][4], float& p0, float& p1,
-                                             float& p2, float& p3) {
-  float mx0 = fmaxf(s0, s2), mx1 = fmaxf(s1, s3);
-  const bool need = (mx0 > m_ref0 + 4.0f) || (mx1 > m_ref1 + 4.0f);
-  if (__any_sync(0xFFFFFFFFu, need)) {
-#pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-      mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, o));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, o));
-    }
-    const float n0 = fmaxf(m_ref0, mx0), n1 = fmaxf(m_ref1, mx1);
-    const float f0 = ex2((m_ref0 - n0) * kLog2e), f1 = ex2((m_ref1 - n1) * kLog2e);
-    l0 *= f0; l1 *= f1;
-#pragma unroll
-    for (int i = 0; i < NT; ++i) { oacc[i][0] *= f0; oacc[i][1] *= f1; oacc[i][2] *= f0; oacc[i][3] *= f1; }
-    m_ref0 = n0; m_ref1 = n1;
-  }
-  const float mb0 = m_ref0 * kLog2e, mb1 = m_ref1 * kLog2e;
-  p0 = ex2(fmaf(s0, kLog2e, -mb0)); p1 = ex2(fmaf(s1, kLog2e, -mb1));
-  p2 = ex2(fmaf(s2, kLog2e, -mb0)); p3 = ex2(fmaf(s3, kLog2e, -mb1));
-  l0 += p0 + p2;
-  l1 += p1 + p3;
 }
 
 // parts: 0 = scores and output partials, 1 = scores and softmax sums only, 2 = output partials from

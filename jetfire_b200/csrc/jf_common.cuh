@@ -185,6 +185,11 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
+// 16 bytes at [src + OFF] to [dst + OFF] (shared-memory address)
+template <int OFF>
+__device__ __forceinline__ void cp_async_16_off(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0+%2], [%1+%2], 16;" ::"r"(dst), "l"(src), "n"(OFF) : "memory");
+}
 __device__ __forceinline__ void bulk_g2s_u32_hint(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar,
                                                   uint64_t policy) {
   asm volatile(
