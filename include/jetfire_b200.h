@@ -137,6 +137,18 @@ jf_status_t jf_pack_append_kv_mirror(const void* key_tok, const void* value_tok,
                                      int64_t num_slots, int32_t k_bits, int32_t v_bits,
                                      int32_t group_size, void* k_mirror, void* v_mirror,
                                      jf_stream_t stream);
+/* The append of a layer's cache store in one launch: jf_pack_append_kv_mirror that also records the
+ * written slots, filled[slot] = 1 (num_slots bytes, device; the reference's slot_filled,
+ * jetfire_vllm/adapter/cache_store.py:686-759).  k_mirror / v_mirror may both be NULL, so may filled. */
+jf_status_t jf_store_append(const void* key_tok, const void* value_tok, int32_t dtype,
+                            int64_t T, int32_t H_kv,
+                            int64_t k_stride_t, int64_t k_stride_h,
+                            int64_t v_stride_t, int64_t v_stride_h,
+                            const int64_t* slots,
+                            uint8_t* k_data, void* k_scales, uint8_t* v_data, void* v_scales,
+                            int64_t num_slots, int32_t k_bits, int32_t v_bits,
+                            int32_t group_size, void* k_mirror, void* v_mirror, uint8_t* filled,
+                            jf_stream_t stream);
 jf_status_t jf_mirror_append_ctx_create(void* k_shadow, void* v_shadow, int32_t H_kv,
                                         int64_t num_slots, int64_t max_tokens, int64_t* handle);
 jf_status_t jf_mirror_append_ctx_destroy(int64_t handle);
@@ -406,6 +418,26 @@ jf_status_t jf_submit_ctx_unwatch(int64_t handle);
 jf_status_t jf_stream_signal_host(jf_stream_t stream, int64_t* done_dev, int64_t* trigger_dev);
 jf_status_t jf_stream_wait_host_flag(jf_stream_t stream, const int64_t* flag_dev, int32_t timeout_ms,
                                      void* status_record);
+
+/* The two ends of a stream-ordered decode step around jf_decode_fused (the reference's input copies,
+ * flag handling, merge and status read of its graph-mode decode, adapter/decode_path.py:2253-2492),
+ * one kernel each, capturable.
+ * begin: q (B, H_q, 128) 16-bit, sequences q_stride elements apart (a multiple of 8), to q_dev and to
+ *   q_host_dev (mapped pinned memory); `width` entries per row of block_table (int64, or int32 with
+ *   bt_is_i32) to bt_dev (row stride bt_dev_stride); seq_lens (int64, or int32) to lens_dev; *done_dev = 0.
+ * end: raises *trigger_dev (NULL: the correction was started earlier), waits for *done_dev at most
+ *   timeout_ms (then JF_ERR_TIMEOUT in the status record, and the stream goes on),
+ *   out = dtype(o_hat + W * o_new - o_old_unnorm) with sequences out_stride elements apart (a multiple
+ *   of 4), and the first JF_STATUS_RECORD_BYTES of the workspace to status_host_dev. */
+jf_status_t jf_step_begin(const void* q, int64_t q_stride, void* q_dev, void* q_host_dev,
+                          const void* block_table, int32_t bt_is_i32, int64_t bt_stride, int32_t width,
+                          int64_t* bt_dev, int32_t bt_dev_stride, const void* seq_lens,
+                          int32_t lens_are_i32, int32_t* lens_dev, int64_t* done_dev, int32_t B,
+                          int32_t H_q, jf_stream_t stream);
+jf_status_t jf_step_end(const float* o_hat, const float* o_old_unnorm, const float* W, const void* o_new,
+                        void* out, int64_t out_stride, int32_t dtype, int32_t B, int32_t H_q,
+                        const int64_t* done_dev, int64_t* trigger_dev, int32_t timeout_ms,
+                        void* status_record, void* status_host_dev, jf_stream_t stream);
 
 /* Pinned host memory mapped into the device address space
  * (alloc_mapped_pinned_pair, jetfire_vllm/csrc/cpu_topk_attn.cpp:958-1040). */

@@ -63,6 +63,16 @@ _SIGS = {
                                              C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                              C.c_int64, C.c_int32, C.c_int32, C.c_int32,
                                              C.c_void_p, C.c_void_p, C.c_void_p]),
+    "jf_store_append": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32,
+                                    C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_void_p,
+                                    C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
+                                    C.c_int64, C.c_int32, C.c_int32, C.c_int32,
+                                    C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "jf_step_begin": (C.c_int32, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32,
+                                  C.c_void_p, C.c_int32, C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_int32,
+                                  C.c_int32, C.c_void_p]),
+    "jf_step_end": (C.c_int32, [C.c_void_p] * 5 + [C.c_int64] + [C.c_int32] * 3 + [C.c_void_p, C.c_void_p, C.c_int32] +
+                    [C.c_void_p] * 3),
     "jf_mirror_append_ctx_create": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int64,
                                                 C.POINTER(C.c_int64)]),
     "jf_mirror_append_ctx_destroy": (C.c_int32, [C.c_int64]),

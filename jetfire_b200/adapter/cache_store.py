@@ -48,16 +48,16 @@ class JetFireCacheStore:
         self.v_data = torch.zeros(num_kv_heads, self.num_slots, head_dim * self.v_nbits // 8, dtype=torch.uint8, **dev)
         self.k_scales = torch.zeros(num_kv_heads, self.num_slots, ng, dtype=torch.bfloat16, **dev)
         self.v_scales = torch.zeros(num_kv_heads, self.num_slots, ng, dtype=torch.bfloat16, **dev)
-        # one spare entry at the end takes the writes of padding / out-of-range slots, so that the
-        # bookkeeping below is a plain scatter with no host step (and can be captured in a graph)
-        self._filled_buf = torch.zeros(self.num_slots + 1, dtype=torch.bool, **dev)
-        self.slot_filled = self._filled_buf[:self.num_slots]
+        # written by the packing kernel (a byte per slot), so the bookkeeping has no launch of its own
+        self._filled_buf = torch.zeros(self.num_slots, dtype=torch.bool, **dev)
+        self.slot_filled = self._filled_buf
         self.written_count = 0
         self.shadow_enabled = bool(shadow_enabled)
         self.mirror_append = mirror_append
         self._k_shadow_dev = self._v_shadow_dev = None
         self._append_ctx = None
         self._pending_event = None
+        self._event: torch.cuda.Event | None = None
         # memory node of the mirrors (and of the workers that gather from them): the GPU's own on a
         # host with several nodes, unless configured otherwise
         self.numa_node = -1
@@ -90,18 +90,14 @@ class JetFireCacheStore:
         padding and are skipped on both sides (jetfire_vllm/kernels/fused_quant_write.py:150-152)."""
         if key_tok.shape != value_tok.shape or key_tok.dim() != 3:
             raise RuntimeError("write_slots: key/value must be (T, H_kv, 128) and match")
-        slot_idx = slot_idx.to(torch.int64)
-        mapped = self.shadow_enabled and self.mirror_append == "mapped"
-        if mapped:
-            ops.fused_quant_write_kv_mirror(key_tok, value_tok, slot_idx, self.k_data, self.k_scales, self.v_data,
-                                            self.v_scales, self.group_size, self.k_nbits, self.v_nbits,
-                                            self._k_shadow_dev, self._v_shadow_dev)
-        else:
-            ops.fused_quant_write_kv(key_tok, value_tok, slot_idx, self.k_data, self.k_scales, self.v_data,
-                                     self.v_scales, self.group_size, self.k_nbits, self.v_nbits)
-        live = (slot_idx >= 0) & (slot_idx < self.num_slots)   # what the packing kernel wrote
-        self._filled_buf.index_fill_(0, torch.where(live, slot_idx, self.num_slots), True)
-        self.written_count += int(key_tok.shape[0])
+        if slot_idx.dtype != torch.int64:
+            slot_idx = slot_idx.to(torch.int64)
+        # one launch: packed rows, the mapped mirror's rows where there is one, the record of filled slots
+        # (padding and out-of-range slots are skipped in all three)
+        ops.store_append(key_tok, value_tok, slot_idx, self.k_data, self.k_scales, self.v_data, self.v_scales,
+                         self.group_size, self.k_nbits, self.v_nbits, self._k_shadow_dev, self._v_shadow_dev,
+                         self.slot_filled)
+        self.written_count += key_tok.shape[0]
         if self.shadow_enabled and self.mirror_append == "stream":
             self._append_ctx.append(key_tok, value_tok, slot_idx)
         if self.shadow_enabled and self.mirror_append != "sync":
@@ -109,9 +105,10 @@ class JetFireCacheStore:
             # the graph orders host reads of the mirror against it, and no event is recorded here
             # (the reference's graph path skips its bookkeeping as well, cache_store.py:611-614).
             if not torch.cuda.is_current_stream_capturing():
-                ev = torch.cuda.Event()
-                ev.record()
-                self._pending_event = ev
+                if self._event is None:
+                    self._event = torch.cuda.Event()
+                self._event.record()
+                self._pending_event = self._event
             return
         if self.shadow_enabled:
             idx_cpu = slot_idx.to("cpu")                       # host sync, as in the reference's eager path

@@ -113,7 +113,11 @@ def _set_worker_count(cfg: JetFireConfig, node: int = -1) -> None:
 class _StreamStep:
     """Buffers and calls of one layer's stream-ordered decode step for one (batch, top-k) shape.
     Everything the kernels and the host correction read or write sits at fixed addresses, so the
-    step can be captured once and replayed; the per-step inputs are copied in on the stream."""
+    step can be captured once and replayed; the per-step inputs are copied in on the stream.
+
+    With flags a step is four launches (ops.AdapterStep): one kernel brings the inputs in and sends the
+    query to the host, scan and select (which writes the selected slots straight into mapped memory),
+    and one that starts the correction, waits for it and merges it into the caller's output."""
 
     def __init__(self, store: JetFireCacheStore, cfg: JetFireConfig, B: int, H_q: int, top_k: int,
                  max_blocks: int, max_S: int, dtype, device, scale: float):
@@ -121,15 +125,34 @@ class _StreamStep:
         self.q = torch.zeros(B, H_q, 128, dtype=dtype, device=device)
         self.block_table = torch.zeros(B, max_blocks, dtype=torch.int64, device=device)
         self.seq_lens = torch.zeros(B, dtype=torch.int32, device=device)
+        self.flags = cfg.stream_signal == "flags"
+        slot_dtype = torch.int32 if cfg.slots_i32 else torch.int64
+        out = None
+        if self.flags:
+            # one mapped block: trigger and completion words (a line apart), status record, query, result, slots
+            sizes = (128, 128, self.q.numel() * 2, self.q.numel() * 2, B * H_q * top_k * slot_dtype.itemsize)
+            offs = [0]
+            for n in sizes:
+                offs.append(offs[-1] + (n + 255) // 256 * 256)
+            self.mapped = ops.alloc_mapped_pinned_pair((offs[-1],), torch.uint8)
+            part = lambda side, i, dt, shape: self.mapped[side][offs[i]:offs[i] + sizes[i]].view(dt).reshape(shape)
+            self.mapped[0].zero_()
+            (self.words_host, self.words_dev) = (part(s, 0, torch.int64, (16,)) for s in (0, 1))
+            (self.status_host, status_dev) = (part(s, 1, torch.uint8, (128,)) for s in (0, 1))
+            (self.q_host, q_host_dev) = (part(s, 2, dtype, (B, H_q, 128)) for s in (0, 1))
+            (self.o_new_host, self.o_new) = (part(s, 3, dtype, (B, H_q, 128)) for s in (0, 1))
+            (self.slots_host, slots_host_dev) = (part(s, 4, slot_dtype, (B, H_q, top_k)) for s in (0, 1))
+            # the list the correction reads is written where the host finds it; the other width stays on the device
+            out = ops.DecodeCall.make_out(B, H_q, top_k, device)
+            if cfg.slots_i32:
+                out["topk_slots_i32"] = slots_host_dev
+                self.slots_dev = out["topk_slots"]
+            else:
+                out["topk_slots"] = slots_host_dev
+                self.slots_dev = out["topk_slots_i32"] = torch.empty(B, H_q, top_k, dtype=torch.int32, device=device)
         self.call = ops.DecodeCall(cfg.kernel_mode, self.q, store.k_data, store.k_scales, store.v_data,
                                    store.v_scales, self.block_table, self.seq_lens, max_S, H_q, store.num_kv_heads,
-                                   store.block_size, top_k, scale, slots_i32=cfg.slots_i32)
-        slot_dtype = torch.int32 if cfg.slots_i32 else torch.int64
-        self.slots_dev = self.call.out["topk_slots_i32"] if cfg.slots_i32 else self.call.out["topk_slots"]
-        self.q_host = torch.zeros(B, H_q, 128, dtype=dtype).pin_memory()
-        self.slots_host = torch.zeros(B, H_q, top_k, dtype=slot_dtype).pin_memory()
-        self.out = torch.zeros(B, H_q, 128, dtype=dtype, device=device)
-        self.flags = cfg.stream_signal == "flags"
+                                   store.block_size, top_k, scale, out=out, slots_i32=cfg.slots_i32)
         # rows [cut, B * H_q) of the correction are the GPU's (read from the mapped mirror over the host
         # link while the workers do the others): only with flags, where the kernel that waits for the
         # workers comes after it on the stream
@@ -137,39 +160,48 @@ class _StreamStep:
         self.rows, self.cut = rows, rows
         if self.flags and cfg.gpu_correction_share > 0.0 and store._k_shadow_dev is not None:
             self.cut = max(1, rows - int(round(min(cfg.gpu_correction_share, 0.5) * rows)))
-        self.mirrors_dev = (store._k_shadow_dev, store._v_shadow_dev)
-        self.scale = scale
         if self.flags:
-            # the correction is started and joined through two words in mapped memory (a line apart),
-            # and its result is read by the merge kernel where the workers wrote it
-            self.words_host, self.words_dev = ops.alloc_mapped_pinned_pair((16,), torch.int64)
-            self.words_host.zero_()
-            self.o_new_host, self.o_new = ops.alloc_mapped_pinned_pair((B, H_q, 128), dtype)
-            self.o_new_host.zero_()
+            # the correction is started and joined through two words in mapped memory,
+            # and its result is read by the merging kernel where the workers wrote it
             self.host = ops.HostCorrectionCall(self.q_host, store.k_shadow, store.v_shadow, None, self.slots_host,
                                                self.o_new_host, scale, done_flag=self.words_host[8:9],
                                                rows=(0, self.cut) if self.cut < rows else None)
             self.host.watch(self.words_host[0:1])
+            gpu_rows = (store._k_shadow_dev, store._v_shadow_dev, self.slots_dev, self.cut) if self.cut < rows else None
+            self.native = ops.AdapterStep(self.call, self.q, self.block_table, self.seq_lens, q_host_dev, self.o_new,
+                                          self.words_dev, self.status_host, status_dev, self.host, _HOST_WAIT_MS, gpu_rows)
         else:
+            self.slots_dev = self.call.out["topk_slots_i32"] if cfg.slots_i32 else self.call.out["topk_slots"]
+            self.q_host = torch.zeros(B, H_q, 128, dtype=dtype).pin_memory()
+            self.slots_host = torch.zeros(B, H_q, top_k, dtype=slot_dtype).pin_memory()
             self.o_new_host = torch.zeros(B, H_q, 128, dtype=dtype).pin_memory()
             self.o_new = torch.zeros(B, H_q, 128, dtype=dtype, device=device)
+            self.out = torch.zeros(B, H_q, 128, dtype=dtype, device=device)
             self.host = ops.HostCorrectionCall(self.q_host, store.k_shadow, store.v_shadow, None, self.slots_host,
                                                self.o_new_host, scale)
-        self.status_host = torch.zeros(ops.STATUS_RECORD_BYTES, dtype=torch.uint8).pin_memory()
-        self.status_event: torch.cuda.Event | None = None
+            self.status_host = torch.zeros(ops.STATUS_RECORD_BYTES, dtype=torch.uint8).pin_memory()
+            self.status_event: torch.cuda.Event | None = None
         self.captured = False
 
     def check_previous(self) -> None:
-        """Raise if the previous eager run of this step recorded an error.  Looks only at what has
-        already arrived on the host: the record's copy once its event has completed, and the
-        correction context's own status.  Never waits."""
-        ev = self.status_event
-        if ev is not None and ev.query():
+        """Raise if an earlier eager run of this step recorded an error.  Looks only at what has
+        already arrived on the host: the record's copy (with callbacks: once its event has completed),
+        and the correction context's own status.  Never waits.  (``run`` does the same first.)"""
+        if not self.flags:
+            if self.status_event is None or not self.status_event.query():
+                return
             self.status_event = None
-            ops.decode_status_of_copy(self.status_host)
-            self.host.stream_status()
+        self.status()
 
-    def run(self, query: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor, out_view: torch.Tensor) -> None:
+    def run(self, query: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor, output: torch.Tensor) -> None:
+        """``query`` / ``output``: at least B rows of H_q * 128 elements."""
+        if self.flags:
+            self.captured = self.native.run(query, block_table, seq_lens, output) or self.captured
+        else:
+            self._run_with_callbacks(query[:self.B].view(self.B, self.H_q, 128), block_table, seq_lens,
+                                     output[:self.B].view(self.B, self.H_q, 128))
+
+    def _run_with_callbacks(self, query, block_table, seq_lens, out_view) -> None:
         capturing = torch.cuda.is_current_stream_capturing()
         if not capturing:
             self.check_previous()
@@ -180,16 +212,9 @@ class _StreamStep:
         self.call.fused()
         self.q_host.copy_(self.q, non_blocking=True)
         self.slots_host.copy_(self.slots_dev, non_blocking=True)
-        if self.flags:
-            ops.stream_signal_host(self.words_dev[8:9], self.words_dev[0:1])
-            if self.cut < self.rows:        # the GPU's rows, while the workers do theirs
-                ops.gpu_topk_attn_rows(self.q, self.mirrors_dev[0], self.mirrors_dev[1], self.slots_dev, self.o_new,
-                                       self.scale, (self.cut, self.rows))
-            ops.stream_wait_host_flag(self.words_dev[8:9], _HOST_WAIT_MS, self.call.status_record())
-        else:
-            self.host.stream_submit()
-            self.host.stream_wait()
-            self.o_new.copy_(self.o_new_host, non_blocking=True)
+        self.host.stream_submit()
+        self.host.stream_wait()
+        self.o_new.copy_(self.o_new_host, non_blocking=True)
         res = self.call.out
         if out_view.is_contiguous():
             ops.blend_unnorm_into(res["o_hat"], res["o_old_unnorm"], res["W"], self.o_new, out_view)
@@ -210,9 +235,13 @@ class _StreamStep:
         self.host.stream_status()
 
     def close(self) -> None:
-        """Release the correction context (the dispatcher stops polling its trigger word).  Only
-        once nothing queued on a stream, and no graph, refers to this step any more."""
+        """Release the correction context (the dispatcher stops polling its trigger word) and the mapped
+        block.  Only once nothing queued on a stream, and no graph, refers to this step any more."""
         self.host.close()
+        if self.flags and self.mapped is not None:
+            self.native = None
+            ops.free_mapped_pinned_pair(self.mapped[0])
+            self.mapped = None
 
 
 _MAX_S_STEP = 4096      # a step object serves row lengths up to the next multiple of this
@@ -257,7 +286,7 @@ def decode_batched_stream_ordered(*, store: JetFireCacheStore, query: torch.Tens
         _set_worker_count(cfg, getattr(store, "numa_node", -1))
         step = steps[key] = _StreamStep(store, cfg, B, num_heads, top_k, max_S // store.block_size, max_S,
                                         query.dtype, query.device, float(scale))
-    step.run(query[:B], block_table, seq_lens, output[:B].view(B, num_heads, 128))
+    step.run(query, block_table, seq_lens, output)
     return output
 
 

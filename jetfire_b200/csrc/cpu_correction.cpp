@@ -713,7 +713,7 @@ class Dispatcher {
  public:
   ~Dispatcher() { stop(); }
   void watch(SubmitCtx* c, int64_t* trigger) {
-    std::lock_guard<std::mutex> g(mu_);
+    Turn g(*this);
     c->trigger = trigger;
     reinterpret_cast<std::atomic<int64_t>*>(trigger)->store(0, std::memory_order_release);
     bool present = false;
@@ -726,14 +726,14 @@ class Dispatcher {
     }
   }
   void unwatch(SubmitCtx* c) {
-    std::lock_guard<std::mutex> g(mu_);
+    Turn g(*this);
     for (size_t i = 0; i < watched_.size(); ++i)
       if (watched_[i] == c) { watched_.erase(watched_.begin() + static_cast<long>(i)); break; }
     c->trigger = nullptr;
   }
   void stop() {
     {
-      std::lock_guard<std::mutex> g(mu_);
+      Turn g(*this);
       if (!running_) return;
       running_ = false;
       quit_.store(true);
@@ -742,10 +742,22 @@ class Dispatcher {
   }
 
  private:
+  // The list's mutex for everyone but the loop, which releases it for a moment only between sweeps: it
+  // is told to stay out until the turn has begun (left to chance that took milliseconds).
+  struct Turn {
+    Dispatcher& d;
+    std::unique_lock<std::mutex> lock;
+    explicit Turn(Dispatcher& d_) : d(d_), lock(d_.mu_, std::defer_lock) {
+      d.waiting_.fetch_add(1, std::memory_order_acq_rel);
+      lock.lock();
+      d.waiting_.fetch_sub(1, std::memory_order_acq_rel);
+    }
+  };
   void loop() {
     auto last_hit = std::chrono::steady_clock::now();
     for (uint64_t sweep = 0; !quit_.load(std::memory_order_acquire); ++sweep) {
       bool hit = false;
+      while (waiting_.load(std::memory_order_acquire) != 0) _mm_pause();   // someone wants to change the list
       {
         std::lock_guard<std::mutex> g(mu_);
         for (SubmitCtx* c : watched_) {
@@ -770,6 +782,7 @@ class Dispatcher {
   std::vector<SubmitCtx*> watched_;
   std::thread thread_;
   std::atomic<bool> quit_{false};
+  std::atomic<int> waiting_{0};
   bool running_ = false;
 };
 

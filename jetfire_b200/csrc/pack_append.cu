@@ -375,3 +375,21 @@ extern "C" jf_status_t jf_pack_append_kv_mirror(const void* key_tok, const void*
   return jf::launch_pack(k, &v, dtype, T, H_kv, slots, num_slots, group_size,
                          static_cast<cudaStream_t>(stream));
 }
+
+extern "C" jf_status_t jf_store_append(const void* key_tok, const void* value_tok, int32_t dtype, int64_t T, int32_t H_kv,
+                                       int64_t k_stride_t, int64_t k_stride_h, int64_t v_stride_t, int64_t v_stride_h,
+                                       const int64_t* slots, uint8_t* k_data, void* k_scales, uint8_t* v_data,
+                                       void* v_scales, int64_t num_slots, int32_t k_bits, int32_t v_bits,
+                                       int32_t group_size, void* k_mirror, void* v_mirror, uint8_t* filled,
+                                       jf_stream_t stream) {
+  jf_status_t st = jf::check_side(key_tok, k_stride_t, k_stride_h, k_data, k_scales, k_bits);
+  if (st != JF_OK) return st;
+  st = jf::check_side(value_tok, v_stride_t, v_stride_h, v_data, v_scales, v_bits);
+  if (st != JF_OK) return st;
+  if ((k_mirror == nullptr) != (v_mirror == nullptr) || !jf::aligned(k_mirror, 16) || !jf::aligned(v_mirror, 16)) return JF_ERR_ARG;
+  jf::PackSide k{key_tok, k_stride_t, k_stride_h, k_data, static_cast<uint16_t*>(k_scales), k_bits,
+                 static_cast<uint16_t*>(k_mirror)};
+  jf::PackSide v{value_tok, v_stride_t, v_stride_h, v_data, static_cast<uint16_t*>(v_scales), v_bits,
+                 static_cast<uint16_t*>(v_mirror)};
+  return jf::launch_pack(k, &v, dtype, T, H_kv, slots, num_slots, group_size, static_cast<cudaStream_t>(stream), filled);
+}

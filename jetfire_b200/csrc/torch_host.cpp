@@ -13,12 +13,15 @@
 #include <Python.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/empty_like.h>
 #include <ATen/ops/empty.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -164,10 +167,10 @@ void check_mirror(const at::Tensor& m, const at::Tensor& key, const at::Tensor& 
 }
 
 // quant_write_kv(name, key, value, slot_idx, k_data, k_scales, v_data, v_scales, group_size, k_bits, v_bits,
-//                k_mirror | None, v_mirror | None)
+//                k_mirror | None, v_mirror | None, filled | None)
 PyObject* quant_write_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
-    expect_args(n, 13, "quant_write_kv");
+    expect_args(n, 14, "quant_write_kv");
     const char* name = text(a[0]);
     const at::Tensor &key = tensor(a[1], name, "key_tok"), &value = tensor(a[2], name, "value_tok"),
                      &slots_in = tensor(a[3], name, "slot_idx"), &kd = tensor(a[4], name, "k_data"),
@@ -188,6 +191,13 @@ PyObject* quant_write_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
       km = ptr(k_mirror);
       vm = ptr(v_mirror);
     }
+    uint8_t* filled = nullptr;
+    if (a[13] != Py_None) {
+      const at::Tensor& f = tensor(a[13], name, "filled");
+      require(f.is_cuda() && f.is_contiguous() && f.element_size() == 1 && f.numel() >= kd.size(1), name,
+              "filled must hold a byte per slot");
+      filled = static_cast<uint8_t*>(ptr(f));
+    }
     at::Tensor keep;
     const at::Tensor& slots = contiguous(slots_in, keep);
     const int dt = dtype_id(key);
@@ -195,10 +205,10 @@ PyObject* quant_write_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const auto* sl = static_cast<const int64_t*>(ptr(slots));
     const auto h = static_cast<int32_t>(key.size(1));
     return PyLong_FromLong(unlocked([&] {
-      if (mirrored)
-        return jf_pack_append_kv_mirror(ptr(key), ptr(value), dt, key.size(0), h, key.stride(0), key.stride(1), value.stride(0),
-                                        value.stride(1), sl, static_cast<uint8_t*>(ptr(kd)), ptr(ks), static_cast<uint8_t*>(ptr(vd)),
-                                        ptr(vs), kd.size(1), kb, vb, static_cast<int32_t>(group), km, vm, st);
+      if (mirrored || filled)
+        return jf_store_append(ptr(key), ptr(value), dt, key.size(0), h, key.stride(0), key.stride(1), value.stride(0),
+                               value.stride(1), sl, static_cast<uint8_t*>(ptr(kd)), ptr(ks), static_cast<uint8_t*>(ptr(vd)),
+                               ptr(vs), kd.size(1), kb, vb, static_cast<int32_t>(group), km, vm, filled, st);
       return jf_pack_append_kv(ptr(key), ptr(value), dt, key.size(0), h, key.stride(0), key.stride(1), value.stride(0),
                                value.stride(1), sl, static_cast<uint8_t*>(ptr(kd)), ptr(ks), static_cast<uint8_t*>(ptr(vd)), ptr(vs),
                                kd.size(1), kb, vb, static_cast<int32_t>(group), st);
@@ -480,10 +490,137 @@ PyObject* blend(PyObject*, PyObject* const* p, Py_ssize_t n) {
   });
 }
 
+// ---- the adapter's decode step ----------------------------------------------------------
+
+// Everything of a kept step that does not change from call to call.
+struct Step {
+  const jf_decode_args* a;
+  at::Tensor q, block_table, seq_lens;      // device buffers the argument block names
+  at::Tensor keep[8];                       // mapped views and outputs whose addresses follow
+  void *q_host_dev, *o_new_dev, *status_host_dev;
+  const void* status_host;
+  int64_t *done_dev, *trigger_dev;
+  int64_t ctx;                              // submit context of the host correction
+  int64_t H_q;
+  int32_t timeout_ms;
+  // rows [cut, rows) of the correction on the GPU, when cut < rows
+  const void *k_mirror = nullptr, *v_mirror = nullptr, *slots = nullptr;
+  int32_t slots_i32 = 0;
+  int64_t cut = 0, rows = 0;
+};
+constexpr const char* kStepName = "jetfire_b200._host.Step";
+void step_free(PyObject* o) { delete static_cast<Step*>(PyCapsule_GetPointer(o, kStepName)); }
+
+// step_create(address of the jf_decode_args, q, block_table, seq_lens, q_host_dev, o_new_dev, words_dev (int64: trigger at
+//   0, completion at 8), status_host (CPU), status_host_dev, submit context, timeout_ms,
+//   (k_mirror_dev, v_mirror_dev, slots_dev, cut) | None) -> capsule
+PyObject* step_create(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    const char* name = "decode_step";
+    expect_args(n, 12, "step_create");
+    auto* s = new Step();
+    PyObject* cap = PyCapsule_New(s, kStepName, step_free);
+    if (!cap) { delete s; return nullptr; }
+    try {
+      s->a = reinterpret_cast<const jf_decode_args*>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLong(p[0])));
+      s->q = tensor(p[1], name, "q"); s->block_table = tensor(p[2], name, "block_table"); s->seq_lens = tensor(p[3], name, "seq_lens");
+      for (int i = 0; i < 5; ++i) s->keep[i] = tensor(p[4 + i], name, "step buffer");
+      s->q_host_dev = ptr(s->keep[0]); s->o_new_dev = ptr(s->keep[1]);
+      auto* words = static_cast<int64_t*>(ptr(s->keep[2]));
+      s->trigger_dev = words; s->done_dev = words + 8;
+      s->status_host = ptr(s->keep[3]); s->status_host_dev = ptr(s->keep[4]);
+      s->ctx = integer(p[9]);
+      s->timeout_ms = int32(p[10]);
+      s->H_q = s->q.size(1);
+      s->rows = s->cut = s->q.size(0) * s->H_q;
+      if (p[11] != Py_None) {
+        for (int i = 0; i < 3; ++i) s->keep[5 + i] = tensor(PyTuple_GetItem(p[11], i), name, "correction buffer");
+        s->k_mirror = ptr(s->keep[5]); s->v_mirror = ptr(s->keep[6]); s->slots = ptr(s->keep[7]);
+        s->slots_i32 = s->keep[7].scalar_type() == at::kInt;
+        s->cut = integer(PyTuple_GetItem(p[11], 3));
+      }
+    } catch (...) {
+      Py_DECREF(cap);
+      throw;
+    }
+    return cap;
+  });
+}
+
+// step_run(capsule, query, block_table, seq_lens, output) -> (status, 1 if the stream is capturing, merged output that
+//   still has to be copied into `output` | None).  Nothing here waits on the host.
+PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    const char* name = "decode_step";
+    expect_args(n, 5, "step_run");
+    auto* s = static_cast<Step*>(PyCapsule_GetPointer(p[0], kStepName));
+    if (!s) return nullptr;
+    const int64_t B = s->q.size(0), H = s->H_q, row = H * JF_HEAD_DIM;
+    const jf_stream_t st = current_stream();
+    const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    jf_status_t r = JF_OK;
+    if (!capturing) {   // an error of an earlier run, as far as it has arrived
+      r = jf_decode_status_of_copy(s->status_host);
+      if (r == JF_OK) r = jf_submit_ctx_status(s->ctx);
+    }
+    at::Tensor q = tensor(p[1], name, "query"), bt = tensor(p[2], name, "block_table"), lens = tensor(p[3], name, "seq_lens"),
+               out = tensor(p[4], name, "output");
+    require(q.is_cuda() && bt.is_cuda() && lens.is_cuda() && out.is_cuda(), name, "tensors must be CUDA");
+    require(q.scalar_type() == s->q.scalar_type() && out.scalar_type() == s->q.scalar_type(), name, "query / output dtype mismatch");
+    // rows of H_q * 128 elements, whatever the leading dimensions are called
+    auto rows_ok = [&](const at::Tensor& t, int64_t mult, uintptr_t align) {
+      const bool two = t.dim() == 2 && t.size(1) == row && t.stride(1) == 1;
+      const bool three = t.dim() == 3 && t.size(1) == H && t.size(2) == JF_HEAD_DIM && t.stride(2) == 1 && t.stride(1) == JF_HEAD_DIM;
+      return (two || three) && t.stride(0) % mult == 0 && reinterpret_cast<uintptr_t>(ptr(t)) % align == 0;
+    };
+    require(q.dim() >= 2 && q.size(0) >= B && q.numel() == q.size(0) * row, name, "query must be (B, H_q, 128)");
+    require(out.dim() >= 2 && out.size(0) >= B && out.numel() == out.size(0) * row, name, "output must be (B, H_q * 128)");
+    if (!rows_ok(q, 8, 16)) q = q.contiguous().clone();
+    require(bt.dim() == 2 && bt.size(0) >= B && lens.dim() == 1 && lens.size(0) >= B, name, "block_table / seq_lens shape mismatch");
+    if ((bt.scalar_type() != at::kLong && bt.scalar_type() != at::kInt) || bt.stride(1) != 1) bt = bt.to(at::kLong).contiguous();
+    if ((lens.scalar_type() != at::kLong && lens.scalar_type() != at::kInt) || lens.stride(0) != 1) lens = lens.to(at::kInt).contiguous();
+    const int64_t width = std::min<int64_t>(bt.size(1), s->block_table.size(1));
+    at::Tensor merged;
+    if (!rows_ok(out, 4, 8)) merged = at::empty_like(s->q);
+    const at::Tensor& dst = merged.defined() ? merged : out;
+    const int64_t dst_stride = merged.defined() ? row : dst.stride(0);
+    const int dt = dtype_id(s->q);
+    if (r == JF_OK) {
+      r = unlocked([&] {
+        jf_status_t e = jf_step_begin(ptr(q), q.stride(0), ptr(s->q), s->q_host_dev, ptr(bt), bt.scalar_type() == at::kInt, bt.stride(0),
+                                      static_cast<int32_t>(width), static_cast<int64_t*>(ptr(s->block_table)),
+                                      static_cast<int32_t>(s->block_table.size(1)), ptr(lens), lens.scalar_type() == at::kInt,
+                                      static_cast<int32_t*>(ptr(s->seq_lens)), s->done_dev, static_cast<int32_t>(B),
+                                      static_cast<int32_t>(H), st);
+        if (e == JF_OK) e = jf_decode_fused(s->a, st);
+        int64_t* trigger = s->trigger_dev;
+        if (e == JF_OK && s->cut < s->rows) {   // the GPU's rows, while the workers do theirs
+          e = jf_stream_signal_host(st, s->done_dev, s->trigger_dev);
+          trigger = nullptr;
+          if (e == JF_OK)
+            e = jf_gpu_topk_attn_rows(ptr(s->q), s->k_mirror, s->v_mirror, s->slots, s->slots_i32, s->o_new_dev, dt, s->a->B, s->a->H_q,
+                                      s->a->H_kv, s->a->num_slots, s->a->top_k, s->a->attn_scale, s->cut, s->rows, st);
+        }
+        if (e == JF_OK)
+          e = jf_step_end(s->a->o_hat, s->a->o_old_unnorm, s->a->W, s->o_new_dev, ptr(dst), dst_stride, dt, s->a->B, s->a->H_q,
+                          s->done_dev, trigger, s->timeout_ms, s->a->workspace, s->status_host_dev, st);
+        return e;
+      });
+    }
+    PyObject* res = PyTuple_New(3);
+    if (!res) return nullptr;
+    PyTuple_SET_ITEM(res, 0, PyLong_FromLong(r));
+    PyTuple_SET_ITEM(res, 1, PyLong_FromLong(capturing));
+    PyTuple_SET_ITEM(res, 2, THPVariable_Wrap(merged));
+    return res;
+  });
+}
+
 #define JF_METHOD(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(f)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
     JF_METHOD(quant_write), JF_METHOD(quant_write_kv), JF_METHOD(fused_attn), JF_METHOD(stage_a), JF_METHOD(stage_b),
-    JF_METHOD(decode), JF_METHOD(get_workspace), JF_METHOD(blend), {nullptr, nullptr, 0, nullptr}};
+    JF_METHOD(decode), JF_METHOD(get_workspace), JF_METHOD(blend), JF_METHOD(step_create), JF_METHOD(step_run),
+    {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "tensor-taking half of jetfire_b200.ops", -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

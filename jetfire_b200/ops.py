@@ -77,7 +77,7 @@ def fused_quant_write_kv(key_tok, value_tok, slot_idx, k_data, k_scales, v_data,
     """K and V of the same tokens in one launch, any bit pair."""
     check("fused_quant_write_kv",
           _host.quant_write_kv("fused_quant_write_kv", key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
-                               group_size, k_bits, v_bits, None, None))
+                               group_size, k_bits, v_bits, None, None, None))
 
 
 def fused_quant_write_int4_sym_kv(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
@@ -94,7 +94,15 @@ def fused_quant_write_kv_mirror(key_tok, value_tok, slot_idx, k_data, k_scales, 
     index_copy_ (jetfire_vllm/adapter/cache_store.py:746-756)."""
     name = "fused_quant_write_kv_mirror"
     check(name, _host.quant_write_kv(name, key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales, group_size, k_bits,
-                                     v_bits, k_mirror_dev, v_mirror_dev))
+                                     v_bits, k_mirror_dev, v_mirror_dev, None))
+
+
+def store_append(key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales, group_size, k_bits, v_bits,
+                 k_mirror_dev, v_mirror_dev, filled) -> None:
+    """``fused_quant_write_kv_mirror`` (mirrors may be None) that also marks the written slots in
+    ``filled`` (a byte per slot): a cache store's append in one launch."""
+    check("store_append", _host.quant_write_kv("store_append", key_tok, value_tok, slot_idx, k_data, k_scales, v_data, v_scales,
+                                               group_size, k_bits, v_bits, k_mirror_dev, v_mirror_dev, filled))
 
 
 def map_host_tensor(host: torch.Tensor) -> torch.Tensor:
@@ -259,14 +267,7 @@ class DecodeCall:
         ws_bytes = workspace.numel() - (ws_ptr - workspace.data_ptr())
         f32 = dict(dtype=torch.float32, device=dev)
         if out is None:
-            out = dict(
-                o_hat=torch.empty(B, H_q, 128, **f32), o_old_unnorm=torch.empty(B, H_q, 128, **f32),
-                W=torch.empty(B, H_q, **f32), softmax_m=torch.empty(B, H_q, **f32),
-                softmax_inv_z=torch.empty(B, H_q, **f32),
-                topk_slots=torch.empty(B, H_q, top_k, dtype=torch.int64, device=dev),
-            )
-            out["topk_idx"] = topk_idx if topk_idx is not None else \
-                torch.empty(B, H_q, top_k, dtype=torch.int64, device=dev)
+            out = self.make_out(B, H_q, top_k, dev, topk_idx)
         if scores is not None:
             _require(scores.is_cuda and scores.dtype == torch.float32 and scores.is_contiguous()
                      and tuple(scores.shape) == (B, H_q, max_S), f"{name}: scores must be contiguous f32 (B, H_q, max_S)")
@@ -304,6 +305,15 @@ class DecodeCall:
         a.topk_slots_i32 = ptr(s32)
         self.args = a
         self._addr = C.addressof(a)
+
+    @staticmethod
+    def make_out(B, H_q, top_k, device, topk_idx=None) -> dict:
+        """Fresh output tensors (the default of ``out``)."""
+        f32, i64 = dict(dtype=torch.float32, device=device), dict(dtype=torch.int64, device=device)
+        return dict(o_hat=torch.empty(B, H_q, 128, **f32), o_old_unnorm=torch.empty(B, H_q, 128, **f32),
+                    W=torch.empty(B, H_q, **f32), softmax_m=torch.empty(B, H_q, **f32),
+                    softmax_inv_z=torch.empty(B, H_q, **f32), topk_slots=torch.empty(B, H_q, top_k, **i64),
+                    topk_idx=topk_idx if topk_idx is not None else torch.empty(B, H_q, top_k, **i64))
 
     def scan(self):
         check("jf_decode_scan", _host.decode(1, self._addr))
@@ -344,6 +354,31 @@ class DecodeCall:
         o = self.out
         return FusedAttnOut(o["o_hat"], o["topk_slots"], o["o_old_unnorm"], o["W"], o["topk_idx"],
                             o["softmax_m"], o["softmax_inv_z"], self.scores)
+
+
+class AdapterStep:
+    """A stream-ordered decode step over kept buffers, everything of it in one native call: inputs in,
+    ``call`` (scan, select), the host correction started and joined through words in mapped memory,
+    merge.  ``words_dev``: trigger at 0, completion word at 8; ``status_host`` / ``status_dev``: the
+    record's copy in mapped memory; ``gpu_rows``: (K mirror, V mirror, slot list, first row) of the
+    correction's rows that the GPU computes."""
+
+    def __init__(self, call: DecodeCall, q, block_table, seq_lens, q_host_dev, o_new_dev, words_dev, status_host, status_dev,
+                 host: "HostCorrectionCall", timeout_ms: int, gpu_rows=None):
+        self._keep = (call, host)
+        self._step = _host.step_create(C.addressof(call.args), q, block_table, seq_lens, q_host_dev, o_new_dev, words_dev,
+                                       status_host, status_dev, host._handle(), timeout_ms, gpu_rows)
+
+    def run(self, query, block_table, seq_lens, output) -> bool:
+        """Queues the step; True when the stream is being captured.  Raises for an error that an earlier
+        run recorded and that has arrived on the host."""
+        st, capturing, merged = _host.step_run(self._step, query, block_table, seq_lens, output)
+        if st:
+            check("decode_step", st)
+        if merged is not None:     # rows the merging kernel cannot address
+            B = merged.shape[0]
+            output[:B].view(merged.shape).copy_(merged)
+        return bool(capturing)
 
 
 STATUS_RECORD_BYTES = 16
@@ -831,3 +866,8 @@ def alloc_mapped_pinned_pair(shape, dtype, node: int = -1):
     device = torch.as_tensor(_DevView(), device="cuda").view(dtype)[:n].reshape(*shape)
     host._jf_mapped = (buf, h.value)  # keep the ctypes view alive with the tensor
     return host, device
+
+
+def free_mapped_pinned_pair(host: torch.Tensor) -> None:
+    """Gives the block of an ``alloc_mapped_pinned_pair`` back; neither tensor may be used afterwards."""
+    check("free_mapped_pinned_pair", lib.jf_free_mapped(host._jf_mapped[1]))

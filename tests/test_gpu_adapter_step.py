@@ -1,0 +1,55 @@
+"""The kernels at the two ends of the adapter's stream-ordered step: the forms of inputs and outputs they
+address themselves, and the ones that go through a copy, all give the bits of the plain form."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from jf_testlib import Case
+
+pytestmark = pytest.mark.gpu
+
+
+def _store(case, cfg):
+    from jetfire_b200.adapter.cache_store import JetFireCacheStore
+    st = JetFireCacheStore(num_blocks=case.n_blocks, num_kv_heads=case.H_kv, head_dim=128, cfg=cfg, device="cuda",
+                           dtype=case.dtype, mirror_append="mapped")
+    st.write_slots(case.k_full.transpose(0, 1).contiguous().cuda(), case.v_full.transpose(0, 1).contiguous().cuda(),
+                   torch.arange(case.num_slots, dtype=torch.int32, device="cuda"))      # converted by the store
+    return st
+
+
+@pytest.mark.parametrize("B,H_q,dtype", [(1, 2, torch.bfloat16), (3, 8, torch.float16), (2, 32, torch.bfloat16)])
+def test_step_takes_the_forms_a_caller_has(B, H_q, dtype):
+    from jetfire_b200.adapter.config import JetFireConfig
+    from jetfire_b200.adapter.decode_path import make_decode_metadata, try_jetfire_decode
+    case = Case("k3v2", B, H_q, 2, 200, seed=61 + B, dtype=dtype)
+    cfg = JetFireConfig(mode="SymInt3K_SymInt2V", top_k=32, group_size=64, cpu_attn_threads=2)
+    st = _store(case, cfg)
+    assert bool(st.slot_filled.all())
+    impl = SimpleNamespace(scale=case.attn_scale, attn_type=SimpleNamespace(name="DECODER"))
+    layer = SimpleNamespace(num_heads=H_q, num_kv_heads=2, head_size=128, layer_name="l0")
+    bt, lens, q = case.block_table.cuda(), case.seq_lens.cuda(), case.q.cuda()
+    row = H_q * 128
+
+    def run(query, block_table, seq_lens, out):
+        md = make_decode_metadata(seq_lens, block_table)
+        assert try_jetfire_decode(impl=impl, layer=layer, query=query, attn_metadata=md, output=out, store=st, cfg=cfg) is out
+        torch.cuda.synchronize()
+        return out[:B].reshape(B, row).clone()
+
+    want = run(q, bt, lens, torch.zeros(B, row, dtype=dtype, device="cuda"))
+    wide = torch.full((B + 2, row + 8), 3.0, dtype=dtype, device="cuda")
+    odd = torch.zeros(B, row + 3, dtype=dtype, device="cuda")
+    q_pad = torch.zeros(B + 1, H_q, 128, dtype=dtype, device="cuda")
+    q_pad[:B] = q
+    q_odd = torch.zeros(B * row + 1, dtype=dtype, device="cuda")[1:].view(B, H_q, 128)   # 2-byte aligned
+    q_odd.copy_(q)
+    forms = [(q.view(B, row), bt.to(torch.int32), lens.to(torch.int64), wide[:, :row]),
+             (q_pad, bt, lens, torch.zeros(B, H_q, 128, dtype=dtype, device="cuda")),
+             (q_odd, torch.cat([bt, bt], 1), lens, odd[:, 3:])]
+    for query, table, length, out in forms:
+        if query.dim() == 2:
+            query = query.view(B, H_q, 128)
+        assert torch.equal(run(query, table, length, out), want)
+    assert bool((wide[B:] == 3.0).all()) and bool((wide[:, row:] == 3.0).all())
