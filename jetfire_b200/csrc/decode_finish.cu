@@ -26,24 +26,24 @@ decode_finish_kernel(const FinishParams p, const TailParams tp) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   TailSmem<MODE>& tsm = *reinterpret_cast<TailSmem<MODE>*>(smem_raw);
   __shared__ float sm_m[kSelWarps];
-  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  __shared__ SplitSums splits;
+  const int h = blockIdx.x, b = blockIdx.y;
   const int hkv = h / tp.G, hi = h - hkv * tp.G;
   const int64_t bh = static_cast<int64_t>(b) * tp.H_q + h;
   const int64_t pbase = (static_cast<int64_t>(b) * tp.H_kv + hkv) * tp.splits;
   pdl_wait();
-  SplitPre<kSelThreads> pre;
-  split_preload<kSelThreads>(tp, pbase, hi, tid, pre);
   const int n = min(p.seq_lens[b], tp.max_S);
   const float M = block_max_of_splits(tp.part_m, pbase, hi, tp.splits, sm_m);
+  merge_splits(tp, splits, pbase, hi, M);
   const int64_t* sel = p.topk_idx + bh * tp.top_k;
-  finish_tail<MODE, kSelThreads>(tp, tsm, TailPrefetch{}, pre, M, n, b, h, p.block_table + static_cast<int64_t>(b) * p.max_blocks,
-                    [&](int kk, int& pos, int& cidx) {
-                      const int64_t v = sel[kk];
-                      if (v < 0 || v >= n) return false;
-                      pos = static_cast<int>(v);
-                      cidx = -1;
-                      return true;
-                    });
+  finish_tail<MODE, kSelThreads, false>(tp, tsm, TailPrefetch{}, splits, M, n, b, h,
+                                        p.block_table + static_cast<int64_t>(b) * p.max_blocks, [&](int kk, int& pos, int& cidx) {
+                                          const int64_t v = sel[kk];
+                                          if (v < 0 || v >= n) return false;
+                                          pos = static_cast<int>(v);
+                                          cidx = -1;
+                                          return true;
+                                        });
 }
 
 // Exact row maximum and 1 / sum exp(s - max) of a stored score row, as the reference's

@@ -10,11 +10,16 @@
 // size: a block of NT threads plays the 1024 thread-items and the 32 warps of the widest
 // block one after the other, so every kernel that runs this code gives the same bits.
 //
-// The selected set's sum runs on the tensor cores like the scan's P.V: sixteen staged entries
-// are a "page" (their packed V rows lie one after the other in shared memory), the masked code
-// fields go to mma.sync.m16n8k16 as subnormal fp16 numbers without arithmetic, the weights
-// (times the V group scale, rounded to fp16 as the scan rounds its P operand) are the other
-// operand -- one column of it; the codes' offset leaves through a sum-of-weights tile.
+// The selected set's sum runs on the tensor cores like the scan's P.V: sixteen entries are a "page",
+// the masked code fields of their packed V rows go to mma.sync.m16n8k16 as subnormal fp16 numbers
+// without arithmetic, the weights (times the V group scale, rounded to fp16 as the scan rounds its P
+// operand) are the other operand -- one column of it; the codes' offset leaves through a
+// sum-of-weights tile.
+//
+// What bounds it: latency -- one row per block, a chain of phases.  So there are two barriers for any
+// top-k: the V words are read where they lie (the candidates' rows in shared memory, or the cache)
+// instead of being brought into order first, a warp's groups accumulate in the MMA's registers, and the
+// merge of the scan's partials is apart, for the caller to place where it waits for memory anyway.
 #pragma once
 
 #include "decode_common.cuh"
@@ -23,10 +28,7 @@ namespace jf {
 
 constexpr int kSelThreads = 1024;                        // widest block; the unit of the fixed orders below
 constexpr int kSelWarps = kSelThreads / 32;
-constexpr int kSplitGroups = kSelThreads / JF_HEAD_DIM;  // split partials are summed in 8 strided groups
-constexpr int kSplitPre = 4;                             // partials per thread fetched ahead of use (all its items together)
-constexpr int kTailChunk = 256;                          // selected entries staged per round
-constexpr int kTailPerWarp = kTailChunk / kSelWarps;
+constexpr int kSplitGroups = 16;                         // split partials are summed in 16 strided groups, a warp each
 
 struct TailParams {
   const float* scores;
@@ -47,282 +49,230 @@ struct TailParams {
 
 template <int MODE>
 struct TailSmem {
-  static constexpr int VW = (MODE == JF_MODE_K3V2) ? 8 : 16;  // 32-bit words per packed V row
-  uint32_t v[kTailChunk * VW];                                 // first: 16-byte aligned
-  int64_t slot[kTailChunk];
-  int cidx[kTailChunk];      // candidate index in the prefetched arrays, or -1
-  float wv[kTailChunk][2];   // weight * v scale (per group)
-  float red[kSelWarps][JF_HEAD_DIM];
-  float sum[kSelWarps];
+  static constexpr int VW = (MODE == JF_MODE_K3V2) ? 8 : 16;    // 32-bit words per packed V row
+  static constexpr int kParts = (MODE == JF_MODE_K3V2) ? 2 : 4; // channel ranges (64 / 32 channels), one per warp item
+  static constexpr int kRows = kSelWarps / kParts;              // warps of the widest block per range
+  float red[kRows][JF_HEAD_DIM];
+  float sum[JF_MAX_TOP_K / 32];                                 // weights' sums of 32 entries each
+  int32_t ref[JF_MAX_TOP_K];                                    // entry -> its V row: candidate, or slot
+  uint16_t w[JF_MAX_TOP_K * ((MODE == JF_MODE_K3V2) ? 2 : 1)];  // weight * V scale as fp16 (K3V2: per group)
+};
+
+// The scan's partials of a row merged over the splits, unnormalised: sixteen partial sums per channel.
+struct alignas(16) SplitSums {
   float o[kSplitGroups][JF_HEAD_DIM];
   float z[kSplitGroups];
 };
-
-// The first kSplitPre split partials of thread (group, d), loaded before they are needed so
-// that their latency hides behind other work.
-// Thread-item `it` = (group it >> 7, channel it & 127) of the 1024; a thread of an NT-wide block
-// owns items tid, tid + NT, ... and preloads the first kSplitPre * NT / 1024 splits of each.
-template <int NT>
-struct SplitPre {
-  static constexpr int kItems = kSelThreads / NT, kPer = kSplitPre / kItems;
-  float m[kItems][kPer], l[kItems][kPer], o[kItems][kPer];
-};
-
-template <int NT>
-__device__ __forceinline__ void split_preload(const TailParams& p, int64_t pbase, int hi, int tid, SplitPre<NT>& r) {
-#pragma unroll
-  for (int k = 0; k < SplitPre<NT>::kItems; ++k) {
-    const int it = tid + k * NT;
-    const int d = it & (JF_HEAD_DIM - 1), grp = it >> 7;
-#pragma unroll
-    for (int i = 0; i < SplitPre<NT>::kPer; ++i) {
-      const int s = grp + i * kSplitGroups;
-      r.m[k][i] = kMinusBig; r.l[k][i] = 0.f; r.o[k][i] = 0.f;
-      if (s < p.splits) {
-        const int64_t e = (pbase + s) * kHeadsPad + hi;
-        r.m[k][i] = p.part_m[e];
-        r.l[k][i] = p.part_l[e];
-        r.o[k][i] = p.part_o[e * JF_HEAD_DIM + d];
-      }
-    }
+// Warp w < 16 sums splits w, w + 16, ...: four channels a lane (a 512-byte row per load), the weight worked
+// out by every lane from a broadcast load; two splits are in flight.
+__device__ __forceinline__ void merge_splits(const TailParams& p, SplitSums& out, int64_t pbase, int hi, float M) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= kSplitGroups) return;
+  float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+  float Z = 0.f;
+  for (int s = warp; s < p.splits; s += 2 * kSplitGroups) {
+    const bool two = s + kSplitGroups < p.splits;
+    const int64_t e0 = (pbase + s) * kHeadsPad + hi, e1 = two ? e0 + kSplitGroups * kHeadsPad : e0;
+    const float m0 = p.part_m[e0], m1 = p.part_m[e1], l0 = p.part_l[e0], l1 = p.part_l[e1];
+    const float4 a = reinterpret_cast<const float4*>(p.part_o + e0 * JF_HEAD_DIM)[lane];
+    const float4 c = reinterpret_cast<const float4*>(p.part_o + e1 * JF_HEAD_DIM)[lane];
+    const float w0 = ex2((m0 - M) * kLog2e), w1 = two ? ex2((m1 - M) * kLog2e) : 0.f;
+    Z = fmaf(l0, w0, Z);
+    o.x = fmaf(a.x, w0, o.x); o.y = fmaf(a.y, w0, o.y); o.z = fmaf(a.z, w0, o.z); o.w = fmaf(a.w, w0, o.w);
+    Z = fmaf(l1, w1, Z);
+    o.x = fmaf(c.x, w1, o.x); o.y = fmaf(c.y, w1, o.y); o.z = fmaf(c.z, w1, o.z); o.w = fmaf(c.w, w1, o.w);
   }
-}
-
-// code - bias as a float without an integer-to-float conversion: 2^23 + code is the float
-// with `code` in its low mantissa bits.
-__device__ __forceinline__ float small_code_to_f32(uint32_t code, float bias) {
-  return __uint_as_float(0x4B000000u | code) - (8388608.0f + bias);
+  reinterpret_cast<float4*>(out.o[warp])[lane] = o;
+  if (lane == 0) out.z[warp] = Z;
 }
 
 // What the fused kernel already holds in shared memory per candidate (null pointers in the
 // stand-alone kernel): slot, scan score, V scales, packed V row.  The values are the ones
 // the stand-alone kernel reads from global memory, so both give the same bits.
 struct TailPrefetch {
-  const int64_t* slot;
+  const int32_t* slot;
   const float* score;
   const uint32_t* vsc;    // K3: both group scales; K4: the aligned pair of scales that holds this slot's
   const uint32_t* vrows;
 };
 
-// `src(kk, pos, cidx)` yields the kk-th selected entry (rank order): its position and its
-// index in the prefetched arrays (-1: none); false if there is no such entry.  M = max over
-// the splits of the scan's reference points.  n = sequence length.
-template <int MODE, int NT, typename Src>
-__device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>& sm, const TailPrefetch& pf,
-                                            const SplitPre<NT>& pre, float M, int n, int b, int h, const int64_t* bt,
-                                            Src src) {
-  constexpr int VW = TailSmem<MODE>::VW;
-  constexpr int kW = NT / 32;                 // warps of this block
-  constexpr int kPre = SplitPre<NT>::kPer;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int hkv = h / p.G, hi = h - hkv * p.G;
-  const int64_t bh = static_cast<int64_t>(b) * p.H_q + h;
-  const int64_t pbase = (static_cast<int64_t>(b) * p.H_kv + hkv) * p.splits;
+__device__ __forceinline__ uint32_t f16_bits_sat(float x) { return pack_f16x2_sat(x, 0.f) & 0xFFFFu; }
 
-  // ---- merge splits (unnormalised): thread (group, d) sums splits group, group + 8, ... ----
+// PPW channel ranges (part0 ...) of the selected set's weighted V sum, by one warp: groups of sixteen
+// entries g0, g0 + step, ... of `top_k`.  `row(e)` = address of entry e's packed V row.
+template <int MODE, int PPW, typename RowFn>
+__device__ __forceinline__ void tail_part(const TailSmem<MODE>& sm, float* red, int part0, int g0, int step, int top_k, RowFn row) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  constexpr int NT_ = (MODE == JF_MODE_K3V2) ? 4 : 2;   // output tiles per part, and one for the sum of weights
+  float t[PPW][NT_ + 1][4];
 #pragma unroll
-  for (int k = 0; k < SplitPre<NT>::kItems; ++k) {
-    const int it = tid + k * NT;
-    const int d = it & (JF_HEAD_DIM - 1), grp = it >> 7;
-    float o = 0.f, Z = 0.f;
+  for (int k = 0; k < PPW; ++k)
 #pragma unroll
-    for (int i = 0; i < kPre; ++i) {
-      if (grp + i * kSplitGroups < p.splits) {
-        const float w = ex2((pre.m[k][i] - M) * kLog2e);
-        Z = fmaf(pre.l[k][i], w, Z);
-        o = fmaf(pre.o[k][i], w, o);
+    for (int i = 0; i <= NT_; ++i) t[k][i][0] = t[k][i][1] = t[k][i][2] = t[k][i][3] = 0.f;
+  // entries of the k-slots 2tig, 2tig+1, 2tig+8, 2tig+9, as in the scan's V path of the mode
+  const int e_a = (MODE == JF_MODE_K3V2) ? tig : ((2 * tig >> 2) & 1) | (((2 * tig >> 1) & 1) << 2) | ((2 * tig & 1) << 1);
+  const int e_b = (MODE == JF_MODE_K3V2) ? tig + 4
+                                         : (((2 * tig + 1) >> 2) & 1) | ((((2 * tig + 1) >> 1) & 1) << 2) | (((2 * tig + 1) & 1) << 1);
+  for (int grp = g0; 16 * grp < top_k; grp += step) {
+    const int e0 = 16 * grp;   // entries past top_k have a place in the arrays and weigh nothing
+    const uint8_t *ra = row(e0 + e_a), *rb = row(e0 + e_b), *rc = row(e0 + e_a + 8), *rd = row(e0 + e_b + 8);
+    if (MODE == JF_MODE_K3V2) {
+      uint32_t wa = 0u, wb = 0u, wc = 0u, wd = 0u;   // {group 0, group 1} weights
+      if (g == 0) {   // the one column of the weight operand
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(sm.w) + e0;
+        wa = w[e_a]; wb = w[e_b]; wc = w[e_a + 8]; wd = w[e_b + 8];
+      }
+#pragma unroll
+      for (int k = 0; k < PPW; ++k) {
+        const int part = part0 + k, at = 16 * part + 2 * g;
+        const uint32_t Ha = *reinterpret_cast<const uint16_t*>(ra + at), Hb = *reinterpret_cast<const uint16_t*>(rb + at);
+        const uint32_t Hc = *reinterpret_cast<const uint16_t*>(rc + at), Hd = *reinterpret_cast<const uint16_t*>(rd + at);
+        const uint32_t sel = part ? 0x7632u : 0x5410u;
+        const uint32_t b0 = prmt(wa, wb, sel), b1 = prmt(wc, wd, sel);
+        const uint32_t XA = Ha | (Hb << 16), XB = Hc | (Hd << 16);
+        const uint32_t XA2 = XA >> 10, XB2 = XB >> 10;
+        constexpr uint32_t m0 = 0x00030003u;
+        mma_f16_16816(t[k][0], XA & m0, XA & (m0 << 2), XB & m0, XB & (m0 << 2), b0, b1);
+        mma_f16_16816(t[k][1], XA & (m0 << 4), XA & (m0 << 6), XB & (m0 << 4), XB & (m0 << 6), b0, b1);
+        mma_f16_16816(t[k][2 % NT_], XA & (m0 << 8), XA2 & m0, XB & (m0 << 8), XB2 & m0, b0, b1);
+        mma_f16_16816(t[k][3 % NT_], XA2 & (m0 << 2), XA2 & (m0 << 4), XB2 & (m0 << 2), XB2 & (m0 << 4), b0, b1);
+        mma_f16_16816(t[k][NT_], 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, b0, b1);
+      }
+    } else {
+      uint32_t b0 = 0u, b1 = 0u;
+      if (g == 0) {
+        b0 = sm.w[e0 + e_a] | (static_cast<uint32_t>(sm.w[e0 + e_b]) << 16);
+        b1 = sm.w[e0 + e_a + 8] | (static_cast<uint32_t>(sm.w[e0 + e_b + 8]) << 16);
+      }
+#pragma unroll
+      for (int k = 0; k < PPW; ++k) {
+        const int wi = (part0 + k) & 1, bp = (part0 + k) >> 1, at = 8 * g + 4 * wi;   // channels 16g + 8wi ..
+        const uint32_t wa = *reinterpret_cast<const uint32_t*>(ra + at), wb = *reinterpret_cast<const uint32_t*>(rb + at);
+        const uint32_t wc = *reinterpret_cast<const uint32_t*>(rc + at), wd = *reinterpret_cast<const uint32_t*>(rd + at);
+        const uint32_t sel = bp ? 0x7632u : 0x5410u;
+        const uint32_t XA = prmt(wa, wb, sel), XB = prmt(wc, wd, sel);
+        const uint32_t XA2 = XA >> 8, XB2 = XB >> 8;
+        constexpr uint32_t m0 = 0x000F000Fu;
+        mma_f16_16816(t[k][0], XA & m0, XA & (m0 << 4), XB & m0, XB & (m0 << 4), b0, b1);
+        mma_f16_16816(t[k][1], XA2 & m0, XA2 & (m0 << 4), XB2 & m0, XB2 & (m0 << 4), b0, b1);
+        mma_f16_16816(t[k][NT_], 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, b0, b1);
       }
     }
-    // the remaining splits four at a time: the twelve loads first (with many splits -- few
-    // (sequence, KV head) pairs on the GPU -- one load after the other made this the longest part
-    // of the stage), then the sums in the same ascending order as before
-    for (int s = grp + kPre * kSplitGroups; s < p.splits; s += 4 * kSplitGroups) {
-      float pm[4], pl[4], po[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int su = s + u * kSplitGroups;
-        pm[u] = kMinusBig; pl[u] = 0.f; po[u] = 0.f;
-        if (su < p.splits) {
-          const int64_t e = (pbase + su) * kHeadsPad + hi;
-          pm[u] = p.part_m[e];
-          pl[u] = p.part_l[e];
-          po[u] = p.part_o[e * JF_HEAD_DIM + d];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (s + u * kSplitGroups < p.splits) {
-          const float w = ex2((pm[u] - M) * kLog2e);
-          Z = fmaf(pl[u], w, Z);
-          o = fmaf(po[u], w, o);
-        }
-      }
-    }
-    sm.o[grp][d] = o;
-    if (d == 0) sm.z[grp] = Z;
   }
+  if (tig != 0) return;
+#pragma unroll
+  for (int k = 0; k < PPW; ++k) {
+    const int part = part0 + k;
+    const float* sums = t[k][NT_];
+    if (MODE == JF_MODE_K3V2) {   // column 0: rows g (fields 2ml) and g + 8 (fields 2ml + 1)
+#pragma unroll
+      for (int ml = 0; ml < NT_; ++ml) {
+        const int fa = 2 * ml, fb = 2 * ml + 1;
+        // bit position of field f in its 16-bit half (after the shift by 10 for f >= 5) and its channel
+        const int pa = fa <= 4 ? 2 * fa : 2 * fa - 10, pb = fb <= 4 ? 2 * fb : 2 * fb - 10;
+        const int da = 64 * part + 8 * g + 4 * (fa >> 2) + 3 - (fa & 3), db = 64 * part + 8 * g + 4 * (fb >> 2) + 3 - (fb & 3);
+        red[da] = fmaf(t[k][ml][0], 16777216.0f / static_cast<float>(1 << pa), -2.0f * sums[0]);
+        red[db] = fmaf(t[k][ml][2], 16777216.0f / static_cast<float>(1 << pb), -2.0f * sums[2]);
+      }
+    } else {   // low nibble -> row g (odd channel), high nibble -> row g + 8 (even channel)
+      const int wi = part & 1, bp = part >> 1;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int dlo = 16 * g + 8 * wi + 4 * bp + 2 * e + 1;
+        red[dlo] = fmaf(t[k][e][0], 16777216.0f, -8.0f * sums[0]);
+        red[dlo - 1] = fmaf(t[k][e][2], 1048576.0f, -8.0f * sums[2]);
+      }
+    }
+  }
+}
 
-  // ---- selected set: weights from the scan's scores ----
+// `src(kk, pos, cidx)` yields the kk-th selected entry (rank order): its position and its
+// index in the prefetched arrays; false if there is no such entry.  PRE: the prefetched arrays are there.
+// M = max over the splits of the scan's reference points.  n = sequence length.  `splits` = the merged
+// partials, written before the block's last barrier or by the same threads as here.
+template <int MODE, int NT, bool PRE, typename Src>
+__device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>& sm, const TailPrefetch& pf,
+                                            const SplitSums& splits, float M, int n, int b, int h, const int64_t* bt, Src src) {
+  constexpr int VW = TailSmem<MODE>::VW, kRows = TailSmem<MODE>::kRows;
+  constexpr int kW = NT / 32;                 // warps of this block
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int hkv = h / p.G;
+  const int64_t bh = static_cast<int64_t>(b) * p.H_q + h;
   const ModeInfo mi = mode_info(MODE);
   const uint8_t* v_rows = p.v_data + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.v_row;
   const uint16_t* v_sc = p.v_scales + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.ng;
   const float* srow = p.scores + bh * p.max_S;
-  constexpr int kVW = kSelWarps / kW;   // warps of the widest block this warp plays: warp, warp + kW, ...
-  for (int i = tid; i < kSelWarps * JF_HEAD_DIM; i += NT) (&sm.red[0][0])[i] = 0.f;
-  if (tid < kSelWarps) sm.sum[tid] = 0.f;
-  __syncthreads();
-  for (int k0 = 0; k0 < p.top_k; k0 += kTailChunk) {
-    const int kend = min(kTailChunk, p.top_k - k0);
-    if (tid < kTailChunk) {
+
+  // ---- selected set: weights from the scan's scores, 32 entries per warp and step ----
+  for (int k0 = 32 * warp; k0 < p.top_k; k0 += NT) {
+    const int kk = k0 + lane;
+    int ref = 0;
+    float w = 0.f, vs0 = 0.f, vs1 = 0.f;
+    int pos = -1, cidx = 0;
+    if (kk < p.top_k && n > 0 && src(kk, pos, cidx) && pos >= 0 && pos < n) {
+      float approx;
+      uint32_t sw = 0u;
       int64_t slot = -1;
-      float w = 0.f, vs0 = 0.f, vs1 = 0.f;
-      int pos = -1, cidx = -1;
-      if (tid < kend && n > 0 && src(k0 + tid, pos, cidx) && pos >= 0 && pos < n) {
-        float approx = 0.f;
-        uint32_t sw = 0u;
-        if (cidx >= 0) {
-          slot = pf.slot[cidx];
-          approx = pf.score[cidx];
-          sw = pf.vsc[cidx];
-          if (MODE == JF_MODE_K4V4) sw = (slot & 1) ? (sw >> 16) : (sw & 0xFFFFu);  // the pair that holds the scale
-        } else {
-          const int64_t blk = bt[pos >> 4];
-          approx = srow[pos];  // independent of the block-table lookup
-          if (blk >= 0 && blk < (p.num_slots >> 4)) {
-            slot = blk * 16 + (pos & 15);
-            if (MODE == JF_MODE_K3V2) sw = __ldg(reinterpret_cast<const uint32_t*>(v_sc + slot * 2));
-            else sw = __ldg(v_sc + slot);
-          }
-        }
-        if (slot >= 0) {
-          w = ex2((approx - M) * kLog2e);
-          if (MODE == JF_MODE_K3V2) {
-            vs0 = __uint_as_float(sw << 16);
-            vs1 = __uint_as_float(sw & 0xFFFF0000u);
-          } else {
-            vs0 = vs1 = __uint_as_float(sw << 16);
-          }
+      if (PRE) {
+        slot = pf.slot[cidx];
+        approx = pf.score[cidx];
+        sw = pf.vsc[cidx];
+        if (MODE == JF_MODE_K4V4) sw = (slot & 1) ? (sw >> 16) : (sw & 0xFFFFu);  // the pair that holds the scale
+        ref = cidx;
+      } else {
+        const int64_t blk = bt[pos >> 4];
+        approx = srow[pos];  // independent of the block-table lookup
+        if (blk >= 0 && blk < (p.num_slots >> 4)) {
+          slot = blk * 16 + (pos & 15);
+          ref = static_cast<int>(slot);
+          if (MODE == JF_MODE_K3V2) sw = __ldg(reinterpret_cast<const uint32_t*>(v_sc + slot * 2));
+          else sw = __ldg(v_sc + slot);
         }
       }
-      sm.slot[tid] = slot;
-      sm.cidx[tid] = cidx;
-      sm.wv[tid][0] = w * vs0; sm.wv[tid][1] = w * vs1;
-      // the weights' sum: whole warps are here (kTailChunk is a multiple of 32); fixed order
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
-      if (lane == 0) sm.sum[warp] += w;
-    }
-    __syncthreads();
-    // packed V rows, one 16-byte load per thread
-    for (int u = tid; u < kend * (VW / 4); u += NT) {
-      const int c = u / (VW / 4), part = u - c * (VW / 4);
-      const int64_t slot = sm.slot[c];
-      const int cidx = sm.cidx[c];
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
       if (slot >= 0) {
-        if (cidx >= 0) v = reinterpret_cast<const uint4*>(pf.vrows)[cidx * (VW / 4) + part];
-        else v = __ldg(reinterpret_cast<const uint4*>(v_rows + slot * (VW * 4)) + part);
-      }
-      reinterpret_cast<uint4*>(sm.v)[u] = v;
-    }
-    __syncthreads();
-    // Work item (group of 16 staged entries, quarter of the channels) -> warp item & 31 of the
-    // widest block; its four output tiles and the sum-of-weights tile are added to the warp's own
-    // row of sm.red (no other warp touches it).
-    {
-      const int g = lane >> 2, tig = lane & 3;
-      constexpr int kGroups = kTailChunk / 16;
-      constexpr int kParts = (MODE == JF_MODE_K3V2) ? 2 : 4;          // channel ranges per group: 64 / 32 channels
-      static_assert(kGroups * kParts <= 2 * kSelWarps, "work items per round");
-#pragma unroll
-      for (int k = 0; k < kVW * (kGroups * kParts / kSelWarps); ++k) {
-        const int item = warp + k * kW;                  // 0 .. kGroups * kParts - 1
-        const int grp = item % kGroups, part = item / kGroups;
-        if (16 * grp >= kend) continue;                  // warp-uniform: no live entry in the group
-        const int e0 = 16 * grp;
-        float t[5][4];
-#pragma unroll
-        for (int i = 0; i < 5; ++i) t[i][0] = t[i][1] = t[i][2] = t[i][3] = 0.f;
-        float* red = sm.red[item & (kSelWarps - 1)];
-        if (MODE == JF_MODE_K3V2) {
-          // as the scan's V path (k-slots 2tig, 2tig+1, 2tig+8, 2tig+9 <-> entries tig, tig+4, tig+8, tig+12)
-          const int qh = part;
-          const uint8_t* page = reinterpret_cast<const uint8_t*>(sm.v + e0 * VW) + 16 * qh + 2 * g;
-          const uint32_t Ha = *reinterpret_cast<const uint16_t*>(page + tig * 32);
-          const uint32_t Hb = *reinterpret_cast<const uint16_t*>(page + (tig + 4) * 32);
-          const uint32_t Hc = *reinterpret_cast<const uint16_t*>(page + (tig + 8) * 32);
-          const uint32_t Hd = *reinterpret_cast<const uint16_t*>(page + (tig + 12) * 32);
-          uint32_t b0 = 0u, b1 = 0u;
-          if (g == 0) {   // the one column of the weight operand
-            b0 = pack_f16x2_sat(sm.wv[e0 + tig][qh], sm.wv[e0 + tig + 4][qh]);
-            b1 = pack_f16x2_sat(sm.wv[e0 + tig + 8][qh], sm.wv[e0 + tig + 12][qh]);
-          }
-          const uint32_t XA = Ha | (Hb << 16), XB = Hc | (Hd << 16);
-          const uint32_t XA2 = XA >> 10, XB2 = XB >> 10;
-          constexpr uint32_t m0 = 0x00030003u;
-          mma_f16_16816(t[0], XA & m0, XA & (m0 << 2), XB & m0, XB & (m0 << 2), b0, b1);
-          mma_f16_16816(t[1], XA & (m0 << 4), XA & (m0 << 6), XB & (m0 << 4), XB & (m0 << 6), b0, b1);
-          mma_f16_16816(t[2], XA & (m0 << 8), XA2 & m0, XB & (m0 << 8), XB2 & m0, b0, b1);
-          mma_f16_16816(t[3], XA2 & (m0 << 2), XA2 & (m0 << 4), XB2 & (m0 << 2), XB2 & (m0 << 4), b0, b1);
-          mma_f16_16816(t[4], 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, b0, b1);
-          if (tig == 0) {   // column 0: rows g (fields 2ml) and g + 8 (fields 2ml + 1)
-#pragma unroll
-            for (int ml = 0; ml < 4; ++ml) {
-              const int fa = 2 * ml, fb = 2 * ml + 1;
-              // bit position of field f in its 16-bit half (after the shift by 10 for f >= 5) and its channel
-              const int pa = fa <= 4 ? 2 * fa : 2 * fa - 10, pb = fb <= 4 ? 2 * fb : 2 * fb - 10;
-              const int da = 64 * qh + 8 * g + 4 * (fa >> 2) + 3 - (fa & 3), db = 64 * qh + 8 * g + 4 * (fb >> 2) + 3 - (fb & 3);
-              red[da] += fmaf(t[ml][0], 16777216.0f / static_cast<float>(1 << pa), -2.0f * t[4][0]);
-              red[db] += fmaf(t[ml][2], 16777216.0f / static_cast<float>(1 << pb), -2.0f * t[4][2]);
-            }
-          }
-        } else {
-          // as the K4V4 scan's V path: k-slots 2tig, 2tig+1 (+8) <-> entries tokA, tokB (+8)
-          const int wi = part & 1, bp = part >> 1;
-          const int tokA = ((2 * tig >> 2) & 1) | (((2 * tig >> 1) & 1) << 2) | ((2 * tig & 1) << 1);
-          const int tokB = (((2 * tig + 1) >> 2) & 1) | ((((2 * tig + 1) >> 1) & 1) << 2) | (((2 * tig + 1) & 1) << 1);
-          const uint8_t* page = reinterpret_cast<const uint8_t*>(sm.v + e0 * VW) + 8 * g + 4 * wi;   // channels 16g + 8wi ..
-          const uint32_t wa = *reinterpret_cast<const uint32_t*>(page + tokA * 64);
-          const uint32_t wb = *reinterpret_cast<const uint32_t*>(page + tokB * 64);
-          const uint32_t wc = *reinterpret_cast<const uint32_t*>(page + (tokA + 8) * 64);
-          const uint32_t wd = *reinterpret_cast<const uint32_t*>(page + (tokB + 8) * 64);
-          uint32_t b0 = 0u, b1 = 0u;
-          if (g == 0) {
-            b0 = pack_f16x2_sat(sm.wv[e0 + tokA][0], sm.wv[e0 + tokB][0]);
-            b1 = pack_f16x2_sat(sm.wv[e0 + tokA + 8][0], sm.wv[e0 + tokB + 8][0]);
-          }
-          const uint32_t sel = bp ? 0x7632u : 0x5410u;
-          const uint32_t XA = prmt(wa, wb, sel), XB = prmt(wc, wd, sel);
-          const uint32_t XA2 = XA >> 8, XB2 = XB >> 8;
-          constexpr uint32_t m0 = 0x000F000Fu;
-          mma_f16_16816(t[0], XA & m0, XA & (m0 << 4), XB & m0, XB & (m0 << 4), b0, b1);
-          mma_f16_16816(t[1], XA2 & m0, XA2 & (m0 << 4), XB2 & m0, XB2 & (m0 << 4), b0, b1);
-          mma_f16_16816(t[4], 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, b0, b1);
-          if (tig == 0) {   // low nibble -> row g (odd channel), high nibble -> row g + 8 (even channel)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int dlo = 16 * g + 8 * wi + 4 * bp + 2 * e + 1;
-              red[dlo] += fmaf(t[e][0], 16777216.0f, -8.0f * t[4][0]);
-              red[dlo - 1] += fmaf(t[e][2], 1048576.0f, -8.0f * t[4][2]);
-            }
-          }
-        }
+        w = ex2((approx - M) * kLog2e);
+        vs0 = __uint_as_float(sw << 16);
+        vs1 = __uint_as_float(sw & 0xFFFF0000u);
       }
     }
-    __syncthreads();
+    sm.ref[kk] = ref;     // the arrays hold a whole number of 32 entries: the last group's padding weighs nothing
+    if (MODE == JF_MODE_K3V2)
+      reinterpret_cast<uint32_t*>(sm.w)[kk] = pack_f16x2_sat(w * vs0, w * vs1);
+    else
+      sm.w[kk] = static_cast<uint16_t>(f16_bits_sat(w * vs0));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
+    if (lane == 0) sm.sum[k0 >> 5] = w;
+  }
+  __syncthreads();
+  const int groups = (p.top_k + 15) / 16;
+  {
+    constexpr int PPW = kSelWarps / kW;   // ranges per warp: two in a block of 512 threads
+    const int r = warp % kRows, part0 = (warp / kRows) * PPW;
+    if (r < groups) {
+      if (PRE)
+        tail_part<MODE, PPW>(sm, sm.red[r], part0, r, kRows, p.top_k,
+                             [&](int e) { return reinterpret_cast<const uint8_t*>(pf.vrows + sm.ref[e] * VW); });
+      else
+        tail_part<MODE, PPW>(sm, sm.red[r], part0, r, kRows, p.top_k,
+                             [&](int e) { return v_rows + static_cast<int64_t>(sm.ref[e]) * (4 * VW); });
+    }
   }
   __syncthreads();
   if (tid < JF_HEAD_DIM) {
-    float acc_old = 0.f, ws = 0.f, o = 0.f, Z = 0.f;
+    float acc_old = 0.f, o = 0.f, Z = 0.f;
 #pragma unroll
-    for (int w = 0; w < kSelWarps; ++w) { acc_old += sm.red[w][tid]; ws += sm.sum[w]; }
+    for (int r = 0; r < kRows; ++r)
+      if (r < groups) acc_old += sm.red[r][tid];
 #pragma unroll
-    for (int gI = 0; gI < kSplitGroups; ++gI) { o += sm.o[gI][tid]; Z += sm.z[gI]; }
+    for (int gI = 0; gI < kSplitGroups; ++gI) { o += splits.o[gI][tid]; Z += splits.z[gI]; }
     const bool live = (Z > 0.f) && (n > 0);
     const float inv_z = live ? (1.0f / Z) : 0.f;
     p.o_hat[bh * JF_HEAD_DIM + tid] = o * inv_z;
     p.o_old[bh * JF_HEAD_DIM + tid] = acc_old * inv_z;
     if (tid == 0) {
+      float ws = 0.f;
+      for (int i = 0; 32 * i < p.top_k; ++i) ws += sm.sum[i];
       p.W[bh] = ws * inv_z;
       if (p.softmax_m) p.softmax_m[bh] = live ? M : 0.f;
       if (p.softmax_inv_z) p.softmax_inv_z[bh] = inv_z;

@@ -173,6 +173,13 @@ __device__ __forceinline__ void cp_async_16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_4(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
+// the same, or zeros when `have` is false (the source is then not read, but has to be a valid address)
+__device__ __forceinline__ void cp_async_16_zfill(void* dst, const void* src, bool have) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(have ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_4_zfill(void* dst, const void* src, bool have) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(have ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 // until at most N of this thread's most recent groups are still in flight

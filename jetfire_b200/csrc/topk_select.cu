@@ -18,6 +18,16 @@
 // band does not fit the sort buffer (massive ties, degenerate scales) a slow exact path
 // radix-selects on the 64-bit key (canonical score, ~position) computed on the fly.
 // Slot translation and -1 padding follow csrc/int3_qk_scores.cu:399-417.
+//
+// What bounds it: instructions and the latency of a row's phases, one after the other on one
+// multiprocessor (82 k warp instructions for a row of 32768 positions in blocks of 1024 threads, a fifth
+// of the stalls waiting for instructions).  Hence blocks of 512 threads, two group maxima per
+// thread, no barrier between a candidate's slot, its rows and its score, ranks instead of moved keys.
+// One row alone on its multiprocessor, scan's end to output: 2048 positions 26.8 k -> 20.7 k cycles,
+// 32768 positions 30.9 k -> 24.7 k; 256 rows of 65536 (top-k 512): 60.0 k -> 54.2 k, bound by the
+// scattered reads of the candidates' rows (0.7 M accesses of 64 bytes a layer).
+#include <algorithm>
+
 #include "finish_tail.cuh"
 
 namespace jf {
@@ -46,6 +56,7 @@ struct TopkParams {
   int kv_shift;   // cache head = KV head >> kv_shift (see head_geom)
   int hm_chunks;  // score chunks whose per-float4 maxima fit the shared-memory side table (0: none)
   int np_stride;  // entries per row of pmax
+  int region0;    // bytes of the first shared-memory region
   float attn_scale;
 };
 
@@ -104,17 +115,18 @@ __device__ __forceinline__ float canon_score_k3(const float* q, const uint8_t* r
 // Every lane of the warp must call this; lanes of a candidate get the same value.
 __device__ __forceinline__ float canon_score_k3_x8(const float (&qv)[16], const uint32_t* row, float attn, int lane) {
   const int sub = lane & 7;
+  const bool early = sub <= 4;
+  const uint4 hi4 = *reinterpret_cast<const uint4*>(row + (early ? 0 : 4)), lo4 = *reinterpret_cast<const uint4*>(row + (early ? 4 : 8));
+  const uint32_t hv[4] = {hi4.x, hi4.y, hi4.z, hi4.w}, lv[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
   const uint32_t sw = row[12];
   const uint32_t sc0 = prmt(sw, sw, 0x1010u), sc1 = prmt(sw, sw, 0x3232u);   // each group scale in both halves
   const uint32_t S0 = mul_bf16x2(sc0, 0x71807180u), C0 = mul_bf16x2(sc0, 0xB000B000u);   // * 2^100, * -2^-31
   const uint32_t S1 = mul_bf16x2(sc1, 0x71807180u), C1 = mul_bf16x2(sc1, 0xB000B000u);
-  const bool early = sub <= 4;
   const int sh = early ? 13 - 3 * sub : 21 - 3 * sub;
   float part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const uint32_t p0 = row[r], p1 = row[4 + r], p2 = row[8 + r];
-    const uint32_t hi = early ? p0 : p1, lo = early ? p1 : p2;
+    const uint32_t hi = hv[r], lo = lv[r];
     const uint32_t c01 = (prmt(lo, hi, 0x5140u) >> sh) & 0x00070007u;   // groups 4r, 4r+1
     const uint32_t c23 = (prmt(lo, hi, 0x7362u) >> sh) & 0x00070007u;   // groups 4r+2, 4r+3
     const uint32_t k01 = fma_bf16x2(c01, (r < 2) ? S0 : S1, (r < 2) ? C0 : C1);
@@ -181,21 +193,21 @@ __device__ __forceinline__ int score_bin(float top64, float s) {
 
 // candidates staged in shared memory per round: a top-k of 512 and its band in one (K4V4 has no band to speak of)
 template <int MODE> struct RowChunk { static constexpr int v = (MODE == JF_MODE_K3V2) ? 768 : 576; };
-constexpr int kChunkVec = 8;                   // float4 reads per thread and pass over a chunk
 // 32-bit words per staged K row: K3V2 holds 12 of data and one of scales in a 64-byte slot (16-byte copies land aligned)
 template <int MODE> struct RowWords { static constexpr int v = 16; };
 
 struct SelSmemFixed {
+  SplitSums splits;           // the scan's partials of the row, merged
   uint64_t bar;               // mbarrier of the score-chunk copy
   unsigned long long prefix;
   int hist[kBins];
   float q[JF_HEAD_DIM];
   float qs[4];
   int8_t qi[JF_HEAD_DIM];
-  float w3[kSelWarps][3];
+  float w3[3][kSelWarps];     // per warp: largest reference point, K scales
   float red[4];
   int wsum[kSelWarps];
-  int ncand, tbin, remaining, pad_;
+  int ncand, nlist, tbin, remaining;
 };
 
 // What lives in the score chunk's shared memory once the candidates are collected.
@@ -206,24 +218,25 @@ struct SelSmemLate {
     uint32_t rows[(MODE == JF_MODE_K3V2) ? RowChunk<MODE>::v * RowWords<MODE>::v : 4];   // K3V2: packed K rows + scales (K4V4 re-scores nothing)
   };
   uint32_t vrows[RowChunk<MODE>::v * TailSmem<MODE>::VW];  // packed V rows of the candidates (fused kernel)
-  int64_t cand_slot[RowChunk<MODE>::v];
+  int32_t cand_slot[RowChunk<MODE>::v];                    // slots fit 32 bits (see validate_decode_args)
   uint32_t vsc[RowChunk<MODE>::v];                         // V scales
 };
 
-__host__ __device__ constexpr size_t hm_chunk_bytes(int nt) { return static_cast<size_t>(kChunkVec) * nt * 2; }   // side table of one chunk
+__host__ __device__ constexpr size_t hm_chunk_bytes(int nt, int vec) { return static_cast<size_t>(vec) * nt * 2; }   // side table of one chunk
 constexpr size_t kSelSmemLimit = 227 * 1024;
-// Bytes of the first shared-memory region: the resident score chunk (whose memory the late
-// structures reuse), or -- lean kernel, which never stages the scores -- the late structures alone.
-template <int MODE, bool LEAN, int NT>
-__host__ __device__ constexpr size_t sel_region0_bytes() {
+// Bytes of the first shared-memory region: the resident score chunk (whose memory the late structures
+// reuse; `positions` of it, as many as a row can have), or -- lean kernel, which never stages the scores --
+// the late structures alone.
+template <int MODE>
+__host__ __device__ constexpr size_t sel_region0_bytes(int positions) {
   constexpr size_t late = ((sizeof(SelSmemLate<MODE>) + 127) / 128) * 128;
-  constexpr size_t chunk = static_cast<size_t>(4 * kChunkVec * NT) * 4;   // the resident chunk of an NT-wide block
-  return LEAN ? late : (chunk > late ? chunk : late);
+  const size_t chunk = static_cast<size_t>(positions) * 4;
+  return chunk > late ? chunk : late;
 }
-__host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, int hm_chunks = 0, int nt = kSelThreads) {
+__host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, size_t side_table = 0) {
   // region 0 | fixed | keys[sort_n] | cand_score[sort_n] | perm[sort_n] | bucket[sort_n] | hm16[hm_chunks]
   return region0 + sizeof(SelSmemFixed) + static_cast<size_t>(sort_n) * 8 +
-         static_cast<size_t>(sort_n) * 4 + static_cast<size_t>(sort_n) * 4 + static_cast<size_t>(hm_chunks) * hm_chunk_bytes(nt);
+         static_cast<size_t>(sort_n) * 4 + static_cast<size_t>(sort_n) * 4 + side_table;
 }
 
 // One CTA per (query head, batch element).  The row's approximate scores are pulled into
@@ -235,21 +248,24 @@ __host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, 
 // K-th largest of them is a lower bound of the K-th largest score), and only the pairs whose
 // maximum passes it are fetched -- a few hundred 128-byte reads instead of two passes over
 // the row.  Rows the bins do not fit take the radix tier over global memory.
-// NT: threads per block -- 1024, or (lean only) 512 with two blocks per multiprocessor, so that
-// one row's chains of dependent memory round trips run under the other's arithmetic.
-template <int MODE, int DT, bool FUSED, bool LEAN, int NT>
-__global__ void __launch_bounds__(NT, kSelThreads / NT)
+// NT, VEC: threads per block, and float4s per thread of a resident chunk.  A row is a chain of phases
+// that every warp goes through, so the number of warps sets the instructions a row costs and sixteen
+// are enough to hide the memory: 512 threads -- with VEC 8 two blocks share a multiprocessor, so
+// that one row's round trips run under the other's arithmetic -- and 1024 only for sort buffers
+// beyond 1024 entries, which are sorted by all threads.
+template <int MODE, int DT, bool FUSED, bool LEAN, int NT, int VEC>
+__global__ void __launch_bounds__(NT, (NT == 512 && VEC == 8) ? 2 : 1)
 topk_select_kernel(const TopkParams p, const TailParams tp) {
   constexpr int kW = NT / 32;                   // warps of this block
+  constexpr int kChunkVec = VEC;
   constexpr int kChunkPos = 4 * kChunkVec * NT; // positions per pass over a chunk
   constexpr int W = RowWords<MODE>::v;         // 32-bit words staged per candidate: data + scales
-  constexpr size_t kRegion0 = sel_region0_bytes<MODE, LEAN, NT>();
   constexpr int kRowChunk = RowChunk<MODE>::v;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* chunk = reinterpret_cast<float*>(smem_raw);
   SelSmemLate<MODE>& late = *reinterpret_cast<SelSmemLate<MODE>*>(smem_raw);
-  SelSmemFixed& sm = *reinterpret_cast<SelSmemFixed*>(smem_raw + kRegion0);
-  uint64_t* keys = reinterpret_cast<uint64_t*>(smem_raw + kRegion0 + sizeof(SelSmemFixed));  // [sort_n]
+  SelSmemFixed& sm = *reinterpret_cast<SelSmemFixed*>(smem_raw + p.region0);
+  uint64_t* keys = reinterpret_cast<uint64_t*>(smem_raw + p.region0 + sizeof(SelSmemFixed));  // [sort_n]
   float* cand_score = reinterpret_cast<float*>(keys + p.sort_n);  // [sort_n] scan score per candidate
   uint16_t* perm = reinterpret_cast<uint16_t*>(cand_score + p.sort_n);             // [sort_n] rank -> candidate
   uint16_t* bucket = perm + p.sort_n;                                              // [sort_n] candidates grouped by bin
@@ -270,8 +286,9 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   // ---- score chunks: bulk copy (16-byte aligned rows) or plain loads ----
   const bool vec = ((p.max_S & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.scores) & 15) == 0);
   uint32_t phase = 0;
-  auto issue_chunk = [&](int ci) {  // the row's allocation covers max_S positions
-    const int cnt = min(kChunkPos, p.max_S - ci * kChunkPos);
+  int n_seq = 0;
+  auto issue_chunk = [&](int ci) {  // whole float4s of the row (its allocation covers max_S positions)
+    const int cnt = min(kChunkPos, vec ? ((n_seq + 3) & ~3) - ci * kChunkPos : n_seq - ci * kChunkPos);
     if (vec) {
       if (tid == 0) {
         fence_proxy_async();
@@ -282,8 +299,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       for (int i = tid; i < cnt; i += NT) chunk[i] = srow[static_cast<int64_t>(ci) * kChunkPos + i];
     }
   };
-  // Block-wide; positions past the sequence read as -inf afterwards.  False (for every
-  // thread) if the copy did not arrive within the wait's budget.
+  // Block-wide; positions past the sequence read as -inf afterwards, up to the last float4 that any pass
+  // over the chunk touches.  False (for every thread) if the copy did not arrive within the wait's budget.
   auto wait_chunk = [&](int ci, int n) {
     bool ok = true;
     if (vec) {
@@ -293,7 +310,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     }
     const int valid = max(0, min(n - ci * kChunkPos, kChunkPos));
     if (!vec) __syncthreads();
-    for (int i = valid + tid; i < kChunkPos; i += NT) chunk[i] = -INFINITY;
+    const int used = min((valid + 4 * NT - 1) / (4 * NT) * (4 * NT), kChunkPos);
+    for (int i = valid + tid; i < used; i += NT) chunk[i] = -INFINITY;
     return __syncthreads_and(ok ? 1 : 0) != 0;
   };
   if (tid == 0) {
@@ -308,7 +326,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   uint16_t q_bits = 0;
   if (tid < JF_HEAD_DIM) q_bits = reinterpret_cast<const uint16_t*>(p.q)[bh * JF_HEAD_DIM + tid];
   const int n_seq_raw = p.seq_lens[b];
-  const int n_seq = min(n_seq_raw, p.max_S);
+  n_seq = max(min(n_seq_raw, p.max_S), 0);
   int64_t* out_idx = p.topk_idx + bh * K;
   int64_t* out_slot = p.topk_slots ? p.topk_slots + bh * K : nullptr;
   int32_t* out_slot32 = p.topk_slots_i32 ? p.topk_slots_i32 + bh * K : nullptr;
@@ -333,7 +351,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     }
     if (lane == 0) sm.red[warp] = s1;
   }
-  if (tid == 0) { sm.ncand = 0; sm.tbin = -1; }
+  if (tid == 0) { sm.ncand = 0; sm.nlist = 0; sm.tbin = -1; }
   for (int i = tid; i < kBins; i += NT) hist[i] = 0;
   for (int i = tid; i < p.sort_n; i += NT) keys[i] = 0ull;
 
@@ -350,21 +368,19 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     if (lane < 8) prefetch_l2(first);
   }
 
-  // ---- the scan's results: split statistics first (small), then the 128 KB score chunk ----
+  // ---- the scan's results: the score chunk's copy is started, then the split statistics are read ----
   if (FUSED) pdl_wait();
+  if (!LEAN && n_seq > 0) issue_chunk(0);
   float top = kMinusBig, sm0 = 0.f, sm1 = 0.f;
   if (tid < p.splits) {  // the first split of this thread; the loop below takes the rest
     top = p.part_m[(pbase + tid) * kHeadsPad + hi];
     sm0 = p.part_smax[(pbase + tid) * 2];
     sm1 = p.part_smax[(pbase + tid) * 2 + 1];
   }
-  SplitPre<NT> pre;
-  if (FUSED) split_preload<NT>(tp, pbase, hi, tid, pre);
   // lean: the scan's maxima of groups of pages -- K3V2: pairs of pages, K4V4: single pages
   constexpr int kGroupPages = (MODE == JF_MODE_K3V2) ? 2 : 1;
   const int n_pages = (n_seq + 15) >> 4, n_groups = (n_pages + kGroupPages - 1) / kGroupPages;
   const float4* pm4 = reinterpret_cast<const float4*>(p.pmax + bh * p.np_stride);
-  if (!LEAN) issue_chunk(0);
   {
     for (int s = tid + NT; s < p.splits; s += NT) {
       top = fmaxf(top, p.part_m[(pbase + s) * kHeadsPad + hi]);
@@ -377,7 +393,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       sm0 = fmaxf(sm0, __shfl_xor_sync(0xFFFFFFFFu, sm0, o));
       sm1 = fmaxf(sm1, __shfl_xor_sync(0xFFFFFFFFu, sm1, o));
     }
-    if (lane == 0) { sm.w3[warp][0] = top; sm.w3[warp][1] = sm0; sm.w3[warp][2] = sm1; }
+    if (lane == 0) { sm.w3[0][warp] = top; sm.w3[1][warp] = sm0; sm.w3[2][warp] = sm1; }
   }
   __syncthreads();
 
@@ -390,12 +406,17 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   ctx.num_slots = p.num_slots;
   ctx.attn = p.attn_scale;
 
-  float row_max = kMinusBig;  // max over the splits of the scan's reference points
+  // max over the splits of the scan's reference points, by every warp for itself
+  auto over_warps = [&](const float (&v)[kSelWarps], float none) {
+    float x = lane < kW ? v[lane] : none;
 #pragma unroll
-  for (int w = 0; w < kW; ++w) row_max = fmaxf(row_max, sm.w3[w][0]);
+    for (int o = kW / 2; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
+    return __shfl_sync(0xFFFFFFFFu, x, 0);
+  };
+  const float row_max = over_warps(sm.w3[0], kMinusBig);
 
   // the copy issued at the top must have landed before its shared memory is reused
-  bool copied = LEAN ? true : wait_chunk(0, n_seq);
+  bool copied = (LEAN || n_seq == 0) ? true : wait_chunk(0, n_seq);
   if (!copied && tid == 0) report_status(p.status, JF_ERR_TIMEOUT);
   if (LEAN && p.status[4] != kPageMaxTag) {   // the scan before this call left no page maxima: arguments do not match
     if (tid == 0) report_status(p.status, JF_ERR_STATE);
@@ -404,7 +425,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   const int n = copied ? n_seq : 0;   // a row whose scores did not arrive selects nothing
 
   int m_sel = 0;  // entries of keys[] that hold the ranked result
-  bool prefetch = false;
+  bool prefetch = false, merged = false;
+  const bool by_rank = p.sort_n <= kSelThreads;   // the result is perm[]: rank -> entry of keys[]; else keys[] itself is sorted
   if (n > 0) {
     int ncand = 0;
     int cand_last = kBins;  // bound on the candidates' canonical-score bin, when one is known
@@ -415,9 +437,6 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       for (int i = tid; i < n; i += NT) { keys[i] = static_cast<uint64_t>(i); cand_score[i] = LEAN ? srow[i] : chunk[i]; }
       ncand = n;
     } else {
-      float sm0 = 0.f, sm1 = 0.f;
-#pragma unroll
-      for (int w = 0; w < kW; ++w) { sm0 = fmaxf(sm0, sm.w3[w][1]); sm1 = fmaxf(sm1, sm.w3[w][2]); }
       const float top = row_max + 4.0f;  // the scan lets its reference point lag the true maximum by at most 4
       const float top64 = top * kBinsPerUnit;
       float delta = 0.f;
@@ -428,7 +447,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         // truncating).  sum|q_d k_hat_d| <= sum_g 3 * scale_g * sum_{d in g} |q_d|.  A factor 32
         // covers both paths with slack; the last term covers the final multiply by attn_scale.
         const float q1a = sm.red[0] + sm.red[1], q1b = sm.red[2] + sm.red[3];
-        const float mag = fabsf(p.attn_scale) * (sm0 * q1a + sm1 * q1b) * 3.0f;
+        const float mag = fabsf(p.attn_scale) * (over_warps(sm.w3[1], 0.f) * q1a + over_warps(sm.w3[2], 0.f) * q1b) * 3.0f;
         delta = mag * (32.0f / 16777216.0f) + mag * (4.0f / 16777216.0f) + 1e-7f;
       }
       float nbf = ceilf(2.0f * delta * kBinsPerUnit) + 1.0f;
@@ -436,7 +455,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       const int nb = (MODE == JF_MODE_K3V2) ? static_cast<int>(nbf) : 0;  // K4: scan scores are canonical
       const int n_chunks = (n + kChunkPos - 1) / kChunkPos;
       const float4* chunk4 = reinterpret_cast<const float4*>(chunk);
-      // element (j, c) of thread tid is chunk position 4 * (j * 1024 + tid) + c
+      // element (j, c) of thread tid is chunk position 4 * (j * NT + tid) + c; float4s per thread that hold any
+      auto vecs_of = [&](int ci) { return min(kChunkVec, (n - ci * kChunkPos + 4 * NT - 1) / (4 * NT)); };
       auto next_chunk = [&](int ci) {  // block-wide: replace the resident chunk by chunk ci
         __syncthreads();
         issue_chunk(ci);
@@ -459,17 +479,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         }
         if (lane == 31) sm.wsum[warp] = incl;
         __syncthreads();
-        if (warp == 0) {
-          int t = (lane < kW) ? sm.wsum[lane] : 0, inc2 = t;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xFFFFFFFFu, inc2, o);
-            if (lane >= o) inc2 += u;
-          }
-          if (lane < kW) sm.wsum[lane] = inc2 - t;  // exclusive prefix of the warp totals
-        }
-        __syncthreads();
-        int run = sm.wsum[warp] + incl - v;   // count in the bins above this thread's
+        // count in the bins above this thread's (every warp adds up the totals of those before it)
+        int run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? sm.wsum[lane] : 0) + incl - v;
 #pragma unroll
         for (int i = 0; i < kPer; ++i) {
           if (run < want && run + hv[i] >= want) sm.tbin = kPer * tid + i;
@@ -479,114 +490,137 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         __syncthreads();
       };
       // Block-wide: positions whose score passes the test against `thr` (kind 0: greater, 1: greater
-      // or equal, 2: equal) go to keys[off0 ...], in position order (offsets from a warp scan and a
-      // block scan, no atomics); entries at or past `cap` are dropped.  Returns how many passed.
+      // or equal, 2: equal) go to keys[off0 ...], in position order (one block scan per float4 of a thread,
+      // no atomics); entries at or past `cap` are dropped.  Returns how many passed.
       float hm[kChunkVec];  // per float4 of the resident chunk: its largest score (tier 1a's pass)
       bool have_hm = false;
-      auto collect = [&](float thr, int kind, int off0, int cap, bool use16 = false) {
-        int running = 0;  // candidates found in earlier chunks
-        const uint32_t thr16 = float_order_key(thr) >> 16;
-        const bool glob = LEAN || use16;   // the scores come straight from memory
+      auto collect = [&](float thr, int kind, int off0, int cap) {
+        int running = 0;  // candidates found so far
         for (int ci = 0; ci < n_chunks; ++ci) {
-          if (n_chunks > 1 && !glob) next_chunk(ci);
-          uint32_t mask = 0u;
-          // which of the thread's float4s can hold a candidate at all (branch-free; most threads
-          // find none and skip the loads altogether)
-          uint32_t hits = (1u << kChunkVec) - 1u;
-          if (LEAN) {
-#pragma unroll
-            for (int j = 0; j < kChunkVec; ++j)
-              if (ci * kChunkPos + 4 * (j * NT + tid) >= n) hits &= ~(1u << j);
-          } else if (have_hm && kind == 0) {
-            hits = 0u;
-#pragma unroll
-            for (int j = 0; j < kChunkVec; ++j) hits |= static_cast<uint32_t>(hm[j] > thr) << j;
-          } else if (use16) {
-            hits = 0u;
-#pragma unroll
-            for (int j = 0; j < kChunkVec; ++j)
-              hits |= static_cast<uint32_t>(hm16[(ci * kChunkVec + j) * NT + tid] >= thr16) << j;
-          }
-          while (hits) {
-            const int j = __ffs(hits) - 1;
-            hits &= hits - 1u;
-            float4 v;
-            if (glob) {    // straight from memory; positions at or past the length read as -inf
-              const int pos = ci * kChunkPos + 4 * (j * NT + tid);
-              v = *reinterpret_cast<const float4*>(srow + pos);
-              if (pos >= n) v.x = -INFINITY;
-              if (pos + 1 >= n) v.y = -INFINITY;
-              if (pos + 2 >= n) v.z = -INFINITY;
-              if (pos + 3 >= n) v.w = -INFINITY;
-            } else {
-              v = chunk4[j * NT + tid];
+          if (n_chunks > 1 && !LEAN) next_chunk(ci);
+          for (int j = 0; j < vecs_of(ci); ++j) {
+            const int at = 4 * (j * NT + tid), pos = ci * kChunkPos + at;
+            float e[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            if (pos < n) {
+              const float4 v = LEAN ? *reinterpret_cast<const float4*>(srow + pos) : chunk4[j * NT + tid];
+              e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
             }
-            uint32_t m4;
-            if (kind == 0)
-              m4 = static_cast<uint32_t>(v.x > thr) | (static_cast<uint32_t>(v.y > thr) << 1) |
-                   (static_cast<uint32_t>(v.z > thr) << 2) | (static_cast<uint32_t>(v.w > thr) << 3);
-            else if (kind == 1)
-              m4 = static_cast<uint32_t>(v.x >= thr) | (static_cast<uint32_t>(v.y >= thr) << 1) |
-                   (static_cast<uint32_t>(v.z >= thr) << 2) | (static_cast<uint32_t>(v.w >= thr) << 3);
-            else
-              m4 = static_cast<uint32_t>(v.x == thr) | (static_cast<uint32_t>(v.y == thr) << 1) |
-                   (static_cast<uint32_t>(v.z == thr) << 2) | (static_cast<uint32_t>(v.w == thr) << 3);
-            mask |= m4 << (4 * j);
-          }
-          const int cnt = __popc(mask);
-          int incl = cnt;
+            uint32_t mask = 0u;
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += t;
-          }
-          // warp totals -> every warp's offset (no atomics: 32 same-address atomics with a
-          // return value cost more than the whole pass)
-          __syncthreads();   // the previous round's (or caller's) reads of wsum are done
-          if (lane == 31) sm.wsum[warp] = incl;
-          __syncthreads();
-          int wt = (lane < kW) ? sm.wsum[lane] : 0, winc = wt;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xFFFFFFFFu, winc, o);
-            if (lane >= o) winc += t;
-          }
-          const int base = running + __shfl_sync(0xFFFFFFFFu, winc - wt, warp);
-          running += __shfl_sync(0xFFFFFFFFu, winc, 31);
-          int o = off0 + base + incl - cnt;
-          while (mask) {
-            const int e = __ffs(mask) - 1;
-            mask &= mask - 1u;
-            const int at = 4 * ((e >> 2) * NT + tid) + (e & 3);
-            if (o < cap) {
-              keys[o] = static_cast<uint64_t>(ci * kChunkPos + at);
-              cand_score[o] = glob ? srow[ci * kChunkPos + at] : chunk[at];
+            for (int c = 0; c < 4; ++c) {
+              const bool hit = kind == 0 ? e[c] > thr : kind == 1 ? e[c] >= thr : e[c] == thr;
+              if (hit && pos + c < n) mask |= 1u << c;
             }
-            ++o;
+            const int cnt = __popc(mask);
+            int incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+              if (lane >= o) incl += t;
+            }
+            __syncthreads();   // the previous step's (or caller's) reads of wsum are done
+            if (lane == 31) sm.wsum[warp] = incl;
+            __syncthreads();
+            const int wt = (lane < kW) ? sm.wsum[lane] : 0;
+            int o = off0 + running + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wt : 0) + incl - cnt;
+            running += __reduce_add_sync(0xFFFFFFFFu, wt);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              if (mask & (1u << c)) {
+                if (o < cap) { keys[o] = static_cast<uint64_t>(pos + c); cand_score[o] = e[c]; }
+                ++o;
+              }
+            }
           }
         }
         __syncthreads();
         return running;
       };
 
+      // A warp's hits to keys[] / cand_score[]: lane's element c (score e[c], position pos + c) if bit c of `m4`
+      // is set.  Places come from ballots and one shared-memory atomic per call; those past sort_n are dropped.
+      auto append_hits = [&](uint32_t m4, const float (&e)[4], int pos) {
+        uint32_t below = 0u, total = 0u, at[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t v = __ballot_sync(0xFFFFFFFFu, (m4 >> c) & 1u);
+          at[c] = total + __popc(v & ((1u << lane) - 1u));
+          total += __popc(v);
+        }
+        if (lane == 0) below = atomicAdd(&sm.ncand, static_cast<int>(total));
+        below = __shfl_sync(0xFFFFFFFFu, below, 0);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t o = below + at[c];
+          if (((m4 >> c) & 1u) && o < static_cast<uint32_t>(p.sort_n)) { keys[o] = static_cast<uint64_t>(pos + c); cand_score[o] = e[c]; }
+        }
+      };
+      auto above4 = [&](const float4& v, float thr) {
+        return static_cast<uint32_t>(v.x > thr) | (static_cast<uint32_t>(v.y > thr) << 1) | (static_cast<uint32_t>(v.z > thr) << 2) |
+               (static_cast<uint32_t>(v.w > thr) << 3);
+      };
+      // Tier 1a's collection: positions whose score exceeds `thr`, in any order (the ranking does not depend
+      // on it), with no barrier but the last.  Returns how many there are; those past sort_n are dropped.
+      auto collect_any = [&](float thr, bool use16) {
+        const uint32_t thr16 = float_order_key(thr) >> 16;
+        for (int ci = 0; ci < n_chunks; ++ci) {
+          if (n_chunks > 1 && !use16) next_chunk(ci);
+          // which of the thread's float4s hold a candidate
+          uint32_t hits = 0u;
+          if (use16) {
+#pragma unroll
+            for (int j = 0; j < kChunkVec; ++j) hits |= static_cast<uint32_t>(hm16[(ci * kChunkVec + j) * NT + tid] >= thr16) << j;
+          } else if (have_hm) {
+#pragma unroll
+            for (int j = 0; j < kChunkVec; ++j) hits |= static_cast<uint32_t>(hm[j] > thr) << j;
+          } else {
+            hits = (1u << vecs_of(ci)) - 1u;
+          }
+          while (__any_sync(0xFFFFFFFFu, hits != 0u)) {
+            const int j = hits ? __ffs(hits) - 1 : 0;
+            const int pos = ci * kChunkPos + 4 * (j * NT + tid);
+            uint32_t m4 = 0u;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (hits && pos < n) {
+              v = use16 ? *reinterpret_cast<const float4*>(srow + pos) : chunk4[j * NT + tid];
+              m4 = above4(v, thr);
+              if (n - pos < 4) m4 &= (1u << (n - pos)) - 1u;
+            }
+            hits &= hits - 1u;
+            const float e[4] = {v.x, v.y, v.z, v.w};
+            append_hits(m4, e, pos);
+          }
+        }
+        __syncthreads();
+        return sm.ncand;
+      };
+
       const bool use_hm16 = vec && n_chunks > 1 && n_chunks <= p.hm_chunks;
-      // ---- tier 1a: a bound from group maxima.  Each thread holds four groups of positions
-      //      per chunk (stride 4096 inside a group); the K-th largest group maximum is a lower
-      //      bound of the K-th largest score, and far fewer values enter the histogram. ----
+      // ---- tier 1a: a bound from group maxima.  Each thread holds two or four groups of positions
+      //      per chunk; the K-th largest group maximum is a lower bound of the K-th largest
+      //      score, and far fewer values enter the histogram.  Two groups are enough (a ninth more
+      //      candidates than top_k, half the shared-memory atomics of four) while there are at least
+      //      four per selected entry. ----
+      const bool two = (n >= 4 * NT ? 2 * NT * max(1, n / kChunkPos) : n / 2) >= 4 * K;
       for (int ci = 0; !LEAN && ci < n_chunks; ++ci) {
         if (ci > 0) next_chunk(ci);
         float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        const int jn = vecs_of(ci);
 #pragma unroll
         for (int j = 0; j < kChunkVec; ++j) {
-          const float4 v = chunk4[j * NT + tid];
-          gm[0] = fmaxf(gm[0], v.x); gm[1] = fmaxf(gm[1], v.y); gm[2] = fmaxf(gm[2], v.z); gm[3] = fmaxf(gm[3], v.w);
-          hm[j] = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+          hm[j] = -INFINITY;
+          if (j < jn) {
+            const float4 v = chunk4[j * NT + tid];
+            gm[0] = fmaxf(gm[0], v.x); gm[1] = fmaxf(gm[1], v.y); gm[2] = fmaxf(gm[2], v.z); gm[3] = fmaxf(gm[3], v.w);
+            hm[j] = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+          }
           if (use_hm16) {
             const uint32_t k32 = float_order_key(hm[j]);
             hm16[(ci * kChunkVec + j) * NT + tid] =
                 static_cast<uint16_t>(min(0xFFFFu, (k32 >> 16) + ((k32 & 0xFFFFu) ? 1u : 0u)));
           }
         }
+        if (two) { gm[0] = fmaxf(gm[0], gm[1]); gm[1] = fmaxf(gm[2], gm[3]); gm[2] = gm[3] = -INFINITY; }
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (gm[c] > -INFINITY) atomicAdd(&hist[score_bin(top64, gm[c])], 1);
@@ -646,7 +680,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
                 if (lane >= o) incl += t;
               }
               int base = 0;
-              if (lane == 31 && incl > 0) base = atomicAdd(&sm.ncand, incl);
+              if (lane == 31 && incl > 0) base = atomicAdd(&sm.nlist, incl);
               int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
               while (flags) {
                 const int i = __ffs(flags) - 1;   // bit i: page kGroupPages * 4 * i4 + i
@@ -656,47 +690,34 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
               }
             }
             __syncthreads();
-            const int n_list = sm.ncand;
-            __syncthreads();
-            if (tid == 0) sm.ncand = 0;
-            __syncthreads();
+            const int n_list = sm.nlist;
             if (n_list <= list_cap) {
-              // the listed pages come into the (still unused) late region with asynchronous copies,
-              // all in flight at once: one trip to the scores instead of one per round of threads
-              float* stage = reinterpret_cast<float*>(smem_raw);
+              // The listed pages come into the (still unused) late region with asynchronous copies, all in
+              // flight at once, a quarter of a page per lane; a lane looks at the quarters it copied, so
+              // there is no barrier in between.
+              float4* stage = reinterpret_cast<float4*>(smem_raw);
               constexpr int kStageCap = static_cast<int>(sizeof(SelSmemLate<MODE>) / 64);
               for (int b0 = 0; b0 < n_list; b0 += kStageCap) {
-                const int nb = min(kStageCap, n_list - b0);
-                for (int u = tid; u < 4 * nb; u += NT) {
-                  const int l = u >> 2, q4 = u & 3;
-                  cp_async_16(stage + 16 * l + 4 * q4, srow + 16 * static_cast<int>(page_list[b0 + l]) + 4 * q4);
-                }
+                const int nq = 4 * min(kStageCap, n_list - b0);
+                for (int u = tid; u < nq; u += NT)
+                  cp_async_16(stage + u, srow + 16 * static_cast<int>(page_list[b0 + (u >> 2)]) + 4 * (u & 3));
                 cp_async_commit();
                 cp_async_wait_all();
-                __syncthreads();
-                for (int lb = 0; lb < nb; lb += NT) {
-                  const int l = lb + tid;
-                  uint32_t m16 = 0u;
-                  int pos0 = 0;
-                  if (l < nb) {
-                    pos0 = 16 * static_cast<int>(page_list[b0 + l]);
-                    // the four float4s of the page, starting at a different one in neighbouring
-                    // threads: the pages lie 64 bytes apart, and read in step they would collide
-                    // on two groups of banks
-                    const float4* s4 = reinterpret_cast<const float4*>(stage + 16 * l);
-                    const int rot = (l >> 1) & 3;
+                // eight quarters of a lane at a time, four bits each: one scan and one atomic for them all
+                for (int u0 = tid; u0 - lane < nq; u0 += 8 * NT) {   // warp-uniform trip count
+                  uint32_t mask = 0u;
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                      const int q4 = (j + rot) & 3;
-                      const float4 v = s4[q4];
-                      const uint32_t m4 = static_cast<uint32_t>(v.x > thr) | (static_cast<uint32_t>(v.y > thr) << 1) |
-                                          (static_cast<uint32_t>(v.z > thr) << 2) | (static_cast<uint32_t>(v.w > thr) << 3);
-                      m16 |= m4 << (4 * q4);
+                  for (int k = 0; k < 8; ++k) {
+                    const int u = u0 + k * NT;
+                    if (u < nq) {
+                      uint32_t m4 = above4(stage[u], thr);
+                      const int live = n - (16 * static_cast<int>(page_list[b0 + (u >> 2)]) + 4 * (u & 3));   // tokens inside the sequence
+                      if (live < 4) m4 &= (1u << max(live, 0)) - 1u;
+                      mask |= m4 << (4 * k);
                     }
-                    const int live = n - pos0;   // tokens of the page inside the sequence
-                    if (live < 16) m16 &= (1u << max(live, 0)) - 1u;
                   }
-                  const int cnt = __popc(m16);
+                  if (!__any_sync(0xFFFFFFFFu, mask != 0u)) continue;
+                  const int cnt = __popc(mask);
                   int incl = cnt;
 #pragma unroll
                   for (int o = 1; o < 32; o <<= 1) {
@@ -704,24 +725,25 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
                     if (lane >= o) incl += t;
                   }
                   int base = 0;
-                  if (lane == 31 && incl > 0) base = atomicAdd(&sm.ncand, incl);
+                  if (lane == 31) base = atomicAdd(&sm.ncand, incl);
                   int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
-                  while (m16) {   // one candidate per listed page, as a rule
-                    const int t = __ffs(m16) - 1;
-                    m16 &= m16 - 1u;
-                    if (o < p.sort_n) { keys[o] = static_cast<uint64_t>(pos0 + t); cand_score[o] = stage[16 * l + t]; }
+                  while (mask) {
+                    const int e = __ffs(mask) - 1, u = u0 + (e >> 2) * NT;
+                    mask &= mask - 1u;
+                    const int pos = 16 * static_cast<int>(page_list[b0 + (u >> 2)]) + 4 * (u & 3) + (e & 3);
+                    if (o < p.sort_n) {
+                      keys[o] = static_cast<uint64_t>(pos);
+                      cand_score[o] = reinterpret_cast<const float*>(stage + u)[e & 3];
+                    }
                     ++o;
                   }
                 }
-                __syncthreads();
               }
-              total = sm.ncand;
-            } else {
-              total = n_list;   // too many: the row does not fit this tier
             }
             __syncthreads();
+            total = n_list <= list_cap ? sm.ncand : n_list;   // a longer list: the row does not fit this tier
           } else {
-            total = collect(thr, 0, 0, p.sort_n, use_hm16);
+            total = collect_any(thr, use_hm16);
           }
           ok = total <= p.sort_n;
           ncand = total;
@@ -747,19 +769,19 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           __syncthreads();
           for (int ci = 0; ci < n_chunks; ++ci) {
             if (n_chunks > 1 && !LEAN) next_chunk(ci);
+            const int jn = vecs_of(ci);
 #pragma unroll
             for (int j = 0; j < kChunkVec; ++j) {
-              float4 v;
+              float4 v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
               if (LEAN) {
                 const int pos = ci * kChunkPos + 4 * (j * NT + tid);
-                v = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
                 if (pos < n) {
                   v = *reinterpret_cast<const float4*>(srow + pos);
                   if (pos + 1 >= n) v.y = -INFINITY;
                   if (pos + 2 >= n) v.z = -INFINITY;
                   if (pos + 3 >= n) v.w = -INFINITY;
                 }
-              } else {
+              } else if (j < jn) {
                 v = chunk4[j * NT + tid];
               }
               const float e[4] = {v.x, v.y, v.z, v.w};
@@ -807,92 +829,87 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
     // the fused finish stage takes slots, scores and V rows of the candidates from shared memory
     prefetch = FUSED && !slow && ncand <= kRowChunk && p.sort_n <= kSelThreads;
+    for (int i = tid; i < kBins; i += NT) hist[i] = 0;   // for the ranking
     if (!slow) {
-      // ---- re-score the candidates canonically: slots, then their packed rows into shared
-      //      memory with independent 16-byte loads, then the canonical arithmetic ----
+      // ---- re-score the candidates canonically.  Every warp works on its own: four candidates per round,
+      //      their slots, the copies of their packed rows into shared memory, the canonical
+      //      arithmetic -- no barrier until all are done, so one warp's wait for memory is not
+      //      every warp's. ----
       for (int base = 0; base < ncand; base += kRowChunk) {
         const int cn = min(kRowChunk, ncand - base);
-        for (int c = tid; c < cn; c += NT) late.cand_slot[c] = slot_of(ctx, static_cast<int>(keys[base + c]));
-        __syncthreads();
-        {
-          // Every candidate's packed K row and scales (K3V2) and, when the finish stage will use
-          // them, its V row and scales, as asynchronous 16- and 4-byte copies: the K side in
-          // kGroups groups of candidates, the V side as a last group.  The canonical scores of a
-          // group are computed while the later groups are still on their way.
-          constexpr int kGroups = 3;
-          constexpr int VW = TailSmem<MODE>::VW;
-          constexpr int kVParts = VW / 4;
-          const uint8_t* v_rows = tp.v_data + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.v_row;
-          const uint16_t* v_sc = tp.v_scales + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.ng;
-          const int per = (cn + kGroups - 1) / kGroups;
-          if (MODE == JF_MODE_K3V2) {
+        const int rounds = (cn + 4 * kW - 1) / (4 * kW);
+        auto cand_of = [&](int i) { return (i >> 2) * (4 * kW) + 4 * warp + (i & 3); };   // the warp's i-th candidate
+        for (int i = lane; i < 4 * rounds; i += 32) {
+          const int c = cand_of(i);
+          if (c < cn) late.cand_slot[c] = static_cast<int32_t>(slot_of(ctx, static_cast<int>(keys[base + c])));
+        }
+        __syncwarp();
+        // Packed K rows and scales (K3V2) and, when the finish stage will use them, V rows and scales, as
+        // asynchronous 16- and 4-byte copies, four lanes per candidate, in kGroups groups of rounds.
+        // The canonical scores of a group are computed while the later ones are on their way.  (A candidate
+        // without a slot copies nothing and gets zeros.)
+        constexpr int kGroups = 3;
+        constexpr int VW = TailSmem<MODE>::VW;
+        constexpr int kVParts = VW / 4;
+        const int per = (rounds + kGroups - 1) / kGroups;
+        const int part = lane & 3;
+        const uint8_t* k_src = ctx.k_rows + 16 * part;
+        const uint8_t* v_src = tp.v_data + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.v_row + 16 * part;
+        const uint16_t* v_sc = tp.v_scales + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.ng;
 #pragma unroll
-            for (int g = 0; g < kGroups; ++g) {
-              const int c_lo = g * per, c_n = max(0, min(cn, c_lo + per) - c_lo);
-              for (int u = tid; u < 4 * c_n; u += NT) {
-                const int c = c_lo + (u >> 2), part = u & 3;
-                const int64_t slot = late.cand_slot[c];
-                uint32_t* r = late.rows + c * W;
-                if (part < 3) {
-                  if (slot >= 0) cp_async_16(r + 4 * part, ctx.k_rows + slot * 48 + 16 * part);
-                  else *reinterpret_cast<uint4*>(r + 4 * part) = make_uint4(0u, 0u, 0u, 0u);
-                } else {
-                  if (slot >= 0) cp_async_4(r + 12, ctx.k_sc + slot * 2);
-                  else r[12] = 0u;
-                }
-              }
-              cp_async_commit();
+        for (int g = 0; g < kGroups; ++g) {
+          for (int i = 4 * g * per + (lane >> 2); i < 4 * min((g + 1) * per, rounds); i += 8) {
+            const int c = cand_of(i);
+            if (c >= cn) continue;
+            const int32_t slot32 = late.cand_slot[c];
+            const bool have = slot32 >= 0;
+            const uint32_t slot = have ? static_cast<uint32_t>(slot32) : 0u;
+            if (MODE == JF_MODE_K3V2) {
+              uint32_t* r = late.rows + c * W;
+              if (part < 3) cp_async_16_zfill(r + 4 * part, k_src + static_cast<uint64_t>(slot) * 48u, have);
+              else cp_async_4_zfill(r + 12, ctx.k_sc + static_cast<uint64_t>(slot) * 2u, have);
             }
-          }
-          if (prefetch) {
-            for (int u = tid; u < 4 * cn; u += NT) {
-              const int c = u >> 2, part = u & 3;
-              const int64_t slot = late.cand_slot[c];
-              if (part < kVParts) {
-                uint4* dst = reinterpret_cast<uint4*>(late.vrows + c * VW) + part;
-                if (slot >= 0) cp_async_16(dst, reinterpret_cast<const uint4*>(v_rows + slot * (16 * kVParts)) + part);
-                else *dst = make_uint4(0u, 0u, 0u, 0u);
-              }
+            if (prefetch) {
+              if (part < kVParts) cp_async_16_zfill(late.vrows + c * VW + 4 * part, v_src + static_cast<uint64_t>(slot) * (16u * kVParts), have);
               // the scales: K3V2 both groups' (4 bytes); K4V4 the aligned 4-byte pair that holds the 2-byte scale
-              if (part == ((MODE == JF_MODE_K3V2) ? 2 : 0)) {
-                if (slot < 0) late.vsc[c] = 0u;
-                else if (MODE == JF_MODE_K3V2) cp_async_4(&late.vsc[c], v_sc + slot * 2);
-                else cp_async_4(&late.vsc[c], v_sc + (slot & ~static_cast<int64_t>(1)));
-              }
+              if (MODE == JF_MODE_K3V2) { if (part == 2) cp_async_4_zfill(&late.vsc[c], v_sc + static_cast<uint64_t>(slot) * 2u, have); }
+              else if (part == 0) cp_async_4_zfill(&late.vsc[c], v_sc + (slot & ~1u), have);
             }
           }
           cp_async_commit();
-          if (MODE == JF_MODE_K4V4) {
-            // K4: the scan's score is the canonical one bit for bit (exact integer dot products,
-            // the same fp32 rescale order), so nothing is recomputed
-            for (int c = tid; c < cn; c += NT) {
-              const int pos = static_cast<int>(keys[base + c]);
-              keys[base + c] = make_key(late.cand_slot[c] >= 0 ? cand_score[base + c] : -INFINITY, pos);
-            }
-          } else {
-            // eight lanes per candidate, four candidates per warp and round
-            float qv[16];
+        }
+        if (FUSED && !merged) {   // under the copies
+          merge_splits(tp, sm.splits, pbase, hi, row_max);
+          merged = true;
+        }
+        if (MODE == JF_MODE_K4V4) {
+          // K4: the scan's score is the canonical one bit for bit (exact integer dot products,
+          // the same fp32 rescale order), so nothing is recomputed
+          for (int i = lane; i < 4 * rounds; i += 32) {
+            const int c = cand_of(i);
+            if (c < cn) keys[base + c] = make_key(late.cand_slot[c] >= 0 ? cand_score[base + c] : -INFINITY, static_cast<int>(keys[base + c]));
+          }
+        } else {
+          // eight lanes per candidate, four candidates per warp and round
+          float qv[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) qv[i] = sm.q[32 * (i >> 2) + 8 * (i & 3) + (lane & 7)] * 8589934592.0f;   // 2^33, see canon_score_k3_x8
+          for (int i = 0; i < 16; ++i) qv[i] = sm.q[32 * (i >> 2) + 8 * (i & 3) + (lane & 7)] * 8589934592.0f;   // 2^33, see canon_score_k3_x8
 #pragma unroll
-            for (int g = 0; g < kGroups; ++g) {
-              // groups 0..g have landed once at most (kGroups - 1 - g) K groups and the V group are in flight
-              if (g == 0) cp_async_wait_group<kGroups>();
-              else if (g == 1) cp_async_wait_group<kGroups - 1>();
-              else cp_async_wait_group<kGroups - 2>();
-              __syncthreads();
-              const int c_lo = g * per, c_hi = min(cn, c_lo + per);
-              for (int c0 = c_lo + 4 * warp; c0 < c_hi; c0 += 4 * kW) {
-                const int c = c0 + (lane >> 3);
-                const int cc = min(c, c_hi - 1);        // lanes past the end keep the shuffles company
-                const float s = canon_score_k3_x8(qv, late.rows + cc * W, ctx.attn, lane);
-                if (c < c_hi && (lane & 7) == 0)
-                  keys[base + c] = make_key(late.cand_slot[c] >= 0 ? s : -INFINITY, static_cast<int>(keys[base + c]));
-              }
+          for (int g = 0; g < kGroups; ++g) {
+            // groups 0..g have landed once at most (kGroups - 1 - g) are in flight
+            if (g == 0) cp_async_wait_group<kGroups - 1>();
+            else if (g == 1) cp_async_wait_group<kGroups - 2>();
+            else cp_async_wait_group<0>();
+            __syncwarp();
+            for (int r = g * per; r < min((g + 1) * per, rounds); ++r) {
+              const int c = cand_of(4 * r + (lane >> 3)), cc = min(c, cn - 1);   // lanes past the end keep the shuffles company
+              const float s = canon_score_k3_x8(qv, late.rows + cc * W, ctx.attn, lane);
+              if (c < cn && (lane & 7) == 0)
+                keys[base + c] = make_key(late.cand_slot[c] >= 0 ? s : -INFINITY, static_cast<int>(keys[base + c]));
             }
           }
         }
-        __syncthreads();
+        __syncwarp();
       }
     } else {
       // ---- slow exact path: 8-level radix select on the 64-bit canonical key ----
@@ -935,19 +952,22 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     __syncthreads();
 
     // ---- order the candidates: best first ----
-    if (p.sort_n <= kSelThreads) {
+    if (by_rank) {
       // Rank by buckets: a candidate's rank is the number of candidates in finer score bins
       // above its own plus the number of larger keys inside its bin.  Bins are `f` times finer
       // than the selection histogram's (the candidates span few of those); a larger canonical
       // score never lands in a later bin, so the result is the exact order of the keys, and
       // crowded bins (massive ties) only cost time.  A thread owns candidates tid, tid + NT, ...
+      // The keys stay where they are; perm[rank] names them.
       constexpr int kCand = kSelThreads / NT;
       int f = 1;
       while (f < 16 && (cand_last + 2) * f * 2 <= kBins) f *= 2;
       const float fscale = kBinsPerUnit * static_cast<float>(f);
       const float ftop = (row_max + 4.0f) * fscale;
-      for (int i = tid; i < kBins; i += NT) hist[i] = 0;
-      __syncthreads();
+      if (slow) {   // its passes used the bins
+        for (int i = tid; i < kBins; i += NT) hist[i] = 0;
+        __syncthreads();
+      }
       unsigned long long mine[kCand];
       int fb[kCand], arrival[kCand];
 #pragma unroll
@@ -978,17 +998,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         }
         if (lane == 31) sm.wsum[warp] = incl;
         __syncthreads();
-        if (warp == 0) {
-          int t = (lane < kW) ? sm.wsum[lane] : 0, inc2 = t;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xFFFFFFFFu, inc2, o);
-            if (lane >= o) inc2 += u;
-          }
-          if (lane < kW) sm.wsum[lane] = inc2 - t;
-        }
-        __syncthreads();
-        int run = sm.wsum[warp] + incl - v;
+        int run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? sm.wsum[lane] : 0) + incl - v;
 #pragma unroll
         for (int i = 0; i < kPer; ++i) { hist[kPer * tid + i] = run; run += hv[i]; }
       }
@@ -999,22 +1009,15 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         if (c < ncand) bucket[hist[fb[k]] + arrival[k]] = static_cast<uint16_t>(c);
       }
       __syncthreads();
-      int r[kCand];
-#pragma unroll
-      for (int k = 0; k < kCand; ++k) {
-        r[k] = 0;
-        if (tid + k * NT < ncand) {
-          const int lo = hist[fb[k]], hi2 = (fb[k] == kBins - 1) ? ncand : hist[fb[k] + 1];
-          int above = 0;
-          for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
-          r[k] = min(lo + above, ncand - 1);
-        }
-      }
-      __syncthreads();
 #pragma unroll
       for (int k = 0; k < kCand; ++k) {
         const int c = tid + k * NT;
-        if (c < ncand) { keys[r[k]] = mine[k]; perm[r[k]] = static_cast<uint16_t>(c); }
+        if (c < ncand) {
+          const int lo = hist[fb[k]], hi2 = (fb[k] == kBins - 1) ? ncand : hist[fb[k] + 1];
+          int above = 0;
+          for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
+          perm[min(lo + above, ncand - 1)] = static_cast<uint16_t>(c);
+        }
       }
       __syncthreads();
     } else {
@@ -1038,11 +1041,13 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   }
 
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
+  auto pos_of_key = [&](int c) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(keys[c] & 0xFFFFFFFFull)); };
   for (int r = tid; r < K; r += NT) {
     int64_t idx = -1, slot = -1;
     if (r < m_sel) {
-      idx = static_cast<int64_t>(0xFFFFFFFFu - static_cast<uint32_t>(keys[r] & 0xFFFFFFFFull));
-      slot = prefetch ? late.cand_slot[perm[r]] : slot_of(ctx, static_cast<int>(idx));
+      const int c = by_rank ? perm[r] : r;
+      idx = pos_of_key(c);
+      slot = prefetch ? late.cand_slot[c] : slot_of(ctx, static_cast<int>(idx));
     }
     out_idx[r] = idx;
     if (out_slot) out_slot[r] = slot;
@@ -1050,16 +1055,21 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   }
 
   if (FUSED) {
+    if (!merged) merge_splits(tp, sm.splits, pbase, hi, row_max);
     cp_async_wait_all();
     __syncthreads();
-    TailPrefetch pf{};
-    if (prefetch) { pf.slot = late.cand_slot; pf.score = cand_score; pf.vsc = late.vsc; pf.vrows = late.vrows; }
-    finish_tail<MODE, NT>(tp, late.tail, pf, pre, row_max, n_seq, b, h, ctx.bt, [&](int kk, int& pos, int& cidx) {
+    auto entry = [&](int kk, int& pos, int& cidx) {
       if (kk >= m_sel) return false;
-      pos = static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(keys[kk] & 0xFFFFFFFFull));
-      cidx = prefetch ? static_cast<int>(perm[kk]) : -1;
+      cidx = by_rank ? perm[kk] : kk;
+      pos = pos_of_key(cidx);
       return true;
-    });
+    };
+    if (prefetch) {
+      const TailPrefetch pf{late.cand_slot, cand_score, late.vsc, late.vrows};
+      finish_tail<MODE, NT, true>(tp, late.tail, pf, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
+    } else {
+      finish_tail<MODE, NT, false>(tp, late.tail, TailPrefetch{}, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
+    }
   }
 }
 
@@ -1068,30 +1078,54 @@ int pow2_ceil(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 // What one of two co-resident blocks may use: half of the multiprocessor's 228 KB, less the 1 KB the system keeps per block.
 constexpr size_t kTwoBlockBytes = 228 * 1024 / 2 - 1024;
 
-template <int MODE, int DT, bool LEAN, int NT>
-jf_status_t launch_select_variant(const TopkParams& sp, const TailParams& tp, dim3 grid, cudaStream_t stream, bool fused) {
-  constexpr size_t kRegion0 = sel_region0_bytes<MODE, LEAN, NT>();
-  const size_t smem = sel_smem_bytes(kRegion0, sp.sort_n, LEAN ? 0 : sp.hm_chunks, NT);
-  static_assert(sel_smem_bytes(kRegion0, 2 * (LEAN ? JF_MAX_TOP_K : kStagedTopK)) <= kSelSmemLimit || NT != kSelThreads,
-                "select kernel shared memory");
-  static_assert(NT == kSelThreads || sel_smem_bytes(kRegion0, 1024) <= kTwoBlockBytes, "two narrow blocks per multiprocessor");
-  if (smem > kSelSmemLimit) return JF_ERR_UNSUPPORTED;
+template <int MODE, int DT, bool LEAN, int NT, int VEC>
+jf_status_t launch_select_variant(const TopkParams& sp, const TailParams& tp, dim3 grid, size_t smem, cudaStream_t stream, bool fused) {
   if (fused) {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, true, LEAN, NT>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, true, LEAN, NT>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, true, LEAN, NT, VEC>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, true, LEAN, NT, VEC>, grid, dim3(NT), smem, stream, sp, tp));
   } else {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, false, LEAN, NT>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, false, LEAN, NT>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, false, LEAN, NT, VEC>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, false, LEAN, NT, VEC>, grid, dim3(NT), smem, stream, sp, tp));
   }
-  JF_CUDA_TRY(cudaGetLastError());
   return JF_OK;
 }
 
-template <int MODE, bool LEAN, int NT>
-jf_status_t launch_select_dtype(const jf_decode_args* a, const TopkParams& sp, const TailParams& tp, dim3 grid,
-                                cudaStream_t stream, bool fused) {
-  return a->q_dtype == JF_DTYPE_BF16 ? launch_select_variant<MODE, JF_DTYPE_BF16, LEAN, NT>(sp, tp, grid, stream, fused)
-                                     : launch_select_variant<MODE, JF_DTYPE_FP16, LEAN, NT>(sp, tp, grid, stream, fused);
+template <int MODE, bool LEAN, int NT, int VEC>
+jf_status_t launch_select_dtype(const jf_decode_args* a, TopkParams& sp, const TailParams& tp, dim3 grid, cudaStream_t stream, bool fused) {
+  constexpr int kStep = 4 * NT;
+  const int chunk = LEAN ? 0 : std::min(VEC * kStep, (a->max_S + kStep - 1) / kStep * kStep);
+  const size_t region0 = sel_region0_bytes<MODE>(chunk);
+  static_assert(sel_smem_bytes(sel_region0_bytes<MODE>(LEAN ? 0 : VEC * kStep), NT == 512 ? 1024 : 2 * (LEAN ? JF_MAX_TOP_K : kStagedTopK)) <=
+                    kSelSmemLimit, "select kernel shared memory");
+  static_assert(NT != 512 || VEC != 8 || sel_smem_bytes(sel_region0_bytes<MODE>(LEAN ? 0 : VEC * kStep), 1024) <= kTwoBlockBytes,
+                "two blocks per multiprocessor");
+  sp.region0 = static_cast<int>(region0);
+  // staged rows of 2..4 chunks get the side table of float4 maxima if it fits
+  sp.hm_chunks = 0;
+  size_t side = 0;
+  const int chunks = (a->max_S + VEC * kStep - 1) / (VEC * kStep);
+  if (!LEAN && chunks >= 2 && chunks <= 4 &&
+      sel_smem_bytes(region0, sp.sort_n, chunks * hm_chunk_bytes(NT, VEC)) <= ((NT == 512 && VEC == 8) ? kTwoBlockBytes : kSelSmemLimit)) {
+    sp.hm_chunks = chunks;
+    side = chunks * hm_chunk_bytes(NT, VEC);
+  }
+  const size_t smem = sel_smem_bytes(region0, sp.sort_n, side);
+  if (smem > kSelSmemLimit) return JF_ERR_UNSUPPORTED;
+  return a->q_dtype == JF_DTYPE_BF16 ? launch_select_variant<MODE, JF_DTYPE_BF16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused)
+                                     : launch_select_variant<MODE, JF_DTYPE_FP16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused);
+}
+
+// The block of a call: 512 threads while the sort buffer allows; a staged row that does not fit the chunk
+// of a half multiprocessor has the whole one to itself when there are no more rows than those.
+template <int MODE>
+jf_status_t launch_select_mode(const jf_decode_args* a, const SelectPlan& plan, TopkParams& sp, const TailParams& tp, dim3 grid,
+                               cudaStream_t stream, bool fused) {
+  if (sp.sort_n > kSelThreads)
+    return plan.lean ? launch_select_dtype<MODE, true, kSelThreads, 8>(a, sp, tp, grid, stream, fused)
+                     : launch_select_dtype<MODE, false, kSelThreads, 8>(a, sp, tp, grid, stream, fused);
+  if (plan.lean) return launch_select_dtype<MODE, true, 512, 8>(a, sp, tp, grid, stream, fused);
+  return (plan.narrow || a->max_S <= 32 * 512) ? launch_select_dtype<MODE, false, 512, 8>(a, sp, tp, grid, stream, fused)
+                                               : launch_select_dtype<MODE, false, 512, 16>(a, sp, tp, grid, stream, fused);
 }
 
 }  // namespace
@@ -1139,37 +1173,10 @@ jf_status_t launch_select(const jf_decode_args* a, cudaStream_t stream, bool fus
   sp.attn_scale = a->attn_scale;
   const TailParams tp = make_tail_params(a, ws);
   const dim3 grid(a->H_q, a->B);
-  // With more rows than multiprocessors the 512-thread block runs two rows per multiprocessor (one
-  // row's chains of dependent memory round trips under the other's arithmetic); otherwise a row's
-  // latency is what counts and the 1024-thread block takes it.
   const SelectPlan plan = select_plan(a, sp.scores);
   if (!plan.supported) return JF_ERR_UNSUPPORTED;
-  const bool many = plan.narrow, lean = plan.lean;
-  // resident-row kernel: rows of 2..4 score chunks get the side table of float4 maxima if it fits
-  auto side_table = [&](int nt, size_t region0, size_t budget) {
-    const int chunks = (a->max_S + 32 * nt - 1) / (32 * nt);
-    return (chunks >= 2 && chunks <= 4 && sel_smem_bytes(region0, sp.sort_n, chunks, nt) <= budget) ? chunks : 0;
-  };
-  if (a->mode == JF_MODE_K3V2) {
-    if (lean && many) return launch_select_dtype<JF_MODE_K3V2, true, 512>(a, sp, tp, grid, stream, fused);
-    if (lean) return launch_select_dtype<JF_MODE_K3V2, true, kSelThreads>(a, sp, tp, grid, stream, fused);
-    constexpr size_t r512 = sel_region0_bytes<JF_MODE_K3V2, false, 512>();
-    if (many && sel_smem_bytes(r512, sp.sort_n, 0, 512) <= kTwoBlockBytes) {
-      sp.hm_chunks = side_table(512, r512, kTwoBlockBytes);
-      return launch_select_dtype<JF_MODE_K3V2, false, 512>(a, sp, tp, grid, stream, fused);
-    }
-    sp.hm_chunks = side_table(kSelThreads, sel_region0_bytes<JF_MODE_K3V2, false, kSelThreads>(), kSelSmemLimit);
-    return launch_select_dtype<JF_MODE_K3V2, false, kSelThreads>(a, sp, tp, grid, stream, fused);
-  }
-  if (lean && many) return launch_select_dtype<JF_MODE_K4V4, true, 512>(a, sp, tp, grid, stream, fused);
-  if (lean) return launch_select_dtype<JF_MODE_K4V4, true, kSelThreads>(a, sp, tp, grid, stream, fused);
-  constexpr size_t r512 = sel_region0_bytes<JF_MODE_K4V4, false, 512>();
-  if (many && sel_smem_bytes(r512, sp.sort_n, 0, 512) <= kTwoBlockBytes) {
-    sp.hm_chunks = side_table(512, r512, kTwoBlockBytes);
-    return launch_select_dtype<JF_MODE_K4V4, false, 512>(a, sp, tp, grid, stream, fused);
-  }
-  sp.hm_chunks = side_table(kSelThreads, sel_region0_bytes<JF_MODE_K4V4, false, kSelThreads>(), kSelSmemLimit);
-  return launch_select_dtype<JF_MODE_K4V4, false, kSelThreads>(a, sp, tp, grid, stream, fused);
+  return a->mode == JF_MODE_K3V2 ? launch_select_mode<JF_MODE_K3V2>(a, plan, sp, tp, grid, stream, fused)
+                                 : launch_select_mode<JF_MODE_K4V4>(a, plan, sp, tp, grid, stream, fused);
 }
 
 }  // namespace jf
