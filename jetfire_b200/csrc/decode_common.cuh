@@ -34,20 +34,96 @@ __host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype) {
   return (mode == JF_MODE_K3V2 && q_dtype == JF_DTYPE_FP16) ? 3 : 4;
 }
 
-// How many splits of the page range one (b, h_kv) pair is cut into: as many as fit in ONE
-// wave of resident CTAs (a second, partial wave would idle most of the GPU), but at least
-// two pages per warp.  Depends only on its arguments, so every launch agrees.
+// ---- how the scan's work is cut -----------------------------------------------------------
+// The unit of work is two 16-token pages of a sequence.  A launch has B * splits CTAs per KV head.
+// `splits`: as many as fill one wave of resident CTAs, or two waves where that leaves fewer of them idle
+// -- a CTA costs about eight units besides its own (start, merge: 3-4 us) -- with at least one unit per
+// warp.  (K4V4, 16 sequences x 8 KV heads x 131072 positions: four splits fill 86 % of a wave, nine 97 %
+// of two, 511 -> 478 us.)
+constexpr int kSliceOverhead = 8;
 inline int scan_splits(int mode, int q_dtype, int B, int H_kv, int max_S) {
-  const int pages = (max_S + JF_BLOCK_SIZE - 1) / JF_BLOCK_SIZE;
-  const int pairs = B * H_kv;
-  int target = (num_sms() * scan_ctas_per_sm(mode, q_dtype)) / pairs;
-  int cap = pages / 8;
+  const int units = ((max_S + JF_BLOCK_SIZE - 1) / JF_BLOCK_SIZE + 1) / 2;
+  const int pairs = B * H_kv, wave = num_sms() * scan_ctas_per_sm(mode, q_dtype);
+  int cap = units / 4;
+  if (cap > 512) cap = 512;
   if (cap < 1) cap = 1;
-  if (target > cap) target = cap;
-  if (target > 512) target = 512;
-  if (target < 1) target = 1;
-  return target;
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int w = 1; w <= 2; ++w) {
+    int s = w * wave / pairs;
+    if (s > cap) s = cap;
+    if (s < 1) s = 1;
+    const int64_t waves = (static_cast<int64_t>(pairs) * s + wave - 1) / wave;
+    const int64_t cost = waves * ((units + s - 1) / s + kSliceOverhead);
+    if (cost < best_cost) { best = s; best_cost = cost; }
+  }
+  return best;
 }
+
+// A long ragged K3V2 batch shares the B * splits CTAs of a KV head out among its sequences in proportion
+// to their lengths: with the same number for each, the short ones' CTAs left a third of the GPU idle
+// (8 sequences of 5k-32k: 38.8 -> 34.0 us).  The lengths are only known on the device, so scan, select
+// and finish work the shares out from them, each for itself and to the same result.  That costs a CTA
+// about a microsecond, the work of two or three units, and gains a fraction of the scan: taken from
+// kShareMin units a CTA on.  (Shares whatever the length: 1.3 us lost on a 2k row of one sequence, 3.6 us
+// on three rows of 3-6k.)  Where all sequences have the units of the longest possible row -- a full
+// batch -- the shares are equal again.  K4V4 keeps equal shares: its CTA has no registers left for the
+// other case, which cost the scan of a full batch 2-5 %.
+constexpr int kShareMin = 24;
+struct SliceGeom {
+  int splits, units;          // CTAs per sequence; units of a row of max_S positions
+  int units_per_split;        // ceil(units / splits)
+  int even;                   // every sequence has `splits` CTAs, whatever its length
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t slice_units(int len) { return len > 0 ? static_cast<uint32_t>((((len + 15) >> 4) + 1) >> 1) : 0u; }
+// Length of sequence `lane` of the 32 from b0 on (0 past B), clamped to the row.
+__device__ __forceinline__ int slice_len(const int32_t* seq_lens, int B, int max_S, int b0, int lane) {
+  return b0 + lane < B ? max(min(seq_lens[b0 + lane], max_S), 0) : 0;
+}
+// Whole warp: total units and non-empty sequences, and whether every sequence has the units of max_S.
+// `my_len`: slice_len of the first 32 sequences.
+struct SliceSums { uint32_t total, live; bool equal; };
+__device__ __forceinline__ SliceSums slice_sums(const SliceGeom& g, const int32_t* seq_lens, int B, int max_S, int lane, int my_len) {
+  SliceSums r{0u, 0u, true};
+  for (int b0 = 0; b0 < B; b0 += 32) {
+    const uint32_t u = slice_units(b0 == 0 ? my_len : slice_len(seq_lens, B, max_S, b0, lane));
+    if (__any_sync(0xFFFFFFFFu, b0 + lane < B && u != static_cast<uint32_t>(g.units))) r.equal = false;
+    r.total += u;
+    r.live += u > 0u ? 1u : 0u;
+  }
+  if (!r.equal) {
+    r.total = __reduce_add_sync(0xFFFFFFFFu, r.total);
+    r.live = __reduce_add_sync(0xFFFFFFFFu, r.live);
+  }
+  return r;
+}
+// CTAs of a sequence of `units` units: one, and its share of the rest (so that they add up to no more than
+// there are); never more than units.
+__device__ __forceinline__ uint32_t slice_count(const SliceGeom& g, const SliceSums& s, int B, uint32_t units) {
+  if (units == 0u) return 0u;
+  return min(1u + units * (static_cast<uint32_t>(B * g.splits) - s.live) / s.total, units);
+}
+// Whole warp: where the partials of (KV head, sequence) lie -- the first one's index and how many.  (The
+// partial of CTA i of a KV head is number hkv * B * splits + i.)
+__device__ __forceinline__ void slice_partials(const SliceGeom& g, const int32_t* seq_lens, int B, int max_S, int hkv, int b, int lane,
+                                               int& first, int& count) {
+  first = (hkv * B + b) * g.splits;
+  count = g.splits;
+  if (g.even) return;
+  const int my_len = slice_len(seq_lens, B, max_S, 0, lane);
+  const SliceSums s = slice_sums(g, seq_lens, B, max_S, lane, my_len);
+  if (s.equal) return;
+  uint32_t before = 0u, mine = 0u;
+  for (int b0 = 0; b0 <= b; b0 += 32) {
+    const uint32_t n = slice_count(g, s, B, slice_units(b0 == 0 ? my_len : slice_len(seq_lens, B, max_S, b0, lane)));
+    before += __reduce_add_sync(0xFFFFFFFFu, b0 + lane < b ? n : 0u);
+    mine = __shfl_sync(0xFFFFFFFFu, n, b & 31);
+  }
+  first = hkv * B * g.splits + static_cast<int>(before);
+  count = static_cast<int>(mine);
+}
+#endif
 
 // Which select kernel a call takes -- decided from the arguments alone, so that the scan (which
 // then leaves the maxima of groups of pages: K3V2 pairs of pages, K4V4 pages) and the select
@@ -78,10 +154,10 @@ inline SelectPlan select_plan(const jf_decode_args* a, const float* scores) {
 
 struct Workspace {
   int32_t* status;   // status record: 64-bit tag, then the error code (see report_status)
-  float* part_o;     // [B][H_kv][splits][8][128]
-  float* part_m;     // [B][H_kv][splits][8]
-  float* part_l;     // [B][H_kv][splits][8]
-  float* part_smax;  // [B][H_kv][splits][2]  largest K group scale seen (per group)
+  float* part_o;     // [H_kv][B * splits][8][128], see SliceGeom
+  float* part_m;     // [H_kv][B * splits][8]
+  float* part_l;     // [H_kv][B * splits][8]
+  float* part_smax;  // [H_kv][B * splits][2]  largest K group scale seen (per group)
   float* pmax;       // [B][H_q][page_max_stride] largest approximate score of every pair of 16-token pages (K3V2) / every page (K4V4)
   float* scores;     // [B][H_q][max_S] approximate scores
   uint64_t bytes;
@@ -95,10 +171,11 @@ __host__ __device__ inline int page_max_stride(int mode, int max_S) {
   return (((max_S + group - 1) / group) + 3) & ~3;
 }
 
-// Sized for the variant with the most splits (bf16 query), so one workspace serves both dtypes.
+// Sized for the query type with the most splits, so one workspace serves both.
 inline Workspace carve_workspace(void* base, int mode, int B, int H_q, int H_kv, int max_S, int /*top_k*/, bool need_scores) {
   const HeadGeom hg = head_geom(H_q, H_kv);
-  const uint64_t splits = scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, max_S);
+  const int s0 = scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, max_S), s1 = scan_splits(mode, JF_DTYPE_FP16, B, hg.H_kv, max_S);
+  const uint64_t splits = s0 > s1 ? s0 : s1;
   const uint64_t pairs = static_cast<uint64_t>(B) * hg.H_kv * splits;
   uint64_t off = 0;
   uint8_t* p = static_cast<uint8_t*>(base);
@@ -134,6 +211,8 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
 #endif
 
 jf_status_t validate_decode_args(const jf_decode_args* a);
+// the cut of a call's work (the same for its scan, select and finish)
+SliceGeom slice_geom(const jf_decode_args* a);
 // device address of the library's built-in scratch array on the current device (decode_static.cu)
 jf_status_t static_scratch_address(void** out);
 

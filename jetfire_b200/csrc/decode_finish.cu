@@ -30,11 +30,12 @@ decode_finish_kernel(const FinishParams p, const TailParams tp) {
   const int h = blockIdx.x, b = blockIdx.y;
   const int hkv = h / tp.G, hi = h - hkv * tp.G;
   const int64_t bh = static_cast<int64_t>(b) * tp.H_q + h;
-  const int64_t pbase = (static_cast<int64_t>(b) * tp.H_kv + hkv) * tp.splits;
   pdl_wait();
+  int pbase, n_splits;   // by every warp for itself
+  slice_partials(tp.geom, p.seq_lens, tp.B, tp.max_S, hkv, b, threadIdx.x & 31, pbase, n_splits);
   const int n = min(p.seq_lens[b], tp.max_S);
-  const float M = block_max_of_splits(tp.part_m, pbase, hi, tp.splits, sm_m);
-  merge_splits(tp, splits, pbase, hi, M);
+  const float M = block_max_of_splits(tp.part_m, pbase, hi, n_splits, sm_m);
+  merge_splits(tp, splits, pbase, n_splits, hi, M);
   const int64_t* sel = p.topk_idx + bh * tp.top_k;
   finish_tail<MODE, kSelThreads, false>(tp, tsm, TailPrefetch{}, splits, M, n, b, h,
                                         p.block_table + static_cast<int64_t>(b) * p.max_blocks, [&](int kk, int& pos, int& cidx) {

@@ -386,7 +386,7 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
 // ------------------------------------------------------------------------------------
 // K3V2
 // ------------------------------------------------------------------------------------
-template <int DT, int kParts>
+template <int DT, int kParts, bool kShares>
 __global__ void __launch_bounds__(kScanWarps * 32, (DT == JF_DTYPE_FP16) ? 3 : 4)
 scan_k3v2_kernel(const ScanParams p) {
   using T = Tile<JF_MODE_K3V2>;
@@ -397,7 +397,7 @@ scan_k3v2_kernel(const ScanParams p) {
   // compiler so, and lets slot addresses live in uniform registers
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
-  const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
+  const int hkv = blockIdx.z;
 
   const uint32_t smem_base = smem_u32(smem);
   constexpr int kRingBytes = kScanWarps * T::kSlots * T::kSlotBytes;
@@ -408,15 +408,16 @@ scan_k3v2_kernel(const ScanParams p) {
 
   pdl_wait();  // nothing above reads global memory
 
-  const int len = min(p.seq_lens[b], p.max_S);
-  const int n_pages = (len + 15) >> 4;
+  const ScanSlice slice = scan_slice<kShares>(p, lane);
+  const int b = slice.b, len = slice.len, n_pages = (len + 15) >> 4;
   // Warp w owns a contiguous quarter of the split's pages, so its block-table entries are
   // contiguous too: sixteen lanes fetch sixteen entries with one load, a whole chunk ahead of
   // its use, and park them in shared memory.  (A load issued while megabytes of page copies are
   // queued in the memory system takes microseconds; fetched one entry at a time, a page or two
   // ahead, those loads stalled the loop.)
-  const int pg_first = split * p.pages_per_split + warp * p.pages_per_warp;
-  const int my_n = max(0, min(min(pg_first + p.pages_per_warp, (split + 1) * p.pages_per_split), n_pages) - pg_first);
+  const int per_warp = 2 * ((slice.hi - slice.lo + kScanWarps - 1) / kScanWarps);   // whole units: pairs of pages
+  const int pg_first = 2 * slice.lo + warp * per_warp;
+  const int my_n = max(0, min(min(pg_first + per_warp, 2 * slice.hi), n_pages) - pg_first);
   const int64_t* bt_w = p.block_table + static_cast<int64_t>(b) * p.max_blocks + pg_first;
   const int bt_avail = p.max_blocks - pg_first;   // entries of the row from this warp's first page on
   auto bt_load = [&](int chunk) -> int64_t {   // lanes 0..15: entry 16 * chunk + lane (never read when out of range)
@@ -593,7 +594,7 @@ scan_k3v2_kernel(const ScanParams p) {
   float l0, l1;
   unpair_f32(st.l2, l0, l1);
   cta_merge_store(p, smem, l0, l1, st.m_ref0, st.m_ref1, __uint_as_float((st.smax2 & 0x7FFFu) << 16),
-                  __uint_as_float(st.smax2 & 0x7FFF0000u), split, hkv, b);
+                  __uint_as_float(st.smax2 & 0x7FFF0000u));
 }
 
 // ------------------------------------------------------------------------------------
@@ -630,13 +631,28 @@ jf_status_t validate_decode_args(const jf_decode_args* a) {
   return JF_OK;
 }
 
+SliceGeom slice_geom(const jf_decode_args* a) {
+  const HeadGeom hg = head_geom(a->H_q, a->H_kv);
+  SliceGeom g{};
+  g.splits = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S);
+  g.units = ((a->max_S + 15) / 16 + 1) / 2;
+  g.units_per_split = (g.units + g.splits - 1) / g.splits;
+  g.even = a->mode != JF_MODE_K3V2 || a->B == 1 || g.units_per_split < kShareMin;
+  return g;
+}
+
 template <int DT, int kParts>
 jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
   using T = Tile<JF_MODE_K3V2>;
   const size_t smem = kScanWarps * T::kSlots * T::kSlotBytes + kScanWarps * 2 * kBtChunk * 8;  // ring, block-table chunks
   static_assert(kScanWarps * T::kSlots * T::kSlotBytes >= kMergeBytes, "merge buffer");
-  JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts>), smem);
-  JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts>, grid, dim3(kScanWarps * 32), smem, stream, sp));
+  if (sp.geom.even) {
+    JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts, false>), smem);
+    JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts, false>, grid, dim3(kScanWarps * 32), smem, stream, sp));
+  } else {
+    JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts, true>), smem);
+    JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts, true>, grid, dim3(kScanWarps * 32), smem, stream, sp));
+  }
   JF_CUDA_TRY(cudaGetLastError());
   return JF_OK;
 }
@@ -679,19 +695,10 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   const HeadGeom hg = head_geom(a->H_q, a->H_kv);
   sp.B = a->B; sp.H_q = a->H_q; sp.H_kv = hg.H_kv; sp.G = hg.G; sp.kv_shift = hg.shift;
   sp.max_S = a->max_S; sp.max_blocks = a->max_blocks;
-  sp.splits = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S);
-  const int pages = (a->max_S + 15) / 16;
-  sp.pages_per_split = (pages + sp.splits - 1) / sp.splits;
-  sp.pages_per_warp = (sp.pages_per_split + kScanWarps - 1) / kScanWarps;
-  if (a->mode == JF_MODE_K3V2) {
-    // every warp's range starts at an even page, so that the pairs of pages a round takes are the
-    // pairs (2m, 2m+1) of the row -- the groups of the page maxima
-    sp.pages_per_split = (sp.pages_per_split + 1) & ~1;
-    sp.pages_per_warp = (((sp.pages_per_split + kScanWarps - 1) / kScanWarps) + 1) & ~1;
-  }
+  sp.geom = slice_geom(a);
   sp.attn_scale = a->attn_scale;
   sp.q_dtype = a->q_dtype;
-  dim3 grid(sp.splits, hg.H_kv, a->B);
+  dim3 grid(sp.geom.splits, a->B, hg.H_kv);
   if (a->mode == JF_MODE_K3V2) {
     // the query's type only matters where the query is read
     const int dt = a->scan_parts == JF_SCAN_V_ONLY ? JF_DTYPE_BF16 : a->q_dtype;

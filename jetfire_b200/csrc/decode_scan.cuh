@@ -47,16 +47,63 @@ struct ScanParams {
   float* part_smax;
   int32_t* status;
   int64_t num_slots;
-  int B, H_q, H_kv, G, max_S, max_blocks, splits, pages_per_split;
-  int pages_per_warp;   // a warp's contiguous share of a split: ceil(pages_per_split / kScanWarps)
+  int B, H_q, H_kv, G, max_S, max_blocks;
   float attn_scale;
   int q_dtype;
   int kv_shift;         // cache head = KV head >> kv_shift (see head_geom)
   int np_stride;        // entries per row of pmax
+  SliceGeom geom;       // how the work is cut
   // K4V4: work is cut into two-page tiles (see scan_k4v4_kernel)
   int n_tiles, tiles_per_split, tiles_per_warp, ref_chunk;
   int tile_base[9];
 };
+
+// This CTA's slice: units [lo, hi) of sequence b, whose length is len.  CTA (x, y) of a KV head is number
+// y * splits + x; with equal shares that is slice x of sequence y.  Whole warp, the same for all lanes.
+struct ScanSlice { int b, len, lo, hi; };
+template <bool kShares>
+__device__ __forceinline__ ScanSlice scan_slice(const ScanParams& p, int lane) {
+  const SliceGeom& g = p.geom;
+  ScanSlice r;
+  r.b = blockIdx.y;
+  r.lo = blockIdx.x * g.units_per_split;
+  r.hi = r.lo + g.units_per_split;   // (the sequence may end before)
+  if (!kShares) {
+    r.len = min(p.seq_lens[r.b], p.max_S);
+    return r;
+  }
+  // the one load that everything waits for: a sequence's length per lane
+  const int my_len = slice_len(p.seq_lens, p.B, p.max_S, 0, lane);
+  const SliceSums s = slice_sums(g, p.seq_lens, p.B, p.max_S, lane, my_len);
+  if (!s.equal) {
+    uint32_t i = blockIdx.y * g.splits + blockIdx.x;   // CTAs left before this one
+    r.b = r.lo = r.hi = 0;
+    for (int b0 = 0; b0 < p.B; b0 += 32) {
+      const uint32_t units = slice_units(b0 == 0 ? my_len : slice_len(p.seq_lens, p.B, p.max_S, b0, lane));
+      const uint32_t n = slice_count(g, s, p.B, units);
+      uint32_t incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const uint32_t hit = __ballot_sync(0xFFFFFFFFu, i < incl);
+      if (hit) {
+        const int l = __ffs(hit) - 1;
+        const uint32_t k = i - incl + n;   // slice k of n, on the lane of the sequence
+        const uint32_t lo = k * units / max(n, 1u), hi = (k + 1) * units / max(n, 1u);
+        r.b = b0 + l;
+        r.lo = __shfl_sync(0xFFFFFFFFu, static_cast<int>(lo), l);
+        r.hi = __shfl_sync(0xFFFFFFFFu, static_cast<int>(hi), l);
+        break;
+      }
+      i -= __shfl_sync(0xFFFFFFFFu, incl, 31);
+    }
+  }
+  r.len = __shfl_sync(0xFFFFFFFFu, my_len, r.b & 31);
+  if (r.b >= 32) r.len = max(min(p.seq_lens[r.b], p.max_S), 0);
+  return r;
+}
 
 constexpr int kBtChunk = 16;              // block-table entries fetched per load (one per lane of a half-warp)
 
@@ -68,8 +115,7 @@ constexpr int kMergeBytes = (kScanWarps * kHeadsPad * JF_HEAD_DIM + 3 * kScanWar
 // the lane's partial softmax sums for heads 2*tig and 2*tig+1, m_ref0/1 its reference
 // points, smax0/1 the largest K group scales it saw.
 __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* smem, float l0, float l1,
-                                                float m_ref0, float m_ref1, float smax0, float smax1,
-                                                int split, int hkv, int b) {
+                                                float m_ref0, float m_ref1, float smax0, float smax1) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
   float* sm_o = reinterpret_cast<float*>(smem);               // [4 warps][8][128]
@@ -92,7 +138,7 @@ __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* sm
   }
   if (lane == 0) { sm_s[warp * 2] = smax0; sm_s[warp * 2 + 1] = smax1; }
   __syncthreads();
-  const int64_t pidx = (static_cast<int64_t>(b) * p.H_kv + hkv) * p.splits + split;
+  const int64_t pidx = (static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   float* po = p.part_o + pidx * (kHeadsPad * JF_HEAD_DIM);
   for (int i = threadIdx.x; i < kHeadsPad * JF_HEAD_DIM; i += blockDim.x) {
     const int h = i >> 7;

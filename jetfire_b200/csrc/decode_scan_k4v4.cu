@@ -351,7 +351,7 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // uniform by construction
   const int g = lane >> 2, tig = lane & 3;
-  const int split = blockIdx.x, hkv = blockIdx.y, b = blockIdx.z;
+  const int split = blockIdx.x, b = blockIdx.y, hkv = blockIdx.z;
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t slots0 = smem_base + warp * (T4::kSlots * T4::kSlotBytes);
@@ -637,7 +637,7 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
       wo[(2 * tig + 1) * JF_HEAD_DIM + dhi] = fmaf(st.oacc[mt][3], 1048576.0f, -8.0f * st.oacc[8][3]);
     }
   }
-  cta_merge_store(p, smem, st.l0, st.l1, st.m_ref0, st.m_ref1, 0.f, 0.f, split, hkv, b);
+  cta_merge_store(p, smem, st.l0, st.l1, st.m_ref0, st.m_ref1, 0.f, 0.f);
 }
 
 // ---- tensor maps -----------------------------------------------------------------------
@@ -730,7 +730,7 @@ jf_status_t launch_scan_k4v4(ScanParams sp, bool int8p, int parts, dim3 grid, cu
     sp.n_tiles = ((sp.max_S + 15) / 16 + 1) / 2;
     for (int s = 0; s <= 8; ++s) sp.tile_base[s] = s ? sp.n_tiles : 0;
   }
-  sp.tiles_per_split = (sp.n_tiles + sp.splits - 1) / sp.splits;
+  sp.tiles_per_split = (sp.n_tiles + sp.geom.splits - 1) / sp.geom.splits;
   sp.tiles_per_warp = (sp.tiles_per_split + kScanWarps - 1) / kScanWarps;
   // a tensor map of a tensor the call does not read is never used by the kernel; the other one stands in
   const void* k_base = sp.k_data ? static_cast<const void*>(sp.k_data) : static_cast<const void*>(sp.v_data);

@@ -43,7 +43,8 @@ struct TailParams {
   float* softmax_m;
   float* softmax_inv_z;
   int64_t num_slots;
-  int H_q, H_kv, G, max_S, splits, top_k;
+  int H_q, H_kv, G, max_S, B, top_k;
+  SliceGeom geom;   // where the scan's partials lie (slice_partials)
   int kv_shift;   // cache head = KV head >> kv_shift (see head_geom)
 };
 
@@ -65,13 +66,13 @@ struct alignas(16) SplitSums {
 };
 // Warp w < 16 sums splits w, w + 16, ...: four channels a lane (a 512-byte row per load), the weight worked
 // out by every lane from a broadcast load; two splits are in flight.
-__device__ __forceinline__ void merge_splits(const TailParams& p, SplitSums& out, int64_t pbase, int hi, float M) {
+__device__ __forceinline__ void merge_splits(const TailParams& p, SplitSums& out, int64_t pbase, int splits, int hi, float M) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp >= kSplitGroups) return;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   float Z = 0.f;
-  for (int s = warp; s < p.splits; s += 2 * kSplitGroups) {
-    const bool two = s + kSplitGroups < p.splits;
+  for (int s = warp; s < splits; s += 2 * kSplitGroups) {
+    const bool two = s + kSplitGroups < splits;
     const int64_t e0 = (pbase + s) * kHeadsPad + hi, e1 = two ? e0 + kSplitGroups * kHeadsPad : e0;
     const float m0 = p.part_m[e0], m1 = p.part_m[e1], l0 = p.part_l[e0], l1 = p.part_l[e1];
     const float4 a = reinterpret_cast<const float4*>(p.part_o + e0 * JF_HEAD_DIM)[lane];

@@ -52,12 +52,13 @@ struct TopkParams {
   int32_t* topk_slots_i32;
   int32_t* status;
   int64_t num_slots;
-  int B, H_q, H_kv, G, max_S, max_blocks, splits, top_k, sort_n, q_dtype;
+  int B, H_q, H_kv, G, max_S, max_blocks, top_k, sort_n, q_dtype;
   int kv_shift;   // cache head = KV head >> kv_shift (see head_geom)
   int hm_chunks;  // score chunks whose per-float4 maxima fit the shared-memory side table (0: none)
   int np_stride;  // entries per row of pmax
   int region0;    // bytes of the first shared-memory region
   float attn_scale;
+  SliceGeom geom; // where the scan's partials lie (slice_partials)
 };
 
 struct RowCtx {
@@ -208,6 +209,7 @@ struct SelSmemFixed {
   float red[4];
   int wsum[kSelWarps];
   int ncand, nlist, tbin, remaining;
+  int part_first, part_count;   // the row's partials of the scan
 };
 
 // What lives in the score chunk's shared memory once the candidates are collected.
@@ -281,7 +283,6 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   const int K = p.top_k;
   const int64_t bh = static_cast<int64_t>(b) * p.H_q + h;
   const float* srow = p.scores + bh * p.max_S;
-  const int64_t pbase = (static_cast<int64_t>(b) * p.H_kv + hkv) * p.splits;
 
   // ---- score chunks: bulk copy (16-byte aligned rows) or plain loads ----
   const bool vec = ((p.max_S & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.scores) & 15) == 0);
@@ -333,7 +334,14 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
   // ---- query row (exact values), per-group L1 norms, INT8 model for K4 ----
   if (tid < JF_HEAD_DIM) sm.q[tid] = Elem<DT>::to_f32(q_bits);
+  if (warp == kW - 1) {
+    int first, count;
+    slice_partials(p.geom, p.seq_lens, p.B, p.max_S, hkv, b, lane, first, count);
+    if (lane == 0) { sm.part_first = first; sm.part_count = count; }
+  }
   __syncthreads();
+  const int64_t pbase = sm.part_first;
+  const int n_splits = sm.part_count;
   if (warp < 4) {  // warp w handles channels 32w..32w+31
     const float v = sm.q[32 * warp + lane];
     float a = fabsf(v), s1 = fabsf(v) + 0.001953125f;
@@ -372,7 +380,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   if (FUSED) pdl_wait();
   if (!LEAN && n_seq > 0) issue_chunk(0);
   float top = kMinusBig, sm0 = 0.f, sm1 = 0.f;
-  if (tid < p.splits) {  // the first split of this thread; the loop below takes the rest
+  if (tid < n_splits) {  // the first split of this thread; the loop below takes the rest
     top = p.part_m[(pbase + tid) * kHeadsPad + hi];
     sm0 = p.part_smax[(pbase + tid) * 2];
     sm1 = p.part_smax[(pbase + tid) * 2 + 1];
@@ -382,7 +390,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   const int n_pages = (n_seq + 15) >> 4, n_groups = (n_pages + kGroupPages - 1) / kGroupPages;
   const float4* pm4 = reinterpret_cast<const float4*>(p.pmax + bh * p.np_stride);
   {
-    for (int s = tid + NT; s < p.splits; s += NT) {
+    for (int s = tid + NT; s < n_splits; s += NT) {
       top = fmaxf(top, p.part_m[(pbase + s) * kHeadsPad + hi]);
       sm0 = fmaxf(sm0, p.part_smax[(pbase + s) * 2]);
       sm1 = fmaxf(sm1, p.part_smax[(pbase + s) * 2 + 1]);
@@ -879,7 +887,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           cp_async_commit();
         }
         if (FUSED && !merged) {   // under the copies
-          merge_splits(tp, sm.splits, pbase, hi, row_max);
+          merge_splits(tp, sm.splits, pbase, n_splits, hi, row_max);
           merged = true;
         }
         if (MODE == JF_MODE_K4V4) {
@@ -1055,7 +1063,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   }
 
   if (FUSED) {
-    if (!merged) merge_splits(tp, sm.splits, pbase, hi, row_max);
+    if (!merged) merge_splits(tp, sm.splits, pbase, n_splits, hi, row_max);
     cp_async_wait_all();
     __syncthreads();
     auto entry = [&](int kk, int& pos, int& cidx) {
@@ -1141,7 +1149,8 @@ TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws) {
   const HeadGeom hg = head_geom(a->H_q, a->H_kv);
   tp.H_q = a->H_q; tp.H_kv = hg.H_kv; tp.G = hg.G; tp.kv_shift = hg.shift;
   tp.max_S = a->max_S;
-  tp.splits = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S);
+  tp.B = a->B;
+  tp.geom = slice_geom(a);
   tp.top_k = a->top_k;
   return tp;
 }
@@ -1165,13 +1174,13 @@ jf_status_t launch_select(const jf_decode_args* a, cudaStream_t stream, bool fus
   const HeadGeom hg = head_geom(a->H_q, a->H_kv);
   sp.B = a->B; sp.H_q = a->H_q; sp.H_kv = hg.H_kv; sp.G = hg.G; sp.kv_shift = hg.shift;
   sp.max_S = a->max_S; sp.max_blocks = a->max_blocks;
-  sp.splits = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S);
   sp.top_k = a->top_k;
   sp.sort_n = pow2_ceil(2 * a->top_k);
   if (sp.sort_n < 512) sp.sort_n = 512;
   sp.q_dtype = a->q_dtype;
   sp.attn_scale = a->attn_scale;
   const TailParams tp = make_tail_params(a, ws);
+  sp.geom = tp.geom;
   const dim3 grid(a->H_q, a->B);
   const SelectPlan plan = select_plan(a, sp.scores);
   if (!plan.supported) return JF_ERR_UNSUPPORTED;
