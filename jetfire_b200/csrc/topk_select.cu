@@ -1117,8 +1117,12 @@ jf_status_t launch_select_dtype(const jf_decode_args* a, TopkParams& sp, const T
     sp.hm_chunks = chunks;
     side = chunks * hm_chunk_bytes(NT, VEC);
   }
-  const size_t smem = sel_smem_bytes(region0, sp.sort_n, side);
+  size_t smem = sel_smem_bytes(region0, sp.sort_n, side);
   if (smem > kSelSmemLimit) return JF_ERR_UNSUPPORTED;
+  // No more rows than multiprocessors: ask for more than half of one's shared memory, so that every row has its
+  // own.  Blocks launched while the scan's last ones leave would go two to the first multiprocessors that are
+  // free (a step of 32 rows of 2048 positions: 22.5 -> 19.1 us; 72 rows of 8000: 34.2 -> 27.1).
+  if (static_cast<int>(grid.x * grid.y) <= num_sms()) smem = std::max(smem, kTwoBlockBytes + 4096);
   return a->q_dtype == JF_DTYPE_BF16 ? launch_select_variant<MODE, JF_DTYPE_BF16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused)
                                      : launch_select_variant<MODE, JF_DTYPE_FP16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused);
 }
