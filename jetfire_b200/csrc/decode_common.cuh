@@ -9,6 +9,13 @@ constexpr int kScanWarps = 4;         // consumer warps per scan CTA; each owns 
 constexpr int kHeadsPad = 8;          // query heads of one KV head, padded to the MMA N
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMinusBig = -1.0e30f; // finite stand-in for "no score seen yet"
+#ifdef __CUDACC__
+// A softmax reference point in the base-2 domain, as the scan's exp2(fma(s, log2(e), -ref)) uses it.  Every
+// factor between two reference points and every weight of a selected entry is formed from this rounded
+// product (not contracted into an fma), so that its rounding -- 2^-24 of it, 1e-6 of a weight at scores of
+// 50 -- cancels between W, o_old and the normaliser.
+__device__ __forceinline__ float ref_log2(float m) { return __fmul_rn(m, kLog2e); }
+#endif
 
 struct ModeInfo {
   int k_bits, v_bits, group_size, ng, k_row, v_row;

@@ -329,7 +329,7 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
       mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, o));
     }
     const float n0 = fmaxf(st.m_ref0, mx0), n1 = fmaxf(st.m_ref1, mx1);
-    const float f0 = ex2((st.m_ref0 - n0) * kLog2e), f1 = ex2((st.m_ref1 - n1) * kLog2e);
+    const float f0 = ex2(ref_log2(st.m_ref0) - ref_log2(n0)), f1 = ex2(ref_log2(st.m_ref1) - ref_log2(n1));
     st.l2 = mul2(st.l2, pair_f32(f0, f1));
     if (kDoV) {
 #pragma unroll
@@ -337,7 +337,7 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
     }
     st.m_ref0 = n0; st.m_ref1 = n1;
   }
-  const uint64_t c2 = pair_f32(kLog2e, kLog2e), mb2 = pair_f32(-st.m_ref0 * kLog2e, -st.m_ref1 * kLog2e);
+  const uint64_t c2 = pair_f32(kLog2e, kLog2e), mb2 = pair_f32(-ref_log2(st.m_ref0), -ref_log2(st.m_ref1));
   float pA[4], pB[4];
   unpair_f32(fma2(pair_f32(sA[0], sA[1]), c2, mb2), pA[0], pA[1]);
   unpair_f32(fma2(pair_f32(sA[2], sA[3]), c2, mb2), pA[2], pA[3]);

@@ -173,7 +173,7 @@ __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* sm
     float acc = 0.f;
 #pragma unroll
     for (int w = 0; w < kScanWarps; ++w)
-      acc = fmaf(sm_o[w * (kHeadsPad * JF_HEAD_DIM) + i], ex2((sm_m[w * 8 + h] - M) * kLog2e), acc);
+      acc = fmaf(sm_o[w * (kHeadsPad * JF_HEAD_DIM) + i], ex2(ref_log2(sm_m[w * 8 + h]) - ref_log2(M)), acc);
     po[i] = acc;
   }
   if (threadIdx.x < kHeadsPad) {
@@ -181,7 +181,7 @@ __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* sm
     float M = kMinusBig;
     for (int w = 0; w < kScanWarps; ++w) M = fmaxf(M, sm_m[w * 8 + h]);
     float L = 0.f;
-    for (int w = 0; w < kScanWarps; ++w) L += sm_l[w * 8 + h] * ex2((sm_m[w * 8 + h] - M) * kLog2e);
+    for (int w = 0; w < kScanWarps; ++w) L += sm_l[w * 8 + h] * ex2(ref_log2(sm_m[w * 8 + h]) - ref_log2(M));
     p.part_m[pidx * kHeadsPad + h] = M;
     p.part_l[pidx * kHeadsPad + h] = L;
   }

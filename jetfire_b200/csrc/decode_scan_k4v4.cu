@@ -274,7 +274,7 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, o));
       }
       const float n0 = fmaxf(st.m_ref0, mx0), n1 = fmaxf(st.m_ref1, mx1);
-      const float f0 = ex2((st.m_ref0 - n0) * kLog2e), f1 = ex2((st.m_ref1 - n1) * kLog2e);
+      const float f0 = ex2(ref_log2(st.m_ref0) - ref_log2(n0)), f1 = ex2(ref_log2(st.m_ref1) - ref_log2(n1));
       st.l2 = mul2(st.l2, pair_f32(f0, f1));
       if (kDoV) {
 #pragma unroll
@@ -282,7 +282,7 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
       }
       st.m_ref0 = n0; st.m_ref1 = n1;
     }
-    const uint64_t c2 = pair_f32(kLog2e, kLog2e), mb2 = pair_f32(-st.m_ref0 * kLog2e, -st.m_ref1 * kLog2e);
+    const uint64_t c2 = pair_f32(kLog2e, kLog2e), mb2 = pair_f32(-ref_log2(st.m_ref0), -ref_log2(st.m_ref1));
     pA01 = ex2_pair(fma2(pair_f32(sA[0], sA[1]), c2, mb2)); pB01 = ex2_pair(fma2(pair_f32(sB[0], sB[1]), c2, mb2));
     pA23 = ex2_pair(fma2(pair_f32(sA[2], sA[3]), c2, mb2)); pB23 = ex2_pair(fma2(pair_f32(sB[2], sB[3]), c2, mb2));
     st.l2 = add2(st.l2, add2(add2(pA01, pA23), add2(pB01, pB23)));

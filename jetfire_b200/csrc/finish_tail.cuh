@@ -77,7 +77,7 @@ __device__ __forceinline__ void merge_splits(const TailParams& p, SplitSums& out
     const float m0 = p.part_m[e0], m1 = p.part_m[e1], l0 = p.part_l[e0], l1 = p.part_l[e1];
     const float4 a = reinterpret_cast<const float4*>(p.part_o + e0 * JF_HEAD_DIM)[lane];
     const float4 c = reinterpret_cast<const float4*>(p.part_o + e1 * JF_HEAD_DIM)[lane];
-    const float w0 = ex2((m0 - M) * kLog2e), w1 = two ? ex2((m1 - M) * kLog2e) : 0.f;
+    const float w0 = ex2(ref_log2(m0) - ref_log2(M)), w1 = two ? ex2(ref_log2(m1) - ref_log2(M)) : 0.f;
     Z = fmaf(l0, w0, Z);
     o.x = fmaf(a.x, w0, o.x); o.y = fmaf(a.y, w0, o.y); o.z = fmaf(a.z, w0, o.z); o.w = fmaf(a.w, w0, o.w);
     Z = fmaf(l1, w1, Z);
@@ -231,7 +231,7 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
         }
       }
       if (slot >= 0) {
-        w = ex2((approx - M) * kLog2e);
+        w = ex2(__fmaf_rn(approx, kLog2e, -ref_log2(M)));
         vs0 = __uint_as_float(sw << 16);
         vs1 = __uint_as_float(sw & 0xFFFF0000u);
       }
