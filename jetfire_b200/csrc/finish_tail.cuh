@@ -261,19 +261,29 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
   }
   __syncthreads();
   if (tid < JF_HEAD_DIM) {
-    float acc_old = 0.f, o = 0.f, Z = 0.f;
+    // the normaliser and the sum of weights pairwise: a running sum would round once per term at its full size
+    float acc_old = 0.f, o[kSplitGroups], z[kSplitGroups];
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
       if (r < groups) acc_old += sm.red[r][tid];
 #pragma unroll
-    for (int gI = 0; gI < kSplitGroups; ++gI) { o += splits.o[gI][tid]; Z += splits.z[gI]; }
+    for (int gI = 0; gI < kSplitGroups; ++gI) { o[gI] = splits.o[gI][tid]; z[gI] = splits.z[gI]; }
+#pragma unroll
+    for (int d = kSplitGroups / 2; d > 0; d >>= 1)
+#pragma unroll
+      for (int gI = 0; gI < d; ++gI) { o[gI] += o[gI + d]; z[gI] += z[gI + d]; }
+    const float Z = z[0];
     const bool live = (Z > 0.f) && (n > 0);
     const float inv_z = live ? (1.0f / Z) : 0.f;
-    p.o_hat[bh * JF_HEAD_DIM + tid] = o * inv_z;
+    p.o_hat[bh * JF_HEAD_DIM + tid] = o[0] * inv_z;
     p.o_old[bh * JF_HEAD_DIM + tid] = acc_old * inv_z;
+    float ws = 0.f;
+    if (warp == 0) {
+      for (int i = lane; 32 * i < p.top_k; i += 32) ws += sm.sum[i];
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) ws += __shfl_xor_sync(0xFFFFFFFFu, ws, d);
+    }
     if (tid == 0) {
-      float ws = 0.f;
-      for (int i = 0; 32 * i < p.top_k; ++i) ws += sm.sum[i];
       p.W[bh] = ws * inv_z;
       if (p.softmax_m) p.softmax_m[bh] = live ? M : 0.f;
       if (p.softmax_inv_z) p.softmax_inv_z[bh] = inv_z;

@@ -27,3 +27,18 @@ def test_weights_sum_with_large_scores(mode, dtype, lens):
     assert res.scores.amax() > 60.0
     err = ((res.W.double() - want) / want).abs().max().item()
     assert err < LIMIT, f"{err:.2e}"
+
+
+@pytest.mark.parametrize("mode", ["k3v2", "k4v4"])
+def test_many_weights_of_one_size(mode):
+    """4096 nearly equal weights: a running sum of their 128 partial sums rounds once per term at the full size
+    (1.8e-7 rms over the rows), pairwise sums seven times; with the scan's own sums 7.5e-8 is left, 2^-23 allowed."""
+    from jetfire_b200 import ops
+    case = Case(mode, 2, 32, 4, 8192, lens=[8192, 8000], seed=33)
+    kd, ks, vd, vs = case.device_cache()
+    res = ops.fused_attn_topk(mode, case.q.cuda(), kd, ks, vd, vs, case.block_table.cuda(), case.seq_lens.cuda(), case.ctx,
+                              32, 4, 16, 4096, 0.02 * case.attn_scale, want_scores=True)
+    p = torch.softmax(res.scores.double(), dim=-1)
+    want = torch.gather(p, 2, res.topk_idx.clamp_min(0)).mul(res.topk_idx >= 0).sum(-1)
+    rms = ((res.W.double() - want) / want).square().mean().sqrt().item()
+    assert rms < 1.2e-7, f"{rms:.2e}"
