@@ -136,7 +136,7 @@ class _StreamStep:
                 offs.append(offs[-1] + (n + 255) // 256 * 256)
             self.mapped = ops.alloc_mapped_pinned_pair((offs[-1],), torch.uint8)
             part = lambda side, i, dt, shape: self.mapped[side][offs[i]:offs[i] + sizes[i]].view(dt).reshape(shape)
-            self.mapped[0].zero_()
+            ops.zero_host(self.mapped[0])
             (self.words_host, self.words_dev) = (part(s, 0, torch.int64, (16,)) for s in (0, 1))
             (self.status_host, status_dev) = (part(s, 1, torch.uint8, (128,)) for s in (0, 1))
             (self.q_host, q_host_dev) = (part(s, 2, dtype, (B, H_q, 128)) for s in (0, 1))

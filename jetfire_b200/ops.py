@@ -868,6 +868,14 @@ def alloc_mapped_pinned_pair(shape, dtype, node: int = -1):
     return host, device
 
 
+def zero_host(host: torch.Tensor) -> None:
+    """Zeroes a small contiguous CPU tensor on this thread alone.  A torch fill of more than 32768 elements
+    goes through OpenMP, whose threads then spin for 4 ms on every processor: the correction's dispatcher
+    and workers wait that long for theirs (first call of an adapter step 0.4 -> 3.8 ms)."""
+    _require(not host.is_cuda and host.is_contiguous(), "zero_host: contiguous CPU tensor expected")
+    C.memset(host.data_ptr(), 0, host.numel() * host.element_size())
+
+
 def free_mapped_pinned_pair(host: torch.Tensor) -> None:
     """Gives the block of an ``alloc_mapped_pinned_pair`` back; neither tensor may be used afterwards."""
     check("free_mapped_pinned_pair", lib.jf_free_mapped(host._jf_mapped[1]))

@@ -1,5 +1,6 @@
 """The kernels at the two ends of the adapter's stream-ordered step: the forms of inputs and outputs they
 address themselves, and the ones that go through a copy, all give the bits of the plain form."""
+import time
 from types import SimpleNamespace
 
 import pytest
@@ -53,3 +54,25 @@ def test_step_takes_the_forms_a_caller_has(B, H_q, dtype):
             query = query.view(B, H_q, 128)
         assert torch.equal(run(query, table, length, out), want)
     assert bool((wide[B:] == 3.0).all()) and bool((wide[:, row:] == 3.0).all())
+
+
+def test_building_a_step_leaves_the_processors_free():
+    """No thread may still be busy once a step object is built: its first run needs the processors for the
+    dispatcher and the workers.  (Fifteen OpenMP threads spinning for 4 ms are 60 ms of processor time.)"""
+    from jetfire_b200.adapter import decode_path as dp
+    from jetfire_b200.adapter.config import JetFireConfig
+    if torch.get_num_threads() < 8:
+        pytest.skip("fewer than eight OpenMP threads: nothing to see")
+    torch.zeros(1 << 20).add_(1.0)                               # the OpenMP threads exist
+    cfg = JetFireConfig(mode="SymInt3K_SymInt2V", top_k=256, group_size=64, cpu_attn_threads=2)
+    st = _store(Case("k3v2", 1, 8, 2, 4096, seed=5), cfg)
+    step = dp._StreamStep(st, cfg, 4, 32, 256, 256, 4096, torch.bfloat16, torch.device("cuda"), 1.0)
+    step.close()                                                 # dispatcher and allocator have been used once
+    time.sleep(0.2)
+    step = dp._StreamStep(st, cfg, 4, 32, 256, 256, 4096, torch.bfloat16, torch.device("cuda"), 1.0)
+    busy = time.process_time()
+    time.sleep(0.006)
+    busy = time.process_time() - busy
+    torch.cuda.synchronize()
+    step.close()
+    assert busy < 0.02, f"{1e3 * busy:.1f} ms of processor time in the 6 ms after the step was built"
