@@ -428,7 +428,8 @@ jf_status_t jf_stream_wait_host_flag(jf_stream_t stream, const int64_t* flag_dev
  * end: raises *trigger_dev (NULL: the correction was started earlier), waits for *done_dev at most
  *   timeout_ms (then JF_ERR_TIMEOUT in the status record, and the stream goes on),
  *   out = dtype(o_hat + W * o_new - o_old_unnorm) with sequences out_stride elements apart (a multiple
- *   of 4), and the first JF_STATUS_RECORD_BYTES of the workspace to status_host_dev. */
+ *   of 4).  A record that holds an error moves to status_host_dev: JF_STATUS_RECORD_BYTES there, which
+ *   are left alone otherwise and are the host's to clear, and the record in the workspace is cleared. */
 jf_status_t jf_step_begin(const void* q, int64_t q_stride, void* q_dev, void* q_host_dev,
                           const void* block_table, int32_t bt_is_i32, int64_t bt_stride, int32_t width,
                           int64_t* bt_dev, int32_t bt_dev_stride, const void* seq_lens,

@@ -230,8 +230,13 @@ class _StreamStep:
             self.status_event = ev
 
     def status(self) -> None:
-        """For the owner of a graph, after synchronising a replay: raise if the step recorded an error."""
-        ops.decode_status_of_copy(self.status_host)
+        """For the owner of a graph, after synchronising a replay: raise if the step recorded an error
+        (with flags: once per error)."""
+        record = self.status_host
+        if self.flags:      # the kernel leaves an error there for the host to take
+            record = self.status_host.clone()
+            ops.zero_host(self.status_host)
+        ops.decode_status_of_copy(record)
         self.host.stream_status()
 
     def close(self) -> None:

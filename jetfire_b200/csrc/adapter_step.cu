@@ -11,7 +11,7 @@
 //        conversion to 64 bits, the lengths -- and clears the completion word.  Bound by launch latency.
 // end    raises the trigger word (everything the correction reads has been written by earlier kernels
 //        of the stream), waits for the completion word (bounded), merges the correction into the
-//        caller's output and leaves the status record's copy on the host.  Bound by the host's work.
+//        caller's output and hands a recorded error over to the host.  Bound by the host's work.
 // The selected slots need no copy: the select kernel writes them to mapped memory itself.
 #include "decode_common.cuh"
 
@@ -100,8 +100,13 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p
     __threadfence_system();     // what the host wrote before the word is read after it
     if (!ok) report_status(p.status, JF_ERR_TIMEOUT);
     if (blockIdx.x == 0) {
-      const volatile int32_t* s = p.status;
-      *p.status_host = make_uint4(s[0], s[1], s[2], s[3]);
+      // an error that a kernel of the stream recorded is handed over: the host's copy keeps it until the host
+      // has seen it, the record is free again (layers share the workspace, one of them reports)
+      volatile int32_t* s = p.status;
+      if (*reinterpret_cast<volatile unsigned long long*>(s) == kStatusTag) {
+        *p.status_host = make_uint4(s[0], s[1], s[2], s[3]);
+        s[0] = s[1] = 0;
+      }
     }
   }
   __syncthreads();

@@ -22,6 +22,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -498,7 +499,7 @@ struct Step {
   at::Tensor q, block_table, seq_lens;      // device buffers the argument block names
   at::Tensor keep[8];                       // mapped views and outputs whose addresses follow
   void *q_host_dev, *o_new_dev, *status_host_dev;
-  const void* status_host;
+  void* status_host;
   int64_t *done_dev, *trigger_dev;
   int64_t ctx;                              // submit context of the host correction
   int64_t H_q;
@@ -562,6 +563,7 @@ PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (!capturing) {   // an error of an earlier run, as far as it has arrived
       r = jf_decode_status_of_copy(s->status_host);
       if (r == JF_OK) r = jf_submit_ctx_status(s->ctx);
+      else std::memset(s->status_host, 0, JF_STATUS_RECORD_BYTES);   // reported once; the next call runs
     }
     at::Tensor q = tensor(p[1], name, "query"), bt = tensor(p[2], name, "block_table"), lens = tensor(p[3], name, "seq_lens"),
                out = tensor(p[4], name, "output");

@@ -370,8 +370,8 @@ class AdapterStep:
                                        status_host, status_dev, host._handle(), timeout_ms, gpu_rows)
 
     def run(self, query, block_table, seq_lens, output) -> bool:
-        """Queues the step; True when the stream is being captured.  Raises for an error that an earlier
-        run recorded and that has arrived on the host."""
+        """Queues the step; True when the stream is being captured.  Raises, once and without queueing
+        anything, for an error that an earlier run recorded and that has arrived on the host."""
         st, capturing, merged = _host.step_run(self._step, query, block_table, seq_lens, output)
         if st:
             check("decode_step", st)

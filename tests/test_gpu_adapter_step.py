@@ -56,6 +56,63 @@ def test_step_takes_the_forms_a_caller_has(B, H_q, dtype):
     assert bool((wide[B:] == 3.0).all()) and bool((wide[:, row:] == 3.0).all())
 
 
+def _one_step(top_k=32):
+    """A store with one sequence and a callable that runs its step."""
+    from jetfire_b200.adapter import decode_path as dp
+    from jetfire_b200.adapter.config import JetFireConfig
+    case = Case("k3v2", 1, 8, 2, 200, seed=71)
+    cfg = JetFireConfig(mode="SymInt3K_SymInt2V", top_k=top_k, group_size=64, cpu_attn_threads=2)
+    st = _store(case, cfg)
+    impl = SimpleNamespace(scale=case.attn_scale)
+    layer = SimpleNamespace(num_heads=8, num_kv_heads=2, head_size=128)
+    md = dp.make_decode_metadata(case.seq_lens.cuda(), case.block_table.cuda())
+    q = case.q.cuda()
+
+    def run():
+        out = torch.zeros(1, 8 * 128, dtype=case.dtype, device="cuda")
+        assert dp.try_jetfire_decode(impl=impl, layer=layer, query=q, attn_metadata=md, output=out, store=st, cfg=cfg) is out
+        torch.cuda.synchronize()
+        return out
+    return st, run
+
+
+TAGGED = torch.tensor([0x4A46535441545553, 2], dtype=torch.int64)      # a status record that says JF_ERR_TIMEOUT
+
+
+def test_a_recorded_error_is_reported_once():
+    """An error in the workspace's record reaches the host with the step's end, raises from the next call
+    (or from ``status()``) and from no later one; the calls after that run."""
+    from jetfire_b200._lib import JetFireError
+    from jetfire_b200.adapter.decode_path import stream_steps
+    st, run = _one_step()
+    want = run()
+    step = stream_steps(st)[0]
+    record = step.call.status_record().view(torch.int64)
+    for read in (run, step.status):
+        record.copy_(TAGGED)
+        assert torch.equal(run(), want)            # carries the record to the host
+        with pytest.raises(JetFireError, match="bounded wait"):
+            read()
+        assert torch.equal(run(), want) and torch.equal(run(), want)
+        step.status()
+    # a record that came over while the host did not look stays until it does
+    record.copy_(TAGGED)
+    graph = torch.cuda.CUDAGraph()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        step.run(step.q.clone(), step.block_table.clone(), step.seq_lens.clone(), torch.zeros_like(want))
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    with pytest.raises(JetFireError, match="bounded wait"):
+        step.status()
+    graph.replay()
+    torch.cuda.synchronize()
+    step.status()
+    del graph
+
+
 def test_building_a_step_leaves_the_processors_free():
     """No thread may still be busy once a step object is built: its first run needs the processors for the
     dispatcher and the workers.  (Fifteen OpenMP threads spinning for 4 ms are 60 ms of processor time.)"""
