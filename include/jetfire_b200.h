@@ -425,8 +425,10 @@ jf_status_t jf_stream_wait_host_flag(jf_stream_t stream, const int64_t* flag_dev
  * begin: q (B, H_q, 128) 16-bit, sequences q_stride elements apart (a multiple of 8), to q_dev and to
  *   q_host_dev (mapped pinned memory); `width` entries per row of block_table (int64, or int32 with
  *   bt_is_i32) to bt_dev (row stride bt_dev_stride); seq_lens (int64, or int32) to lens_dev; *done_dev = 0.
- * end: raises *trigger_dev (NULL: the correction was started earlier), waits for *done_dev at most
- *   timeout_ms (then JF_ERR_TIMEOUT in the status record, and the stream goes on),
+ * end: clears *done_dev and raises *trigger_dev (NULL: the correction was started earlier, both are
+ *   left alone), waits for *done_dev at most timeout_ms (then JF_ERR_TIMEOUT in the status record, and
+ *   the stream goes on), status_record being the start of the workspace of a jf_decode_fused or
+ *   jf_decode_scan before it in the stream; then
  *   out = dtype(o_hat + W * o_new - o_old_unnorm) with sequences out_stride elements apart (a multiple
  *   of 4).  A record that holds an error moves to status_host_dev: JF_STATUS_RECORD_BYTES there, which
  *   are left alone otherwise and are the host's to clear, and the record in the workspace is cleared. */
@@ -437,7 +439,7 @@ jf_status_t jf_step_begin(const void* q, int64_t q_stride, void* q_dev, void* q_
                           int32_t H_q, jf_stream_t stream);
 jf_status_t jf_step_end(const float* o_hat, const float* o_old_unnorm, const float* W, const void* o_new,
                         void* out, int64_t out_stride, int32_t dtype, int32_t B, int32_t H_q,
-                        const int64_t* done_dev, int64_t* trigger_dev, int32_t timeout_ms,
+                        int64_t* done_dev, int64_t* trigger_dev, int32_t timeout_ms,
                         void* status_record, void* status_host_dev, jf_stream_t stream);
 
 /* Pinned host memory mapped into the device address space

@@ -61,7 +61,7 @@ struct EndParams {
   const uint2* o_new;        // four 16-bit channels each; mapped host memory or device memory
   uint16_t* out;
   int64_t out_stride;        // between sequences, in elements
-  const volatile long long* done;
+  volatile long long* done;
   volatile long long* trigger;   // may be null: the correction was started by an earlier kernel
   int32_t* status;
   uint4* status_host;
@@ -86,20 +86,25 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p
     w = p.W[row];
   }
   if (threadIdx.x == 0) {
-    if (blockIdx.x == 0 && p.trigger != nullptr) {
-      __threadfence_system();   // what the correction reads is on the host before the trigger is
-      *p.trigger = 1;
-    }
+    volatile int32_t* const verdict = p.status + kWaitWord;
     const unsigned long long t0 = global_ns();
-    bool ok = false;
-    for (unsigned long long polls = 0; polls < (1ull << 32); ++polls) {
-      if (*p.done != 0) { ok = true; break; }
-      if (global_ns() - t0 > p.budget_ns) break;
-      __nanosleep(polls < 64 ? 50 : 400);
-    }
-    __threadfence_system();     // what the host wrote before the word is read after it
-    if (!ok) report_status(p.status, JF_ERR_TIMEOUT);
     if (blockIdx.x == 0) {
+      // One block waits and decides for the grid: with a budget of its own each, the blocks could differ
+      // around the limit, and those of a later wave would start it afresh.
+      if (p.trigger != nullptr) {
+        *p.done = 0;              // again, as late as can be: a worker of a run that was given up may have set it since
+        __threadfence_system();   // what the correction reads is on the host before the trigger is
+        *p.trigger = 1;
+      }
+      bool ok = false;
+      for (unsigned long long polls = 0; polls < (1ull << 32); ++polls) {
+        if (*p.done != 0) { ok = true; break; }
+        if (global_ns() - t0 > p.budget_ns) break;
+        __nanosleep(polls < 64 ? 50 : 400);
+      }
+      __threadfence_system();     // what the host wrote before the word is read after it, by every block
+      *verdict = ok ? kWaitDone : kWaitRanOut;
+      if (!ok) report_status(p.status, JF_ERR_TIMEOUT);
       // an error that a kernel of the stream recorded is handed over: the host's copy keeps it until the host
       // has seen it, the record is free again (layers share the workspace, one of them reports)
       volatile int32_t* s = p.status;
@@ -107,6 +112,13 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p
         *p.status_host = make_uint4(s[0], s[1], s[2], s[3]);
         s[0] = s[1] = 0;
       }
+    } else {
+      // block 0 started with this one or before it and gives up within the budget
+      for (unsigned long long polls = 0; polls < (1ull << 32); ++polls) {
+        if (*verdict != 0 || global_ns() - t0 > p.budget_ns + 1000000000ull) break;
+        __nanosleep(20);
+      }
+      __threadfence_system();
     }
   }
   __syncthreads();
@@ -145,7 +157,7 @@ extern "C" jf_status_t jf_step_begin(const void* q, int64_t q_stride, void* q_de
 }
 
 extern "C" jf_status_t jf_step_end(const float* o_hat, const float* o_old_unnorm, const float* W, const void* o_new, void* out,
-                                   int64_t out_stride, int32_t dtype, int32_t B, int32_t H_q, const int64_t* done_dev,
+                                   int64_t out_stride, int32_t dtype, int32_t B, int32_t H_q, int64_t* done_dev,
                                    int64_t* trigger_dev, int32_t timeout_ms, void* status_record, void* status_host_dev,
                                    jf_stream_t stream) {
   using namespace jf;
@@ -158,7 +170,7 @@ extern "C" jf_status_t jf_step_end(const float* o_hat, const float* o_old_unnorm
   if (static_cast<int64_t>(B) * H_q > (1 << 25)) return JF_ERR_UNSUPPORTED;
   EndParams p{reinterpret_cast<const float4*>(o_hat), reinterpret_cast<const float4*>(o_old_unnorm), W,
               static_cast<const uint2*>(o_new), static_cast<uint16_t*>(out), out_stride,
-              reinterpret_cast<const volatile long long*>(done_dev), reinterpret_cast<volatile long long*>(trigger_dev),
+              reinterpret_cast<volatile long long*>(done_dev), reinterpret_cast<volatile long long*>(trigger_dev),
               static_cast<int32_t*>(status_record), static_cast<uint4*>(status_host_dev),
               static_cast<unsigned long long>(timeout_ms) * 1000000ull, B * H_q, H_q};
   const dim3 grid((B * H_q * 32 + kEndThreads - 1) / kEndThreads);

@@ -209,6 +209,10 @@ constexpr unsigned long long kStatusTag = 0x4A46535441545553ull;  // "JFSTATUS"
 // and checked by the select kernel that works from them, so that a select whose arguments do not
 // match the scan's reports JF_ERR_STATE (and selects nothing) instead of reading stale maxima.
 constexpr int32_t kPageMaxTag = 0x504D4158;  // "PMAX"
+// Word 8: how the wait of the step's end went, for its other blocks (adapter_step.cu); cleared by every scan
+// that reads K.
+constexpr int kWaitWord = 8;
+constexpr int32_t kWaitDone = 1, kWaitRanOut = 2;
 #ifdef __CUDACC__
 __device__ __forceinline__ void report_status(int32_t* status, int code) {
   status[2] = code;

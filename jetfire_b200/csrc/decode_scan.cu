@@ -548,7 +548,10 @@ scan_k3v2_kernel(const ScanParams p) {
   }
 
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
-  if (kDoK && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) p.status[4] = want_pm ? kPageMaxTag : 0;
+  if (kDoK && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) {
+    p.status[4] = want_pm ? kPageMaxTag : 0;
+    p.status[kWaitWord] = 0;
+  }
 
   // ---------------- CTA merge: 4 warps -> one partial ----------------
   __syncthreads();  // every warp is done with its slots; smem is reused below

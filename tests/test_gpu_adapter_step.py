@@ -113,6 +113,46 @@ def test_a_recorded_error_is_reported_once():
     del graph
 
 
+@pytest.mark.parametrize("B,H_q", [(1, 4), (5, 20)], ids=["one block", "seven blocks"])
+def test_the_wait_at_the_end_runs_out(B, H_q):
+    """jf_step_end with a completion word that nobody sets: the stream goes on after the budget, the error is
+    handed to the host, the record is clear again; the next call, with the word set, leaves no error.  A word
+    left set by a run that was given up does not count once the trigger is raised."""
+    from jetfire_b200 import ops
+    from jetfire_b200._lib import JF_ERR_TIMEOUT, lib
+    g = torch.Generator(device="cuda").manual_seed(3)
+    o_hat, o_old = (torch.randn(B, H_q, 128, generator=g, device="cuda") for _ in range(2))
+    W = torch.rand(B, H_q, generator=g, device="cuda")
+    o_new = torch.randn(B, H_q, 128, generator=g, device="cuda").to(torch.float16)
+    want = torch.empty_like(o_new)
+    ops.blend_unnorm_into(o_hat, o_old, W, o_new, want)
+    host, dev = ops.alloc_mapped_pinned_pair((64,), torch.int64)       # trigger, completion word, record's copy a line apart
+    ops.zero_host(host)
+    word = lambda i: dev.data_ptr() + 8 * i
+    record = torch.zeros(32, dtype=torch.int64, device="cuda")
+
+    def end(trigger):
+        record.zero_()
+        out = torch.zeros_like(o_new)
+        t = time.perf_counter()
+        st = lib.jf_step_end(o_hat.data_ptr(), o_old.data_ptr(), W.data_ptr(), o_new.data_ptr(), out.data_ptr(), H_q * 128,
+                             ops._dtype_id(out), B, H_q, word(16), word(0) if trigger else None, 20, record.data_ptr(), word(32),
+                             torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+        torch.cuda.synchronize()
+        assert time.perf_counter() - t < 1.0 and torch.equal(out, want)
+        assert int(record[0]) == 0
+        code = int(host[33]) & 0xFFFFFFFF if int(host[32]) else 0
+        ops.zero_host(host[32:34])
+        return code
+
+    assert end(False) == JF_ERR_TIMEOUT
+    host[16] = 1
+    assert end(False) == 0 and end(False) == 0
+    assert end(True) == JF_ERR_TIMEOUT and int(host[0]) == 1 and int(host[16]) == 0
+    ops.free_mapped_pinned_pair(host)
+
+
 def test_building_a_step_leaves_the_processors_free():
     """No thread may still be busy once a step object is built: its first run needs the processors for the
     dispatcher and the workers.  (Fifteen OpenMP threads spinning for 4 ms are 60 ms of processor time.)"""
