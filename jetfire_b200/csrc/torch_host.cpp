@@ -225,19 +225,27 @@ ModeShape mode_shape(int mode, const char* name) {
   return mode == JF_MODE_K3V2 ? ModeShape{3, 2, 2} : ModeShape{4, 4, 1};
 }
 
+inline bool capturing_now() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
 // Scratch per (device, stream): grows as needed, one block per pair, bounded in number (the blocks go
 // back to the caching allocator when the table is cleared, which is safe in the order of the stream).
+// A call that is being captured gets a block of its own from the graph's pool, as any temporary of the
+// capture does: the graph keeps its address, and the table's block may be replaced or given back.
 at::Tensor workspace(uint64_t bytes, c10::Device device) {
   static std::mutex mu;
   static auto* table = new std::map<std::pair<int, void*>, at::Tensor>();   // never destroyed: outlives the CUDA context at exit
   constexpr size_t kMaxEntries = 64;
   const int index = device.has_index() ? device.index() : c10::cuda::current_device();
+  auto fresh = [&] {
+    return at::detail::empty_cuda({static_cast<int64_t>(bytes) + 256}, at::kByte, c10::Device(c10::kCUDA, index), c10::nullopt);
+  };
+  if (capturing_now()) return fresh();
   const std::pair<int, void*> key(index, current_stream());
   std::lock_guard<std::mutex> lock(mu);
   auto it = table->find(key);
   if (it != table->end() && static_cast<uint64_t>(it->second.numel()) >= bytes) return it->second;
   if (it == table->end() && table->size() >= kMaxEntries) table->clear();
-  at::Tensor t = at::detail::empty_cuda({static_cast<int64_t>(bytes) + 256}, at::kByte, c10::Device(c10::kCUDA, index), c10::nullopt);
+  at::Tensor t = fresh();
   (*table)[key] = t;
   return t;
 }
@@ -558,7 +566,7 @@ PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (!s) return nullptr;
     const int64_t B = s->q.size(0), H = s->H_q, row = H * JF_HEAD_DIM;
     const jf_stream_t st = current_stream();
-    const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    const bool capturing = capturing_now();
     jf_status_t r = JF_OK;
     if (!capturing) {   // an error of an earlier run, as far as it has arrived
       r = jf_decode_status_of_copy(s->status_host);

@@ -198,8 +198,8 @@ def decode_workspace_bytes(mode, B, H_q, H_kv, max_S, top_k) -> int:
 
 
 def get_workspace(nbytes: int, device) -> torch.Tensor:
-    """Cached scratch (grows monotonically per device and stream); one per current stream is the
-    caller's business when streams overlap."""
+    """Scratch for calls on the current stream, kept per device and stream and grown as needed; two threads
+    that use one stream at a time share it.  Under stream capture: a fresh block of the graph's pool."""
     dev = torch.device(device)
     return _host.get_workspace(nbytes, dev.index if dev.index is not None else torch.cuda.current_device())
 
