@@ -77,7 +77,11 @@ int dtype_id(const at::Tensor& t) {
   PyErr_Format(PyExc_RuntimeError, "expected bfloat16 or float16, got %s", c10::toString(t.scalar_type()));
   throw ArgError();
 }
-inline void* ptr(const at::Tensor& t) { return const_cast<void*>(t.const_data_ptr()); }
+// Addresses are taken with the interpreter lock held: a tensor without storage (a fake, functional or batched
+// one) throws here.  `out_ptr`: of memory that is written.
+inline const void* ptr(const at::Tensor& t) { return t.const_data_ptr(); }
+inline void* out_ptr(const at::Tensor& t) { return const_cast<void*>(t.const_data_ptr()); }
+inline uint8_t* out_bytes(const at::Tensor& t) { return static_cast<uint8_t*>(out_ptr(t)); }
 inline jf_stream_t current_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // The contiguous form of a tensor, kept alive in `keep` when it is a copy.
@@ -87,6 +91,7 @@ inline const at::Tensor& contiguous(const at::Tensor& t, at::Tensor& keep) {
   return keep;
 }
 
+// `f` must not throw: it runs without the interpreter lock.
 template <typename F> jf_status_t unlocked(F&& f) {
   jf_status_t st;
   Py_BEGIN_ALLOW_THREADS
@@ -153,10 +158,14 @@ PyObject* quant_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& slots = contiguous(slots_in, keep);
     const int dt = dtype_id(x);
     const jf_stream_t st = current_stream();
+    const void* xp = ptr(x);
+    const int64_t T = x.size(0), st_t = x.stride(0), st_h = x.stride(1), num_slots = data.size(1);
+    const auto h = static_cast<int32_t>(x.size(1));
+    const auto* sl = static_cast<const int64_t*>(ptr(slots));
+    uint8_t* dp = out_bytes(data);
+    void* sp = out_ptr(scale);
     return PyLong_FromLong(unlocked([&] {
-      return jf_pack_append(ptr(x), dt, x.size(0), static_cast<int32_t>(x.size(1)), x.stride(0), x.stride(1),
-                            static_cast<const int64_t*>(ptr(slots)), static_cast<uint8_t*>(ptr(data)), ptr(scale), data.size(1),
-                            nbits, static_cast<int32_t>(group), st);
+      return jf_pack_append(xp, dt, T, h, st_t, st_h, sl, dp, sp, num_slots, nbits, static_cast<int32_t>(group), st);
     }));
   });
 }
@@ -189,15 +198,15 @@ PyObject* quant_write_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const at::Tensor &k_mirror = tensor(a[11], name, "k_mirror_dev"), &v_mirror = tensor(a[12], name, "v_mirror_dev");
       check_mirror(k_mirror, key, kd, name);
       check_mirror(v_mirror, key, kd, name);
-      km = ptr(k_mirror);
-      vm = ptr(v_mirror);
+      km = out_ptr(k_mirror);
+      vm = out_ptr(v_mirror);
     }
     uint8_t* filled = nullptr;
     if (a[13] != Py_None) {
       const at::Tensor& f = tensor(a[13], name, "filled");
       require(f.is_cuda() && f.is_contiguous() && f.element_size() == 1 && f.numel() >= kd.size(1), name,
               "filled must hold a byte per slot");
-      filled = static_cast<uint8_t*>(ptr(f));
+      filled = out_bytes(f);
     }
     at::Tensor keep;
     const at::Tensor& slots = contiguous(slots_in, keep);
@@ -205,14 +214,17 @@ PyObject* quant_write_kv(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const jf_stream_t st = current_stream();
     const auto* sl = static_cast<const int64_t*>(ptr(slots));
     const auto h = static_cast<int32_t>(key.size(1));
+    const int64_t T = key.size(0), num_slots = kd.size(1), k_t = key.stride(0), k_h = key.stride(1), v_t = value.stride(0),
+                  v_h = value.stride(1);
+    const void *kp = ptr(key), *vp = ptr(value);
+    uint8_t *kdp = out_bytes(kd), *vdp = out_bytes(vd);
+    void *ksp = out_ptr(ks), *vsp = out_ptr(vs);
     return PyLong_FromLong(unlocked([&] {
       if (mirrored || filled)
-        return jf_store_append(ptr(key), ptr(value), dt, key.size(0), h, key.stride(0), key.stride(1), value.stride(0),
-                               value.stride(1), sl, static_cast<uint8_t*>(ptr(kd)), ptr(ks), static_cast<uint8_t*>(ptr(vd)),
-                               ptr(vs), kd.size(1), kb, vb, static_cast<int32_t>(group), km, vm, filled, st);
-      return jf_pack_append_kv(ptr(key), ptr(value), dt, key.size(0), h, key.stride(0), key.stride(1), value.stride(0),
-                               value.stride(1), sl, static_cast<uint8_t*>(ptr(kd)), ptr(ks), static_cast<uint8_t*>(ptr(vd)), ptr(vs),
-                               kd.size(1), kb, vb, static_cast<int32_t>(group), st);
+        return jf_store_append(kp, vp, dt, T, h, k_t, k_h, v_t, v_h, sl, kdp, ksp, vdp, vsp, num_slots, kb, vb,
+                               static_cast<int32_t>(group), km, vm, filled, st);
+      return jf_pack_append_kv(kp, vp, dt, T, h, k_t, k_h, v_t, v_h, sl, kdp, ksp, vdp, vsp, num_slots, kb, vb,
+                               static_cast<int32_t>(group), st);
     }));
   });
 }
@@ -303,7 +315,7 @@ struct Decode {
     const uint64_t bytes = jf_decode_workspace_bytes(a.mode, a.B, a.H_q, a.H_kv, a.max_S, a.top_k);
     require(bytes > 0, name, "bad shape");
     keep[3] = given && given != Py_None ? tensor(given, name, "workspace") : workspace(bytes, device);
-    const auto base = reinterpret_cast<uintptr_t>(ptr(keep[3])), at = (base + 255) / 256 * 256;
+    const auto base = reinterpret_cast<uintptr_t>(out_ptr(keep[3])), at = (base + 255) / 256 * 256;
     a.workspace = reinterpret_cast<void*>(at);
     a.workspace_bytes = static_cast<uint64_t>(keep[3].numel()) * keep[3].element_size() - (at - base);
   }
@@ -341,10 +353,10 @@ PyObject* fused_attn(PyObject*, PyObject* const* p, Py_ssize_t n) {
     at::Tensor o_hat = d.f32({B, H, JF_HEAD_DIM}), o_old = d.f32({B, H, JF_HEAD_DIM}), W = d.f32({B, H}), sm = d.f32({B, H}),
                inv = d.f32({B, H}), slots = d.i64({B, H, K}), idx = d.i64({B, H, K}), scores;
     if (integer(p[16])) scores = d.f32({B, H, d.a.max_S});
-    d.a.o_hat = static_cast<float*>(ptr(o_hat)); d.a.o_old_unnorm = static_cast<float*>(ptr(o_old));
-    d.a.W = static_cast<float*>(ptr(W)); d.a.softmax_m = static_cast<float*>(ptr(sm)); d.a.softmax_inv_z = static_cast<float*>(ptr(inv));
-    d.a.topk_slots = static_cast<int64_t*>(ptr(slots)); d.a.topk_idx = static_cast<int64_t*>(ptr(idx));
-    if (scores.defined()) d.a.scores = static_cast<float*>(ptr(scores));
+    d.a.o_hat = static_cast<float*>(out_ptr(o_hat)); d.a.o_old_unnorm = static_cast<float*>(out_ptr(o_old));
+    d.a.W = static_cast<float*>(out_ptr(W)); d.a.softmax_m = static_cast<float*>(out_ptr(sm)); d.a.softmax_inv_z = static_cast<float*>(out_ptr(inv));
+    d.a.topk_slots = static_cast<int64_t*>(out_ptr(slots)); d.a.topk_idx = static_cast<int64_t*>(out_ptr(idx));
+    if (scores.defined()) d.a.scores = static_cast<float*>(out_ptr(scores));
     const jf_stream_t st = current_stream();
     const jf_status_t r = unlocked([&] { return jf_decode_fused(&d.a, st); });
     return tuple_of(r, {o_hat, slots, o_old, W, idx, sm, inv, scores});
@@ -371,15 +383,15 @@ PyObject* stage_a(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int64_t B = d.B, H = d.H_q, K = d.a.top_k;
     at::Tensor scores = d.f32({B, H, d.a.max_S}), slots = d.i64({B, H, K}), idx = d.i64({B, H, K}), sm, inv;
     if (stats) { sm = d.f32({B, H}); inv = d.f32({B, H}); }
-    d.a.scores = static_cast<float*>(ptr(scores));
-    d.a.topk_slots = static_cast<int64_t*>(ptr(slots)); d.a.topk_idx = static_cast<int64_t*>(ptr(idx));
+    d.a.scores = static_cast<float*>(out_ptr(scores));
+    d.a.topk_slots = static_cast<int64_t*>(out_ptr(slots)); d.a.topk_idx = static_cast<int64_t*>(out_ptr(idx));
     const jf_stream_t st = current_stream();
+    float *smp = stats ? static_cast<float*>(out_ptr(sm)) : nullptr, *invp = stats ? static_cast<float*>(out_ptr(inv)) : nullptr;
     const jf_status_t r = unlocked([&] {
       jf_status_t s = jf_decode_scan(&d.a, st);
       if (s == JF_OK) s = jf_topk_select(&d.a, st);
       if (s == JF_OK && stats)
-        s = jf_softmax_stats(d.a.scores, d.a.seq_lens, static_cast<float*>(ptr(sm)), static_cast<float*>(ptr(inv)), d.a.B, d.a.H_q,
-                             d.a.max_S, st);
+        s = jf_softmax_stats(d.a.scores, d.a.seq_lens, smp, invp, d.a.B, d.a.H_q, d.a.max_S, st);
       return s;
     });
     return stats ? tuple_of(r, {scores, idx, slots, sm, inv}) : tuple_of(r, {scores, idx, slots});
@@ -411,8 +423,9 @@ PyObject* stage_b(PyObject*, PyObject* const* p, Py_ssize_t n) {
     d.scratch(nullptr, name);
     d.a.scan_parts = JF_SCAN_V_ONLY;
     d.a.stage_b = int32(p[2]);
-    d.a.scores = static_cast<float*>(ptr(contiguous(scores_in, d.keep[4])));
-    d.a.topk_idx = static_cast<int64_t*>(ptr(contiguous(idx_in, d.keep[5])));
+    // inputs here: the argument block's type has them writable
+    d.a.scores = static_cast<float*>(const_cast<void*>(ptr(contiguous(scores_in, d.keep[4]))));
+    d.a.topk_idx = static_cast<int64_t*>(const_cast<void*>(ptr(contiguous(idx_in, d.keep[5]))));
     at::Tensor out[3];
     if (p[14] != Py_None) {
       const int64_t want[3] = {B * H * JF_HEAD_DIM, B * H * JF_HEAD_DIM, B * H};
@@ -427,8 +440,8 @@ PyObject* stage_b(PyObject*, PyObject* const* p, Py_ssize_t n) {
       out[1] = d.f32({B, H, JF_HEAD_DIM});
       out[2] = d.f32({B, H});
     }
-    d.a.o_hat = static_cast<float*>(ptr(out[0])); d.a.o_old_unnorm = static_cast<float*>(ptr(out[1]));
-    d.a.W = static_cast<float*>(ptr(out[2]));
+    d.a.o_hat = static_cast<float*>(out_ptr(out[0])); d.a.o_old_unnorm = static_cast<float*>(out_ptr(out[1]));
+    d.a.W = static_cast<float*>(out_ptr(out[2]));
     const jf_stream_t st = current_stream();
     const jf_status_t r = unlocked([&] {
       const jf_status_t s = jf_decode_scan(&d.a, st);
@@ -493,9 +506,9 @@ PyObject* blend(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const void* nw = ptr(contiguous(o_new, keep[3]));
     const int dt = dtype_id(out);
     const jf_stream_t st = current_stream();
-    return PyLong_FromLong(unlocked([&] {
-      return jf_merge_correct(a, b, w, nw, ptr(out), dt, static_cast<int32_t>(shape[0]), static_cast<int32_t>(shape[1]), st);
-    }));
+    void* op = out_ptr(out);
+    const auto B = static_cast<int32_t>(shape[0]), H = static_cast<int32_t>(shape[1]);
+    return PyLong_FromLong(unlocked([&] { return jf_merge_correct(a, b, w, nw, op, dt, B, H, st); }));
   });
 }
 
@@ -506,7 +519,9 @@ struct Step {
   const jf_decode_args* a;
   at::Tensor q, block_table, seq_lens;      // device buffers the argument block names
   at::Tensor keep[8];                       // mapped views and outputs whose addresses follow
-  void *q_host_dev, *o_new_dev, *status_host_dev;
+  void *q_dev, *q_host_dev, *o_new_dev, *status_host_dev;
+  int64_t* bt_dev;
+  int32_t *lens_dev, bt_dev_stride;
   void* status_host;
   int64_t *done_dev, *trigger_dev;
   int64_t ctx;                              // submit context of the host correction
@@ -534,10 +549,12 @@ PyObject* step_create(PyObject*, PyObject* const* p, Py_ssize_t n) {
       s->a = reinterpret_cast<const jf_decode_args*>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLong(p[0])));
       s->q = tensor(p[1], name, "q"); s->block_table = tensor(p[2], name, "block_table"); s->seq_lens = tensor(p[3], name, "seq_lens");
       for (int i = 0; i < 5; ++i) s->keep[i] = tensor(p[4 + i], name, "step buffer");
-      s->q_host_dev = ptr(s->keep[0]); s->o_new_dev = ptr(s->keep[1]);
-      auto* words = static_cast<int64_t*>(ptr(s->keep[2]));
+      s->q_host_dev = out_ptr(s->keep[0]); s->o_new_dev = out_ptr(s->keep[1]);
+      auto* words = static_cast<int64_t*>(out_ptr(s->keep[2]));
       s->trigger_dev = words; s->done_dev = words + 8;
-      s->status_host = ptr(s->keep[3]); s->status_host_dev = ptr(s->keep[4]);
+      s->status_host = out_ptr(s->keep[3]); s->status_host_dev = out_ptr(s->keep[4]);
+      s->q_dev = out_ptr(s->q); s->bt_dev = static_cast<int64_t*>(out_ptr(s->block_table));
+      s->lens_dev = static_cast<int32_t*>(out_ptr(s->seq_lens)); s->bt_dev_stride = static_cast<int32_t>(s->block_table.size(1));
       s->ctx = integer(p[9]);
       s->timeout_ms = int32(p[10]);
       s->H_q = s->q.size(1);
@@ -596,11 +613,13 @@ PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int64_t dst_stride = merged.defined() ? row : dst.stride(0);
     const int dt = dtype_id(s->q);
     if (r == JF_OK) {
+      const void *qp = ptr(q), *btp = ptr(bt), *lp = ptr(lens);
+      void* op = out_ptr(dst);
+      const int64_t q_stride = q.stride(0), bt_stride = bt.stride(0);
+      const int32_t bt_i32 = bt.scalar_type() == at::kInt, lens_i32 = lens.scalar_type() == at::kInt;
       r = unlocked([&] {
-        jf_status_t e = jf_step_begin(ptr(q), q.stride(0), ptr(s->q), s->q_host_dev, ptr(bt), bt.scalar_type() == at::kInt, bt.stride(0),
-                                      static_cast<int32_t>(width), static_cast<int64_t*>(ptr(s->block_table)),
-                                      static_cast<int32_t>(s->block_table.size(1)), ptr(lens), lens.scalar_type() == at::kInt,
-                                      static_cast<int32_t*>(ptr(s->seq_lens)), s->done_dev, static_cast<int32_t>(B),
+        jf_status_t e = jf_step_begin(qp, q_stride, s->q_dev, s->q_host_dev, btp, bt_i32, bt_stride, static_cast<int32_t>(width), s->bt_dev,
+                                      s->bt_dev_stride, lp, lens_i32, s->lens_dev, s->done_dev, static_cast<int32_t>(B),
                                       static_cast<int32_t>(H), st);
         if (e == JF_OK) e = jf_decode_fused(s->a, st);
         int64_t* trigger = s->trigger_dev;
@@ -608,11 +627,11 @@ PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
           e = jf_stream_signal_host(st, s->done_dev, s->trigger_dev);
           trigger = nullptr;
           if (e == JF_OK)
-            e = jf_gpu_topk_attn_rows(ptr(s->q), s->k_mirror, s->v_mirror, s->slots, s->slots_i32, s->o_new_dev, dt, s->a->B, s->a->H_q,
+            e = jf_gpu_topk_attn_rows(s->q_dev, s->k_mirror, s->v_mirror, s->slots, s->slots_i32, s->o_new_dev, dt, s->a->B, s->a->H_q,
                                       s->a->H_kv, s->a->num_slots, s->a->top_k, s->a->attn_scale, s->cut, s->rows, st);
         }
         if (e == JF_OK)
-          e = jf_step_end(s->a->o_hat, s->a->o_old_unnorm, s->a->W, s->o_new_dev, ptr(dst), dst_stride, dt, s->a->B, s->a->H_q,
+          e = jf_step_end(s->a->o_hat, s->a->o_old_unnorm, s->a->W, s->o_new_dev, op, dst_stride, dt, s->a->B, s->a->H_q,
                           s->done_dev, trigger, s->timeout_ms, s->a->workspace, s->status_host_dev, st);
         return e;
       });
