@@ -78,9 +78,9 @@ int dtype_id(const at::Tensor& t) {
   throw ArgError();
 }
 // Addresses are taken with the interpreter lock held: a tensor without storage (a fake, functional or batched
-// one) throws here.  `out_ptr`: of memory that is written.
+// one) throws here.  `out_ptr`: of memory that is written (a lazily copied tensor gets its own first).
 inline const void* ptr(const at::Tensor& t) { return t.const_data_ptr(); }
-inline void* out_ptr(const at::Tensor& t) { return const_cast<void*>(t.const_data_ptr()); }
+inline void* out_ptr(const at::Tensor& t) { return t.mutable_data_ptr(); }
 inline uint8_t* out_bytes(const at::Tensor& t) { return static_cast<uint8_t*>(out_ptr(t)); }
 inline jf_stream_t current_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 

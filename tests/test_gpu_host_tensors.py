@@ -38,3 +38,22 @@ def test_tensors_without_storage_are_refused():
                        cwd=Path(__file__).resolve().parents[1])
     assert r.returncode == 0, r.stderr[-2000:]
     assert r.stdout.split("\n")[:-1] == ["refused"] * 5
+
+
+def test_a_lazy_copy_gets_memory_of_its_own_before_it_is_written():
+    from jetfire_b200 import ops
+    x = torch.randn(4, 2, 128, device="cuda").to(torch.bfloat16)
+    slots = torch.arange(4, device="cuda")
+    caches = [torch.full((2, 64, 48), 0xA5, dtype=torch.uint8, device="cuda"), torch.zeros(2, 64, 2, dtype=torch.bfloat16, device="cuda"),
+              torch.full((2, 64, 32), 0xA5, dtype=torch.uint8, device="cuda"), torch.zeros(2, 64, 2, dtype=torch.bfloat16, device="cuda")]
+    before = [t.clone() for t in caches]
+    copies = [torch._lazy_clone(t) for t in caches]
+    ops.fused_quant_write_kv(x, x, slots, *copies, 64, 3, 2)
+    out = torch.zeros(1, 4, 128, dtype=torch.bfloat16, device="cuda")
+    out_copy = torch._lazy_clone(out)
+    o = torch.ones(1, 4, 128, device="cuda")
+    ops.blend_unnorm_into(o, torch.zeros_like(o), torch.zeros(1, 4, device="cuda"), out, out_copy)
+    torch.cuda.synchronize()
+    for t, b, c in zip(caches, before, copies):
+        assert torch.equal(t, b) and not torch.equal(c, b)
+    assert bool((out == 0).all()) and bool((out_copy == 1).all())
