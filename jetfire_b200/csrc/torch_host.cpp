@@ -584,38 +584,46 @@ PyObject* step_run(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int64_t B = s->q.size(0), H = s->H_q, row = H * JF_HEAD_DIM;
     const jf_stream_t st = current_stream();
     const bool capturing = capturing_now();
-    jf_status_t r = JF_OK;
-    if (!capturing) {   // an error of an earlier run, as far as it has arrived
-      r = jf_decode_status_of_copy(s->status_host);
-      if (r == JF_OK) r = jf_submit_ctx_status(s->ctx);
-      else std::memset(s->status_host, 0, JF_STATUS_RECORD_BYTES);   // reported once; the next call runs
-    }
     at::Tensor q = tensor(p[1], name, "query"), bt = tensor(p[2], name, "block_table"), lens = tensor(p[3], name, "seq_lens"),
                out = tensor(p[4], name, "output");
-    require(q.is_cuda() && bt.is_cuda() && lens.is_cuda() && out.is_cuda(), name, "tensors must be CUDA");
-    require(q.scalar_type() == s->q.scalar_type() && out.scalar_type() == s->q.scalar_type(), name, "query / output dtype mismatch");
+    require(q.is_cuda(), name, "query must be CUDA");
+    require(q.scalar_type() == s->q.scalar_type(), name, "query dtype mismatch");
+    require(q.dim() >= 2 && q.size(0) >= B && q.numel() == q.size(0) * row, name, "query must be (B, H_q, 128)");
+    require(out.dim() >= 2 && out.size(0) >= B && out.numel() == out.size(0) * row, name, "output must be (B, H_q * 128)");
     // rows of H_q * 128 elements, whatever the leading dimensions are called
     auto rows_ok = [&](const at::Tensor& t, int64_t mult, uintptr_t align) {
       const bool two = t.dim() == 2 && t.size(1) == row && t.stride(1) == 1;
       const bool three = t.dim() == 3 && t.size(1) == H && t.size(2) == JF_HEAD_DIM && t.stride(2) == 1 && t.stride(1) == JF_HEAD_DIM;
       return (two || three) && t.stride(0) % mult == 0 && reinterpret_cast<uintptr_t>(ptr(t)) % align == 0;
     };
-    require(q.dim() >= 2 && q.size(0) >= B && q.numel() == q.size(0) * row, name, "query must be (B, H_q, 128)");
-    require(out.dim() >= 2 && out.size(0) >= B && out.numel() == out.size(0) * row, name, "output must be (B, H_q * 128)");
-    if (!rows_ok(q, 8, 16)) q = q.contiguous().clone();
-    require(bt.dim() == 2 && bt.size(0) >= B && lens.dim() == 1 && lens.size(0) >= B, name, "block_table / seq_lens shape mismatch");
+    // an output in place has the step's device and type; any other form is what a copy takes
+    const bool same = out.is_cuda() && out.scalar_type() == s->q.scalar_type();
+    require(same || !out.narrow(0, 0, B).is_contiguous(), name, "output must be a CUDA tensor of the query's dtype");
+    require(bt.dim() == 2 && (bt.size(0) >= B || bt.size(0) == 1) && lens.dim() <= 1 && lens.numel() >= B, name,
+            "block_table / seq_lens shape mismatch");
+    jf_status_t r = JF_OK;
+    if (!capturing) {   // an error of an earlier run, as far as it has arrived
+      r = jf_decode_status_of_copy(s->status_host);
+      if (r == JF_OK) r = jf_submit_ctx_status(s->ctx);
+      else std::memset(s->status_host, 0, JF_STATUS_RECORD_BYTES);   // reported once; the next call runs
+    }
+    // forms that the kernels do not address go through a copy
+    if (!rows_ok(q, 8, 16)) q = at::empty({B, row}, s->q.options()).copy_(q.narrow(0, 0, B).reshape({B, row}));
+    if (!bt.is_cuda()) bt = bt.to(s->q.device());
     if ((bt.scalar_type() != at::kLong && bt.scalar_type() != at::kInt) || bt.stride(1) != 1) bt = bt.to(at::kLong).contiguous();
+    if (!lens.is_cuda()) lens = lens.to(s->q.device());
+    if (lens.dim() == 0) lens = lens.reshape({1});
     if ((lens.scalar_type() != at::kLong && lens.scalar_type() != at::kInt) || lens.stride(0) != 1) lens = lens.to(at::kInt).contiguous();
     const int64_t width = std::min<int64_t>(bt.size(1), s->block_table.size(1));
     at::Tensor merged;
-    if (!rows_ok(out, 4, 8)) merged = at::empty_like(s->q);
+    if (!same || !rows_ok(out, 4, 8)) merged = at::empty_like(s->q);
     const at::Tensor& dst = merged.defined() ? merged : out;
     const int64_t dst_stride = merged.defined() ? row : dst.stride(0);
     const int dt = dtype_id(s->q);
     if (r == JF_OK) {
       const void *qp = ptr(q), *btp = ptr(bt), *lp = ptr(lens);
       void* op = out_ptr(dst);
-      const int64_t q_stride = q.stride(0), bt_stride = bt.stride(0);
+      const int64_t q_stride = q.stride(0), bt_stride = bt.size(0) < B ? 0 : bt.stride(0);   // one row for all: broadcast
       const int32_t bt_i32 = bt.scalar_type() == at::kInt, lens_i32 = lens.scalar_type() == at::kInt;
       r = unlocked([&] {
         jf_status_t e = jf_step_begin(qp, q_stride, s->q_dev, s->q_host_dev, btp, bt_i32, bt_stride, static_cast<int32_t>(width), s->bt_dev,

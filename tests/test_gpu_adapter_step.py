@@ -37,7 +37,7 @@ def test_step_takes_the_forms_a_caller_has(B, H_q, dtype):
         md = make_decode_metadata(seq_lens, block_table)
         assert try_jetfire_decode(impl=impl, layer=layer, query=query, attn_metadata=md, output=out, store=st, cfg=cfg) is out
         torch.cuda.synchronize()
-        return out[:B].reshape(B, row).clone()
+        return out[:B].reshape(B, row).cuda()
 
     want = run(q, bt, lens, torch.zeros(B, row, dtype=dtype, device="cuda"))
     wide = torch.full((B + 2, row + 8), 3.0, dtype=dtype, device="cuda")
@@ -48,12 +48,21 @@ def test_step_takes_the_forms_a_caller_has(B, H_q, dtype):
     q_odd.copy_(q)
     forms = [(q.view(B, row), bt.to(torch.int32), lens.to(torch.int64), wide[:, :row]),
              (q_pad, bt, lens, torch.zeros(B, H_q, 128, dtype=dtype, device="cuda")),
-             (q_odd, torch.cat([bt, bt], 1), lens, odd[:, 3:])]
+             (q_odd, torch.cat([bt, bt], 1), lens, odd[:, 3:]),
+             (q, bt.cpu(), lens.cpu(), torch.zeros(B, row, dtype=dtype, device="cuda")),
+             (q, bt, lens.double(), torch.zeros(B, 2 * row, dtype=dtype)[:, ::2])]
+    if B == 1:       # strides of a dimension of one element mean nothing; lengths without a dimension
+        forms.append((q.view(H_q, 128, 1).clone().permute(2, 0, 1), bt, lens[0], torch.zeros(1, row, dtype=dtype, device="cuda")))
     for query, table, length, out in forms:
         if query.dim() == 2:
             query = query.view(B, H_q, 128)
         assert torch.equal(run(query, table, length, out), want)
     assert bool((wide[B:] == 3.0).all()) and bool((wide[:, row:] == 3.0).all())
+    same = run(q, bt[:1].expand(B, -1).contiguous(), lens, torch.zeros(B, row, dtype=dtype, device="cuda"))
+    assert torch.equal(run(q, bt[:1], lens, torch.zeros(B, row, dtype=dtype, device="cuda")), same)    # one table for all
+    for bad in (torch.zeros(B, row, device="cuda"), torch.zeros(B, row, dtype=dtype)):
+        with pytest.raises(RuntimeError, match="output"):
+            run(q, bt, lens, bad)
 
 
 def _one_step(top_k=32):
