@@ -61,10 +61,24 @@ int32_t int32(PyObject* o) {
   }
   return static_cast<int32_t>(v);
 }
+// What int(x) and float(x) take, where the op's Python form converted its arguments with them.
+struct Owned {
+  PyObject* o;
+  explicit Owned(PyObject* p) : o(p) { if (!o) throw ArgError(); }
+  ~Owned() { Py_DECREF(o); }
+};
+int32_t as_int32(PyObject* o) {
+  if (PyLong_CheckExact(o)) return int32(o);
+  return int32(Owned(PyNumber_Long(o)).o);
+}
 double real(PyObject* o) {
-  const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw ArgError();
-  return v;
+  if (PyFloat_CheckExact(o)) return PyFloat_AS_DOUBLE(o);
+  return PyFloat_AS_DOUBLE(Owned(PyNumber_Float(o)).o);
+}
+bool truth(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw ArgError();
+  return v != 0;
 }
 const char* text(PyObject* o) {
   const char* s = PyUnicode_AsUTF8(o);
@@ -343,7 +357,7 @@ PyObject* fused_attn(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const ModeShape m = mode_shape(mode, name);
     Decode d;
     d.common(mode, tensor(p[7], name, "block_table"), tensor(p[8], name, "seq_lens"), int32(p[9]), int32(p[10]), int32(p[11]),
-             int32(p[12]), int32(p[13]), real(p[14]), name);
+             as_int32(p[12]), int32(p[13]), real(p[14]), name);
     d.query(tensor(p[2], name, "q"), name);
     d.side(tensor(p[3], name, "k_data"), tensor(p[4], name, "k_scales"), m.k_bits, m.groups, true, name);
     d.side(tensor(p[5], name, "v_data"), tensor(p[6], name, "v_scales"), m.v_bits, m.groups, false, name);
@@ -352,7 +366,7 @@ PyObject* fused_attn(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int64_t B = d.B, H = d.H_q, K = d.a.top_k;
     at::Tensor o_hat = d.f32({B, H, JF_HEAD_DIM}), o_old = d.f32({B, H, JF_HEAD_DIM}), W = d.f32({B, H}), sm = d.f32({B, H}),
                inv = d.f32({B, H}), slots = d.i64({B, H, K}), idx = d.i64({B, H, K}), scores;
-    if (integer(p[16])) scores = d.f32({B, H, d.a.max_S});
+    if (truth(p[16])) scores = d.f32({B, H, d.a.max_S});
     d.a.o_hat = static_cast<float*>(out_ptr(o_hat)); d.a.o_old_unnorm = static_cast<float*>(out_ptr(o_old));
     d.a.W = static_cast<float*>(out_ptr(W)); d.a.softmax_m = static_cast<float*>(out_ptr(sm)); d.a.softmax_inv_z = static_cast<float*>(out_ptr(inv));
     d.a.topk_slots = static_cast<int64_t*>(out_ptr(slots)); d.a.topk_idx = static_cast<int64_t*>(out_ptr(idx));
@@ -371,15 +385,15 @@ PyObject* stage_a(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const char* name = text(p[0]);
     const int mode = int32(p[1]);
     const ModeShape m = mode_shape(mode, name);
-    require(integer(p[10]) == JF_BLOCK_SIZE, name, "block_size must be 16");
+    require(as_int32(p[10]) == JF_BLOCK_SIZE, name, "block_size must be 16");
     Decode d;
-    d.common(mode, tensor(p[5], name, "block_table"), tensor(p[6], name, "seq_lens"), int32(p[7]), int32(p[8]), int32(p[9]),
-             int32(p[10]), int32(p[12]), real(p[11]), name);
+    d.common(mode, tensor(p[5], name, "block_table"), tensor(p[6], name, "seq_lens"), as_int32(p[7]), as_int32(p[8]), as_int32(p[9]),
+             JF_BLOCK_SIZE, as_int32(p[12]), real(p[11]), name);
     d.query(tensor(p[2], name, "q"), name);
     d.side(tensor(p[3], name, "k_data"), tensor(p[4], name, "k_scales"), m.k_bits, m.groups, true, name);
     d.scratch(nullptr, name);
     d.a.scan_parts = JF_SCAN_K_ONLY;
-    const bool stats = integer(p[13]) != 0;
+    const bool stats = truth(p[13]);
     const int64_t B = d.B, H = d.H_q, K = d.a.top_k;
     at::Tensor scores = d.f32({B, H, d.a.max_S}), slots = d.i64({B, H, K}), idx = d.i64({B, H, K}), sm, inv;
     if (stats) { sm = d.f32({B, H}); inv = d.f32({B, H}); }
@@ -406,15 +420,15 @@ PyObject* stage_b(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const char* name = text(p[0]);
     const int mode = int32(p[1]);
     const ModeShape m = mode_shape(mode, name);
-    require(integer(p[12]) == JF_BLOCK_SIZE, name, "block_size must be 16");
+    require(as_int32(p[12]) == JF_BLOCK_SIZE, name, "block_size must be 16");
     const at::Tensor &scores_in = tensor(p[3], name, "scores"), &idx_in = tensor(p[8], name, "topk_idx");
     require(scores_in.is_cuda() && scores_in.scalar_type() == at::kFloat && scores_in.dim() == 3, name, "scores must be f32 (B,H_q,max_S)");
-    const int64_t K = int32(p[13]);
+    const int64_t K = as_int32(p[13]);
     require(idx_in.is_cuda() && idx_in.scalar_type() == at::kLong && idx_in.dim() == 3 && idx_in.size(2) == K, name,
             "topk_idx must be int64 (B,H_q,top_k)");
     Decode d;
-    d.common(mode, tensor(p[6], name, "block_table"), tensor(p[7], name, "seq_lens"), int32(p[9]), int32(p[10]), int32(p[11]),
-             int32(p[12]), K, 1.0, name);
+    d.common(mode, tensor(p[6], name, "block_table"), tensor(p[7], name, "seq_lens"), as_int32(p[9]), as_int32(p[10]), as_int32(p[11]),
+             JF_BLOCK_SIZE, K, 1.0, name);
     d.side(tensor(p[4], name, "v_data"), tensor(p[5], name, "v_scales"), m.v_bits, m.groups, false, name);
     const int64_t B = d.B, H = d.H_q;
     require(scores_in.size(0) == B && scores_in.size(1) == H && scores_in.size(2) == d.a.max_S, name,

@@ -1,4 +1,5 @@
 """The native half of ``ops``: argument errors are RuntimeErrors that name the op, before any launch."""
+import numpy as np
 import pytest
 import torch
 
@@ -17,3 +18,22 @@ from jetfire_b200 import ops
 def test_host_tensors_are_refused_by_name(call):
     with pytest.raises(RuntimeError, match=r"^[a-z0-9_]+: "):
         call(torch.zeros(1, 8, 128))
+
+
+@pytest.mark.parametrize("call", [
+    lambda t, n: ops.int3_qk_scores_topk(t, t, t, t, t, n(16), n(8), n(2), n(16), n(1), n(32)),
+    lambda t, n: ops.int8tc_qk_scores_topk_stats(t, t, t, t, t, n(16), n(8), n(2), n(16), n(1), n(32)),
+    lambda t, n: ops.fused_attn_topk("k3v2", t, t, t, t, t, t, t, 16, 8, 2, n(16), 32, n(1)),
+])
+@pytest.mark.parametrize("number", [float, np.float32, torch.tensor, lambda v: torch.tensor(float(v)), str],
+                         ids=["float", "numpy", "tensor", "float tensor", "text"])
+def test_numbers_are_what_int_and_float_take(call, number):
+    """The ops that convert their sizes with int() and float() get as far as the tensors."""
+    with pytest.raises(RuntimeError, match="must be CUDA"):
+        call(torch.zeros(1, 8, 128), number)
+
+
+def test_a_number_that_is_none_is_an_error_of_its_own():
+    t = torch.zeros(1, 8, 128)
+    with pytest.raises((TypeError, ValueError)):
+        ops.int3_qk_scores_topk(t, t, t, t, t, "sixteen", 8, 2, 16, 1.0, 32)
