@@ -228,8 +228,14 @@ typedef struct jf_decode_args {
                               size; topk_slots may then be NULL.  No counterpart in the reference. */
 } jf_decode_args;
 
+/* The workspace a call requires, and what it can make use of: with the second much, long rows are cut
+ * into two waves of blocks where that is faster (the last bits of o_hat follow the cut).  The first does
+ * not shrink as max_S grows, the second not as B or max_S do: a workspace for the largest call of a
+ * program serves the others. */
 uint64_t    jf_decode_workspace_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
                                       int32_t max_S, int32_t top_k);
+uint64_t    jf_decode_workspace_useful_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
+                                             int32_t max_S, int32_t top_k);
 /* scan: dequantise, Q.K^T, online softmax, P.V over the packed cache; leaves split
  * partials, approximate scores (also in args->scores if given) and, for long rows, the largest
  * score of every group of 16-token pages in the workspace (what the select kernel of the same

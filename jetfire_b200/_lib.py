@@ -89,6 +89,7 @@ _SIGS = {
     "jf_map_host": (C.c_int32, [C.c_void_p, C.c_uint64, C.POINTER(C.c_void_p)]),
     "jf_unmap_host": (C.c_int32, [C.c_void_p]),
     "jf_decode_workspace_bytes": (C.c_uint64, [C.c_int32] * 6),
+    "jf_decode_workspace_useful_bytes": (C.c_uint64, [C.c_int32] * 6),
     "jf_decode_scan": (C.c_int32, [C.POINTER(DecodeArgs), C.c_void_p]),
     "jf_topk_select": (C.c_int32, [C.POINTER(DecodeArgs), C.c_void_p]),
     "jf_decode_finish": (C.c_int32, [C.POINTER(DecodeArgs), C.c_void_p]),

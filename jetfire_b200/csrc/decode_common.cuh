@@ -46,17 +46,17 @@ __host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype) {
 // `splits`: as many as fill one wave of resident CTAs, or two waves where that leaves fewer of them idle
 // -- a CTA costs about eight units besides its own (start, merge: 3-4 us) -- with at least one unit per
 // warp.  (K4V4, 16 sequences x 8 KV heads x 131072 positions: four splits fill 86 % of a wave, nine 97 %
-// of two, 511 -> 478 us.)
+// of two, 511 -> 478 us.)  Two waves only where the workspace has room for their partials (`most_waves`):
+// what a call requires is the one wave's, which does not shrink as the row grows.
 constexpr int kSliceOverhead = 8;
-inline int scan_splits(int mode, int q_dtype, int B, int H_kv, int max_S) {
-  const int units = ((max_S + JF_BLOCK_SIZE - 1) / JF_BLOCK_SIZE + 1) / 2;
+inline int scan_units(int max_S) { return ((max_S + JF_BLOCK_SIZE - 1) / JF_BLOCK_SIZE + 1) / 2; }
+inline int scan_split_cap(int units) { return units < 8 ? 1 : units > 4 * 512 ? 512 : units / 4; }
+inline int scan_splits(int mode, int q_dtype, int B, int H_kv, int max_S, int most_waves) {
+  const int units = scan_units(max_S), cap = scan_split_cap(units);
   const int pairs = B * H_kv, wave = num_sms() * scan_ctas_per_sm(mode, q_dtype);
-  int cap = units / 4;
-  if (cap > 512) cap = 512;
-  if (cap < 1) cap = 1;
   int best = 1;
   int64_t best_cost = INT64_MAX;
-  for (int w = 1; w <= 2; ++w) {
+  for (int w = 1; w <= most_waves; ++w) {
     int s = w * wave / pairs;
     if (s > cap) s = cap;
     if (s < 1) s = 1;
@@ -178,26 +178,46 @@ __host__ __device__ inline int page_max_stride(int mode, int max_S) {
   return (((max_S + group - 1) / group) + 3) & ~3;
 }
 
-// Sized for the query type with the most splits, so one workspace serves both.
-inline Workspace carve_workspace(void* base, int mode, int B, int H_q, int H_kv, int max_S, int /*top_k*/, bool need_scores) {
-  const HeadGeom hg = head_geom(H_q, H_kv);
-  const int s0 = scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, max_S), s1 = scan_splits(mode, JF_DTYPE_FP16, B, hg.H_kv, max_S);
-  const uint64_t splits = s0 > s1 ? s0 : s1;
-  const uint64_t pairs = static_cast<uint64_t>(B) * hg.H_kv * splits;
+// With room for `partials` partials of the scan (CTAs).
+inline Workspace carve_workspace(void* base, int mode, int B, int H_q, int max_S, uint64_t partials) {
   uint64_t off = 0;
   uint8_t* p = static_cast<uint8_t*>(base);
   Workspace w{};
   w.status = reinterpret_cast<int32_t*>(p + off);   off = align_up(off + 256, 256);
-  w.part_o = reinterpret_cast<float*>(p + off);     off = align_up(off + pairs * kHeadsPad * JF_HEAD_DIM * 4, 256);
-  w.part_m = reinterpret_cast<float*>(p + off);     off = align_up(off + pairs * kHeadsPad * 4, 256);
-  w.part_l = reinterpret_cast<float*>(p + off);     off = align_up(off + pairs * kHeadsPad * 4, 256);
-  w.part_smax = reinterpret_cast<float*>(p + off);  off = align_up(off + pairs * 2 * 4, 256);
+  w.part_o = reinterpret_cast<float*>(p + off);     off = align_up(off + partials * kHeadsPad * JF_HEAD_DIM * 4, 256);
+  w.part_m = reinterpret_cast<float*>(p + off);     off = align_up(off + partials * kHeadsPad * 4, 256);
+  w.part_l = reinterpret_cast<float*>(p + off);     off = align_up(off + partials * kHeadsPad * 4, 256);
+  w.part_smax = reinterpret_cast<float*>(p + off);  off = align_up(off + partials * 2 * 4, 256);
   w.pmax = reinterpret_cast<float*>(p + off);
   off = align_up(off + static_cast<uint64_t>(B) * H_q * page_max_stride(mode, max_S) * 4, 256);
   w.scores = reinterpret_cast<float*>(p + off);
-  if (need_scores) off = align_up(off + static_cast<uint64_t>(B) * H_q * max_S * 4, 256);
+  off = align_up(off + static_cast<uint64_t>(B) * H_q * max_S * 4, 256);
   w.bytes = off;
   return w;
+}
+// Least partials a call needs room for (one wave, the query type with more CTAs, so one workspace serves
+// both), and the most any call of up to these sizes makes use of (neither shrinks as B or max_S grows but
+// for the remainder of a wave in the first).
+inline uint64_t partials_needed(int mode, int B, int H_q, int H_kv, int max_S) {
+  const HeadGeom hg = head_geom(H_q, H_kv);
+  return static_cast<uint64_t>(B) * hg.H_kv * scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, max_S, 1);
+}
+inline uint64_t partials_useful(int mode, int B, int H_q, int H_kv, int max_S) {
+  const uint64_t pairs = static_cast<uint64_t>(B) * head_geom(H_q, H_kv).H_kv, capped = pairs * scan_split_cap(scan_units(max_S));
+  const uint64_t waves = 2ull * num_sms() * scan_ctas_per_sm(mode, JF_DTYPE_BF16), most = capped < waves ? capped : waves;
+  return most > pairs ? most : pairs;
+}
+// CTAs per sequence and KV head of a call (the same for its scan, select and finish), and its workspace.
+inline int call_splits(const jf_decode_args* a) {
+  const HeadGeom hg = head_geom(a->H_q, a->H_kv);
+  const int two = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S, 2);
+  const uint64_t partials = static_cast<uint64_t>(a->B) * hg.H_kv * two;
+  if (carve_workspace(nullptr, a->mode, a->B, a->H_q, a->max_S, partials).bytes <= a->workspace_bytes) return two;
+  return scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S, 1);
+}
+inline Workspace call_workspace(const jf_decode_args* a, int splits) {
+  return carve_workspace(a->workspace, a->mode, a->B, a->H_q, a->max_S,
+                         static_cast<uint64_t>(a->B) * head_geom(a->H_q, a->H_kv).H_kv * splits);
 }
 
 // Status record at the start of the workspace.  A kernel whose bounded wait ran out writes
@@ -222,8 +242,8 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
 #endif
 
 jf_status_t validate_decode_args(const jf_decode_args* a);
-// the cut of a call's work (the same for its scan, select and finish)
-SliceGeom slice_geom(const jf_decode_args* a);
+// the cut of a call's work (`splits`: call_splits)
+SliceGeom slice_geom(const jf_decode_args* a, int splits);
 // device address of the library's built-in scratch array on the current device (decode_static.cu)
 jf_status_t static_scratch_address(void** out);
 

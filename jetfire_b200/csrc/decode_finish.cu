@@ -107,11 +107,12 @@ extern "C" jf_status_t jf_decode_finish(const jf_decode_args* a, jf_stream_t str
   if (st != JF_OK) return st;
   if (!a->topk_idx || !a->o_hat || !a->o_old_unnorm || !a->W) return JF_ERR_ARG;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  Workspace ws = carve_workspace(a->workspace, a->mode, a->B, a->H_q, a->H_kv, a->max_S, a->top_k, true);
+  const int splits = call_splits(a);
+  Workspace ws = call_workspace(a, splits);
   FinishParams fp{};
   fp.block_table = a->block_table; fp.seq_lens = a->seq_lens; fp.topk_idx = a->topk_idx;
   fp.max_blocks = a->max_blocks;
-  const TailParams tp = make_tail_params(a, ws);
+  const TailParams tp = make_tail_params(a, ws, splits);
   dim3 grid(a->H_q, a->B);
   if (a->mode == JF_MODE_K3V2) {
     JF_ENSURE_SMEM((decode_finish_kernel<JF_MODE_K3V2>), sizeof(TailSmem<JF_MODE_K3V2>));

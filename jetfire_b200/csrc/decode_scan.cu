@@ -610,11 +610,10 @@ jf_status_t validate_decode_args(const jf_decode_args* a) {
   return JF_OK;
 }
 
-SliceGeom slice_geom(const jf_decode_args* a) {
-  const HeadGeom hg = head_geom(a->H_q, a->H_kv);
+SliceGeom slice_geom(const jf_decode_args* a, int splits) {
   SliceGeom g{};
-  g.splits = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S);
-  g.units = ((a->max_S + 15) / 16 + 1) / 2;
+  g.splits = splits;
+  g.units = scan_units(a->max_S);
   g.units_per_split = (g.units + g.splits - 1) / g.splits;
   g.even = a->mode != JF_MODE_K3V2 || a->B == 1 || g.units_per_split < kShareMin;
   return g;
@@ -648,7 +647,15 @@ __global__ void fill_neg_inf_tail_kernel(float* scores, const int32_t* seq_lens,
 extern "C" uint64_t jf_decode_workspace_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
                                               int32_t max_S, int32_t top_k) {
   if (B <= 0 || H_q <= 0 || H_kv <= 0 || max_S <= 0 || top_k <= 0) return 0;
-  return jf::carve_workspace(nullptr, mode, B, H_q, H_kv, max_S, top_k, true).bytes;
+  return jf::carve_workspace(nullptr, mode, B, H_q, max_S, jf::partials_needed(mode, B, H_q, H_kv, max_S)).bytes;
+}
+
+extern "C" uint64_t jf_decode_workspace_useful_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
+                                                     int32_t max_S, int32_t top_k) {
+  if (B <= 0 || H_q <= 0 || H_kv <= 0 || max_S <= 0 || top_k <= 0) return 0;
+  const uint64_t most = jf::carve_workspace(nullptr, mode, B, H_q, max_S, jf::partials_useful(mode, B, H_q, H_kv, max_S)).bytes;
+  const uint64_t least = jf_decode_workspace_bytes(mode, B, H_q, H_kv, max_S, top_k);
+  return most > least ? most : least;
 }
 
 extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t stream_) {
@@ -656,7 +663,8 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   jf_status_t st = validate_decode_args(a);
   if (st != JF_OK) return st;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  Workspace ws = carve_workspace(a->workspace, a->mode, a->B, a->H_q, a->H_kv, a->max_S, a->top_k, true);
+  const int splits = call_splits(a);
+  Workspace ws = call_workspace(a, splits);
   ScanParams sp{};
   sp.q = a->q;
   sp.k_data = a->k_data;  sp.k_scales = static_cast<const uint16_t*>(a->k_scales);
@@ -674,7 +682,7 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   const HeadGeom hg = head_geom(a->H_q, a->H_kv);
   sp.B = a->B; sp.H_q = a->H_q; sp.H_kv = hg.H_kv; sp.G = hg.G; sp.kv_shift = hg.shift;
   sp.max_S = a->max_S; sp.max_blocks = a->max_blocks;
-  sp.geom = slice_geom(a);
+  sp.geom = slice_geom(a, splits);
   sp.attn_scale = a->attn_scale;
   sp.q_dtype = a->q_dtype;
   dim3 grid(sp.geom.splits, a->B, hg.H_kv);

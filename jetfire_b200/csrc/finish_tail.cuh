@@ -307,7 +307,7 @@ __device__ __forceinline__ float block_max_of_splits(const float* part_m, int64_
 }
 
 struct Workspace;
-TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws);
+TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws, int splits);
 jf_status_t launch_select(const jf_decode_args* a, cudaStream_t stream, bool fused);
 
 }  // namespace jf

@@ -1142,7 +1142,7 @@ jf_status_t launch_select_mode(const jf_decode_args* a, const SelectPlan& plan, 
 
 }  // namespace
 
-TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws) {
+TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws, int splits) {
   TailParams tp{};
   tp.scores = a->scores ? a->scores : ws.scores;
   tp.part_o = ws.part_o; tp.part_m = ws.part_m; tp.part_l = ws.part_l;
@@ -1154,7 +1154,7 @@ TailParams make_tail_params(const jf_decode_args* a, const Workspace& ws) {
   tp.H_q = a->H_q; tp.H_kv = hg.H_kv; tp.G = hg.G; tp.kv_shift = hg.shift;
   tp.max_S = a->max_S;
   tp.B = a->B;
-  tp.geom = slice_geom(a);
+  tp.geom = slice_geom(a, splits);
   tp.top_k = a->top_k;
   return tp;
 }
@@ -1166,7 +1166,8 @@ jf_status_t launch_select(const jf_decode_args* a, cudaStream_t stream, bool fus
   if (!a->topk_idx || (!a->topk_slots && !a->topk_slots_i32)) return JF_ERR_ARG;
   if (a->topk_slots_i32 && a->num_slots > 0x7FFFFFFFll) return JF_ERR_ARG;
   if (fused && (!a->o_hat || !a->o_old_unnorm || !a->W)) return JF_ERR_ARG;
-  Workspace ws = carve_workspace(a->workspace, a->mode, a->B, a->H_q, a->H_kv, a->max_S, a->top_k, true);
+  const int splits = call_splits(a);
+  Workspace ws = call_workspace(a, splits);
   TopkParams sp{};
   sp.scores = a->scores ? a->scores : ws.scores;
   sp.pmax = ws.pmax; sp.np_stride = page_max_stride(a->mode, a->max_S);
@@ -1183,7 +1184,7 @@ jf_status_t launch_select(const jf_decode_args* a, cudaStream_t stream, bool fus
   if (sp.sort_n < 512) sp.sort_n = 512;
   sp.q_dtype = a->q_dtype;
   sp.attn_scale = a->attn_scale;
-  const TailParams tp = make_tail_params(a, ws);
+  const TailParams tp = make_tail_params(a, ws, splits);
   sp.geom = tp.geom;
   const dim3 grid(a->H_q, a->B);
   const SelectPlan plan = select_plan(a, sp.scores);

@@ -326,7 +326,7 @@ struct Decode {
     a.q = ptr(contiguous(q, keep[2]));
   }
   void scratch(PyObject* given, const char* name) {
-    const uint64_t bytes = jf_decode_workspace_bytes(a.mode, a.B, a.H_q, a.H_kv, a.max_S, a.top_k);
+    const uint64_t bytes = jf_decode_workspace_useful_bytes(a.mode, a.B, a.H_q, a.H_kv, a.max_S, a.top_k);
     require(bytes > 0, name, "bad shape");
     keep[3] = given && given != Py_None ? tensor(given, name, "workspace") : workspace(bytes, device);
     const auto base = reinterpret_cast<uintptr_t>(out_ptr(keep[3])), at = (base + 255) / 256 * 256;

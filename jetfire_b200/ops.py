@@ -193,8 +193,10 @@ _STAGE_B = {"fp32": _lib.JF_STAGE_B_FP32, "int8p": _lib.JF_STAGE_B_INT8P}
 
 
 def decode_workspace_bytes(mode, B, H_q, H_kv, max_S, top_k) -> int:
-    return int(lib.jf_decode_workspace_bytes(MODE_IDS[mode] if isinstance(mode, str) else mode,
-                                             B, H_q, H_kv, max_S, top_k))
+    """Scratch for calls of up to these sizes; a smaller workspace serves down to what
+    ``jf_decode_workspace_bytes`` says, with the scan cut into one wave of blocks."""
+    return int(lib.jf_decode_workspace_useful_bytes(MODE_IDS[mode] if isinstance(mode, str) else mode,
+                                                    B, H_q, H_kv, max_S, top_k))
 
 
 def get_workspace(nbytes: int, device) -> torch.Tensor:
