@@ -241,12 +241,18 @@ class _StreamStep:
 
     def close(self) -> None:
         """Release the correction context (the dispatcher stops polling its trigger word) and the mapped
-        block.  Only once nothing queued on a stream, and no graph, refers to this step any more."""
+        block.  Only once nothing queued on a stream, and no graph, refers to this step any more.  A job
+        that outlasted its run's wait may still be with the workers, who read and write the block: it goes
+        back when they are through, and stays allocated if they are not."""
         self.host.close()
         if self.flags and self.mapped is not None:
             self.native = None
-            ops.free_mapped_pinned_pair(self.mapped[0])
-            self.mapped = None
+            mapped, self.mapped = self.mapped, None
+            try:
+                ops.cpu_topk_attn_wait(30000)
+            except RuntimeError:
+                return
+            ops.free_mapped_pinned_pair(mapped[0])
 
 
 _MAX_S_STEP = 4096      # a step object serves row lengths up to the next multiple of this

@@ -90,3 +90,25 @@ def test_decode_gate_reasons():
     assert _decode_unsupported(attn_metadata=md, **{**args, "layer": layer12}) == "gqa_ratio"
     layer32 = SimpleNamespace(layer_name="l0", num_heads=64, num_kv_heads=2, head_size=128)
     assert _decode_unsupported(attn_metadata=md, **{**args, "layer": layer32}) == "gqa_ratio"
+
+
+@pytest.mark.parametrize("workers_finish", [True, False])
+def test_a_closed_step_gives_its_block_back_after_the_workers(monkeypatch, workers_finish):
+    """The mapped block is what a correction job reads and writes: it is freed once the workers are through
+    with every job, never before, and not at all if they do not finish."""
+    from jetfire_b200 import ops
+    from jetfire_b200.adapter import decode_path as dp
+    events = []
+
+    def wait(timeout_ms):
+        events.append("wait")
+        if not workers_finish:
+            raise RuntimeError("cpu_topk_attn_wait failed: status 2 (a bounded wait ran out)")
+    monkeypatch.setattr(ops, "cpu_topk_attn_wait", wait)
+    monkeypatch.setattr(ops, "free_mapped_pinned_pair", lambda host: events.append("free"))
+    step = dp._StreamStep.__new__(dp._StreamStep)
+    step.flags, step.mapped, step.native = True, (torch.zeros(1), None), None
+    step.host = SimpleNamespace(close=lambda: events.append("unwatch"))
+    step.close()
+    step.close()
+    assert events == ["unwatch", "wait"] + (["free"] if workers_finish else []) + ["unwatch"]
