@@ -5,7 +5,8 @@
 The library is plain C ABI (``include/jetfire_b200.h``); Python loads it with ctypes
 (``jetfire_b200._lib``).  Beside it ``_host.so`` is built from ``csrc/torch_host.cpp``: the
 tensor-taking half of ``ops.py``, a CPython extension against the installed torch and this
-library.  The build is skipped when both are newer than every source file.
+library.  The build is skipped when both are newer than every source file and ``_host.so`` was built against
+the installed torch.
 """
 from __future__ import annotations
 
@@ -32,8 +33,14 @@ def nvcc_path() -> str:
     return cand
 
 
+def torch_stamp() -> str:
+    """What ``_host.so`` is built against, as text inside it: torch's interfaces change with its version."""
+    import torch
+    return f"jetfire_b200._host for torch {torch.__version__}"
+
+
 def up_to_date() -> bool:
-    if not LIB.exists() or not HOST.exists():
+    if not LIB.exists() or not HOST.exists() or (torch_stamp() + "\0").encode() not in HOST.read_bytes():
         return False
     t = min(LIB.stat().st_mtime, HOST.stat().st_mtime)
     deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + list(CSRC.glob("*.h")) + \
@@ -50,7 +57,8 @@ def host_command(nvcc: str) -> list[str]:
     cuda = Path(nvcc).resolve().parents[1]
     inc = [base / "include", base / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{i}" for i in inc),
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DJF_TORCH_STAMP="{torch_stamp()}"',
+            *(f"-I{i}" for i in inc),
             str(CSRC / "torch_host.cpp"), "-o", str(HOST), f"-L{base / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
             "-ltorch", "-lc10_cuda", "-lc10", f"-L{PKG}", "-ljetfire_b200", "-Wl,-rpath,$ORIGIN"]
 

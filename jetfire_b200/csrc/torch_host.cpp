@@ -676,4 +676,11 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "tensor-taking half of je
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__host() {
+  PyObject* m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "built_for", JF_TORCH_STAMP) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -23,7 +23,32 @@ import torch
 
 from . import _lib
 from ._lib import DecodeArgs, JetFireError, check, lib
-from . import _host   # after the library it is linked to
+
+
+class _NoHost:
+    """Stands in for ``_host.so`` where it cannot be used: the host-side ops (correction workers, placement)
+    need only the library, every op that needs the module says why it is not there."""
+
+    def __init__(self, why):
+        self._why = why
+
+    def __getattr__(self, name):
+        raise ImportError(f"jetfire_b200/_host.so cannot be used ({self._why}): build it with `python -m jetfire_b200.build` "
+                          "(there is no fallback path)")
+
+
+def _load_host():
+    from .build import torch_stamp
+    try:
+        from . import _host   # after the library it is linked to
+    except ImportError as e:
+        return _NoHost(e)
+    if getattr(_host, "built_for", "") != torch_stamp():
+        return _NoHost(f"it is {getattr(_host, 'built_for', 'of an unknown torch')!r}, installed is {torch.__version__}")
+    return _host
+
+
+_host = _load_host()
 
 MODE_IDS = {"k3v2": _lib.JF_MODE_K3V2, "k4v4": _lib.JF_MODE_K4V4,
             "SymInt3K_SymInt2V": _lib.JF_MODE_K3V2, "SymInt4K_SymInt4V": _lib.JF_MODE_K4V4}

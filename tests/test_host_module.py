@@ -1,4 +1,8 @@
 """The native half of ``ops``: argument errors are RuntimeErrors that name the op, before any launch."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -37,3 +41,35 @@ def test_a_number_that_is_none_is_an_error_of_its_own():
     t = torch.zeros(1, 8, 128)
     with pytest.raises((TypeError, ValueError)):
         ops.int3_qk_scores_topk(t, t, t, t, t, "sixteen", 8, 2, 16, 1.0, 32)
+
+
+@pytest.mark.parametrize("module", ["None", "types.SimpleNamespace(built_for='jetfire_b200._host for torch 0.1')"],
+                         ids=["missing", "of another torch"])
+def test_the_host_ops_need_only_the_library(module):
+    """Without a usable ``_host.so`` the package imports, the ops of the correction workers run, and an op
+    that needs the module says how to build it."""
+    code = f"""
+import sys, types
+sys.modules["jetfire_b200._host"] = {module}
+import torch, jetfire_b200
+if {module} is not None: jetfire_b200._host = {module}
+from jetfire_b200 import ops
+assert ops.get_cpu_attn_threads() > 0 and ops.numa_node_count() >= 1
+t = torch.zeros(1, 8, 128)
+try:
+    ops.blend_unnorm_into(t, t, t, t, t)
+except ImportError as e:
+    assert "jetfire_b200.build" in str(e), e
+    print("refused")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=Path(__file__).resolve().parents[1])
+    assert r.returncode == 0 and r.stdout == "refused\n", r.stdout + r.stderr
+
+
+def test_a_module_for_another_torch_is_not_up_to_date(monkeypatch):
+    from jetfire_b200 import build
+    if not build.up_to_date():
+        pytest.skip("the sources are newer than the build")
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".1")
+    assert not build.up_to_date()
