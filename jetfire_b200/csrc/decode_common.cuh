@@ -135,12 +135,19 @@ __device__ __forceinline__ void slice_partials(const SliceGeom& g, const int32_t
 // Which select kernel a call takes -- decided from the arguments alone, so that the scan (which
 // then leaves the maxima of groups of pages: K3V2 pairs of pages, K4V4 pages) and the select
 // kernel (which then takes its threshold from them and never stages the row) agree.
-//   narrow: more rows than multiprocessors -> 512-thread blocks, two per multiprocessor;
-//   lean:   the row does not fit one resident chunk of that block (32 positions per thread), there
-//           are enough groups for the K-th largest group maximum to be a tight bound, and the
-//           score rows are whole pages that 16-byte loads can read.
-// Rows of one chunk stay with the kernel that stages them: it is as fast there, and the scan
-// saves the few per cent the maxima cost it.
+//   narrow: more rows than multiprocessors -> two blocks share one, and a staged chunk is 16384
+//           positions; otherwise a row has a multiprocessor to itself and a chunk of 32768;
+//   lean:   the row does not fit one staged chunk, there are enough groups for the K-th largest group
+//           maximum to be a tight bound, and the score rows are whole pages that 16-byte loads can read.
+// Rows of one chunk stay with the kernel that stages them.  Scan + select, staged / from maxima, us, top-k
+// 256 (64 where there are too few groups for that):
+//   128 rows   K4V4 16384 29.2 / 29.6, 32768 41.3 / 41.7, 40960 50.4 / 48.1;  K3V2 8192 22.9 / 23.3,
+//              16384 31.4 / 30.5, 32768 52.1 / 49.8, 40960 62.7 / 56.7
+//    32 rows   K4V4 32768 24.0 / 23.7, 40960 29.3 / 25.8;  K3V2 32768 26.0 / 26.0, 40960 31.5 / 28.0
+//   256 rows   (8 KV heads x 8 sequences) K4V4 16384 44.3 / 44.2, 20480 53.0 / 50.0;  K3V2 12288 39.5 / 39.5,
+//              16384 49.1 / 47.8, 20480 64.1 / 54.7
+// so the line is right for K4V4 and within 2 % up to there, and K3V2 would gain up to 5 % from half of it on.
+// The maxima cost the scan 0.4 % (K3V2, whose warps form them anyway) and 4-5 % (K4V4).
 constexpr int kStagedTopK = 2048;   // widest top-k of the kernel that stages the row
 struct SelectPlan { bool narrow, lean, supported; };
 inline SelectPlan select_plan(const jf_decode_args* a, const float* scores) {

@@ -18,10 +18,12 @@
 // shared memory together with what the copies need, so that the loop never waits for a global
 // load and the warp-uniform work per page stays small.
 //
-// What bounds it: instruction issue and the half-rate logic pipe (a field mask is two issue
-// cycles), not memory.  Measured per pipe: LOP3 2 cycles, HFMA2.BF16 2, HMMA 16816 8; the 72 + 32 +
-// 18 of a page alone are 255 cycles of a scheduler.  On a layer of 4 sequences x 8 KV heads x 65536
-// positions: 352 -> 277 warp instructions per page, 74.4 -> 62.4 us (0.46 of the copy peak).
+// What bounds it: instruction issue and a warp's dependent chain, not memory.  A page is 280 warp
+// instructions (352 before), so 280 cycles of its scheduler at one a cycle; of these 64 are field masks (one
+// per two codes) and as many more go to the same half-rate pipe that it is busy for 273 cycles; the 18 MMAs
+// hold theirs for 144.  On a layer of 4 sequences x 8 KV heads x 65536 positions a page takes ~ 520 cycles
+// (pipe 53 % busy, 58 % of the issue slots used, four warps a scheduler, DRAM at 41 % of its peak): 74.4 ->
+// 62.4 us, 0.46 of the copy peak; the 280 cycles alone would be 32 us.
 //
 // Compute: tokens sit on the MMA M axis and the (<= 8) query heads on N = 8.  Packed codes
 // are expanded in registers straight into the A fragments of mma.sync.m16n8k16 (the

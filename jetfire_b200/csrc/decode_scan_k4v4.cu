@@ -262,7 +262,7 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
     if (pm && (!kMasked || !pb || ((mask >> 20) & 3) == 2)) *pm = v;   // lanes with bit 2 clear of a live head; page B only if present
   }
 
-  // ---- one online-softmax step over both pages (same arithmetic per score as softmax_step) ----
+  // ---- one online-softmax step over both pages (the arithmetic per score of the K3V2 scan) ----
   uint64_t pA01, pA23, pB01, pB23;
   {
     float mx0 = fmaxf(fmaxf(sA[0], sA[2]), fmaxf(sB[0], sB[2])), mx1 = fmaxf(fmaxf(sA[1], sA[3]), fmaxf(sB[1], sB[3]));
