@@ -375,7 +375,8 @@ scan_k3v2_kernel(const ScanParams p) {
   // compiler so, and lets slot addresses live in uniform registers
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
-  const int hkv = blockIdx.z;
+  const ScanBlock blk = scan_block(p);
+  const int hkv = blk.hkv;
 
   const uint32_t smem_base = smem_u32(smem);
   constexpr int kRingBytes = kScanWarps * T::kSlots * T::kSlotBytes;
@@ -386,7 +387,7 @@ scan_k3v2_kernel(const ScanParams p) {
 
   pdl_wait();  // nothing above reads global memory
 
-  const ScanSlice slice = scan_slice<kShares>(p, lane);
+  const ScanSlice slice = scan_slice<kShares>(p, blk.b, lane);
   const int b = slice.b, len = slice.len, n_pages = (len + 15) >> 4;
   // Warp w owns a contiguous quarter of the split's pages, so its block-table entries are
   // contiguous too: sixteen lanes fetch sixteen entries with one load, a whole chunk ahead of
@@ -687,7 +688,7 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   sp.geom = slice_geom(a, splits);
   sp.attn_scale = a->attn_scale;
   sp.q_dtype = a->q_dtype;
-  dim3 grid(sp.geom.splits, a->B, hg.H_kv);
+  const dim3 grid = scan_grid(sp);
   if (a->mode == JF_MODE_K3V2) {
     // the query's type only matters where the query is read
     const int dt = a->scan_parts == JF_SCAN_V_ONLY ? JF_DTYPE_BF16 : a->q_dtype;

@@ -58,14 +58,28 @@ struct ScanParams {
   int tile_base[9];
 };
 
-// This CTA's slice: units [lo, hi) of sequence b, whose length is len.  CTA (x, y) of a KV head is number
-// y * splits + x; with equal shares that is slice x of sequence y.  Whole warp, the same for all lanes.
+// Grid (splits, sequences, KV heads), or (1, KV heads, sequences) with one CTA per pair: there are so many pairs
+// then that they take about a wave or more, and with the sequences slowest blocks of one length follow one
+// another, the short ones of falling lengths at the end (128 sequences of 700 and less x 8 KV heads, K4V4: 18
+// us, 23 with the KV heads slowest, in no order slower).  With more CTAs a pair it is the other way round
+// (16 ragged sequences of 65536 x 8, K4V4: 198 us, 204 with the sequences slowest).
+struct ScanBlock { int b, hkv; };
+__device__ __forceinline__ ScanBlock scan_block(const ScanParams& p) {
+  const bool one = p.geom.splits == 1;
+  return ScanBlock{static_cast<int>(one ? blockIdx.z : blockIdx.y), static_cast<int>(one ? blockIdx.y : blockIdx.z)};
+}
+inline dim3 scan_grid(const ScanParams& p) {
+  return p.geom.splits == 1 ? dim3(1, p.H_kv, p.B) : dim3(p.geom.splits, p.B, p.H_kv);
+}
+
+// This CTA's slice: units [lo, hi) of sequence b, whose length is len.  CTA x of sequence y of a KV head is its
+// number y * splits + x; with equal shares that is slice x of sequence y.  Whole warp, the same for all lanes.
 struct ScanSlice { int b, len, lo, hi; };
 template <bool kShares>
-__device__ __forceinline__ ScanSlice scan_slice(const ScanParams& p, int lane) {
+__device__ __forceinline__ ScanSlice scan_slice(const ScanParams& p, int y, int lane) {
   const SliceGeom& g = p.geom;
   ScanSlice r;
-  r.b = blockIdx.y;
+  r.b = y;
   r.lo = blockIdx.x * g.units_per_split;
   r.hi = r.lo + g.units_per_split;   // (the sequence may end before)
   if (!kShares) {
@@ -76,7 +90,7 @@ __device__ __forceinline__ ScanSlice scan_slice(const ScanParams& p, int lane) {
   const int my_len = slice_len(p.seq_lens, p.B, p.max_S, 0, lane);
   const SliceSums s = slice_sums(g, p.seq_lens, p.B, p.max_S, lane, my_len);
   if (!s.equal) {
-    uint32_t i = blockIdx.y * g.splits + blockIdx.x;   // CTAs left before this one
+    uint32_t i = y * g.splits + blockIdx.x;   // CTAs left before this one
     r.b = r.lo = r.hi = 0;
     for (int b0 = 0; b0 < p.B; b0 += 32) {
       const uint32_t units = slice_units(b0 == 0 ? my_len : slice_len(p.seq_lens, p.B, p.max_S, b0, lane));
@@ -163,7 +177,8 @@ __device__ __forceinline__ void cta_merge_store(const ScanParams& p, uint8_t* sm
   }
   if (lane == 0) { sm_s[warp * 2] = smax0; sm_s[warp * 2 + 1] = smax1; }
   __syncthreads();
-  const int64_t pidx = (static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const ScanBlock blk = scan_block(p);
+  const int64_t pidx = (static_cast<int64_t>(blk.hkv) * p.B + blk.b) * gridDim.x + blockIdx.x;
   float* po = p.part_o + pidx * (kHeadsPad * JF_HEAD_DIM);
   for (int i = threadIdx.x; i < kHeadsPad * JF_HEAD_DIM; i += blockDim.x) {
     const int h = i >> 7;

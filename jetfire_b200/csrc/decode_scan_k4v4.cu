@@ -361,7 +361,8 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // uniform by construction
   const int g = lane >> 2, tig = lane & 3;
-  const int split = blockIdx.x, b = blockIdx.y, hkv = blockIdx.z;
+  const ScanBlock blk = scan_block(p);
+  const int split = blockIdx.x, b = blk.b, hkv = blk.hkv;
 
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t slots0 = smem_base + warp * (T4::kSlots * T4::kSlotBytes);
