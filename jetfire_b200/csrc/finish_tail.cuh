@@ -292,17 +292,18 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
 }
 
 // Shared by both kernels: the merged reference point M = max over the splits, block-wide.
-// `red` = 32 floats of shared memory.  Ends with a barrier.  For a block of kSelThreads threads.
+// `red` = a float of shared memory per warp.  Ends with a barrier.  NT: threads of the block.
+template <int NT>
 __device__ __forceinline__ float block_max_of_splits(const float* part_m, int64_t pbase, int hi, int splits, float* red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float M = kMinusBig;
-  for (int s = tid; s < splits; s += kSelThreads) M = fmaxf(M, part_m[(pbase + s) * kHeadsPad + hi]);
+  for (int s = tid; s < splits; s += NT) M = fmaxf(M, part_m[(pbase + s) * kHeadsPad + hi]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, o));
   if (lane == 0) red[warp] = M;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < kSelWarps; ++w) M = fmaxf(M, red[w]);
+  for (int w = 0; w < NT / 32; ++w) M = fmaxf(M, red[w]);
   return M;
 }
 
