@@ -584,19 +584,55 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           } else {
             hits = (1u << vecs_of(ci)) - 1u;
           }
-          while (__any_sync(0xFFFFFFFFu, hits != 0u)) {
-            const int j = hits ? __ffs(hits) - 1 : 0;
-            const int pos = ci * kChunkPos + 4 * (j * NT + tid);
-            uint32_t m4 = 0u;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (hits && pos < n) {
-              v = use16 ? *reinterpret_cast<const float4*>(srow + pos) : chunk4[j * NT + tid];
-              m4 = above4(v, thr);
-              if (n - pos < 4) m4 &= (1u << (n - pos)) - 1u;
+          // Places: from votes, a float4 of every lane at a time -- or, for the two to eight float4s a lane of the
+          // smaller chunk has, from one scan over four bits for each.  (Votes on a row of 16384: 1 k cycles more.
+          // The scan on a row of 2048: 0.6 k more, its dense hits being written one after the other; on one of
+          // 32768 alone on its multiprocessor no difference but the code.)
+          if (kChunkVec > 8 || vecs_of(ci) == 1) {
+            while (__any_sync(0xFFFFFFFFu, hits != 0u)) {
+              const int j = hits ? __ffs(hits) - 1 : 0;
+              const int pos = ci * kChunkPos + 4 * (j * NT + tid);
+              uint32_t m4 = 0u;
+              float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (hits && pos < n) {
+                v = use16 ? *reinterpret_cast<const float4*>(srow + pos) : chunk4[j * NT + tid];
+                m4 = above4(v, thr);
+                if (n - pos < 4) m4 &= (1u << (n - pos)) - 1u;
+              }
+              hits &= hits - 1u;
+              const float e[4] = {v.x, v.y, v.z, v.w};
+              append_hits(m4, e, pos);
             }
+            continue;
+          }
+          uint32_t mask = 0u;
+          while (hits) {
+            const int j = __ffs(hits) - 1, pos = ci * kChunkPos + 4 * (j * NT + tid);
             hits &= hits - 1u;
-            const float e[4] = {v.x, v.y, v.z, v.w};
-            append_hits(m4, e, pos);
+            if (pos >= n) continue;
+            uint32_t m4 = above4(use16 ? *reinterpret_cast<const float4*>(srow + pos) : chunk4[j * NT + tid], thr);
+            if (n - pos < 4) m4 &= (1u << (n - pos)) - 1u;
+            mask |= m4 << ((4 * j) & 31);
+          }
+          if (!__any_sync(0xFFFFFFFFu, mask != 0u)) continue;
+          const int cnt = __popc(mask);
+          int incl = cnt;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          int base = 0;
+          if (lane == 31) base = atomicAdd(&sm.ncand, incl);
+          int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
+          while (mask) {
+            const int e = __ffs(mask) - 1, at = 4 * ((e >> 2) * NT + tid) + (e & 3);
+            mask &= mask - 1u;
+            if (o < p.sort_n) {
+              keys[o] = static_cast<uint64_t>(ci * kChunkPos + at);
+              cand_score[o] = use16 ? srow[ci * kChunkPos + at] : chunk[at];
+            }
+            ++o;
           }
         }
         __syncthreads();
@@ -847,7 +883,20 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         const int cn = min(kRowChunk, ncand - base);
         const int rounds = (cn + 4 * kW - 1) / (4 * kW);
         auto cand_of = [&](int i) { return (i >> 2) * (4 * kW) + 4 * warp + (i & 3); };   // the warp's i-th candidate
-        for (int i = lane; i < 4 * rounds; i += 32) {
+        int i0 = lane;
+        if (FUSED && MODE == JF_MODE_K4V4 && !merged) {
+          // K4V4 has no scores to compute under the copies: the merge of the scan's partials runs while the block
+          // ids of the first 32 candidates are on their way
+          const int c = cand_of(lane);
+          const bool any = lane < 4 * rounds && c < cn;
+          const int pos = any ? static_cast<int>(keys[base + c]) : 0;
+          const int64_t blk = any ? ctx.bt[pos >> 4] : -1;
+          merge_splits(tp, sm.splits, pbase, n_splits, hi, row_max);
+          merged = true;
+          if (any) late.cand_slot[c] = static_cast<int32_t>(blk < 0 || blk >= (ctx.num_slots >> 4) ? -1 : blk * 16 + (pos & 15));
+          i0 += 32;
+        }
+        for (int i = i0; i < 4 * rounds; i += 32) {
           const int c = cand_of(i);
           if (c < cn) late.cand_slot[c] = static_cast<int32_t>(slot_of(ctx, static_cast<int>(keys[base + c])));
         }
