@@ -69,21 +69,30 @@ struct EndParams {
   int rows, H_q;             // rows = B * H_q
 };
 
-constexpr int kEndThreads = 512;   // 16 rows of 32 four-channel pieces
+constexpr int kEndThreads = 512;   // 16 rows of 32 four-channel pieces at a time
+constexpr int kEndRows = 2;        // so often per block: 32 rows are one block, which needs no word from another (1.3 us)
 
 template <int DT>
 __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p) {
   pdl_wait();      // the kernels that wrote the slots, the query copy and the attention parts are complete
   pdl_trigger();
-  const int row = blockIdx.x * (kEndThreads / 32) + (threadIdx.x >> 5), piece = threadIdx.x & 31;
-  const bool live = row < p.rows;
+  // again, and late: a worker of a run that was given up may have set it since the step began (ahead of the loads,
+  // so that the fence before the trigger does not wait a trip over the host link for it)
+  if (threadIdx.x == 0 && blockIdx.x == 0 && p.trigger != nullptr) *p.done = 0;
+  const int row0 = blockIdx.x * (kEndRows * kEndThreads / 32) + (threadIdx.x >> 5), piece = threadIdx.x & 31;
   // what the merge needs besides the correction, while that is on its way
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f), o = a;
-  float w = 0.f;
-  if (live) {
-    a = p.o_hat[row * 32 + piece];
-    o = p.o_old[row * 32 + piece];
-    w = p.W[row];
+  float4 a[kEndRows], o[kEndRows];
+  float w[kEndRows];
+#pragma unroll
+  for (int k = 0; k < kEndRows; ++k) {
+    const int row = row0 + k * (kEndThreads / 32);
+    a[k] = o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    w[k] = 0.f;
+    if (row < p.rows) {
+      a[k] = p.o_hat[row * 32 + piece];
+      o[k] = p.o_old[row * 32 + piece];
+      w[k] = p.W[row];
+    }
   }
   if (threadIdx.x == 0) {
     volatile int32_t* const verdict = p.status + kWaitWord;
@@ -92,7 +101,6 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p
       // One block waits and decides for the grid: with a budget of its own each, the blocks could differ
       // around the limit, and those of a later wave would start it afresh.
       if (p.trigger != nullptr) {
-        *p.done = 0;              // again, as late as can be: a worker of a run that was given up may have set it since
         __threadfence_system();   // what the correction reads is on the host before the trigger is
         *p.trigger = 1;
       }
@@ -122,18 +130,31 @@ __global__ void __launch_bounds__(kEndThreads) step_end_kernel(const EndParams p
     }
   }
   __syncthreads();
-  if (!live) return;
-  const volatile uint32_t* nw = reinterpret_cast<const volatile uint32_t*>(p.o_new + row * 32 + piece);
-  const uint32_t n0 = nw[0], n1 = nw[1];
-  const float n[4] = {Elem<DT>::to_f32(static_cast<uint16_t>(n0 & 0xFFFFu)), Elem<DT>::to_f32(static_cast<uint16_t>(n0 >> 16)),
-                      Elem<DT>::to_f32(static_cast<uint16_t>(n1 & 0xFFFFu)), Elem<DT>::to_f32(static_cast<uint16_t>(n1 >> 16))};
-  const float h[4] = {a.x, a.y, a.z, a.w}, old[4] = {o.x, o.y, o.z, o.w};
-  uint16_t r[4];
+  uint32_t n0[kEndRows], n1[kEndRows];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) r[i] = Elem<DT>::from_f32(h[i] + w * n[i] - old[i]);
-  const int b = row / p.H_q, hq = row - b * p.H_q;
-  uint2* dst = reinterpret_cast<uint2*>(p.out + b * p.out_stride + hq * JF_HEAD_DIM) + piece;
-  *dst = make_uint2(r[0] | (static_cast<uint32_t>(r[1]) << 16), r[2] | (static_cast<uint32_t>(r[3]) << 16));
+  for (int k = 0; k < kEndRows; ++k) {
+    const int row = row0 + k * (kEndThreads / 32);
+    n0[k] = n1[k] = 0u;
+    if (row < p.rows) {
+      const volatile uint32_t* nw = reinterpret_cast<const volatile uint32_t*>(p.o_new + row * 32 + piece);
+      n0[k] = nw[0];
+      n1[k] = nw[1];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kEndRows; ++k) {
+    const int row = row0 + k * (kEndThreads / 32);
+    if (row >= p.rows) break;
+    const float n[4] = {Elem<DT>::to_f32(static_cast<uint16_t>(n0[k] & 0xFFFFu)), Elem<DT>::to_f32(static_cast<uint16_t>(n0[k] >> 16)),
+                        Elem<DT>::to_f32(static_cast<uint16_t>(n1[k] & 0xFFFFu)), Elem<DT>::to_f32(static_cast<uint16_t>(n1[k] >> 16))};
+    const float h[4] = {a[k].x, a[k].y, a[k].z, a[k].w}, old[4] = {o[k].x, o[k].y, o[k].z, o[k].w};
+    uint16_t r[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = Elem<DT>::from_f32(h[i] + w[k] * n[i] - old[i]);
+    const int b = row / p.H_q, hq = row - b * p.H_q;
+    uint2* dst = reinterpret_cast<uint2*>(p.out + b * p.out_stride + hq * JF_HEAD_DIM) + piece;
+    *dst = make_uint2(r[0] | (static_cast<uint32_t>(r[1]) << 16), r[2] | (static_cast<uint32_t>(r[3]) << 16));
+  }
 }
 
 }  // namespace
@@ -173,7 +194,8 @@ extern "C" jf_status_t jf_step_end(const float* o_hat, const float* o_old_unnorm
               reinterpret_cast<volatile long long*>(done_dev), reinterpret_cast<volatile long long*>(trigger_dev),
               static_cast<int32_t*>(status_record), static_cast<uint4*>(status_host_dev),
               static_cast<unsigned long long>(timeout_ms) * 1000000ull, B * H_q, H_q};
-  const dim3 grid((B * H_q * 32 + kEndThreads - 1) / kEndThreads);
+  constexpr int per_block = kEndRows * kEndThreads / 32;
+  const dim3 grid((B * H_q + per_block - 1) / per_block);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   JF_CUDA_TRY(dtype == JF_DTYPE_BF16 ? launch_pdl(step_end_kernel<JF_DTYPE_BF16>, grid, dim3(kEndThreads), 0, s, p)
                                      : launch_pdl(step_end_kernel<JF_DTYPE_FP16>, grid, dim3(kEndThreads), 0, s, p));

@@ -122,7 +122,7 @@ def test_a_recorded_error_is_reported_once():
     del graph
 
 
-@pytest.mark.parametrize("B,H_q", [(1, 4), (5, 20)], ids=["one block", "seven blocks"])
+@pytest.mark.parametrize("B,H_q", [(1, 4), (1, 32), (3, 11), (5, 20)], ids=["one block", "a full block", "two blocks", "four blocks"])
 def test_the_wait_at_the_end_runs_out(B, H_q):
     """jf_step_end with a completion word that nobody sets: the stream goes on after the budget, the error is
     handed to the host, the record is clear again; the next call, with the word set, leaves no error.  A word
