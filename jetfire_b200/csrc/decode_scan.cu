@@ -18,12 +18,15 @@
 // shared memory together with what the copies need, so that the loop never waits for a global
 // load and the warp-uniform work per page stays small.
 //
-// What bounds it: instruction issue and a warp's dependent chain, not memory.  A page is 280 warp
-// instructions (352 before), so 280 cycles of its scheduler at one a cycle; of these 64 are field masks (one
-// per two codes) and as many more go to the same half-rate pipe that it is busy for 273 cycles; the 18 MMAs
-// hold theirs for 144.  On a layer of 4 sequences x 8 KV heads x 65536 positions a page takes ~ 520 cycles
-// (pipe 53 % busy, 58 % of the issue slots used, four warps a scheduler, DRAM at 41 % of its peak): 74.4 ->
-// 62.4 us, 0.46 of the copy peak; the 280 cycles alone would be 32 us.
+// What bounds it: the issue of instructions, not memory and not a warp's dependent chain (the keys of the next
+// round gone through beside the softmax and P.V of the last: no difference).  A page is some 270 warp instructions (352
+// with bulk copies, 280 before the codes sat at two bit positions).  On a scheduler of a B200 a logic or integer
+// instruction takes two cycles of its pipe, packed 16-bit arithmetic two of the other, and an mma.sync.m16n8k16 -- 8.6 cycles
+// alone -- does not run under them: beside a dozen others it adds 3.5 to 7 cycles, so that the 18 of a page are about a
+// fifth of its ~ 550.  Of the 62.4 us of a layer of 4 sequences x 8 KV heads x 65536 positions (0.46 of the copy peak;
+// 74.4 with bulk copies) the expansion of the K codes takes 10, of the V codes 4, the copies 8 and the score stores 2.
+// (The same work as 128-token tiles on tcgen05, the expanded codes in tensor memory: 74 us.  A token a thread is 320
+// instructions a page with its stores to tensor memory, and those that turn V over run at a quarter of the rate.)
 //
 // Compute: tokens sit on the MMA M axis and the (<= 8) query heads on N = 8.  Packed codes
 // are expanded in registers straight into the A fragments of mma.sync.m16n8k16 (the
@@ -40,10 +43,9 @@ namespace jf {
 namespace {
 
 // Bit position at which code x (0..7) of an INT3 group is picked up (see the unpack in the
-// kernel): the 3-bit field has to sit inside the 7-bit bf16 mantissa, i.e. at 0..4.
-__device__ __forceinline__ constexpr int k3_pos(int x) {
-  return x == 0 ? 0 : x == 1 ? 3 : x == 2 ? 0 : x == 3 ? 4 : x == 4 ? 1 : x == 5 ? 0 : x == 6 ? 3 : 0;
-}
+// kernel): the 3-bit field has to sit inside the 7-bit bf16 mantissa.  Two positions, so that a
+// (token, group) takes two offset constants.
+__device__ __forceinline__ constexpr int k3_pos(int x) { return (x & 1) ? 0 : 3; }
 // bit position of 2-bit field f (0..7, bit offset 2f of a 16-bit half row word)
 __device__ __forceinline__ constexpr int v2_pos(int f) { return f <= 4 ? 2 * f : 2 * f - 10; }
 // head-dim index inside the 8-wide chunk for field f: bytes are little-endian in the
@@ -60,42 +62,39 @@ __device__ __forceinline__ constexpr int v2_dlocal(int f) { return 4 * (f >> 2) 
 // jetfire_vllm/csrc/int3_qk_scores.cu:94-99.  The factor 2^(POS - 33) is undone by the query
 // operand.  (An 8-bit scale times a 3-bit integer needs at most 10 bits: exact before rounding.)
 struct K3Scale {
-  uint32_t S;     // scale * 2^100, both halves
-  uint32_t C[5];  // -scale * 2^(POS - 31) for POS = 0..4, both halves (POS 2 is unused)
+  uint32_t S;       // scale * 2^100, both halves
+  uint32_t C0, C3;  // -scale * 2^(POS - 31) for POS = 0 and 3, both halves
 };
 __device__ __forceinline__ K3Scale k3_scale(uint32_t scale2) {
   K3Scale k;
-  k.S = mul_bf16x2(scale2, 0x71807180u);        // 2^100
-  k.C[0] = mul_bf16x2(scale2, 0xB000B000u);     // -2^-31
-  k.C[1] = mul_bf16x2(scale2, 0xB080B080u);     // -2^-30
-  k.C[2] = 0u;
-  k.C[3] = mul_bf16x2(scale2, 0xB180B180u);     // -2^-28
-  k.C[4] = mul_bf16x2(scale2, 0xB200B200u);     // -2^-27
+  k.S = mul_bf16x2(scale2, 0x71807180u);    // 2^100
+  k.C0 = mul_bf16x2(scale2, 0xB000B000u);   // -2^-31
+  k.C3 = mul_bf16x2(scale2, 0xB180B180u);   // -2^-28
   return k;
 }
 template <int POS>
 __device__ __forceinline__ uint32_t k3_field(uint32_t v, const K3Scale& k) {
   constexpr uint32_t m = (7u << POS) | (7u << (POS + 16));
-  return fma_bf16x2(v & m, k.S, k.C[POS]);
+  return fma_bf16x2(v & m, k.S, POS == 0 ? k.C0 : k.C3);
 }
 // One 32-bit word of each byte plane (4 INT3 groups = 32 channels of one row) -> 16 bf16x2
 // registers R[pair][code]: pair p holds groups (2p, 2p+1) in its (low, high) halves.
-__device__ __forceinline__ void k3_unpack_row(uint32_t P0, uint32_t P1, uint32_t P2, const K3Scale& scale2,
+__device__ __forceinline__ void k3_unpack_row(uint32_t P0, uint32_t P1, uint32_t P2, const K3Scale& k,
                                               uint32_t (&R)[2][8]) {
 #pragma unroll
   for (int pr = 0; pr < 2; ++pr) {
     const uint32_t sel = pr ? 0x7362u : 0x5140u;
     const uint32_t lo = prmt(P2, P1, sel);  // halves: bits 15..0 of the two 24-bit groups
     const uint32_t hi = prmt(P1, P0, sel);  // halves: bits 23..8
-    const uint32_t lo6 = lo >> 6, hi7 = hi >> 7, hi13 = hi >> 13;
-    R[pr][7] = k3_field<0>(lo, scale2);
-    R[pr][6] = k3_field<3>(lo, scale2);
-    R[pr][5] = k3_field<0>(lo6, scale2);
-    R[pr][4] = k3_field<1>(hi, scale2);
-    R[pr][3] = k3_field<4>(hi, scale2);
-    R[pr][2] = k3_field<0>(hi7, scale2);
-    R[pr][1] = k3_field<3>(hi7, scale2);
-    R[pr][0] = k3_field<0>(hi13, scale2);
+    const uint32_t w5 = lo >> 6, w3 = hi >> 4, w1 = hi >> 10;   // codes 5, 4 | 3, 2 | 1, 0 at bits 0 and 3
+    R[pr][7] = k3_field<0>(lo, k);
+    R[pr][6] = k3_field<3>(lo, k);
+    R[pr][5] = k3_field<0>(w5, k);
+    R[pr][4] = k3_field<3>(w5, k);
+    R[pr][3] = k3_field<0>(w3, k);
+    R[pr][2] = k3_field<3>(w3, k);
+    R[pr][1] = k3_field<0>(w1, k);
+    R[pr][0] = k3_field<3>(w1, k);
   }
 }
 
@@ -164,7 +163,7 @@ __device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t a, uint32_t b) {
 template <int QT>
 struct K3State {
   uint32_t qf[QT][8][2];   // query fragments (B operand of the K MMA)
-  float oacc[10][4];       // output accumulators, O^T fragments; tiles 8, 9: sum of the P operand per V group
+  float oacc[9][4];        // output accumulators, O^T fragments; tile 8: sum of the P operand, rows 0-7 V group 0, rows 8-15 group 1
   float m_ref0, m_ref1;    // softmax reference points of heads 2tig, 2tig+1
   uint64_t l2;             // softmax sums of the two heads
   uint32_t smax2;          // largest K group scales seen (bf16 pair: group 0, group 1; sign bits are noise)
@@ -192,13 +191,16 @@ __device__ __forceinline__ void k3_weights(uint32_t (&B)[4], const float (&p)[4]
 #pragma unroll
   for (int qh = 0; qh < 2; ++qh) {
     const float va = __uint_as_float(qh ? (vsa & 0xFFFF0000u) : (vsa << 16)), vb = __uint_as_float(qh ? (vsb & 0xFFFF0000u) : (vsb << 16));
-    B[2 * qh] = movmatrix_trans(pack_f16x2_sat(p[0] * va, p[1] * va));
-    B[2 * qh + 1] = movmatrix_trans(pack_f16x2_sat(p[2] * vb, p[3] * vb));
+    float w[4];
+    unpair_f32(mul2(pair_f32(p[0], p[1]), pair_f32(va, va)), w[0], w[1]);
+    unpair_f32(mul2(pair_f32(p[2], p[3]), pair_f32(vb, vb)), w[2], w[3]);
+    B[2 * qh] = movmatrix_trans(pack_f16x2_sat(w[0], w[1]));
+    B[2 * qh + 1] = movmatrix_trans(pack_f16x2_sat(w[2], w[3]));
   }
 }
 // One page's (P * vscale).V into the output accumulators.  X = the page's V words, transposed so that a
 // register holds two tokens' halves: {tokens 0-7, tokens 8-15} of channel half 0, then of half 1.
-__device__ __forceinline__ void k3_values(float (&oacc)[10][4], const uint32_t (&B)[4], const uint32_t (&X)[4]) {
+__device__ __forceinline__ void k3_values(float (&oacc)[9][4], const uint32_t (&B)[4], const uint32_t (&X)[4]) {
 #pragma unroll
   for (int qh = 0; qh < 2; ++qh) {
     const uint32_t B0 = B[2 * qh], B1 = B[2 * qh + 1], XA = X[2 * qh], XB = X[2 * qh + 1];
@@ -208,7 +210,7 @@ __device__ __forceinline__ void k3_values(float (&oacc)[10][4], const uint32_t (
     mma_f16_nv(oacc[qh * 4 + 1], v2_field<4>(XA), v2_field<6>(XA), v2_field<4>(XB), v2_field<6>(XB), B0, B1);
     mma_f16_nv(oacc[qh * 4 + 2], v2_field<8>(XA), v2_field<0>(XA2), v2_field<8>(XB), v2_field<0>(XB2), B0, B1);
     mma_f16_nv(oacc[qh * 4 + 3], v2_field<2>(XA2), v2_field<4>(XA2), v2_field<2>(XB2), v2_field<4>(XB2), B0, B1);
-    mma_f16_nv(oacc[8 + qh], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
+    mma_f16_nv(oacc[8], qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, B0, B1);
   }
 }
 
@@ -335,7 +337,7 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
     st.l2 = mul2(st.l2, pair_f32(f0, f1));
     if (kDoV) {
 #pragma unroll
-      for (int i = 0; i < 10; ++i) { st.oacc[i][0] *= f0; st.oacc[i][1] *= f1; st.oacc[i][2] *= f0; st.oacc[i][3] *= f1; }
+      for (int i = 0; i < 9; ++i) { st.oacc[i][0] *= f0; st.oacc[i][1] *= f1; st.oacc[i][2] *= f0; st.oacc[i][3] *= f1; }
     }
     st.m_ref0 = n0; st.m_ref1 = n1;
   }
@@ -497,7 +499,7 @@ scan_k3v2_kernel(const ScanParams p) {
   }
   st.ks_sel = (tig >> 1) ? 0x3232u : 0x1010u;
 #pragma unroll
-  for (int i = 0; i < 10; ++i) { st.oacc[i][0] = st.oacc[i][1] = st.oacc[i][2] = st.oacc[i][3] = 0.f; }
+  for (int i = 0; i < 9; ++i) { st.oacc[i][0] = st.oacc[i][1] = st.oacc[i][2] = st.oacc[i][3] = 0.f; }
   st.m_ref0 = kMinusBig; st.m_ref1 = kMinusBig; st.l2 = 0ull;
   st.smax2 = 0u;
 
@@ -567,10 +569,10 @@ scan_k3v2_kernel(const ScanParams p) {
       const int da = 64 * qh + 8 * g + v2_dlocal(fa), db = 64 * qh + 8 * g + v2_dlocal(fb);
       // 2^(24 - POS) * sum(P * field) - 2 * sum(P): the codes' offset leaves here (see v2_field)
       const float ua = 16777216.0f / static_cast<float>(1 << v2_pos(fa)), ub = 16777216.0f / static_cast<float>(1 << v2_pos(fb));
-      wo[(2 * tig) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][0], ua, -2.0f * st.oacc[8 + qh][0]);
-      wo[(2 * tig + 1) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][1], ua, -2.0f * st.oacc[8 + qh][1]);
-      wo[(2 * tig) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][2], ub, -2.0f * st.oacc[8 + qh][2]);
-      wo[(2 * tig + 1) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][3], ub, -2.0f * st.oacc[8 + qh][3]);
+      wo[(2 * tig) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][0], ua, -2.0f * st.oacc[8][2 * qh]);
+      wo[(2 * tig + 1) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][1], ua, -2.0f * st.oacc[8][2 * qh + 1]);
+      wo[(2 * tig) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][2], ub, -2.0f * st.oacc[8][2 * qh]);
+      wo[(2 * tig + 1) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][3], ub, -2.0f * st.oacc[8][2 * qh + 1]);
     }
   }
   float l0, l1;
