@@ -71,6 +71,7 @@ __device__ __forceinline__ void merge_splits(const TailParams& p, SplitSums& out
   if (warp >= kSplitGroups) return;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
   float Z = 0.f;
+#pragma unroll 1
   for (int s = warp; s < splits; s += 2 * kSplitGroups) {
     const bool two = s + kSplitGroups < splits;
     const int64_t e0 = (pbase + s) * kHeadsPad + hi, e1 = two ? e0 + kSplitGroups * kHeadsPad : e0;
@@ -114,6 +115,7 @@ __device__ __forceinline__ void tail_part(const TailSmem<MODE>& sm, float* red, 
   const int e_a = (MODE == JF_MODE_K3V2) ? tig : ((2 * tig >> 2) & 1) | (((2 * tig >> 1) & 1) << 2) | ((2 * tig & 1) << 1);
   const int e_b = (MODE == JF_MODE_K3V2) ? tig + 4
                                          : (((2 * tig + 1) >> 2) & 1) | ((((2 * tig + 1) >> 1) & 1) << 2) | (((2 * tig + 1) & 1) << 1);
+#pragma unroll 1
   for (int grp = g0; 16 * grp < top_k; grp += step) {
     const int e0 = 16 * grp;   // entries past top_k have a place in the arrays and weigh nothing
     const uint8_t *ra = row(e0 + e_a), *rb = row(e0 + e_b), *rc = row(e0 + e_a + 8), *rd = row(e0 + e_b + 8);
@@ -205,6 +207,7 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
   const float* srow = p.scores + bh * p.max_S;
 
   // ---- selected set: weights from the scan's scores, 32 entries per warp and step ----
+#pragma unroll 1
   for (int k0 = 32 * warp; k0 < p.top_k; k0 += NT) {
     const int kk = k0 + lane;
     int ref = 0;
@@ -279,6 +282,7 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
     p.o_old[bh * JF_HEAD_DIM + tid] = acc_old * inv_z;
     float ws = 0.f;
     if (warp == 0) {
+#pragma unroll 1
       for (int i = lane; 32 * i < p.top_k; i += 32) ws += sm.sum[i];
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) ws += __shfl_xor_sync(0xFFFFFFFFu, ws, d);
@@ -297,6 +301,7 @@ template <int NT>
 __device__ __forceinline__ float block_max_of_splits(const float* part_m, int64_t pbase, int hi, int splits, float* red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float M = kMinusBig;
+#pragma unroll 1
   for (int s = tid; s < splits; s += NT) M = fmaxf(M, part_m[(pbase + s) * kHeadsPad + hi]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, o));

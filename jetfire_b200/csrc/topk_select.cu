@@ -26,6 +26,10 @@
 // One row alone on its multiprocessor, scan's end to output: 2048 positions 26.8 k -> 20.7 k cycles,
 // 32768 positions 30.9 k -> 24.7 k; 256 rows of 65536 (top-k 512): 60.0 k -> 54.2 k, bound by the
 // scattered reads of the candidates' rows (0.7 M accesses of 64 bytes a layer).
+// Run-time loops are not unrolled: they go round once or twice, by four with their remainders the kernel was
+// 153 KB of code, more than the instruction cache (111 KB now; a fused call of 32 rows of 2048: 16.3 -> 15.7 us,
+// K4V4 14.6 -> 13.6, 128 rows of 8192: 24.95 -> 24.6, 512 of 16384: 90.9 -> 89.5, steps of them 0.6-3 us less).
+// A third of the stalls of a row on its own multiprocessor still wait for instructions.
 #include <algorithm>
 
 #include "finish_tail.cuh"
@@ -297,6 +301,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         bulk_g2s(chunk, srow + static_cast<int64_t>(ci) * kChunkPos, static_cast<uint32_t>(cnt) * 4u, &sm.bar);
       }
     } else {
+#pragma unroll 1
       for (int i = tid; i < cnt; i += NT) chunk[i] = srow[static_cast<int64_t>(ci) * kChunkPos + i];
     }
   };
@@ -312,6 +317,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     const int valid = max(0, min(n - ci * kChunkPos, kChunkPos));
     if (!vec) __syncthreads();
     const int used = min((valid + 4 * NT - 1) / (4 * NT) * (4 * NT), kChunkPos);
+#pragma unroll 1
     for (int i = valid + tid; i < used; i += NT) chunk[i] = -INFINITY;
     return __syncthreads_and(ok ? 1 : 0) != 0;
   };
@@ -360,7 +366,9 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     if (lane == 0) sm.red[warp] = s1;
   }
   if (tid == 0) { sm.ncand = 0; sm.nlist = 0; sm.tbin = -1; }
+#pragma unroll 1
   for (int i = tid; i < kBins; i += NT) hist[i] = 0;
+#pragma unroll 1
   for (int i = tid; i < p.sort_n; i += NT) keys[i] = 0ull;
 
   // what this block reads first once the scan is done: warm the address translations now
@@ -390,6 +398,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   const int n_pages = (n_seq + 15) >> 4, n_groups = (n_pages + kGroupPages - 1) / kGroupPages;
   const float4* pm4 = reinterpret_cast<const float4*>(p.pmax + bh * p.np_stride);
   {
+#pragma unroll 1
     for (int s = tid + NT; s < n_splits; s += NT) {
       top = fmaxf(top, p.part_m[(pbase + s) * kHeadsPad + hi]);
       sm0 = fmaxf(sm0, p.part_smax[(pbase + s) * 2]);
@@ -442,6 +451,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
     if (n <= p.sort_n) {
       // short row: every position is a candidate
+#pragma unroll 1
       for (int i = tid; i < n; i += NT) { keys[i] = static_cast<uint64_t>(i); cand_score[i] = LEAN ? srow[i] : chunk[i]; }
       ncand = n;
     } else {
@@ -504,8 +514,10 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       bool have_hm = false;
       auto collect = [&](float thr, int kind, int off0, int cap) {
         int running = 0;  // candidates found so far
+#pragma unroll 1
         for (int ci = 0; ci < n_chunks; ++ci) {
           if (n_chunks > 1 && !LEAN) next_chunk(ci);
+#pragma unroll 1
           for (int j = 0; j < vecs_of(ci); ++j) {
             const int at = 4 * (j * NT + tid), pos = ci * kChunkPos + at;
             float e[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -571,6 +583,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       // on it), with no barrier but the last.  Returns how many there are; those past sort_n are dropped.
       auto collect_any = [&](float thr, bool use16) {
         const uint32_t thr16 = float_order_key(thr) >> 16;
+#pragma unroll 1
         for (int ci = 0; ci < n_chunks; ++ci) {
           if (n_chunks > 1 && !use16) next_chunk(ci);
           // which of the thread's float4s hold a candidate
@@ -589,6 +602,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           // The scan on a row of 2048: 0.6 k more, its dense hits being written one after the other; on one of
           // 32768 alone on its multiprocessor no difference but the code.)
           if (kChunkVec > 8 || vecs_of(ci) == 1) {
+#pragma unroll 1
             while (__any_sync(0xFFFFFFFFu, hits != 0u)) {
               const int j = hits ? __ffs(hits) - 1 : 0;
               const int pos = ci * kChunkPos + 4 * (j * NT + tid);
@@ -606,6 +620,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
             continue;
           }
           uint32_t mask = 0u;
+#pragma unroll 1
           while (hits) {
             const int j = __ffs(hits) - 1, pos = ci * kChunkPos + 4 * (j * NT + tid);
             hits &= hits - 1u;
@@ -625,6 +640,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           int base = 0;
           if (lane == 31) base = atomicAdd(&sm.ncand, incl);
           int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
+#pragma unroll 1
           while (mask) {
             const int e = __ffs(mask) - 1, at = 4 * ((e >> 2) * NT + tid) + (e & 3);
             mask &= mask - 1u;
@@ -646,6 +662,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       //      candidates than top_k, half the shared-memory atomics of four) while there are at least
       //      four per selected entry. ----
       const bool two = (n >= 4 * NT ? 2 * NT * max(1, n / kChunkPos) : n / 2) >= 4 * K;
+#pragma unroll 1
       for (int ci = 0; !LEAN && ci < n_chunks; ++ci) {
         if (ci > 0) next_chunk(ci);
         float gm[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -674,6 +691,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         // the groups are the scan's; their maxima came with it.  +inf marks a K4V4 page whose
         // maximum is not known (it is always fetched below) and does not count here; groups past
         // the sequence were never written.
+#pragma unroll 1
         for (int i4 = tid; 4 * i4 < n_groups; i4 += NT) {
           const float4 v = pm4[i4];
           const float e[4] = {v.x, v.y, v.z, v.w};
@@ -703,6 +721,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
             // fixed, the ranking below does not depend on it.
             uint16_t* page_list = perm;   // perm and bucket, contiguous: 2 * sort_n entries
             const int list_cap = 2 * p.sort_n;
+#pragma unroll 1
             for (int b4 = 0; 4 * b4 < n_groups; b4 += NT) {   // the same trip count for every thread
               const int i4 = b4 + tid;
               uint32_t flags = 0u;   // kGroupPages bits per group: its pages that exist
@@ -726,6 +745,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
               int base = 0;
               if (lane == 31 && incl > 0) base = atomicAdd(&sm.nlist, incl);
               int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
+#pragma unroll 1
               while (flags) {
                 const int i = __ffs(flags) - 1;   // bit i: page kGroupPages * 4 * i4 + i
                 flags &= flags - 1u;
@@ -741,13 +761,16 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
               // there is no barrier in between.
               float4* stage = reinterpret_cast<float4*>(smem_raw);
               constexpr int kStageCap = static_cast<int>(sizeof(SelSmemLate<MODE>) / 64);
+#pragma unroll 1
               for (int b0 = 0; b0 < n_list; b0 += kStageCap) {
                 const int nq = 4 * min(kStageCap, n_list - b0);
+#pragma unroll 1
                 for (int u = tid; u < nq; u += NT)
                   cp_async_16(stage + u, srow + 16 * static_cast<int>(page_list[b0 + (u >> 2)]) + 4 * (u & 3));
                 cp_async_commit();
                 cp_async_wait_all();
                 // eight quarters of a lane at a time, four bits each: one scan and one atomic for them all
+#pragma unroll 1
                 for (int u0 = tid; u0 - lane < nq; u0 += 8 * NT) {   // warp-uniform trip count
                   uint32_t mask = 0u;
 #pragma unroll
@@ -771,6 +794,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
                   int base = 0;
                   if (lane == 31) base = atomicAdd(&sm.ncand, incl);
                   int o = __shfl_sync(0xFFFFFFFFu, base, 31) + incl - cnt;
+#pragma unroll 1
                   while (mask) {
                     const int e = __ffs(mask) - 1, u = u0 + (e >> 2) * NT;
                     mask &= mask - 1u;
@@ -804,13 +828,16 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         have_hm = false;
         uint32_t prefix = 0u;
         int want = K;
+#pragma unroll 1
         for (int level = 0; level < 3; ++level) {
           const int bits = (level == 2) ? 10 : 11, shift = (level == 0) ? 21 : (level == 1) ? 10 : 0;
           const uint32_t dmask = (1u << bits) - 1u;
           __syncthreads();
           if (tid == 0) sm.tbin = -1;
+#pragma unroll 1
           for (int i = tid; i < kBins; i += NT) hist[i] = 0;
           __syncthreads();
+#pragma unroll 1
           for (int ci = 0; ci < n_chunks; ++ci) {
             if (n_chunks > 1 && !LEAN) next_chunk(ci);
             const int jn = vecs_of(ci);
@@ -848,6 +875,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         }
         const float kth = float_from_order_key(prefix);   // the K-th largest approximate score
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < p.sort_n; i += NT) keys[i] = 0ull;
         __syncthreads();
         if (MODE == JF_MODE_K4V4) {
@@ -873,12 +901,14 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
     // the fused finish stage takes slots, scores and V rows of the candidates from shared memory
     prefetch = FUSED && !slow && ncand <= kRowChunk && p.sort_n <= kSelThreads;
+#pragma unroll 1
     for (int i = tid; i < kBins; i += NT) hist[i] = 0;   // for the ranking
     if (!slow) {
       // ---- re-score the candidates canonically.  Every warp works on its own: four candidates per round,
       //      their slots, the copies of their packed rows into shared memory, the canonical
       //      arithmetic -- no barrier until all are done, so one warp's wait for memory is not
       //      every warp's. ----
+#pragma unroll 1
       for (int base = 0; base < ncand; base += kRowChunk) {
         const int cn = min(kRowChunk, ncand - base);
         const int rounds = (cn + 4 * kW - 1) / (4 * kW);
@@ -896,6 +926,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           if (any) late.cand_slot[c] = static_cast<int32_t>(blk < 0 || blk >= (ctx.num_slots >> 4) ? -1 : blk * 16 + (pos & 15));
           i0 += 32;
         }
+#pragma unroll 1
         for (int i = i0; i < 4 * rounds; i += 32) {
           const int c = cand_of(i);
           if (c < cn) late.cand_slot[c] = static_cast<int32_t>(slot_of(ctx, static_cast<int>(keys[base + c])));
@@ -915,6 +946,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         const uint16_t* v_sc = tp.v_scales + static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots * mi.ng;
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
+#pragma unroll 1
           for (int i = 4 * g * per + (lane >> 2); i < 4 * min((g + 1) * per, rounds); i += 8) {
             const int c = cand_of(i);
             if (c >= cn) continue;
@@ -942,6 +974,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         if (MODE == JF_MODE_K4V4) {
           // K4: the scan's score is the canonical one bit for bit (exact integer dot products,
           // the same fp32 rescale order), so nothing is recomputed
+#pragma unroll 1
           for (int i = lane; i < 4 * rounds; i += 32) {
             const int c = cand_of(i);
             if (c < cn) keys[base + c] = make_key(late.cand_slot[c] >= 0 ? cand_score[base + c] : -INFINITY, static_cast<int>(keys[base + c]));
@@ -958,6 +991,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
             else if (g == 1) cp_async_wait_group<kGroups - 2>();
             else cp_async_wait_group<0>();
             __syncwarp();
+#pragma unroll 1
             for (int r = g * per; r < min((g + 1) * per, rounds); ++r) {
               const int c = cand_of(4 * r + (lane >> 3)), cc = min(c, cn - 1);   // lanes past the end keep the shuffles company
               const float s = canon_score_k3_x8(qv, late.rows + cc * W, ctx.attn, lane);
@@ -972,10 +1006,13 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       // ---- slow exact path: 8-level radix select on the 64-bit canonical key ----
       if (tid == 0) { sm.prefix = 0ull; sm.remaining = K; sm.ncand = 0; }
       __syncthreads();
+#pragma unroll 1
       for (int level = 7; level >= 0; --level) {
+#pragma unroll 1
         for (int i = tid; i < 256; i += NT) hist[i] = 0;
         __syncthreads();
         const unsigned long long prefix = sm.prefix;
+#pragma unroll 1
         for (int i = warp; i < n; i += kW) {
           const uint64_t key = canon_key_global<MODE>(ctx, i, lane);
           const bool match = (level == 7) || ((key >> (8 * (level + 1))) == prefix);
@@ -984,6 +1021,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         __syncthreads();
         if (tid == 0) {
           int cum = 0, rem = sm.remaining, cb = 0;
+#pragma unroll 1
           for (int bin = 255; bin >= 0; --bin) {
             if (cum + hist[bin] >= rem) { cb = bin; break; }
             cum += hist[bin];
@@ -994,8 +1032,10 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         __syncthreads();
       }
       const unsigned long long tkey = sm.prefix;  // key of the k-th best; keys are unique
+#pragma unroll 1
       for (int i = tid; i < p.sort_n; i += NT) keys[i] = 0ull;
       __syncthreads();
+#pragma unroll 1
       for (int i = warp; i < n; i += kW) {
         const uint64_t key = canon_key_global<MODE>(ctx, i, lane);
         if (key >= tkey && lane == 0) {
@@ -1018,10 +1058,12 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       // The keys stay where they are; perm[rank] names them.
       constexpr int kCand = kSelThreads / NT;
       int f = 1;
+#pragma unroll 1
       while (f < 16 && (cand_last + 2) * f * 2 <= kBins) f *= 2;
       const float fscale = kBinsPerUnit * static_cast<float>(f);
       const float ftop = (row_max + 4.0f) * fscale;
       if (slow) {   // its passes used the bins
+#pragma unroll 1
         for (int i = tid; i < kBins; i += NT) hist[i] = 0;
         __syncthreads();
       }
@@ -1072,6 +1114,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         if (c < ncand) {
           const int lo = hist[fb[k]], hi2 = (fb[k] == kBins - 1) ? ncand : hist[fb[k] + 1];
           int above = 0;
+#pragma unroll 1
           for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
           perm[min(lo + above, ncand - 1)] = static_cast<uint16_t>(c);
         }
@@ -1079,10 +1122,14 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       __syncthreads();
     } else {
       // bitonic sort, descending, sort_n a power of two
+#pragma unroll 1
       for (int i = ncand + tid; i < p.sort_n; i += NT) keys[i] = 0ull;
       __syncthreads();
+#pragma unroll 1
       for (int size = 2; size <= p.sort_n; size <<= 1) {
+#pragma unroll 1
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
+#pragma unroll 1
           for (int i = tid; i < (p.sort_n >> 1); i += NT) {
             const int lo = 2 * i - (i & (stride - 1));
             const int hi2 = lo + stride;
@@ -1099,6 +1146,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
   auto pos_of_key = [&](int c) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(keys[c] & 0xFFFFFFFFull)); };
+#pragma unroll 1
   for (int r = tid; r < K; r += NT) {
     int64_t idx = -1, slot = -1;
     if (r < m_sel) {

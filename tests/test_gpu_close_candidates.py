@@ -1,0 +1,50 @@
+"""K3V2 rows that share a multiprocessor (more rows than there are): of a row's candidates only those whose scan
+scores are close to another one's are re-scored.  Lists must still be the oracle's where scores tie, crowd
+together or are so large that every candidate is re-scored, and name positions of the row whatever the scores are."""
+import pytest
+import torch
+
+from jf_testlib import Case
+from test_gpu_long_rows import _run
+
+pytestmark = pytest.mark.gpu
+B, H_Q, H_KV = 5, 32, 2    # 160 rows
+
+
+def _few_keys(case, distinct, jitter=0.0):
+    g = torch.Generator().manual_seed(3)
+    rows = case.k_full[:, torch.randperm(case.num_slots, generator=g)[:distinct]]
+    k = rows[:, torch.randint(0, distinct, (case.num_slots,), generator=g)].float()
+    case.k_full = (k * (1.0 + jitter * torch.randn(k.shape[:2] + (1,), generator=g))).to(case.dtype).contiguous()
+    return case
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("ctx,top_k", [(1600, 256), (1601, 64), (17008, 128)])
+def test_lists_are_the_oracles(dtype, ctx, top_k):
+    _run(Case("k3v2", B, H_Q, H_KV, ctx, lens=[ctx, ctx - 1, 513, 512, 33], seed=ctx, dtype=dtype), top_k)
+
+
+@pytest.mark.parametrize("distinct,jitter", [(40, 0.0), (8, 1e-3), (700, 0.0)])
+def test_ties_and_crowds(distinct, jitter):
+    _run(_few_keys(Case("k3v2", B, H_Q, H_KV, 2000, seed=4), distinct, jitter), 128)
+
+
+def test_scores_whose_band_spans_bins():
+    case = Case("k3v2", B, H_Q, H_KV, 1500, seed=5)
+    case.k_full = (case.k_full.float() * 300.0).to(case.dtype)
+    _run(case, 128)
+
+
+def test_scores_of_another_cache_select_positions_of_the_row():
+    from jetfire_b200 import ops
+    calls = []
+    for seed in (6, 7):
+        c = Case("k3v2", B, H_Q, H_KV, 1600, seed=seed)
+        calls.append(ops.DecodeCall("k3v2", c.q.cuda(), *c.device_cache(), c.block_table.cuda(), c.seq_lens.cuda(), c.ctx, H_Q, H_KV, 16,
+                                    256, c.attn_scale))
+    calls[0].scan()              # both calls use the stream's workspace
+    calls[1].select_finish()
+    idx = calls[1].out["topk_idx"].cpu()
+    lens = c.seq_lens[:, None, None]
+    assert ((idx >= 0) & (idx < lens)).all()
