@@ -12,7 +12,7 @@
 //   2. every position whose approximate score can still beat it -- bins <= T + ceil(2*delta*64)
 //      + 1, with delta a bound on |approximate - canonical| (fp32 summation-order error only,
 //      the scan dequantises with the reference's rounding) -- is re-scored in the canonical
-//      arithmetic, and the k best by (canonical score desc, position asc) are emitted in
+//      arithmetic (or only those of them whose order the scan's scores leave open), and the k best by (canonical score desc, position asc) are emitted in
 //      that order.
 // The result is reproducible by a CPU and independent of tensor-core internals.  If the
 // band does not fit the sort buffer (massive ties, degenerate scales) a slow exact path
@@ -40,6 +40,7 @@ namespace {
 
 constexpr int kBins = 2048;
 constexpr float kBinsPerUnit = 64.0f;
+constexpr int kCloseTopK = 256;   // see launch_select_block
 
 struct TopkParams {
   const float* scores;
@@ -117,13 +118,12 @@ __device__ __forceinline__ float canon_score_k3(const float* q, const uint8_t* r
 // a single rounding, and a power of two commutes with it (K scales between 2^-93 and 2^27, or
 // zero -- the scan's dequantisation rests on the same identity).  `qv[4 r + m]` =
 // 2^33 * q[32 r + 8 m + sub], so every product is the exact q * k_hat of the canonical order.
+// `hi4`, `lo4`: the two planes of the lane's window (b0, b1 or b1, b2); `sw`: the two bf16 group scales.
 // Every lane of the warp must call this; lanes of a candidate get the same value.
-__device__ __forceinline__ float canon_score_k3_x8(const float (&qv)[16], const uint32_t* row, float attn, int lane) {
+__device__ __forceinline__ float canon_score_k3_x8(const float (&qv)[16], uint4 hi4, uint4 lo4, uint32_t sw, float attn, int lane) {
   const int sub = lane & 7;
   const bool early = sub <= 4;
-  const uint4 hi4 = *reinterpret_cast<const uint4*>(row + (early ? 0 : 4)), lo4 = *reinterpret_cast<const uint4*>(row + (early ? 4 : 8));
   const uint32_t hv[4] = {hi4.x, hi4.y, hi4.z, hi4.w}, lv[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
-  const uint32_t sw = row[12];
   const uint32_t sc0 = prmt(sw, sw, 0x1010u), sc1 = prmt(sw, sw, 0x3232u);   // each group scale in both halves
   const uint32_t S0 = mul_bf16x2(sc0, 0x71807180u), C0 = mul_bf16x2(sc0, 0xB000B000u);   // * 2^100, * -2^-31
   const uint32_t S1 = mul_bf16x2(sc1, 0x71807180u), C1 = mul_bf16x2(sc1, 0xB000B000u);
@@ -146,6 +146,12 @@ __device__ __forceinline__ float canon_score_k3_x8(const float (&qv)[16], const 
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xFFFFFFFFu, t, o));
   return __fmul_rn(t, attn);
+}
+
+// The `qv` of canon_score_k3_x8.
+__device__ __forceinline__ void canon_query(float (&qv)[16], const float* q, int lane) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) qv[i] = q[32 * (i >> 2) + 8 * (i & 3) + (lane & 7)] * 8589934592.0f;   // 2^33
 }
 
 // Canonical K4/G128 score (jetfire_vllm/csrc/int8tc_qk_scores.cu:445-487): exact int32 dot per
@@ -173,6 +179,8 @@ __device__ __forceinline__ uint64_t make_key(float s, int pos) {
   return (static_cast<uint64_t>(float_order_key(s)) << 32) | (0xFFFFFFFFu - static_cast<uint32_t>(pos));
 }
 
+__device__ __forceinline__ int pos_of(uint64_t key) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(key & 0xFFFFFFFFull)); }
+
 // Key of a position straight from global memory (slow exact path only), whole warp.
 template <int MODE>
 __device__ __forceinline__ uint64_t canon_key_global(const RowCtx& c, int pos, int lane) {
@@ -198,8 +206,7 @@ __device__ __forceinline__ int score_bin(float top64, float s) {
 
 // candidates staged in shared memory per round: a top-k of 512 and its band in one (K4V4 has no band to speak of)
 template <int MODE> struct RowChunk { static constexpr int v = (MODE == JF_MODE_K3V2) ? 768 : 576; };
-// 32-bit words per staged K row: K3V2 holds 12 of data and one of scales in a 64-byte slot (16-byte copies land aligned)
-template <int MODE> struct RowWords { static constexpr int v = 16; };
+constexpr int kRowWords = 12;   // 32-bit words per staged K row (K3V2)
 
 struct SelSmemFixed {
   SplitSums splits;           // the scan's partials of the row, merged
@@ -221,11 +228,13 @@ template <int MODE>
 struct SelSmemLate {
   union {   // the K rows are done with (canonical scores) before the finish stage starts
     TailSmem<MODE> tail;
-    uint32_t rows[(MODE == JF_MODE_K3V2) ? RowChunk<MODE>::v * RowWords<MODE>::v : 4];   // K3V2: packed K rows + scales (K4V4 re-scores nothing)
+    uint32_t rows[(MODE == JF_MODE_K3V2) ? RowChunk<MODE>::v * kRowWords : 4];   // K3V2: packed K rows (K4V4 re-scores nothing)
   };
   uint32_t vrows[RowChunk<MODE>::v * TailSmem<MODE>::VW];  // packed V rows of the candidates (fused kernel)
   int32_t cand_slot[RowChunk<MODE>::v];                    // slots fit 32 bits (see validate_decode_args)
   uint32_t vsc[RowChunk<MODE>::v];                         // V scales
+  uint32_t ksc[(MODE == JF_MODE_K3V2) ? RowChunk<MODE>::v : 4];   // K scales
+  uint16_t close[(MODE == JF_MODE_K3V2) ? kSelThreads : 4];       // candidates whose order their scan scores leave open
 };
 
 __host__ __device__ constexpr size_t hm_chunk_bytes(int nt, int vec) { return static_cast<size_t>(vec) * nt * 2; }   // side table of one chunk
@@ -249,6 +258,7 @@ __host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, 
 // shared memory by one bulk copy per 32768 positions, issued before anything else so that
 // the prologue runs under it; every later pass over the scores reads shared memory.
 // FUSED: the finish stage follows in the same kernel.
+// CLOSE (K3V2): candidates are re-scored only where the order needs it.
 // LEAN (K3V2, long rows): the scores are never staged.  The scan left the largest score of every
 // pair of 16-token pages next to them; the threshold comes from a histogram of those maxima (the
 // K-th largest of them is a lower bound of the K-th largest score), and only the pairs whose
@@ -259,13 +269,12 @@ __host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, 
 // are enough to hide the memory: 512 threads -- with VEC 8 two blocks share a multiprocessor, so
 // that one row's round trips run under the other's arithmetic -- and 1024 only for sort buffers
 // beyond 1024 entries, which are sorted by all threads.
-template <int MODE, int DT, bool FUSED, bool LEAN, int NT, int VEC>
+template <int MODE, bool FUSED, bool LEAN, int NT, int VEC, bool CLOSE>
 __global__ void __launch_bounds__(NT, (NT == 512 && VEC == 8) ? 2 : 1)
 topk_select_kernel(const TopkParams p, const TailParams tp) {
   constexpr int kW = NT / 32;                   // warps of this block
   constexpr int kChunkVec = VEC;
   constexpr int kChunkPos = 4 * kChunkVec * NT; // positions per pass over a chunk
-  constexpr int W = RowWords<MODE>::v;         // 32-bit words staged per candidate: data + scales
   constexpr int kRowChunk = RowChunk<MODE>::v;
   extern __shared__ __align__(128) uint8_t smem_raw[];
   float* chunk = reinterpret_cast<float*>(smem_raw);
@@ -339,7 +348,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   int32_t* out_slot32 = p.topk_slots_i32 ? p.topk_slots_i32 + bh * K : nullptr;
 
   // ---- query row (exact values), per-group L1 norms, INT8 model for K4 ----
-  if (tid < JF_HEAD_DIM) sm.q[tid] = Elem<DT>::to_f32(q_bits);
+  if (tid < JF_HEAD_DIM) sm.q[tid] = p.q_dtype == JF_DTYPE_BF16 ? Elem<JF_DTYPE_BF16>::to_f32(q_bits) : Elem<JF_DTYPE_FP16>::to_f32(q_bits);
   if (warp == kW - 1) {
     int first, count;
     slice_partials(p.geom, p.seq_lens, p.B, p.max_S, hkv, b, lane, first, count);
@@ -443,11 +452,22 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 
   int m_sel = 0;  // entries of keys[] that hold the ranked result
   bool prefetch = false, merged = false;
-  const bool by_rank = p.sort_n <= kSelThreads;   // the result is perm[]: rank -> entry of keys[]; else keys[] itself is sorted
+  constexpr bool by_rank = NT != kSelThreads;   // (sort_n <= 1024) the result is perm[]: rank -> entry of keys[]; else keys[] itself is sorted
   if (n > 0) {
     int ncand = 0;
     int cand_last = kBins;  // bound on the candidates' canonical-score bin, when one is known
     bool slow = false;
+    float delta = 0.f;
+    if (MODE == JF_MODE_K3V2) {
+      // The scan and the canonical order add the same exact products q_d * k_hat_d in fp32,
+      // in different orders: each stays within (roundings) * 2^-24 * sum|q_d k_hat_d| of the
+      // exact sum (canonical: 9 roundings; tensor core: one per k-step, 8, possibly
+      // truncating).  sum|q_d k_hat_d| <= sum_g 3 * scale_g * sum_{d in g} |q_d|.  A factor 32
+      // covers both paths with slack; the last term covers the final multiply by attn_scale.
+      const float q1a = sm.red[0] + sm.red[1], q1b = sm.red[2] + sm.red[3];
+      const float mag = fabsf(p.attn_scale) * (over_warps(sm.w3[1], 0.f) * q1a + over_warps(sm.w3[2], 0.f) * q1b) * 3.0f;
+      delta = mag * (32.0f / 16777216.0f) + mag * (4.0f / 16777216.0f) + 1e-7f;
+    }
 
     if (n <= p.sort_n) {
       // short row: every position is a candidate
@@ -457,17 +477,6 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     } else {
       const float top = row_max + 4.0f;  // the scan lets its reference point lag the true maximum by at most 4
       const float top64 = top * kBinsPerUnit;
-      float delta = 0.f;
-      if (MODE == JF_MODE_K3V2) {
-        // The scan and the canonical order add the same exact products q_d * k_hat_d in fp32,
-        // in different orders: each stays within (roundings) * 2^-24 * sum|q_d k_hat_d| of the
-        // exact sum (canonical: 9 roundings; tensor core: one per k-step, 8, possibly
-        // truncating).  sum|q_d k_hat_d| <= sum_g 3 * scale_g * sum_{d in g} |q_d|.  A factor 32
-        // covers both paths with slack; the last term covers the final multiply by attn_scale.
-        const float q1a = sm.red[0] + sm.red[1], q1b = sm.red[2] + sm.red[3];
-        const float mag = fabsf(p.attn_scale) * (over_warps(sm.w3[1], 0.f) * q1a + over_warps(sm.w3[2], 0.f) * q1b) * 3.0f;
-        delta = mag * (32.0f / 16777216.0f) + mag * (4.0f / 16777216.0f) + 1e-7f;
-      }
       float nbf = ceilf(2.0f * delta * kBinsPerUnit) + 1.0f;
       if (!(nbf < 4096.0f)) nbf = 4096.0f;
       const int nb = (MODE == JF_MODE_K3V2) ? static_cast<int>(nbf) : 0;  // K4: scan scores are canonical
@@ -900,13 +909,16 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     __syncthreads();   // every read of the score chunk is done: its memory is reused from here on
 
     // the fused finish stage takes slots, scores and V rows of the candidates from shared memory
-    prefetch = FUSED && !slow && ncand <= kRowChunk && p.sort_n <= kSelThreads;
+    prefetch = FUSED && by_rank && !slow && ncand <= kRowChunk;
+    // K3V2: every candidate's canonical score ahead of the ranking, or only where the ranking needs it (see there)
+    const float band = 2.002f * delta;
+    const bool rescore_all = MODE == JF_MODE_K3V2 && (!CLOSE || !(band * kBinsPerUnit <= 0.5f));
 #pragma unroll 1
     for (int i = tid; i < kBins; i += NT) hist[i] = 0;   // for the ranking
     if (!slow) {
-      // ---- re-score the candidates canonically.  Every warp works on its own: four candidates per round,
-      //      their slots, the copies of their packed rows into shared memory, the canonical
-      //      arithmetic -- no barrier until all are done, so one warp's wait for memory is not
+      // ---- the candidates' slots, and copies of what later phases read of their rows: V rows and scales, and the packed
+      //      K rows where all candidates are re-scored canonically.  Every warp works on
+      //      its own, four candidates per round -- no barrier until all are done, so one warp's wait for memory is not
       //      every warp's. ----
 #pragma unroll 1
       for (int base = 0; base < ncand; base += kRowChunk) {
@@ -914,8 +926,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         const int rounds = (cn + 4 * kW - 1) / (4 * kW);
         auto cand_of = [&](int i) { return (i >> 2) * (4 * kW) + 4 * warp + (i & 3); };   // the warp's i-th candidate
         int i0 = lane;
-        if (FUSED && MODE == JF_MODE_K4V4 && !merged) {
-          // K4V4 has no scores to compute under the copies: the merge of the scan's partials runs while the block
+        if (FUSED && !rescore_all && !merged) {
+          // no scores to compute under the copies: the merge of the scan's partials runs while the block
           // ids of the first 32 candidates are on their way
           const int c = cand_of(lane);
           const bool any = lane < 4 * rounds && c < cn;
@@ -932,9 +944,8 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           if (c < cn) late.cand_slot[c] = static_cast<int32_t>(slot_of(ctx, static_cast<int>(keys[base + c])));
         }
         __syncwarp();
-        // Packed K rows and scales (K3V2) and, when the finish stage will use them, V rows and scales, as
-        // asynchronous 16- and 4-byte copies, four lanes per candidate, in kGroups groups of rounds.
-        // The canonical scores of a group are computed while the later ones are on their way.  (A candidate
+        // Asynchronous 16- and 4-byte copies, four lanes per candidate, in kGroups groups of rounds: the canonical scores
+        // of a group are computed while the later ones are on their way.  (A candidate
         // without a slot copies nothing and gets zeros.)
         constexpr int kGroups = 3;
         constexpr int VW = TailSmem<MODE>::VW;
@@ -947,16 +958,15 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 #pragma unroll
         for (int g = 0; g < kGroups; ++g) {
 #pragma unroll 1
-          for (int i = 4 * g * per + (lane >> 2); i < 4 * min((g + 1) * per, rounds); i += 8) {
+          for (int i = 4 * g * per + (lane >> 2); (rescore_all || prefetch) && i < 4 * min((g + 1) * per, rounds); i += 8) {
             const int c = cand_of(i);
             if (c >= cn) continue;
             const int32_t slot32 = late.cand_slot[c];
             const bool have = slot32 >= 0;
             const uint32_t slot = have ? static_cast<uint32_t>(slot32) : 0u;
-            if (MODE == JF_MODE_K3V2) {
-              uint32_t* r = late.rows + c * W;
-              if (part < 3) cp_async_16_zfill(r + 4 * part, k_src + static_cast<uint64_t>(slot) * 48u, have);
-              else cp_async_4_zfill(r + 12, ctx.k_sc + static_cast<uint64_t>(slot) * 2u, have);
+            if (rescore_all) {
+              if (part < 3) cp_async_16_zfill(late.rows + c * kRowWords + 4 * part, k_src + static_cast<uint64_t>(slot) * 48u, have);
+              else cp_async_4_zfill(&late.ksc[c], ctx.k_sc + static_cast<uint64_t>(slot) * 2u, have);
             }
             if (prefetch) {
               if (part < kVParts) cp_async_16_zfill(late.vrows + c * VW + 4 * part, v_src + static_cast<uint64_t>(slot) * (16u * kVParts), have);
@@ -971,19 +981,21 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           merge_splits(tp, sm.splits, pbase, n_splits, hi, row_max);
           merged = true;
         }
-        if (MODE == JF_MODE_K4V4) {
-          // K4: the scan's score is the canonical one bit for bit (exact integer dot products,
-          // the same fp32 rescale order), so nothing is recomputed
+        if (!rescore_all) {
+          // K4V4: the scan's score is the canonical one bit for bit (exact integer dot products,
+          // the same fp32 rescale order).  K3V2: it orders the candidates but for those that are close, see below.
 #pragma unroll 1
           for (int i = lane; i < 4 * rounds; i += 32) {
             const int c = cand_of(i);
-            if (c < cn) keys[base + c] = make_key(late.cand_slot[c] >= 0 ? cand_score[base + c] : -INFINITY, static_cast<int>(keys[base + c]));
+            if (c < cn) {
+              if (late.cand_slot[c] < 0) cand_score[base + c] = -INFINITY;
+              keys[base + c] = make_key(cand_score[base + c], static_cast<int>(keys[base + c]));
+            }
           }
         } else {
           // eight lanes per candidate, four candidates per warp and round
           float qv[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) qv[i] = sm.q[32 * (i >> 2) + 8 * (i & 3) + (lane & 7)] * 8589934592.0f;   // 2^33, see canon_score_k3_x8
+          canon_query(qv, sm.q, lane);
 #pragma unroll
           for (int g = 0; g < kGroups; ++g) {
             // groups 0..g have landed once at most (kGroups - 1 - g) are in flight
@@ -994,7 +1006,9 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
 #pragma unroll 1
             for (int r = g * per; r < min((g + 1) * per, rounds); ++r) {
               const int c = cand_of(4 * r + (lane >> 3)), cc = min(c, cn - 1);   // lanes past the end keep the shuffles company
-              const float s = canon_score_k3_x8(qv, late.rows + cc * W, ctx.attn, lane);
+              const uint32_t* row = late.rows + cc * kRowWords + ((lane & 7) <= 4 ? 0 : 4);
+              const float s = canon_score_k3_x8(qv, *reinterpret_cast<const uint4*>(row), *reinterpret_cast<const uint4*>(row + 4), late.ksc[cc],
+                                                ctx.attn, lane);
               if (c < cn && (lane & 7) == 0)
                 keys[base + c] = make_key(late.cand_slot[c] >= 0 ? s : -INFINITY, static_cast<int>(keys[base + c]));
             }
@@ -1051,15 +1065,21 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     // ---- order the candidates: best first ----
     if (by_rank) {
       // Rank by buckets: a candidate's rank is the number of candidates in finer score bins
-      // above its own plus the number of larger keys inside its bin.  Bins are `f` times finer
-      // than the selection histogram's (the candidates span few of those); a larger canonical
-      // score never lands in a later bin, so the result is the exact order of the keys, and
+      // above its own plus the number of better ones inside its bin.  Bins are `f` times finer
+      // than the selection histogram's (the candidates span few of those); a larger
+      // score never lands in a later bin, so the result is the exact order, and
       // crowded bins (massive ties) only cost time.  A thread owns candidates tid, tid + NT, ...
       // The keys stay where they are; perm[rank] names them.
+      //
+      // K3V2: a scan score is within delta of the canonical one, so two candidates whose scan scores are more
+      // than 2 delta apart have the canonical order already.  With CLOSE (launch_select_block) only those that are closer
+      // to another one are re-scored, straight from the cache: at a top-k of 64 / 128 / 256 / 512 of a row that is about
+      // 6 / 12 / 25 / 45 % of them, and their packed K rows are half of a row's scattered DRAM accesses.
       constexpr int kCand = kSelThreads / NT;
+      const bool open = CLOSE && !slow && !rescore_all;   // ordered by scan scores, the close ones looked at again
       int f = 1;
 #pragma unroll 1
-      while (f < 16 && (cand_last + 2) * f * 2 <= kBins) f *= 2;
+      while (f < 16 && (cand_last + 2) * f * 2 <= kBins && (!open || band * (kBinsPerUnit * 2 * f) <= 0.5f)) f *= 2;
       const float fscale = kBinsPerUnit * static_cast<float>(f);
       const float ftop = (row_max + 4.0f) * fscale;
       if (slow) {   // its passes used the bins
@@ -1067,6 +1087,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         for (int i = tid; i < kBins; i += NT) hist[i] = 0;
         __syncthreads();
       }
+      if (tid == 0) sm.nlist = 0;
       unsigned long long mine[kCand];
       int fb[kCand], arrival[kCand];
 #pragma unroll
@@ -1074,6 +1095,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         const int c = tid + k * NT;
         mine[k] = 0ull; fb[k] = 0; arrival[k] = 0;
         if (c < ncand) {
+          perm[c] = static_cast<uint16_t>(c);   // a candidate whatever the ranks are: scores of another call's cache have no order
           mine[k] = keys[c];
           const float sc = float_from_order_key(static_cast<uint32_t>(mine[k] >> 32));
           const float x = fminf(fmaxf(fmaf(sc, -fscale, ftop), 0.0f), static_cast<float>(kBins - 1));
@@ -1108,18 +1130,70 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
         if (c < ncand) bucket[hist[fb[k]] + arrival[k]] = static_cast<uint16_t>(c);
       }
       __syncthreads();
+      bool left[kCand];   // the order of this candidate is open
 #pragma unroll
       for (int k = 0; k < kCand; ++k) {
         const int c = tid + k * NT;
+        left[k] = false;
         if (c < ncand) {
-          const int lo = hist[fb[k]], hi2 = (fb[k] == kBins - 1) ? ncand : hist[fb[k] + 1];
+          // the bins that can hold a close candidate: one more on either side
+          const int b0 = open ? max(fb[k] - 1, 0) : fb[k], b1 = open ? fb[k] + 2 : fb[k] + 1;
+          const int lo = hist[b0], hi2 = b1 >= kBins ? ncand : hist[b1];
           int above = 0;
+          if (open) {
+            const float sc = cand_score[c];
 #pragma unroll 1
-          for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
-          perm[min(lo + above, ncand - 1)] = static_cast<uint16_t>(c);
+            for (int m = lo; m < hi2; ++m) {
+              const int o = bucket[m];
+              const float so = cand_score[o];
+              above += so > sc ? 1 : 0;
+              left[k] |= o != c && !(fabsf(so - sc) > band);
+            }
+            left[k] &= lo < K;   // a rank past the last one is as good as any other
+          } else {
+#pragma unroll 1
+            for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
+          }
+          if (left[k]) late.close[atomicAdd(&sm.nlist, 1)] = static_cast<uint16_t>(c);
+          else perm[min(lo + above, ncand - 1)] = static_cast<uint16_t>(c);
         }
       }
       __syncthreads();
+      if (open && sm.nlist > 0) {
+        // canonical keys, eight lanes a candidate
+        float qv[16];
+        canon_query(qv, sm.q, lane);
+        const int count = sm.nlist;
+#pragma unroll 1
+        for (int r = 4 * warp; r < count; r += 4 * kW) {
+          const int i = min(r + (lane >> 3), count - 1), c = late.close[i], pos = pos_of(keys[c]);
+          const int64_t slot = prefetch ? static_cast<int64_t>(late.cand_slot[c]) : slot_of(ctx, pos);
+          const uint64_t at = slot >= 0 ? static_cast<uint64_t>(slot) : 0ull;
+          const uint4* src = reinterpret_cast<const uint4*>(ctx.k_rows + at * 48u) + ((lane & 7) <= 4 ? 0 : 1);
+          const float sc = canon_score_k3_x8(qv, __ldg(src), __ldg(src + 1), __ldg(reinterpret_cast<const uint32_t*>(ctx.k_sc + at * 2u)), ctx.attn, lane);
+          __syncwarp();   // the lanes have read the position
+          if ((lane & 7) == 0 && r + (lane >> 3) < count) keys[c] = make_key(slot >= 0 ? sc : -INFINITY, pos);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kCand; ++k) {
+          const int c = tid + k * NT;
+          if (left[k]) {
+            const int lo = hist[max(fb[k] - 1, 0)], hi2 = fb[k] + 2 >= kBins ? ncand : hist[fb[k] + 2];
+            const float sc = cand_score[c];
+            const uint64_t key = keys[c];
+            int above = 0;
+#pragma unroll 1
+            for (int m = lo; m < hi2; ++m) {
+              const int o = bucket[m];
+              const float so = cand_score[o];
+              above += (fabsf(so - sc) > band ? so > sc : keys[o] > key) ? 1 : 0;   // both canonical if they are close
+            }
+            perm[min(lo + above, ncand - 1)] = static_cast<uint16_t>(c);
+          }
+        }
+        __syncthreads();
+      }
     } else {
       // bitonic sort, descending, sort_n a power of two
 #pragma unroll 1
@@ -1145,7 +1219,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
   }
 
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
-  auto pos_of_key = [&](int c) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(keys[c] & 0xFFFFFFFFull)); };
+  auto pos_of_key = [&](int c) { return pos_of(keys[c]); };
 #pragma unroll 1
   for (int r = tid; r < K; r += NT) {
     int64_t idx = -1, slot = -1;
@@ -1183,20 +1257,20 @@ int pow2_ceil(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 // What one of two co-resident blocks may use: half of the multiprocessor's 228 KB, less the 1 KB the system keeps per block.
 constexpr size_t kTwoBlockBytes = 228 * 1024 / 2 - 1024;
 
-template <int MODE, int DT, bool LEAN, int NT, int VEC>
+template <int MODE, bool LEAN, int NT, int VEC, bool CLOSE>
 jf_status_t launch_select_variant(const TopkParams& sp, const TailParams& tp, dim3 grid, size_t smem, cudaStream_t stream, bool fused) {
   if (fused) {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, true, LEAN, NT, VEC>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, true, LEAN, NT, VEC>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, true, LEAN, NT, VEC, CLOSE>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, true, LEAN, NT, VEC, CLOSE>, grid, dim3(NT), smem, stream, sp, tp));
   } else {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, DT, false, LEAN, NT, VEC>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, DT, false, LEAN, NT, VEC>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, false, LEAN, NT, VEC, CLOSE>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, false, LEAN, NT, VEC, CLOSE>, grid, dim3(NT), smem, stream, sp, tp));
   }
   return JF_OK;
 }
 
 template <int MODE, bool LEAN, int NT, int VEC>
-jf_status_t launch_select_dtype(const jf_decode_args* a, TopkParams& sp, const TailParams& tp, dim3 grid, cudaStream_t stream, bool fused) {
+jf_status_t launch_select_block(const jf_decode_args* a, TopkParams& sp, const TailParams& tp, dim3 grid, cudaStream_t stream, bool fused) {
   constexpr int kStep = 4 * NT;
   const int chunk = LEAN ? 0 : std::min(VEC * kStep, (a->max_S + kStep - 1) / kStep * kStep);
   const size_t region0 = sel_region0_bytes<MODE>(chunk);
@@ -1220,8 +1294,17 @@ jf_status_t launch_select_dtype(const jf_decode_args* a, TopkParams& sp, const T
   // own.  Blocks launched while the scan's last ones leave would go two to the first multiprocessors that are
   // free (a step of 32 rows of 2048 positions: 22.5 -> 19.1 us; 72 rows of 8000: 34.2 -> 27.1).
   if (static_cast<int>(grid.x * grid.y) <= num_sms()) smem = std::max(smem, kTwoBlockBytes + 4096);
-  return a->q_dtype == JF_DTYPE_BF16 ? launch_select_variant<MODE, JF_DTYPE_BF16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused)
-                                     : launch_select_variant<MODE, JF_DTYPE_FP16, LEAN, NT, VEC>(sp, tp, grid, smem, stream, fused);
+  // Of a K3V2 row's candidates only the close ones are re-scored (see the ranking) where rows share a
+  // multiprocessor and the top-k leaves most of them apart.  Scan + select, all / close only, us:
+  //   512 rows of 1024, top-k 128: 35.3 / 31.5;  of 4096, 256: 52.9 / 50.8;  of 4096, 512: 64.4 / 64.4;  of 16384, 256: 89.2 / 87.0
+  //   256 rows of 65536, top-k 128: 79.6 / 78.9;  256: 85.6 / 84.4;  512: 98.5 / 99.8;  of 32761 (falling), 256: 54.5 / 53.1
+  //   with a multiprocessor each a row's latency counts, to which the second look adds:
+  //   128 rows of 8192, top-k 64: 22.2 / 22.4;  256: 24.7 / 25.9;  32 rows of 32768, 256: 26.3 / 26.7
+  if constexpr (MODE == JF_MODE_K3V2 && NT == 512 && VEC == 8) {
+    if (static_cast<int>(grid.x * grid.y) > num_sms() && a->top_k <= kCloseTopK)
+      return launch_select_variant<MODE, LEAN, NT, VEC, true>(sp, tp, grid, smem, stream, fused);
+  }
+  return launch_select_variant<MODE, LEAN, NT, VEC, false>(sp, tp, grid, smem, stream, fused);
 }
 
 // The block of a call: 512 threads while the sort buffer allows; a staged row that does not fit the chunk
@@ -1230,11 +1313,11 @@ template <int MODE>
 jf_status_t launch_select_mode(const jf_decode_args* a, const SelectPlan& plan, TopkParams& sp, const TailParams& tp, dim3 grid,
                                cudaStream_t stream, bool fused) {
   if (sp.sort_n > kSelThreads)
-    return plan.lean ? launch_select_dtype<MODE, true, kSelThreads, 8>(a, sp, tp, grid, stream, fused)
-                     : launch_select_dtype<MODE, false, kSelThreads, 8>(a, sp, tp, grid, stream, fused);
-  if (plan.lean) return launch_select_dtype<MODE, true, 512, 8>(a, sp, tp, grid, stream, fused);
-  return (plan.narrow || a->max_S <= 32 * 512) ? launch_select_dtype<MODE, false, 512, 8>(a, sp, tp, grid, stream, fused)
-                                               : launch_select_dtype<MODE, false, 512, 16>(a, sp, tp, grid, stream, fused);
+    return plan.lean ? launch_select_block<MODE, true, kSelThreads, 8>(a, sp, tp, grid, stream, fused)
+                     : launch_select_block<MODE, false, kSelThreads, 8>(a, sp, tp, grid, stream, fused);
+  if (plan.lean) return launch_select_block<MODE, true, 512, 8>(a, sp, tp, grid, stream, fused);
+  return (plan.narrow || a->max_S <= 32 * 512) ? launch_select_block<MODE, false, 512, 8>(a, sp, tp, grid, stream, fused)
+                                               : launch_select_block<MODE, false, 512, 16>(a, sp, tp, grid, stream, fused);
 }
 
 }  // namespace

@@ -1,10 +1,13 @@
 """K3V2 rows that share a multiprocessor (more rows than there are): of a row's candidates only those whose scan
 scores are close to another one's are re-scored.  Lists must still be the oracle's where scores tie, crowd
 together or are so large that every candidate is re-scored, and name positions of the row whatever the scores are."""
+import numpy as np
 import pytest
 import torch
 
-from jf_testlib import Case
+from oracle import native
+from jf_testlib import Case, f32_values, to_bits
+from test_gpu_decode_parity import k3_score_bound, run_gpu
 from test_gpu_long_rows import _run
 
 pytestmark = pytest.mark.gpu
@@ -33,7 +36,14 @@ def test_ties_and_crowds(distinct, jitter):
 def test_scores_whose_band_spans_bins():
     case = Case("k3v2", B, H_Q, H_KV, 1500, seed=5)
     case.k_full = (case.k_full.float() * 300.0).to(case.dtype)
-    _run(case, 128)
+    res, (kd, ks, vd, vs) = run_gpu(case, 128)
+    ref = native.c_decode("k3v2", f32_values(case.q), kd.cpu().numpy(), to_bits(ks), vd.cpu().numpy(), to_bits(vs),
+                          case.block_table.numpy(), case.seq_lens.numpy(), case.ctx, 128, case.attn_scale, want_scores=True)
+    assert np.array_equal(res.topk_idx.cpu().numpy(), ref["topk_idx"])
+    for b in range(B):   # sums of terms of some thousands: fp32 orders differ by the bound that the selection goes by
+        n = int(case.seq_lens[b])
+        err = np.abs(res.scores.cpu().numpy()[b, :, :n] - ref["scores"][b, :, :n])
+        assert (err <= k3_score_bound(case, to_bits(ks), b, n)[:, None]).all()
 
 
 def test_scores_of_another_cache_select_positions_of_the_row():
