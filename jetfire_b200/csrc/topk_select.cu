@@ -684,7 +684,10 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
             gm[0] = fmaxf(gm[0], v.x); gm[1] = fmaxf(gm[1], v.y); gm[2] = fmaxf(gm[2], v.z); gm[3] = fmaxf(gm[3], v.w);
             hm[j] = fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
           }
-          if (use_hm16) {
+        }
+        if (use_hm16) {
+#pragma unroll
+          for (int j = 0; j < kChunkVec; ++j) {
             const uint32_t k32 = float_order_key(hm[j]);
             hm16[(ci * kChunkVec + j) * NT + tid] =
                 static_cast<uint16_t>(min(0xFFFFu, (k32 >> 16) + ((k32 & 0xFFFFu) ? 1u : 0u)));
