@@ -34,15 +34,19 @@ decode_finish_kernel(const FinishParams p, const TailParams tp) {
   const int hkv = h / tp.G, hi = h - hkv * tp.G;
   const int64_t bh = static_cast<int64_t>(b) * tp.H_q + h;
   pdl_wait();
+  pdl_trigger();   // the next kernel may start its prologue; it waits for this grid before reading
+  // the thread's first selected position: on its way while the partials are merged
+  const int64_t* sel = p.topk_idx + bh * tp.top_k;
+  const int first = threadIdx.x;
+  const int64_t first_sel = first < tp.top_k ? sel[first] : -1;
   int pbase, n_splits;   // by every warp for itself
   slice_partials(tp.geom, p.seq_lens, tp.B, tp.max_S, hkv, b, threadIdx.x & 31, pbase, n_splits);
   const int n = min(p.seq_lens[b], tp.max_S);
   const float M = block_max_of_splits<kFinishThreads>(tp.part_m, pbase, hi, n_splits, sm_m);
   merge_splits(tp, splits, pbase, n_splits, hi, M);
-  const int64_t* sel = p.topk_idx + bh * tp.top_k;
   finish_tail<MODE, kFinishThreads, false>(tp, tsm, TailPrefetch{}, splits, M, n, b, h,
                                         p.block_table + static_cast<int64_t>(b) * p.max_blocks, [&](int kk, int& pos, int& cidx) {
-                                          const int64_t v = sel[kk];
+                                          const int64_t v = kk == first ? first_sel : sel[kk];
                                           if (v < 0 || v >= n) return false;
                                           pos = static_cast<int>(v);
                                           cidx = -1;
@@ -54,34 +58,47 @@ decode_finish_kernel(const FinishParams p, const TailParams tp) {
 // statistics-emitting select computes them (jetfire_vllm/csrc/int8tc_qk_scores.cu:1790-1800):
 // an empty or all -inf row gives m = 0, and a non-positive sum gives 1/Z = 0.
 // One CTA per (query head, batch element); sums in a fixed order.
-__global__ void __launch_bounds__(256)
+// What bounds it: latency.  A row of up to kStatsHeld positions is read once, all its loads in flight, and stays in
+// registers between the two reductions; longer rows are read a second time for their rest.
+constexpr int kStatsThreads = 512, kStatsPer = 16, kStatsHeld = kStatsThreads * kStatsPer;
+__global__ void __launch_bounds__(kStatsThreads)
 softmax_stats_kernel(const float* __restrict__ scores, const int32_t* __restrict__ seq_lens, float* __restrict__ out_m,
                      float* __restrict__ out_inv_z, int H_q, int max_S) {
-  __shared__ float red[8];
+  constexpr int kW = kStatsThreads / 32;
+  __shared__ float red[kW], red_z[kW];
   const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_wait();
+  pdl_trigger();   // the next kernel may start its prologue; it waits for this grid before reading
   const int n = max(0, min(seq_lens[b], max_S));
   const float* row = scores + (static_cast<int64_t>(b) * H_q + h) * max_S;
-  float m = -INFINITY;
-  for (int i = tid; i < n; i += 256) m = fmaxf(m, row[i]);
+  float v[kStatsPer], m = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < kStatsPer; ++k) {
+    const int i = tid + k * kStatsThreads;
+    v[k] = i < n ? row[i] : -INFINITY;
+  }
+#pragma unroll
+  for (int k = 0; k < kStatsPer; ++k) m = fmaxf(m, v[k]);
+  for (int i = tid + kStatsHeld; i < n; i += kStatsThreads) m = fmaxf(m, row[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
   if (lane == 0) red[warp] = m;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 8; ++w) m = fmaxf(m, red[w]);
+  for (int w = 0; w < kW; ++w) m = fmaxf(m, red[w]);
   if (!isfinite(m)) m = 0.f;
-  __syncthreads();
   float z = 0.f;
-  for (int i = tid; i < n; i += 256) z += __expf(row[i] - m);
+#pragma unroll
+  for (int k = 0; k < kStatsPer; ++k) z += tid + k * kStatsThreads < n ? __expf(v[k] - m) : 0.f;
+  for (int i = tid + kStatsHeld; i < n; i += kStatsThreads) z += __expf(row[i] - m);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xFFFFFFFFu, z, o);
-  if (lane == 0) red[warp] = z;
+  if (lane == 0) red_z[warp] = z;
   __syncthreads();
   if (tid == 0) {
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) t += red[w];
+    for (int w = 0; w < kW; ++w) t += red_z[w];
     out_m[static_cast<int64_t>(b) * H_q + h] = m;
     out_inv_z[static_cast<int64_t>(b) * H_q + h] = t > 0.f ? 1.0f / t : 0.f;
   }
@@ -133,7 +150,7 @@ extern "C" jf_status_t jf_softmax_stats(const float* scores, const int32_t* seq_
                                         jf_stream_t stream_) {
   using namespace jf;
   if (!scores || !seq_lens || !softmax_m || !softmax_inv_z || B <= 0 || H_q <= 0 || max_S <= 0) return JF_ERR_ARG;
-  JF_CUDA_TRY(launch_pdl(softmax_stats_kernel, dim3(H_q, B), dim3(256), 0, static_cast<cudaStream_t>(stream_), scores,
+  JF_CUDA_TRY(launch_pdl(softmax_stats_kernel, dim3(H_q, B), dim3(kStatsThreads), 0, static_cast<cudaStream_t>(stream_), scores,
                          seq_lens, softmax_m, softmax_inv_z, static_cast<int>(H_q), static_cast<int>(max_S)));
   return JF_OK;
 }

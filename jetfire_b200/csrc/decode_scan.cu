@@ -552,6 +552,7 @@ scan_k3v2_kernel(const ScanParams p) {
     slot_off = (slot_off == (T::kSlots - 1) * T::kSlotBytes) ? 0u : slot_off + T::kSlotBytes;
   }
 
+  if (kDoK && p.fill_tail) fill_score_tail(p, blk);
   pdl_trigger();  // the next kernel may start its prologue; it waits for this grid before reading
   if (kDoK && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) {
     p.status[4] = want_pm ? kPageMaxTag : 0;
@@ -640,13 +641,6 @@ jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
   return JF_OK;
 }
 
-__global__ void fill_neg_inf_tail_kernel(float* scores, const int32_t* seq_lens, int H_q, int max_S) {
-  const int bh = blockIdx.x, b = bh / H_q;
-  const int len = min(seq_lens[b], max_S);
-  float* row = scores + static_cast<int64_t>(bh) * max_S;
-  for (int i = len + threadIdx.x; i < max_S; i += blockDim.x) row[i] = -INFINITY;
-}
-
 }  // namespace jf
 
 extern "C" uint64_t jf_decode_workspace_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
@@ -689,6 +683,7 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   sp.max_S = a->max_S; sp.max_blocks = a->max_blocks;
   sp.geom = slice_geom(a, splits);
   sp.attn_scale = a->attn_scale;
+  sp.fill_tail = a->scores != nullptr && a->scan_parts != JF_SCAN_V_ONLY;   // scores the caller sees
   sp.q_dtype = a->q_dtype;
   const dim3 grid = scan_grid(sp);
   if (a->mode == JF_MODE_K3V2) {
@@ -705,10 +700,5 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   } else {
     st = launch_scan_k4v4(sp, a->stage_b == JF_STAGE_B_INT8P, a->scan_parts, grid, stream);
   }
-  if (st != JF_OK) return st;
-  if (a->scores && a->scan_parts != JF_SCAN_V_ONLY) {
-    fill_neg_inf_tail_kernel<<<a->B * a->H_q, 256, 0, stream>>>(a->scores, a->seq_lens, a->H_q, a->max_S);
-    JF_CUDA_TRY(cudaGetLastError());
-  }
-  return JF_OK;
+  return st;
 }

@@ -50,6 +50,7 @@ struct ScanParams {
   int B, H_q, H_kv, G, max_S, max_blocks;
   float attn_scale;
   int q_dtype;
+  bool fill_tail;       // the scores past a sequence's end are set to -inf
   int kv_shift;         // cache head = KV head >> kv_shift (see head_geom)
   int np_stride;        // entries per row of pmax
   SliceGeom geom;       // how the work is cut
@@ -70,6 +71,16 @@ __device__ __forceinline__ ScanBlock scan_block(const ScanParams& p) {
 }
 inline dim3 scan_grid(const ScanParams& p) {
   return p.geom.splits == 1 ? dim3(1, p.H_kv, p.B) : dim3(p.geom.splits, p.B, p.H_kv);
+}
+
+// Scores past the end of the block's sequence: -inf.  The sequence's CTAs of the KV head share the positions out, each
+// for all query heads.  (In a kernel of its own this was a launch, of the two-stage call order's seven.)
+__device__ __forceinline__ void fill_score_tail(const ScanParams& p, const ScanBlock& blk) {
+  const int len = max(min(p.seq_lens[blk.b], p.max_S), 0), rest = p.max_S - len, parts = gridDim.x;
+  const int per = (rest + parts - 1) / parts, lo = len + static_cast<int>(blockIdx.x) * per, hi = min(lo + per, p.max_S);
+  float* row = p.scores + (static_cast<int64_t>(blk.b) * p.H_q + blk.hkv * p.G) * p.max_S;
+  for (int h = 0; h < p.G; ++h, row += p.max_S)
+    for (int i = lo + static_cast<int>(threadIdx.x); i < hi; i += static_cast<int>(blockDim.x)) row[i] = -INFINITY;
 }
 
 // This CTA's slice: units [lo, hi) of sequence b, whose length is len.  CTA x of sequence y of a KV head is its
