@@ -305,7 +305,8 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
       a1 = fmaxf(a1, __shfl_xor_sync(0xFFFFFFFFu, a1, o));
     }
     const float sc0 = a0 * (1.0f / 127.0f), sc1 = a1 * (1.0f / 127.0f);
-    const float in0 = sc0 > 0.f ? __frcp_rn(sc0) : 0.f, in1 = sc1 > 0.f ? __frcp_rn(sc1) : 0.f;
+    // (Weights below 1e-18 are zero as 16-bit floats; the reciprocal of the smallest scales would be infinite.)
+    const float in0 = sc0 > 1e-20f ? __frcp_rn(sc0) : 0.f, in1 = sc1 > 1e-20f ? __frcp_rn(sc1) : 0.f;
     // round to nearest (ties to even) by adding and removing 1.5 * 2^23: 0 <= pv / scale <= 127
     const uint64_t rnd2 = pair_f32(12582912.0f, 12582912.0f), unrnd2 = pair_f32(-12582912.0f, -12582912.0f);
     const uint64_t in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
