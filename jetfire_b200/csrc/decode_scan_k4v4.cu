@@ -102,6 +102,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 __device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
   return pair_f32(__uint_as_float(lo), __uint_as_float(hi));
 }
+__device__ __forceinline__ uint64_t both(float x) { return pair_f32(x, x); }
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t v) {
   float lo, hi;
   unpair_f32(v, lo, hi);
@@ -315,13 +316,14 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
     // and the error against 64 bits stays what it was to five digits (o_hat 2.185e-4).  Correctly rounded ones with their
     // branch for special values were 6 % of the scan (4 sequences of 32768 positions 32.8 -> 31.0 us, 16 of 131072 500 -> 480).
     const float in0 = sc0 > 1e-20f ? rcp_approx(sc0) : 0.f, in1 = sc1 > 1e-20f ? rcp_approx(sc1) : 0.f;
-    // round to nearest (ties to even) by adding and removing 1.5 * 2^23: 0 <= pv / scale <= 127
-    const uint64_t rnd2 = pair_f32(12582912.0f, 12582912.0f), unrnd2 = pair_f32(-12582912.0f, -12582912.0f);
-    const uint64_t in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
-    unpair_f32(mul2(add2(fma2(wA01, in2, rnd2), unrnd2), sc2), wA[0], wA[1]);
-    unpair_f32(mul2(add2(fma2(wA23, in2, rnd2), unrnd2), sc2), wA[2], wA[3]);
-    unpair_f32(mul2(add2(fma2(wB01, in2, rnd2), unrnd2), sc2), wB[0], wB[1]);
-    unpair_f32(mul2(add2(fma2(wB23, in2, rnd2), unrnd2), sc2), wB[2], wB[3]);
+    // round to nearest (ties to even) by adding 2^23, 0 <= pv / scale <= 127; that leaves together with the multiply by
+    // the scale, of which 2^23 times is exact: one rounding, as if they were apart
+    const uint64_t rnd2 = both(8388608.0f), in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
+    const uint64_t unrnd2 = mul2(sc2, both(-8388608.0f));
+    unpair_f32(fma2(fma2(wA01, in2, rnd2), sc2, unrnd2), wA[0], wA[1]);
+    unpair_f32(fma2(fma2(wA23, in2, rnd2), sc2, unrnd2), wA[2], wA[3]);
+    unpair_f32(fma2(fma2(wB01, in2, rnd2), sc2, unrnd2), wB[0], wB[1]);
+    unpair_f32(fma2(fma2(wB23, in2, rnd2), sc2, unrnd2), wB[2], wB[3]);
   }
   const uint32_t A0 = movmatrix_trans(pack_f16x2_sat(wA[0], wA[1]));
   const uint32_t B0 = movmatrix_trans(pack_f16x2_sat(wB[0], wB[1]));
