@@ -35,18 +35,25 @@
 // -- straight into the mirror through a device-visible pointer (mapped pinned host memory),
 // one coalesced 256-byte write per row, so an append is one launch with no host step.  The
 // store's record of filled slots (:686-759) is written by the same launch.
+#include <algorithm>
+
 #include "jf_common.cuh"
 
 namespace jf {
 
 constexpr int kRowsPerHalf = 2;    // rows of K (and of V) a half-warp loads before it processes any
 constexpr int kWarpsPerCta = 4;
-// Batches of rows a block goes through: as many (up to 8) as leave 24 blocks per multiprocessor, four
-// rounds of the six resident ones -- with fewer the last round is nearly empty, with more batches cut
-// short the set-up of a block (20 instructions per row) shows (32768 x 8 rows: 12 / 24 / 36 blocks
-// per multiprocessor 32.3 / 31.1 / 31.3 us).
-constexpr int kMaxBatches = 8;
-constexpr int kBlocksPerSm = 24;
+// Batches of rows a block goes through (it loads one while it works on the one before): as many as leave 1.8 rounds
+// of the six blocks that a multiprocessor holds, up to five; from there on as many (up to 8) as leave four rounds.  One batch a
+// block up to four rounds, and four rounds then, was 15 % slower in the middle: 6500 x 8 rows 9.1 -> 8.1 us, 9000 12.4 ->
+// 11.0, 12000 15.8 -> 13.8, 16000 17.8 -> 17.0; 3001 (4.3 us), 24000 (24.2) and 32768 (31.4) as before.  (A block with n
+// batches takes 1.2 + 1.7 n us of a round: one wave of 0.85 with 3 batches 6.2 us, with 6 batches 11.8, 10 batches 18.2.)
+constexpr int kMaxBatches = 8, kBlocksResident = 6, kBlocksPerSm = 4 * kBlocksResident;
+inline int pack_batches(int64_t units, int sms) {
+  const int64_t round = static_cast<int64_t>(sms) * kBlocksResident, want = (5 * units + round * 9 / 2) / (round * 9);
+  const int64_t most = std::min<int64_t>(std::max<int64_t>(5, units / (static_cast<int64_t>(sms) * kBlocksPerSm)), kMaxBatches);
+  return static_cast<int>(std::max<int64_t>(1, std::min(want, most)));
+}
 constexpr int kTokensPerBatch = kWarpsPerCta * 2 * kRowsPerHalf;   // of a block
 
 struct PackSide {
@@ -310,8 +317,7 @@ static jf_status_t launch_pack(const PackSide& k, const PackSide* v, int dtype, 
   if (dtype != JF_DTYPE_BF16 && dtype != JF_DTYPE_FP16) return JF_ERR_UNSUPPORTED;
   if (T == 0) return JF_OK;
   const int64_t units = (T + kTokensPerBatch - 1) / kTokensPerBatch;
-  const int64_t want = units * H / (static_cast<int64_t>(num_sms()) * kBlocksPerSm);
-  const int batches = static_cast<int>(want < 1 ? 1 : want > kMaxBatches ? kMaxBatches : want);
+  const int batches = pack_batches(units * H, num_sms());
   const int64_t ctas = (units + batches - 1) / batches;
   const int64_t gz = (ctas + 65534) / 65535;       // the y and z extents of a grid end at 65535
   if (gz > 65535) return JF_ERR_UNSUPPORTED;
