@@ -36,9 +36,11 @@ __host__ __device__ inline HeadGeom head_geom(int H_q, int H_kv) {
   return HeadGeom{H_kv << shift, G >> shift, shift};
 }
 
-// Resident scan CTAs per SM (set by registers / shared memory of the kernel variant).
-__host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype) {
-  return (mode == JF_MODE_K3V2 && q_dtype == JF_DTYPE_FP16) ? 3 : 4;
+// Query heads of a KV head up to which the K3V2 scan repeats them on its unused columns (scan_k3v2_kernel, kNarrow).
+constexpr int kNarrowGroup = 4;
+// Resident scan CTAs per SM (set by registers / shared memory of the kernel variant); G: query heads per (virtual) KV head.
+__host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype, int G) {
+  return (mode == JF_MODE_K3V2 && q_dtype == JF_DTYPE_FP16 && G > kNarrowGroup) ? 3 : 4;
 }
 
 // ---- how the scan's work is cut -----------------------------------------------------------
@@ -51,9 +53,9 @@ __host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype) {
 constexpr int kSliceOverhead = 8;
 inline int scan_units(int max_S) { return ((max_S + JF_BLOCK_SIZE - 1) / JF_BLOCK_SIZE + 1) / 2; }
 inline int scan_split_cap(int units) { return units < 8 ? 1 : units > 4 * 512 ? 512 : units / 4; }
-inline int scan_splits(int mode, int q_dtype, int B, int H_kv, int max_S, int most_waves) {
+inline int scan_splits(int mode, int q_dtype, int B, int H_kv, int G, int max_S, int most_waves) {
   const int units = scan_units(max_S), cap = scan_split_cap(units);
-  const int pairs = B * H_kv, wave = num_sms() * scan_ctas_per_sm(mode, q_dtype);
+  const int pairs = B * H_kv, wave = num_sms() * scan_ctas_per_sm(mode, q_dtype, G);
   int best = 1;
   int64_t best_cost = INT64_MAX;
   for (int w = 1; w <= most_waves; ++w) {
@@ -207,20 +209,20 @@ inline Workspace carve_workspace(void* base, int mode, int B, int H_q, int max_S
 // for the remainder of a wave in the first).
 inline uint64_t partials_needed(int mode, int B, int H_q, int H_kv, int max_S) {
   const HeadGeom hg = head_geom(H_q, H_kv);
-  return static_cast<uint64_t>(B) * hg.H_kv * scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, max_S, 1);
+  return static_cast<uint64_t>(B) * hg.H_kv * scan_splits(mode, JF_DTYPE_BF16, B, hg.H_kv, hg.G, max_S, 1);
 }
 inline uint64_t partials_useful(int mode, int B, int H_q, int H_kv, int max_S) {
   const uint64_t pairs = static_cast<uint64_t>(B) * head_geom(H_q, H_kv).H_kv, capped = pairs * scan_split_cap(scan_units(max_S));
-  const uint64_t waves = 2ull * num_sms() * scan_ctas_per_sm(mode, JF_DTYPE_BF16), most = capped < waves ? capped : waves;
+  const uint64_t waves = 2ull * num_sms() * scan_ctas_per_sm(mode, JF_DTYPE_BF16, 1), most = capped < waves ? capped : waves;
   return most > pairs ? most : pairs;
 }
 // CTAs per sequence and KV head of a call (the same for its scan, select and finish), and its workspace.
 inline int call_splits(const jf_decode_args* a) {
   const HeadGeom hg = head_geom(a->H_q, a->H_kv);
-  const int two = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S, 2);
+  const int two = scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, hg.G, a->max_S, 2);
   const uint64_t partials = static_cast<uint64_t>(a->B) * hg.H_kv * two;
   if (carve_workspace(nullptr, a->mode, a->B, a->H_q, a->max_S, partials).bytes <= a->workspace_bytes) return two;
-  return scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, a->max_S, 1);
+  return scan_splits(a->mode, a->q_dtype, a->B, hg.H_kv, hg.G, a->max_S, 1);
 }
 inline Workspace call_workspace(const jf_decode_args* a, int splits) {
   return carve_workspace(a->workspace, a->mode, a->B, a->H_q, a->max_S,

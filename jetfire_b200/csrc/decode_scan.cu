@@ -36,6 +36,12 @@
 // applies offset, group scale and the reference's bf16 rounding together.  The power-of-two
 // factors are undone on the other operand (K: folded into Q) or on the output row (V); the V
 // group scale is folded into P, the V codes' offset leaves through a sum(P) tile at the end.
+//
+// Narrow groups (at most four query heads per KV head, kNarrow): the eight columns would be half empty, so columns 4-7 repeat
+// the heads.  In P.V the two halves carry the weights of the two V groups: half the conversions and transposes and one sum
+// tile.  In the scores they carry the two bf16 terms of an fp16 query: half the MMAs, and four CTAs a multiprocessor instead
+// of three.  32 / 8 heads: bf16 16 falling lengths up to 16384 51.4 -> 49.3 us, 1 x 32768 11.85 -> 11.35; fp16 4 x 32768
+// 39.6 -> 35.3, 1 x 3000 6.6 -> 5.6.
 #include "decode_scan.cuh"
 
 namespace jf {
@@ -168,6 +174,7 @@ struct K3State {
   uint64_t l2;             // softmax sums of the two heads
   uint32_t smax2;          // largest K group scales seen (bf16 pair: group 0, group 1; sign bits are noise)
   uint32_t ks_sel;         // PRMT selector: this lane's K group scale into both halves
+  uint32_t vs_sel;         // narrow: PRMT selector of this lane's V group scale, as a float
 };
 
 // Scores of one page: token g of the lane in acc[0..1] (heads 2tig, 2tig+1), token g + 8 in acc[2..3].
@@ -198,20 +205,31 @@ __device__ __forceinline__ void k3_weights(uint32_t (&B)[4], const float (&p)[4]
     B[2 * qh + 1] = movmatrix_trans(pack_f16x2_sat(w[2], w[3]));
   }
 }
+// Narrow: the lane's columns belong to one V group, `vs_sel` picks its scale; B = {tokens 0-7, tokens 8-15}.
+__device__ __forceinline__ void k3_weights_narrow(uint32_t (&B)[4], const float (&p)[4], uint32_t vsa, uint32_t vsb, uint32_t vs_sel) {
+  const float va = __uint_as_float(prmt(vsa, 0u, vs_sel)), vb = __uint_as_float(prmt(vsb, 0u, vs_sel));
+  float w[4];
+  unpair_f32(mul2(pair_f32(p[0], p[1]), pair_f32(va, va)), w[0], w[1]);
+  unpair_f32(mul2(pair_f32(p[2], p[3]), pair_f32(vb, vb)), w[2], w[3]);
+  B[0] = movmatrix_trans(pack_f16x2_sat(w[0], w[1]));
+  B[1] = movmatrix_trans(pack_f16x2_sat(w[2], w[3]));
+}
 // One page's (P * vscale).V into the output accumulators.  X = the page's V words, transposed so that a
 // register holds two tokens' halves: {tokens 0-7, tokens 8-15} of channel half 0, then of half 1.
+template <bool kNarrow>
 __device__ __forceinline__ void k3_values(float (&oacc)[9][4], const uint32_t (&B)[4], const uint32_t (&X)[4]) {
 #pragma unroll
   for (int qh = 0; qh < 2; ++qh) {
-    const uint32_t B0 = B[2 * qh], B1 = B[2 * qh + 1], XA = X[2 * qh], XB = X[2 * qh + 1];
+    const uint32_t B0 = B[kNarrow ? 0 : 2 * qh], B1 = B[kNarrow ? 1 : 2 * qh + 1], XA = X[2 * qh], XB = X[2 * qh + 1];
     const uint32_t XA2 = XA >> 10, XB2 = XB >> 10;
     // fields 2ml -> output row g, 2ml+1 -> output row g+8
     mma_f16_nv(oacc[qh * 4 + 0], v2_field<0>(XA), v2_field<2>(XA), v2_field<0>(XB), v2_field<2>(XB), B0, B1);
     mma_f16_nv(oacc[qh * 4 + 1], v2_field<4>(XA), v2_field<6>(XA), v2_field<4>(XB), v2_field<6>(XB), B0, B1);
     mma_f16_nv(oacc[qh * 4 + 2], v2_field<8>(XA), v2_field<0>(XA2), v2_field<8>(XB), v2_field<0>(XB2), B0, B1);
     mma_f16_nv(oacc[qh * 4 + 3], v2_field<2>(XA2), v2_field<4>(XA2), v2_field<2>(XB2), v2_field<4>(XB2), B0, B1);
-    mma_f16_nv(oacc[8], qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, B0, B1);
+    if (!kNarrow) mma_f16_nv(oacc[8], qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, qh ? 0u : kOnesF16x2, qh ? kOnesF16x2 : 0u, B0, B1);
   }
+  if (kNarrow) mma_f16_nv(oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B[0], B[1]);
 }
 
 // One round: two 16-token pages (A and B, one ring slot at shared-memory address `sb`).  Rows of the
@@ -222,7 +240,9 @@ __device__ __forceinline__ void k3_values(float (&oacc)[9][4], const uint32_t (&
 // id was invalid, an absent second page: -1); the common instance carries none of that logic.
 // kParts: 0 = scores and output partials; 1 = scores and softmax sums only (no V);
 // 2 = output partials from scores read back from memory (no K).
-template <int QT, bool kMasked, int kParts>
+// kNarrow: the group has at most four query heads, and columns 4-7 repeat them: with the other V group's weights in P.V, with
+// the second term of an fp16 query (kSplitQ) in the scores.
+template <int QT, bool kMasked, int kParts, bool kNarrow, bool kSplitQ>
 __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const uint32_t (&off)[4], int g, int live_a, int live_b,
                                            float attn, float* row0, float* row1, uint32_t at, bool st0, bool st1,
                                            float* pm_row, uint32_t pm_at, bool pm_store, int lane) {
@@ -257,6 +277,13 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
     st.smax2 = absmax_bf16x2(st.smax2, absmax_bf16x2(absmax_bf16x2(ksa0, ksa1), absmax_bf16x2(ksb0, ksb1)));
     k3_scores<QT>(st, sA, ka[0], ka[1], ka[2], ka[3], kc[0], kc[1], ksa0, ksa1);
     k3_scores<QT>(st, sB, kb[0], kb[1], kb[2], kb[3], kc[2], kc[3], ksb0, ksb1);
+    if (kSplitQ) {   // the two terms of a score lie four columns apart
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sA[i] += __shfl_xor_sync(0xFFFFFFFFu, sA[i], 2);
+        sB[i] += __shfl_xor_sync(0xFFFFFFFFu, sB[i], 2);
+      }
+    }
     const uint64_t attn2 = pair_f32(attn, attn);
     unpair_f32(mul2(pair_f32(sA[0], sA[1]), attn2), sA[0], sA[1]);
     unpair_f32(mul2(pair_f32(sA[2], sA[3]), attn2), sA[2], sA[3]);
@@ -354,10 +381,15 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
   // ---------------- (P * vscale).V ----------------
   if (kDoV) {
     uint32_t BA[4], BB[4];
-    k3_weights(BA, pA, vsa0, vsa1);
-    k3_weights(BB, pB, vsb0, vsb1);
-    k3_values(st.oacc, BA, xa);
-    k3_values(st.oacc, BB, xb);
+    if (kNarrow) {
+      k3_weights_narrow(BA, pA, vsa0, vsa1, st.vs_sel);
+      k3_weights_narrow(BB, pB, vsb0, vsb1, st.vs_sel);
+    } else {
+      k3_weights(BA, pA, vsa0, vsa1);
+      k3_weights(BB, pB, vsb0, vsb1);
+    }
+    k3_values<kNarrow>(st.oacc, BA, xa);
+    k3_values<kNarrow>(st.oacc, BB, xb);
   }
 }
 
@@ -366,11 +398,12 @@ __device__ __forceinline__ void k3v2_round(K3State<QT>& st, uint32_t sb, const u
 // ------------------------------------------------------------------------------------
 // K3V2
 // ------------------------------------------------------------------------------------
-template <int DT, int kParts, bool kShares>
-__global__ void __launch_bounds__(kScanWarps * 32, (DT == JF_DTYPE_FP16) ? 3 : 4)
+template <int DT, int kParts, bool kShares, bool kNarrow>
+__global__ void __launch_bounds__(kScanWarps * 32, (DT == JF_DTYPE_FP16 && !kNarrow) ? 3 : 4)
 scan_k3v2_kernel(const ScanParams p) {
   using T = Tile<JF_MODE_K3V2>;
-  constexpr int kQTerms = (DT == JF_DTYPE_FP16) ? 2 : 1;
+  constexpr int kQTerms = (DT == JF_DTYPE_FP16 && !kNarrow) ? 2 : 1;
+  constexpr bool kSplitQ = DT == JF_DTYPE_FP16 && kNarrow;
   constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
   extern __shared__ __align__(128) uint8_t smem[];
   // the warp index is the same for all lanes; routing it through a shuffle tells the
@@ -466,8 +499,8 @@ scan_k3v2_kernel(const ScanParams p) {
   //      (11-bit significand) is split exactly into two bf16 terms, hi + lo. ----
   K3State<kQTerms> st;
   if (kDoK) {
-    const int h = hkv * p.G + g;
-    const bool live = g < p.G;
+    const int col = kNarrow ? (g & 3) : g, h = hkv * p.G + col;
+    const bool live = col < p.G;
     const int64_t qbase = (static_cast<int64_t>(b) * p.H_q + h) * JF_HEAD_DIM;
     // this lane's 32 channels are contiguous: four 16-byte loads
     uint32_t qraw[16];
@@ -494,10 +527,12 @@ scan_k3v2_kernel(const ScanParams p) {
           const float ra = a - __uint_as_float(hi2 << 16), rc = c - __uint_as_float(hi2 & 0xFFFF0000u);
           st.qf[kQTerms - 1][x][half] = pack_bf16x2(ra, rc);
         }
+        if (kSplitQ && g >= 4) st.qf[0][x][half] = pack_bf16x2(a - __uint_as_float(hi2 << 16), c - __uint_as_float(hi2 & 0xFFFF0000u));
       }
     }
   }
   st.ks_sel = (tig >> 1) ? 0x3232u : 0x1010u;
+  st.vs_sel = (tig >> 1) ? 0x3244u : 0x1044u;
 #pragma unroll
   for (int i = 0; i < 9; ++i) { st.oacc[i][0] = st.oacc[i][1] = st.oacc[i][2] = st.oacc[i][3] = 0.f; }
   st.m_ref0 = kMinusBig; st.m_ref1 = kMinusBig; st.l2 = 0ull;
@@ -514,8 +549,11 @@ scan_k3v2_kernel(const ScanParams p) {
   // 2^18 positions: 32 bits reach)
   float* const row0 = p.scores + (static_cast<int64_t>(b) * p.H_q + hkv * p.G) * p.max_S;
   float* const row1 = row0 + p.max_S;
-  uint32_t at = 4u * (2u * tig * static_cast<uint32_t>(p.max_S) + g + 16u * pg_first);
-  const bool st0 = (2 * tig) < p.G, st1 = (2 * tig + 1) < p.G;
+  const int head0 = kNarrow ? 2 * (tig & 1) : 2 * tig;   // of the lane's columns 2tig, 2tig + 1
+  uint32_t at = 4u * (head0 * static_cast<uint32_t>(p.max_S) + g + 16u * pg_first);
+  // (narrow: the lanes of columns 4-7 read scores, but the others write them)
+  const bool mine = !kNarrow || !kDoK || tig < 2;
+  const bool st0 = mine && head0 < p.G, st1 = mine && head0 + 1 < p.G;
   // Page-pair maxima (pages 2m, 2m+1; a warp's range starts at an even page): after the round's
   // butterfly the lanes with bits 2 and 3 clear hold them -- lane bit 4 clear: head 2tig, set: 2tig+1.
   const int pm_head = 2 * tig + (lane >> 4);
@@ -533,9 +571,9 @@ scan_k3v2_kernel(const ScanParams p) {
     const uint32_t sb = slots0 + slot_off;
     const int4 ent = ent_s[(it >> 1) & (kBtChunk - 1)];   // the round's parked entries are still resident
     if (ent.y + ent.w == 32)
-      k3v2_round<kQTerms, false, kParts>(st, sb, off, g, 16, 16, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store, lane);
+      k3v2_round<kQTerms, false, kParts, kNarrow, kSplitQ>(st, sb, off, g, 16, 16, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store, lane);
     else
-      k3v2_round<kQTerms, true, kParts>(st, sb, off, g, ent.y, ent.w, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store,
+      k3v2_round<kQTerms, true, kParts, kNarrow, kSplitQ>(st, sb, off, g, ent.y, ent.w, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store,
                                         lane);
     at += 128u;
     pm_at += 4u;
@@ -570,10 +608,12 @@ scan_k3v2_kernel(const ScanParams p) {
       const int da = 64 * qh + 8 * g + v2_dlocal(fa), db = 64 * qh + 8 * g + v2_dlocal(fb);
       // 2^(24 - POS) * sum(P * field) - 2 * sum(P): the codes' offset leaves here (see v2_field)
       const float ua = 16777216.0f / static_cast<float>(1 << v2_pos(fa)), ub = 16777216.0f / static_cast<float>(1 << v2_pos(fb));
-      wo[(2 * tig) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][0], ua, -2.0f * st.oacc[8][2 * qh]);
-      wo[(2 * tig + 1) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][1], ua, -2.0f * st.oacc[8][2 * qh + 1]);
-      wo[(2 * tig) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][2], ub, -2.0f * st.oacc[8][2 * qh]);
-      wo[(2 * tig + 1) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][3], ub, -2.0f * st.oacc[8][2 * qh + 1]);
+      if (kNarrow && (tig >> 1) != qh) continue;   // the columns of the other group
+      const float* sum = st.oacc[8] + (kNarrow ? 0 : 2 * qh);
+      wo[head0 * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][0], ua, -2.0f * sum[0]);
+      wo[(head0 + 1) * JF_HEAD_DIM + da] = fmaf(st.oacc[mt][1], ua, -2.0f * sum[1]);
+      wo[head0 * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][2], ub, -2.0f * sum[0]);
+      wo[(head0 + 1) * JF_HEAD_DIM + db] = fmaf(st.oacc[mt][3], ub, -2.0f * sum[1]);
     }
   }
   float l0, l1;
@@ -625,20 +665,21 @@ SliceGeom slice_geom(const jf_decode_args* a, int splits) {
   return g;
 }
 
-template <int DT, int kParts>
-jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
+template <int DT, int kParts, bool kShares, bool kNarrow>
+jf_status_t launch_k3v2_variant(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
   using T = Tile<JF_MODE_K3V2>;
   const size_t smem = kScanWarps * T::kSlots * T::kSlotBytes + kScanWarps * 2 * kBtChunk * 8;  // ring, block-table chunks
   static_assert(kScanWarps * T::kSlots * T::kSlotBytes >= kMergeBytes, "merge buffer");
-  if (sp.geom.even) {
-    JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts, false>), smem);
-    JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts, false>, grid, dim3(kScanWarps * 32), smem, stream, sp));
-  } else {
-    JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts, true>), smem);
-    JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts, true>, grid, dim3(kScanWarps * 32), smem, stream, sp));
-  }
+  JF_ENSURE_SMEM((scan_k3v2_kernel<DT, kParts, kShares, kNarrow>), smem);
+  JF_CUDA_TRY(launch_pdl(scan_k3v2_kernel<DT, kParts, kShares, kNarrow>, grid, dim3(kScanWarps * 32), smem, stream, sp));
   JF_CUDA_TRY(cudaGetLastError());
   return JF_OK;
+}
+template <int DT, int kParts>
+jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
+  if (sp.G <= kNarrowGroup)
+    return sp.geom.even ? launch_k3v2_variant<DT, kParts, false, true>(sp, grid, stream) : launch_k3v2_variant<DT, kParts, true, true>(sp, grid, stream);
+  return sp.geom.even ? launch_k3v2_variant<DT, kParts, false, false>(sp, grid, stream) : launch_k3v2_variant<DT, kParts, true, false>(sp, grid, stream);
 }
 
 }  // namespace jf
