@@ -41,6 +41,7 @@ namespace {
 constexpr int kBins = 2048;
 constexpr float kBinsPerUnit = 64.0f;
 constexpr int kCloseTopK = 256;   // see launch_select_block
+constexpr int64_t kL2Bytes = 126ll << 20, kK3RowBytes = 88;   // packed K and V of a position and KV head
 
 struct TopkParams {
   const float* scores;
@@ -258,7 +259,8 @@ __host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, 
 // shared memory by one bulk copy per 32768 positions, issued before anything else so that
 // the prologue runs under it; every later pass over the scores reads shared memory.
 // FUSED: the finish stage follows in the same kernel.
-// CLOSE (K3V2): candidates are re-scored only where the order needs it.
+// KIND (K3V2, rows that share a multiprocessor): kCut: the candidates are cut down to the top-k and its band by their scan
+// scores before anything of them is fetched; kClose: they are re-scored only where the order needs it.
 // LEAN (K3V2, long rows): the scores are never staged.  The scan left the largest score of every
 // pair of 16-token pages next to them; the threshold comes from a histogram of those maxima (the
 // K-th largest of them is a lower bound of the K-th largest score), and only the pairs whose
@@ -269,7 +271,8 @@ __host__ __device__ constexpr size_t sel_smem_bytes(size_t region0, int sort_n, 
 // are enough to hide the memory: 512 threads -- with VEC 8 two blocks share a multiprocessor, so
 // that one row's round trips run under the other's arithmetic -- and 1024 only for sort buffers
 // beyond 1024 entries, which are sorted by all threads.
-template <int MODE, bool FUSED, bool LEAN, int NT, int VEC, bool CLOSE>
+enum RowKind { kPlain = 0, kCut = 1, kClose = 2 };
+template <int MODE, bool FUSED, bool LEAN, int NT, int VEC, int KIND>
 __global__ void __launch_bounds__(NT, (NT == 512 && VEC == 8) ? 2 : 1)
 topk_select_kernel(const TopkParams p, const TailParams tp) {
   constexpr int kW = NT / 32;                   // warps of this block
@@ -828,6 +831,48 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
           ok = total <= p.sort_n;
           ncand = total;
           cand_last = last + nb;
+          if (KIND == kCut && ok && total > K) {
+            // The threshold came from maxima of groups, of which several top scores may share one: a fifth more candidates
+            // than the top-k.  The same histogram over the candidates' own scores, in finer bins, cuts them down to the top-k and
+            // its band, and with them the scattered reads of their rows.
+            constexpr int kCand = kSelThreads / NT;
+            int f = 1;
+            while (f < 16 && (cand_last + 2) * f * 2 <= kBins) f *= 2;
+            const float fscale = kBinsPerUnit * static_cast<float>(f), ftop = top * fscale;
+            if (tid == 0) { sm.tbin = -1; sm.nlist = 0; }   // (sm.ncand may not have been read by every warp yet)
+            for (int i = tid; i < kBins; i += NT) hist[i] = 0;
+            float cs[kCand];
+            uint32_t cpos[kCand];
+            int cbin[kCand];
+#pragma unroll
+            for (int k = 0; k < kCand; ++k) {
+              const int c = tid + k * NT;
+              cs[k] = c < total ? cand_score[c] : -INFINITY;
+              cpos[k] = c < total ? static_cast<uint32_t>(keys[c]) : 0u;
+              const float x = fminf(fmaxf(fmaf(cs[k], -fscale, ftop), 0.0f), static_cast<float>(kBins - 1));
+              cbin[k] = __float_as_int(__fadd_rz(x, 8388608.0f)) & (kBins - 1);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kCand; ++k)
+              if (tid + k * NT < total) atomicAdd(&hist[cbin[k]], 1);
+            __syncthreads();
+            scan_hist(K);
+            // the K-th largest lies in bin tbin or above; a score within 2 delta of it is less than `span` bins further down
+            const float span = ceilf(2.0f * delta * fscale) + 1.0f;
+            const int keep = sm.tbin + (span < 4096.0f ? static_cast<int>(span) : 4096);
+#pragma unroll
+            for (int k = 0; k < kCand; ++k) {
+              const bool in = tid + k * NT < total && cbin[k] <= keep;
+              const uint32_t vote = __ballot_sync(0xFFFFFFFFu, in);
+              int base = 0;
+              if (lane == 0 && vote) base = atomicAdd(&sm.nlist, __popc(vote));
+              base = __shfl_sync(0xFFFFFFFFu, base, 0) + __popc(vote & ((1u << lane) - 1u));
+              if (in) { keys[base] = cpos[k]; cand_score[base] = cs[k]; }
+            }
+            __syncthreads();
+            ncand = sm.nlist;
+          }
         }
       }
       if (!ok) {
@@ -915,7 +960,7 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     prefetch = FUSED && by_rank && !slow && ncand <= kRowChunk;
     // K3V2: every candidate's canonical score ahead of the ranking, or only where the ranking needs it (see there)
     const float band = 2.002f * delta;
-    const bool rescore_all = MODE == JF_MODE_K3V2 && (!CLOSE || !(band * kBinsPerUnit <= 0.5f));
+    const bool rescore_all = MODE == JF_MODE_K3V2 && (KIND != kClose || !(band * kBinsPerUnit <= 0.5f));
 #pragma unroll 1
     for (int i = tid; i < kBins; i += NT) hist[i] = 0;   // for the ranking
     if (!slow) {
@@ -1075,11 +1120,11 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
       // The keys stay where they are; perm[rank] names them.
       //
       // K3V2: a scan score is within delta of the canonical one, so two candidates whose scan scores are more
-      // than 2 delta apart have the canonical order already.  With CLOSE (launch_select_block) only those that are closer
+      // than 2 delta apart have the canonical order already.  With kClose (launch_select_block) only those that are closer
       // to another one are re-scored, straight from the cache: at a top-k of 64 / 128 / 256 / 512 of a row that is about
       // 6 / 12 / 25 / 45 % of them, and their packed K rows are half of a row's scattered DRAM accesses.
       constexpr int kCand = kSelThreads / NT;
-      const bool open = CLOSE && !slow && !rescore_all;   // ordered by scan scores, the close ones looked at again
+      const bool open = KIND == kClose && !slow && !rescore_all;   // ordered by scan scores, the close ones looked at again
       int f = 1;
 #pragma unroll 1
       while (f < 16 && (cand_last + 2) * f * 2 <= kBins && (!open || band * (kBinsPerUnit * 2 * f) <= 0.5f)) f *= 2;
@@ -1260,14 +1305,14 @@ int pow2_ceil(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 // What one of two co-resident blocks may use: half of the multiprocessor's 228 KB, less the 1 KB the system keeps per block.
 constexpr size_t kTwoBlockBytes = 228 * 1024 / 2 - 1024;
 
-template <int MODE, bool LEAN, int NT, int VEC, bool CLOSE>
+template <int MODE, bool LEAN, int NT, int VEC, int KIND>
 jf_status_t launch_select_variant(const TopkParams& sp, const TailParams& tp, dim3 grid, size_t smem, cudaStream_t stream, bool fused) {
   if (fused) {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, true, LEAN, NT, VEC, CLOSE>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, true, LEAN, NT, VEC, CLOSE>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, true, LEAN, NT, VEC, KIND>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, true, LEAN, NT, VEC, KIND>, grid, dim3(NT), smem, stream, sp, tp));
   } else {
-    JF_ENSURE_SMEM((topk_select_kernel<MODE, false, LEAN, NT, VEC, CLOSE>), kSelSmemLimit);
-    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, false, LEAN, NT, VEC, CLOSE>, grid, dim3(NT), smem, stream, sp, tp));
+    JF_ENSURE_SMEM((topk_select_kernel<MODE, false, LEAN, NT, VEC, KIND>), kSelSmemLimit);
+    JF_CUDA_TRY(launch_pdl(topk_select_kernel<MODE, false, LEAN, NT, VEC, KIND>, grid, dim3(NT), smem, stream, sp, tp));
   }
   return JF_OK;
 }
@@ -1304,10 +1349,19 @@ jf_status_t launch_select_block(const jf_decode_args* a, TopkParams& sp, const T
   //   with a multiprocessor each a row's latency counts, to which the second look adds:
   //   128 rows of 8192, top-k 64: 22.2 / 22.4;  256: 24.7 / 25.9;  32 rows of 32768, 256: 26.3 / 26.7
   if constexpr (MODE == JF_MODE_K3V2 && NT == 512 && VEC == 8) {
-    if (static_cast<int>(grid.x * grid.y) > num_sms() && a->top_k <= kCloseTopK)
-      return launch_select_variant<MODE, LEAN, NT, VEC, true>(sp, tp, grid, smem, stream, fused);
+    if (static_cast<int>(grid.x * grid.y) > num_sms()) {
+      if (a->top_k <= kCloseTopK) return launch_select_variant<MODE, LEAN, NT, VEC, kClose>(sp, tp, grid, smem, stream, fused);
+      // A wider top-k of a cache that does not stay in L2: candidates are cut down before their rows are fetched from DRAM.
+      // Scan + select, us, 512 of 65536 x 256 rows (185 MB) 98.2 / 96.3, of 50000 x 512 (282 MB) 180.3 / 180.3; of 32761
+      // falling x 256 (92 MB) 65.1 / 65.7.  (Not worth it at 256, where the rest is half as much: 84.3 / 85.4; nor for staged rows: 4096 x
+      // 512 62.5 / 64.9.)
+      if constexpr (LEAN) {
+        if (static_cast<int64_t>(a->B) * a->H_kv * a->max_S * kK3RowBytes > kL2Bytes)
+          return launch_select_variant<MODE, LEAN, NT, VEC, kCut>(sp, tp, grid, smem, stream, fused);
+      }
+    }
   }
-  return launch_select_variant<MODE, LEAN, NT, VEC, false>(sp, tp, grid, smem, stream, fused);
+  return launch_select_variant<MODE, LEAN, NT, VEC, kPlain>(sp, tp, grid, smem, stream, fused);
 }
 
 // The block of a call: 512 threads while the sort buffer allows; a staged row that does not fit the chunk

@@ -1,6 +1,7 @@
 """K3V2 rows that share a multiprocessor (more rows than there are): of a row's candidates only those whose scan
-scores are close to another one's are re-scored.  Lists must still be the oracle's where scores tie, crowd
-together or are so large that every candidate is re-scored, and name positions of the row whatever the scores are."""
+scores are close to another one's are re-scored, or they are cut down by their scan scores first.  Lists must still be the
+oracle's where scores tie, crowd together or are so large that every candidate is re-scored, and name positions of the
+row whatever the scores are."""
 import numpy as np
 import pytest
 import torch
@@ -44,6 +45,13 @@ def test_scores_whose_band_spans_bins():
         n = int(case.seq_lens[b])
         err = np.abs(res.scores.cpu().numpy()[b, :, :n] - ref["scores"][b, :, :n])
         assert (err <= k3_score_bound(case, to_bits(ks), b, n)[:, None]).all()
+
+
+@pytest.mark.parametrize("few", [False, True])
+def test_wide_top_k_of_a_cache_beyond_l2(few):
+    """5 x 10 KV heads x 33008 positions x 88 bytes = 145 MB: candidates are cut down before their rows are read."""
+    case = Case("k3v2", B, 40, 10, 33008, lens=[33008, 33007, 1025, 300, 20000], seed=12)
+    _run(_few_keys(case, 5000) if few else case, 400)
 
 
 def test_scores_of_another_cache_select_positions_of_the_row():
