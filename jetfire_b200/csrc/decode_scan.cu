@@ -19,7 +19,7 @@
 // load and the warp-uniform work per page stays small.
 //
 // What bounds it: the issue of instructions, not memory and not a warp's dependent chain (the keys of the next
-// round gone through beside the softmax and P.V of the last: no difference).  A page is some 270 warp instructions (352
+// round gone through beside the softmax and P.V of the last: no difference).  A page is 278 warp instructions (352
 // with bulk copies, 280 before the codes sat at two bit positions).  On a scheduler of a B200 a logic or integer
 // instruction takes two cycles of its pipe, packed 16-bit arithmetic two of the other, and an mma.sync.m16n8k16 -- 8.6 cycles
 // alone -- does not run under them: beside a dozen others it adds 3.5 to 7 cycles, so that the 18 of a page are about a
