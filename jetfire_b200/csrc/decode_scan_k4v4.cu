@@ -119,7 +119,8 @@ constexpr int kSmemBytes = kBtOff + kScanWarps * 2 * kBtChunk * 16 + 1024;      
 static_assert(kScanWarps * T4::kSlots * 8 <= 64 && kRingBytes >= kMergeBytes && kBtOff % 16 == 0, "layout");
 
 struct K4State {
-  uint32_t qb[4][2];          // INT8 query fragments (B operand of the K MMA)
+  uint32_t qb[4][2];          // INT8 query fragments (B operand of the K MMA); narrow groups: page A's columns, 0 in page B's
+  uint32_t qb2[4][2];         // narrow groups: page B's columns, 0 in page A's
   uint64_t qs2[4];            // block scales of the two heads this lane's score columns belong to
   int init[4][4];             // -8 * sum(qi) + kAccMagic per block for those heads, laid out as the MMA's C operand
   float oacc[9][4];           // output tiles 0..7; tile 8: sum of the P operand per head (see v4_field)
@@ -351,6 +352,158 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
   mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
 }
 
+// The same tile for a group of at most four query heads: columns 0-3 of every MMA are the heads over page A's tokens,
+// columns 4-7 the heads over page B's.  Each page meets a query (and weights) that are zero in the other page's columns, and
+// both accumulate into the same registers: a lane then holds two heads x two tokens of one page instead of two pages' with half
+// of the lanes' columns empty, so the scaling of scores, the softmax, the weights' rounding and the stores are half the
+// instructions.  32 / 8 heads, scan + select, us: 4 x 32768 42.9 -> 42.55, 16 x 131072 506 -> 491, 1 x 2048 13.4 -> 13.2 (the scan
+// alone 30.95 -> 30.7 and 473 -> 456: instruction issue counts where many tiles follow one another, its chain elsewhere).  Trading
+// the two heads' maxima instead of reducing both: the same.  Groups of five to eight heads have no empty columns.  The reference point is common to both pages; sums and outputs of the pages meet after the loop.
+// (`sb` / `ss`: shared-memory addresses of page A's K tile and scales; t0, spA0, spA1, pm: of this lane's page.)
+template <bool kInt8P, bool kMasked, int kParts>
+__device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint32_t ss, int mask, int t0, float attn, float* sp0,
+                                                 float* sp1, bool st0, bool st1, bool want_pm, float* pm, int lane) {
+  constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
+  const int page = (lane >> 1) & 1;
+  bool lo = true, hi = true;   // are this lane's tokens (rows g, g + 8) in the tile
+  if (kMasked) {
+    const int range = mask >> (10 * page), first = range & 31, end = (range >> 5) & 31;
+    lo = t0 >= first && t0 < end;
+    hi = t0 + 8 >= first && t0 + 8 < end;
+  }
+  const uint32_t sbB = sb + T4::kPageBytes, sa = ss + st.s_off;
+  float sc[4] = {0.f, 0.f, 0.f, 0.f};
+  if (kDoK) {
+    uint32_t kwA[4][2], kwB[4][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t a = sb + st.k_off[c], b = sbB + st.k_off[c];
+      kwA[c][0] = lds32<0>(a); kwA[c][1] = lds32<512>(a);
+      kwB[c][0] = lds32<0>(b); kwB[c][1] = lds32<512>(b);
+    }
+    const uint32_t ks0 = lds16<0>(sa), ks1 = lds16<16>(sa);
+    int accA[4][4], acc[4][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t a0 = kwA[c][0], a1 = kwA[c][1];
+      mma_u8s8_cd(accA[c], st.init[c], (a0 >> 4) & 0x0F0F0F0Fu, (a1 >> 4) & 0x0F0F0F0Fu, a0 & 0x0F0F0F0Fu, a1 & 0x0F0F0F0Fu,
+                  st.qb[c][0], st.qb[c][1]);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t b0 = kwB[c][0], b1 = kwB[c][1];
+      mma_u8s8_cd(acc[c], accA[c], (b0 >> 4) & 0x0F0F0F0Fu, (b1 >> 4) & 0x0F0F0F0Fu, b0 & 0x0F0F0F0Fu, b1 & 0x0F0F0F0Fu,
+                  st.qb2[c][0], st.qb2[c][1]);
+    }
+    uint64_t s01 = 0, s23 = 0;
+    const uint64_t magic2 = both(-12582912.0f), attn2 = both(attn);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      s01 = fma2(add2(pair_bits(acc[c][0], acc[c][1]), magic2), st.qs2[c], s01);
+      s23 = fma2(add2(pair_bits(acc[c][2], acc[c][3]), magic2), st.qs2[c], s23);
+    }
+    unpair_f32(mul2(mul2(s01, pair_bits(ks0 << 16, ks0 << 16)), attn2), sc[0], sc[1]);
+    unpair_f32(mul2(mul2(s23, pair_bits(ks1 << 16, ks1 << 16)), attn2), sc[2], sc[3]);
+  } else {
+    if (st0 && lo) sc[0] = sp0[0];
+    if (st0 && hi) sc[2] = sp0[8];
+    if (st1 && lo) sc[1] = sp1[0];
+    if (st1 && hi) sc[3] = sp1[8];
+  }
+  uint2 WaA, WbA, WcA, WdA, WaB, WbB, WcB, WdB;
+  float vs0 = 0.f, vs1 = 0.f;
+  if (kDoV) {
+    const uint32_t vA0 = sb + st.v_offA, vA1 = sb + st.v_offB, vB0 = sbB + st.v_offA, vB1 = sbB + st.v_offB;
+    WaA = lds64<0>(vA0); WbA = lds64<0>(vA1); WcA = lds64<512>(vA0); WdA = lds64<512>(vA1);
+    WaB = lds64<0>(vB0); WbB = lds64<0>(vB1); WcB = lds64<512>(vB0); WdB = lds64<512>(vB1);
+    vs0 = __uint_as_float(lds16<T4::kVsOff>(sa) << 16); vs1 = __uint_as_float(lds16<T4::kVsOff + 16>(sa) << 16);
+  }
+  if (kMasked) {
+    if (!lo) { sc[0] = sc[1] = -INFINITY; vs0 = 0.f; }
+    if (!hi) { sc[2] = sc[3] = -INFINITY; vs1 = 0.f; }
+  }
+  if (kDoK) {
+    if (st0) { if (lo) sp0[0] = sc[0]; if (hi) sp0[8] = sc[2]; }
+    if (st1) { if (lo) sp1[0] = sc[1]; if (hi) sp1[8] = sc[3]; }
+  }
+  float mx0 = fmaxf(sc[0], sc[2]), mx1 = fmaxf(sc[1], sc[3]);
+  if (kDoK && want_pm) {
+    // the largest score of each page per head (as in k4v4_tile): over the eight lanes that hold a head's tokens of a
+    // page, which trade one head for the other on the way
+    const bool hb = (lane & 16) != 0;
+    float v = fmaxf(hb ? mx1 : mx0, __shfl_xor_sync(0xFFFFFFFFu, hb ? mx0 : mx1, 16));
+    v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 8));
+    v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 4));
+    if (kMasked && (mask & (1 << (22 + page)))) v = INFINITY;
+    if (pm && (!kMasked || !page || ((mask >> 20) & 3) == 2)) *pm = v;
+  }
+  uint64_t p01, p23;
+  {
+    const bool need = (mx0 > st.m_ref0 + 4.0f) || (mx1 > st.m_ref1 + 4.0f);
+    if (__any_sync(0xFFFFFFFFu, need)) {
+#pragma unroll
+      for (int o = 2; o < 32; o <<= 1) {
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, o));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, o));
+      }
+      const float n0 = fmaxf(st.m_ref0, mx0), n1 = fmaxf(st.m_ref1, mx1);
+      const float f0 = ex2(ref_log2(st.m_ref0) - ref_log2(n0)), f1 = ex2(ref_log2(st.m_ref1) - ref_log2(n1));
+      st.l2 = mul2(st.l2, pair_f32(f0, f1));
+      if (kDoV) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) { st.oacc[i][0] *= f0; st.oacc[i][1] *= f1; st.oacc[i][2] *= f0; st.oacc[i][3] *= f1; }
+      }
+      st.m_ref0 = n0; st.m_ref1 = n1;
+    }
+    const uint64_t c2 = both(kLog2e), mb2 = pair_f32(-ref_log2(st.m_ref0), -ref_log2(st.m_ref1));
+    p01 = ex2_pair(fma2(pair_f32(sc[0], sc[1]), c2, mb2));
+    p23 = ex2_pair(fma2(pair_f32(sc[2], sc[3]), c2, mb2));
+    st.l2 = add2(st.l2, add2(p01, p23));
+  }
+  if (!kDoV) return;
+
+  const uint64_t w01 = mul2(p01, both(vs0)), w23 = mul2(p23, both(vs1));
+  float w[4];
+  unpair_f32(w01, w[0], w[1]); unpair_f32(w23, w[2], w[3]);
+  if (kInt8P) {
+    // the tile's largest pv per head: sixteen lanes hold a head's tokens
+    float a0 = fmaxf(w[0], w[2]), a1 = fmaxf(w[1], w[3]);
+#pragma unroll
+    for (int o = 2; o < 32; o <<= 1) {
+      a0 = fmaxf(a0, __shfl_xor_sync(0xFFFFFFFFu, a0, o));
+      a1 = fmaxf(a1, __shfl_xor_sync(0xFFFFFFFFu, a1, o));
+    }
+    const float sc0 = a0 * (1.0f / 127.0f), sc1 = a1 * (1.0f / 127.0f);
+    const float in0 = sc0 > 1e-20f ? rcp_approx(sc0) : 0.f, in1 = sc1 > 1e-20f ? rcp_approx(sc1) : 0.f;   // (see k4v4_tile)
+    const uint64_t rnd2 = both(8388608.0f), in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
+    const uint64_t unrnd2 = mul2(sc2, both(-8388608.0f));
+    unpair_f32(fma2(fma2(w01, in2, rnd2), sc2, unrnd2), w[0], w[1]);
+    unpair_f32(fma2(fma2(w23, in2, rnd2), sc2, unrnd2), w[2], w[3]);
+  }
+  const uint32_t X0 = movmatrix_trans(pack_f16x2_sat(w[0], w[1]));   // column g: a head over page A's tokens (g < 4) or B's
+  const uint32_t X1 = movmatrix_trans(pack_f16x2_sat(w[2], w[3]));
+  const bool colA = lane < 16;
+  const uint32_t A0 = colA ? X0 : 0u, A1 = colA ? X1 : 0u, B0 = colA ? 0u : X0, B1 = colA ? 0u : X1;
+  const uint32_t waA[2] = {WaA.x, WaA.y}, wbA[2] = {WbA.x, WbA.y}, wcA[2] = {WcA.x, WcA.y}, wdA[2] = {WdA.x, WdA.y};
+  const uint32_t waB[2] = {WaB.x, WaB.y}, wbB[2] = {WbB.x, WbB.y}, wcB[2] = {WcB.x, WcB.y}, wdB[2] = {WdB.x, WdB.y};
+#pragma unroll
+  for (int wi = 0; wi < 2; ++wi) {
+#pragma unroll
+    for (int bp = 0; bp < 2; ++bp) {
+      const uint32_t sel = bp ? 0x7632u : 0x5410u;
+      const uint32_t XA = prmt(waA[wi], wbA[wi], sel), XB = prmt(wcA[wi], wdA[wi], sel);
+      const uint32_t YA = prmt(waB[wi], wbB[wi], sel), YB = prmt(wcB[wi], wdB[wi], sel);
+      const uint32_t XA2 = XA >> 8, XB2 = XB >> 8, YA2 = YA >> 8, YB2 = YB >> 8;
+      const int mt = 4 * wi + 2 * bp;
+      mma_f16_16816(st.oacc[mt], v4_field<0>(XA), v4_field<4>(XA), v4_field<0>(XB), v4_field<4>(XB), A0, A1);
+      mma_f16_16816(st.oacc[mt + 1], v4_field<0>(XA2), v4_field<4>(XA2), v4_field<0>(XB2), v4_field<4>(XB2), A0, A1);
+      mma_f16_16816(st.oacc[mt], v4_field<0>(YA), v4_field<4>(YA), v4_field<0>(YB), v4_field<4>(YB), B0, B1);
+      mma_f16_16816(st.oacc[mt + 1], v4_field<0>(YA2), v4_field<4>(YA2), v4_field<0>(YB2), v4_field<4>(YB2), B0, B1);
+    }
+  }
+  mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, X0, X1);
+}
+
 constexpr int kFullTile = (16 << 5) | (16 << 15) | (2 << 20);   // both pages whole
 
 }  // namespace
@@ -361,7 +514,7 @@ constexpr int kFullTile = (16 << 5) | (16 << 15) | (2 << 20);   // both pages wh
 // block (jetfire_vllm/csrc/int8tc_softmax_v_fused.cu:62, 1049-1053); a block that a split boundary
 // cuts belongs to two tiles, each with its own tokens.  p.tile_base[s] = first tile of split s.
 // A CTA takes a contiguous range of tiles, each of its warps a contiguous quarter of it.
-template <bool kInt8P, int kParts>
+template <bool kInt8P, int kParts, bool kNarrow>
 __global__ void __launch_bounds__(kScanWarps * 32, 4)
 scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
                  const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap k_map2,
@@ -460,8 +613,9 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   Pending pend = desc_load(0);
   // warp w prepares the query's 32-channel block w for the whole CTA (see below)
   uint4 q_raw = make_uint4(0u, 0u, 0u, 0u);
-  if (kDoK && g < p.G) {   // the 8 channels 32 w + 8 tig + {0..7} are 16 contiguous bytes
-    const int64_t qbase = (static_cast<int64_t>(b) * p.H_q + hkv * p.G + g) * JF_HEAD_DIM;
+  const int q_head = kNarrow ? (g & 3) : g;
+  if (kDoK && q_head < p.G) {   // the 8 channels 32 w + 8 tig + {0..7} are 16 contiguous bytes
+    const int64_t qbase = (static_cast<int64_t>(b) * p.H_q + hkv * p.G + q_head) * JF_HEAD_DIM;
     q_raw = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q) + qbase + 32 * warp + 8 * tig));
   }
 
@@ -567,8 +721,12 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const uint32_t* src = qx + c * (6 * 32) + lane;
-      st.qb[c][0] = src[0];
-      st.qb[c][1] = src[32];
+      st.qb[c][0] = (kNarrow && g >= 4) ? 0u : src[0];
+      st.qb[c][1] = (kNarrow && g >= 4) ? 0u : src[32];
+      if (kNarrow) {
+        st.qb2[c][0] = g >= 4 ? src[0] : 0u;
+        st.qb2[c][1] = g >= 4 ? src[32] : 0u;
+      }
       st.qs2[c] = pair_bits(src[64], src[96]);
       st.init[c][0] = st.init[c][2] = static_cast<int>(src[128]) + kAccMagic;
       st.init[c][1] = st.init[c][3] = static_cast<int>(src[160]) + kAccMagic;
@@ -588,19 +746,19 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     for (int c = 0; c < 4; ++c) st.k_off[c] = t0 * 64 + 4 * tig + ((c ^ ksw) << 4);
     st.v_offA = T4::kVOff + tA * 64 + ((vchunk ^ ((tA >> 1) & 3)) << 4) + vsub;
     st.v_offB = T4::kVOff + tB * 64 + ((vchunk ^ ((tB >> 1) & 3)) << 4) + vsub;
-    st.s_off = t0 * 2;
+    st.s_off = t0 * 2 + (kNarrow ? 32 * (tig >> 1) : 0);
   }
-  const int h0 = hkv * p.G + 2 * tig;
-  float* sp0 = p.scores + (static_cast<int64_t>(b) * p.H_q + h0) * p.max_S + t0;
+  const int head0 = kNarrow ? 2 * (tig & 1) : 2 * tig;   // of the lane's columns 2tig, 2tig + 1
+  float* sp0 = p.scores + (static_cast<int64_t>(b) * p.H_q + hkv * p.G + head0) * p.max_S + t0 + (kNarrow ? 16 * (tig >> 1) : 0);
   float* sp1 = sp0 + p.max_S;
-  const bool st0 = (2 * tig) < p.G, st1 = (2 * tig + 1) < p.G;
+  const bool st0 = head0 < p.G, st1 = head0 + 1 < p.G;
   const float attn = p.attn_scale;
-  // page maxima: after the tile's exchange the lanes with bit 2 clear hold them -- bit 4: head
-  // 2tig / 2tig+1, bit 3: page A / B
-  const int pm_head = 2 * tig + (lane >> 4);
+  // page maxima: after the tile's exchange the lanes with bit 2 (narrow: and 3) clear hold them -- bit 4: which of
+  // the lane's two heads, bit 3 (narrow: 1): page A / B
+  const int pm_head = head0 + (lane >> 4);
   const bool want_pm = kDoK && p.pmax != nullptr;   // the same for the whole grid
-  float* pm_row = (want_pm && (lane & 4) == 0 && pm_head < p.G)
-                      ? p.pmax + (static_cast<int64_t>(b) * p.H_q + hkv * p.G + pm_head) * p.np_stride + ((lane >> 3) & 1)
+  float* pm_row = (want_pm && (lane & (kNarrow ? 12 : 4)) == 0 && pm_head < p.G)
+                      ? p.pmax + (static_cast<int64_t>(b) * p.H_q + hkv * p.G + pm_head) * p.np_stride + ((lane >> (kNarrow ? 1 : 3)) & 1)
                       : nullptr;
 
   // A round takes one slot: one tile.  Tiles of two whole pages go through the unmasked path.
@@ -619,7 +777,11 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     const uint32_t sb = slots0 + sl * T4::kSlotBytes, ss = sb + T4::kScaleOff;
     float* spA0 = sp0 + static_cast<int64_t>(d.w) * 16;
     float* spA1 = sp1 + static_cast<int64_t>(d.w) * 16;
-    if (d.z == kFullTile)
+    if (kNarrow) {
+      float* const pm = pm_row ? pm_row + d.w : nullptr;
+      if (d.z == kFullTile) k4v4_tile_narrow<kInt8P, false, kParts>(st, sb, ss, d.z, t0, attn, spA0, spA1, st0, st1, want_pm, pm, lane);
+      else k4v4_tile_narrow<kInt8P, true, kParts>(st, sb, ss, d.z, t0, attn, spA0, spA1, st0, st1, want_pm, pm, lane);
+    } else if (d.z == kFullTile)
       k4v4_tile<kInt8P, false, kParts>(st, sb, sb + T4::kPageBytes, ss, ss + 32, d.z, t0, attn, spA0, spA1, st0, st1,
                                        want_pm, pm_row ? pm_row + d.w : nullptr, lane);
     else
@@ -647,6 +809,12 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     p.status[kWaitWord] = 0;
   }
 
+  if (kNarrow) {   // the pages' columns meet
+#pragma unroll
+    for (int i = 0; i < 9; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) st.oacc[i][j] += __shfl_xor_sync(0xFFFFFFFFu, st.oacc[i][j], 2);
+  }
   __syncthreads();
   {
     float* wo = reinterpret_cast<float*>(smem) + warp * (kHeadsPad * JF_HEAD_DIM);
@@ -664,6 +832,10 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   }
   float l0, l1;
   unpair_f32(st.l2, l0, l1);
+  if (kNarrow) {
+    l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
+    l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2);
+  }
   cta_merge_store(p, smem, l0, l1, st.m_ref0, st.m_ref1, 0.f, 0.f);
 }
 
@@ -725,15 +897,22 @@ jf_status_t page_map(const void* base, uint64_t rows, uint32_t box_rows, CUtenso
 
 }  // namespace
 
-template <bool kInt8P, int kParts>
-jf_status_t launch_variant(const ScanParams& sp, dim3 grid, cudaStream_t stream, const CUtensorMap& k_map,
+template <bool kInt8P, int kParts, bool kNarrow>
+jf_status_t launch_typed(const ScanParams& sp, dim3 grid, cudaStream_t stream, const CUtensorMap& k_map,
                            const CUtensorMap& v_map, const CUtensorMap& k_map2, const CUtensorMap& v_map2) {
   const size_t smem = kSmemBytes;
-  JF_ENSURE_SMEM((scan_k4v4_kernel<kInt8P, kParts>), smem);
-  JF_CUDA_TRY(launch_pdl(scan_k4v4_kernel<kInt8P, kParts>, grid, dim3(kScanWarps * 32), smem, stream, sp, k_map, v_map,
+  JF_ENSURE_SMEM((scan_k4v4_kernel<kInt8P, kParts, kNarrow>), smem);
+  JF_CUDA_TRY(launch_pdl(scan_k4v4_kernel<kInt8P, kParts, kNarrow>, grid, dim3(kScanWarps * 32), smem, stream, sp, k_map, v_map,
                          k_map2, v_map2));
   JF_CUDA_TRY(cudaGetLastError());
   return JF_OK;
+}
+
+template <bool kInt8P, int kParts>
+jf_status_t launch_variant(const ScanParams& sp, dim3 grid, cudaStream_t stream, const CUtensorMap& k_map,
+                           const CUtensorMap& v_map, const CUtensorMap& k_map2, const CUtensorMap& v_map2) {
+  return sp.G <= kNarrowGroup ? launch_typed<kInt8P, kParts, true>(sp, grid, stream, k_map, v_map, k_map2, v_map2)
+                              : launch_typed<kInt8P, kParts, false>(sp, grid, stream, k_map, v_map, k_map2, v_map2);
 }
 
 // `sp` arrives with everything but the tile geometry filled in.
