@@ -352,13 +352,17 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
   mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
 }
 
-// The same tile for a group of at most four query heads: columns 0-3 of every MMA are the heads over page A's tokens,
-// columns 4-7 the heads over page B's.  Each page meets a query (and weights) that are zero in the other page's columns, and
-// both accumulate into the same registers: a lane then holds two heads x two tokens of one page instead of two pages' with half
-// of the lanes' columns empty, so the scaling of scores, the softmax, the weights' rounding and the stores are half the
-// instructions.  32 / 8 heads, scan + select, us: 4 x 32768 42.9 -> 42.55, 16 x 131072 506 -> 491, 1 x 2048 13.4 -> 13.2 (the scan
-// alone 30.95 -> 30.7 and 473 -> 456: instruction issue counts where many tiles follow one another, its chain elsewhere).  Trading
-// the two heads' maxima instead of reducing both: the same.  Groups of five to eight heads have no empty columns.  The reference point is common to both pages; sums and outputs of the pages meet after the loop.
+// The same tile for a group of at most four query heads: columns 0-3 of the score MMAs are the heads over page A's tokens,
+// columns 4-7 the heads over page B's.  Each page meets a query that is zero in the other page's columns, and both accumulate
+// into the same registers: a lane then holds two heads x two tokens of one page instead of two pages' with half of the lanes'
+// columns empty, so the scaling of scores, the softmax, the weights' rounding and the stores are half the instructions.
+// P.V and the softmax sums add in the order of k4v4_tile, to the same bits: page A meets the weights as they lie, page B the
+// same turned round by four columns, both in columns 0-3 (4-7 hold what nobody reads).  (Sums kept apart by page until the end
+// of the loop saved two MMAs' turns, and nothing in time: 16 x 131072 the scan alone 462 / 465 us, 4 x 32768 30.5 / 30.3; but where
+// sum(P * code) and 8 * sum(P) nearly cancel, outputs of few and of many heads to a group differed by 4e-4.)
+// 32 / 8 heads, with the columns half empty / like this, scan + select, us: 4 x 32768 42.9 / 42.2, 16 x 131072 506 / 500, 1 x 2048 13.4 /
+// 13.3 (the scan of 16 x 131072 alone 473 / 465: instruction issue counts where many tiles follow one another, its chain
+// elsewhere).  Trading the two heads' maxima instead of reducing both: the same.  Groups of five to eight heads have no empty columns.
 // (`sb` / `ss`: shared-memory addresses of page A's K tile and scales; t0, spA0, spA1, pm: of this lane's page.)
 template <bool kInt8P, bool kMasked, int kParts>
 __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint32_t ss, int mask, int t0, float attn, float* sp0,
@@ -371,15 +375,16 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
     lo = t0 >= first && t0 < end;
     hi = t0 + 8 >= first && t0 + 8 < end;
   }
-  const uint32_t sbB = sb + T4::kPageBytes, sa = ss + st.s_off;
+  constexpr int kB = T4::kPageBytes;   // page B's tiles, from page A's
+  const uint32_t sa = ss + st.s_off;
   float sc[4] = {0.f, 0.f, 0.f, 0.f};
   if (kDoK) {
     uint32_t kwA[4][2], kwB[4][2];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const uint32_t a = sb + st.k_off[c], b = sbB + st.k_off[c];
+      const uint32_t a = (sb + st.k_off[0]) ^ (c << 4);   // slots are whole 512 bytes: k_off[c] = k_off[0] ^ 16 c
       kwA[c][0] = lds32<0>(a); kwA[c][1] = lds32<512>(a);
-      kwB[c][0] = lds32<0>(b); kwB[c][1] = lds32<512>(b);
+      kwB[c][0] = lds32<kB>(a); kwB[c][1] = lds32<kB + 512>(a);
     }
     const uint32_t ks0 = lds16<0>(sa), ks1 = lds16<16>(sa);
     int accA[4][4], acc[4][4];
@@ -413,9 +418,9 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
   uint2 WaA, WbA, WcA, WdA, WaB, WbB, WcB, WdB;
   float vs0 = 0.f, vs1 = 0.f;
   if (kDoV) {
-    const uint32_t vA0 = sb + st.v_offA, vA1 = sb + st.v_offB, vB0 = sbB + st.v_offA, vB1 = sbB + st.v_offB;
-    WaA = lds64<0>(vA0); WbA = lds64<0>(vA1); WcA = lds64<512>(vA0); WdA = lds64<512>(vA1);
-    WaB = lds64<0>(vB0); WbB = lds64<0>(vB1); WcB = lds64<512>(vB0); WdB = lds64<512>(vB1);
+    const uint32_t v0 = sb + st.v_offA, v1 = sb + st.v_offB;
+    WaA = lds64<0>(v0); WbA = lds64<0>(v1); WcA = lds64<512>(v0); WdA = lds64<512>(v1);
+    WaB = lds64<kB>(v0); WbB = lds64<kB>(v1); WcB = lds64<kB + 512>(v0); WdB = lds64<kB + 512>(v1);
     vs0 = __uint_as_float(lds16<T4::kVsOff>(sa) << 16); vs1 = __uint_as_float(lds16<T4::kVsOff + 16>(sa) << 16);
   }
   if (kMasked) {
@@ -458,7 +463,8 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
     const uint64_t c2 = both(kLog2e), mb2 = pair_f32(-ref_log2(st.m_ref0), -ref_log2(st.m_ref1));
     p01 = ex2_pair(fma2(pair_f32(sc[0], sc[1]), c2, mb2));
     p23 = ex2_pair(fma2(pair_f32(sc[2], sc[3]), c2, mb2));
-    st.l2 = add2(st.l2, add2(p01, p23));
+    const uint64_t page_l = add2(p01, p23);
+    st.l2 = add2(st.l2, add2(page_l, __shfl_xor_sync(0xFFFFFFFFu, page_l, 2)));   // with the other page's: the wide tile's sum
   }
   if (!kDoV) return;
 
@@ -482,8 +488,7 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
   }
   const uint32_t X0 = movmatrix_trans(pack_f16x2_sat(w[0], w[1]));   // column g: a head over page A's tokens (g < 4) or B's
   const uint32_t X1 = movmatrix_trans(pack_f16x2_sat(w[2], w[3]));
-  const bool colA = lane < 16;
-  const uint32_t A0 = colA ? X0 : 0u, A1 = colA ? X1 : 0u, B0 = colA ? 0u : X0, B1 = colA ? 0u : X1;
+  const uint32_t A0 = X0, A1 = X1, B0 = __shfl_xor_sync(0xFFFFFFFFu, X0, 16), B1 = __shfl_xor_sync(0xFFFFFFFFu, X1, 16);
   const uint32_t waA[2] = {WaA.x, WaA.y}, wbA[2] = {WbA.x, WbA.y}, wcA[2] = {WcA.x, WcA.y}, wdA[2] = {WdA.x, WdA.y};
   const uint32_t waB[2] = {WaB.x, WaB.y}, wbB[2] = {WbB.x, WbB.y}, wcB[2] = {WcB.x, WcB.y}, wdB[2] = {WdB.x, WdB.y};
 #pragma unroll
@@ -501,7 +506,8 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
       mma_f16_16816(st.oacc[mt + 1], v4_field<0>(YA2), v4_field<4>(YA2), v4_field<0>(YB2), v4_field<4>(YB2), B0, B1);
     }
   }
-  mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, X0, X1);
+  mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, A0, A1);
+  mma_f16_16816(st.oacc[8], kOnesF16x2, kOnesF16x2, kOnesF16x2, kOnesF16x2, B0, B1);
 }
 
 constexpr int kFullTile = (16 << 5) | (16 << 15) | (2 << 20);   // both pages whole
@@ -776,7 +782,7 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     }
     const uint32_t sb = slots0 + sl * T4::kSlotBytes, ss = sb + T4::kScaleOff;
     float* spA0 = sp0 + static_cast<int64_t>(d.w) * 16;
-    float* spA1 = sp1 + static_cast<int64_t>(d.w) * 16;
+    float* spA1 = kNarrow ? spA0 + p.max_S : sp1 + static_cast<int64_t>(d.w) * 16;
     if (kNarrow) {
       float* const pm = pm_row ? pm_row + d.w : nullptr;
       if (d.z == kFullTile) k4v4_tile_narrow<kInt8P, false, kParts>(st, sb, ss, d.z, t0, attn, spA0, spA1, st0, st1, want_pm, pm, lane);
@@ -809,12 +815,6 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     p.status[kWaitWord] = 0;
   }
 
-  if (kNarrow) {   // the pages' columns meet
-#pragma unroll
-    for (int i = 0; i < 9; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) st.oacc[i][j] += __shfl_xor_sync(0xFFFFFFFFu, st.oacc[i][j], 2);
-  }
   __syncthreads();
   {
     float* wo = reinterpret_cast<float*>(smem) + warp * (kHeadsPad * JF_HEAD_DIM);
@@ -832,10 +832,6 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   }
   float l0, l1;
   unpair_f32(st.l2, l0, l1);
-  if (kNarrow) {
-    l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
-    l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2);
-  }
   cta_merge_store(p, smem, l0, l1, st.m_ref0, st.m_ref1, 0.f, 0.f);
 }
 
