@@ -103,6 +103,20 @@ __device__ __forceinline__ uint64_t pair_bits(uint32_t lo, uint32_t hi) {
   return pair_f32(__uint_as_float(lo), __uint_as_float(hi));
 }
 __device__ __forceinline__ uint64_t both(float x) { return pair_f32(x, x); }
+// kInt8P: the unit of a tile's 127 levels for two heads whose largest weights are a0 and a1, and its correctly rounded inverse: the
+// approximation and one Newton step in fma, which rounds correctly from within a unit in the last place (Markstein, IBM J. Res.
+// Dev. 34, 1990; equal to __frcp_rn for all 2^23 significands).  A weight near a tie of two levels takes the
+// level that fp32 arithmetic gives it.  (__frcp_rn itself, with its branch for special values, was 6 % of the scan: 4 sequences of
+// 32768 positions 32.8 us, 31.0 without; the step's three packed instructions: 30.35 -> 30.5, 16 of 131072 464 -> 466.)
+// Units up to 1e-20 count as 0: 127 of them are below what a 16-bit float holds, and the inverse of the smallest would be infinite.
+__device__ __forceinline__ void level_units(float a0, float a1, uint64_t& unit2, uint64_t& inv2) {
+  const float u0 = a0 * (1.0f / 127.0f), u1 = a1 * (1.0f / 127.0f);
+  unit2 = pair_f32(u0, u1);
+  const uint64_t y = pair_f32(rcp_approx(u0), rcp_approx(u1));
+  float i0, i1;
+  unpair_f32(fma2(fma2(pair_f32(-u0, -u1), y, both(1.0f)), y, y), i0, i1);
+  inv2 = pair_f32(u0 > 1e-20f ? i0 : 0.f, u1 > 1e-20f ? i1 : 0.f);
+}
 __device__ __forceinline__ uint64_t ex2_pair(uint64_t v) {
   float lo, hi;
   unpair_f32(v, lo, hi);
@@ -311,15 +325,11 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
       a0 = fmaxf(a0, __shfl_xor_sync(0xFFFFFFFFu, a0, o));
       a1 = fmaxf(a1, __shfl_xor_sync(0xFFFFFFFFu, a1, o));
     }
-    const float sc0 = a0 * (1.0f / 127.0f), sc1 = a1 * (1.0f / 127.0f);
-    // (Weights below 1e-18 are zero as 16-bit floats; the reciprocal of the smallest scales would be infinite.)  The
-    // reciprocals are approximate to an unit of fp32: a level changes where a weight is within 2^-16 of a level of a tie,
-    // and the error against 64 bits stays what it was to five digits (o_hat 2.185e-4).  Correctly rounded ones with their
-    // branch for special values were 6 % of the scan (4 sequences of 32768 positions 32.8 -> 31.0 us, 16 of 131072 500 -> 480).
-    const float in0 = sc0 > 1e-20f ? rcp_approx(sc0) : 0.f, in1 = sc1 > 1e-20f ? rcp_approx(sc1) : 0.f;
+    uint64_t sc2, in2;
+    level_units(a0, a1, sc2, in2);
     // round to nearest (ties to even) by adding 2^23, 0 <= pv / scale <= 127; that leaves together with the multiply by
     // the scale, of which 2^23 times is exact: one rounding, as if they were apart
-    const uint64_t rnd2 = both(8388608.0f), in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
+    const uint64_t rnd2 = both(8388608.0f);
     const uint64_t unrnd2 = mul2(sc2, both(-8388608.0f));
     unpair_f32(fma2(fma2(wA01, in2, rnd2), sc2, unrnd2), wA[0], wA[1]);
     unpair_f32(fma2(fma2(wA23, in2, rnd2), sc2, unrnd2), wA[2], wA[3]);
@@ -479,9 +489,9 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
       a0 = fmaxf(a0, __shfl_xor_sync(0xFFFFFFFFu, a0, o));
       a1 = fmaxf(a1, __shfl_xor_sync(0xFFFFFFFFu, a1, o));
     }
-    const float sc0 = a0 * (1.0f / 127.0f), sc1 = a1 * (1.0f / 127.0f);
-    const float in0 = sc0 > 1e-20f ? rcp_approx(sc0) : 0.f, in1 = sc1 > 1e-20f ? rcp_approx(sc1) : 0.f;   // (see k4v4_tile)
-    const uint64_t rnd2 = both(8388608.0f), in2 = pair_f32(in0, in1), sc2 = pair_f32(sc0, sc1);
+    uint64_t sc2, in2;
+    level_units(a0, a1, sc2, in2);   // (see k4v4_tile)
+    const uint64_t rnd2 = both(8388608.0f);
     const uint64_t unrnd2 = mul2(sc2, both(-8388608.0f));
     unpair_f32(fma2(fma2(w01, in2, rnd2), sc2, unrnd2), w[0], w[1]);
     unpair_f32(fma2(fma2(w23, in2, rnd2), sc2, unrnd2), w[2], w[3]);
