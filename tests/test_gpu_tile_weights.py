@@ -57,3 +57,20 @@ def test_every_pair_of_scales(group):
     # at most in fp32 (2^-8): well within the half that tells two levels apart
     assert np.array_equal(np.rint(got), want)
     assert np.abs(got - want).max() < 0.1
+
+
+@pytest.mark.parametrize("group", [4, 8])
+def test_signed_scales(group):
+    s = bf16_scales(3)
+    s[:, 1::2] *= -1.0
+    want, unit = levels(s)
+    got = tile_weights(s, group) / unit
+    assert np.array_equal(np.rint(got), want)
+    assert np.abs(got - want).max() < 0.1
+
+
+@pytest.mark.parametrize("group", [4, 8])
+def test_scales_whose_weights_saturate(group):
+    s = bf16_scales(9) * np.float32(2.0 ** 115)
+    want, _ = levels(s)
+    assert np.array_equal(tile_weights(s, group), np.where(want > 0, np.float32(65504.0), np.float32(0.0)))
