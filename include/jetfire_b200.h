@@ -212,7 +212,8 @@ typedef struct jf_decode_args {
   const int32_t* seq_lens;     /* (B,)                                             */
   /* outputs */
   float*   scores;        /* optional (B, H_q, max_S): approximate scores, -inf past the
-                             sequence end; NULL keeps them in the workspace only;
+                             sequence end and where block_table names no block of the
+                             cache; NULL keeps them in the workspace only;
                              JF_SCAN_V_ONLY, select and finish read them from here   */
   int64_t* topk_idx;      /* (B, H_q, top_k) positions, (score desc, index asc), -1 pad */
   int64_t* topk_slots;    /* (B, H_q, top_k) physical slots, -1 pad                */

@@ -236,8 +236,8 @@ __device__ __forceinline__ void k3_values(float (&oacc)[9][4], const uint32_t (&
 // pages are MMA rows in order; a lane holds tokens g and g + 8 of both.  ldmatrix does what used to be
 // fourteen scalar loads and four joins per page: untransposed it hands each lane its word of a K byte
 // plane, transposed it pairs two tokens' V halves in one register.
-// kMasked: only the first `live_a` / `live_b` tokens count (the last page of a sequence, a page whose block
-// id was invalid, an absent second page: -1); the common instance carries none of that logic.
+// kMasked: only the first `live_a` / `live_b` tokens count (the last page of a sequence; an absent second page,
+// a page whose block id was invalid: none); the common instance carries none of that logic.
 // kParts: 0 = scores and output partials; 1 = scores and softmax sums only (no V);
 // 2 = output partials from scores read back from memory (no K).
 // kNarrow: the group has at most four query heads, and columns 4-7 repeat them: with the other V group's weights in P.V, with
@@ -417,7 +417,7 @@ scan_k3v2_kernel(const ScanParams p) {
   constexpr int kRingBytes = kScanWarps * T::kSlots * T::kSlotBytes;
   constexpr int kPagesInFlight = 2 * T::kSlots;
   const uint32_t slots0 = smem_base + warp * (T::kSlots * T::kSlotBytes);
-  // parked per page: its index in the cache (over all KV heads) and how many of its 16 tokens are live
+  // parked per page: its index in the cache (over all KV heads) and how many of its 16 tokens are live (see bt_entry)
   int2* bt_s = reinterpret_cast<int2*>(smem + kRingBytes) + warp * (2 * kBtChunk);
 
   pdl_wait();  // nothing above reads global memory
@@ -444,12 +444,23 @@ scan_k3v2_kernel(const ScanParams p) {
   const uint32_t head_page0 = static_cast<uint32_t>(hkv >> p.kv_shift) * static_cast<uint32_t>(n_blocks_phys);
   const int last_pg = (len & 15) ? (n_pages - 1) : -1;   // the only page that can be partial
   // entry e of this warp (page pg_first + e) from its block id, worked out by sixteen lanes at
-  // once when a chunk arrives: an invalid block id reads block 0 and counts no live token; the
-  // sequence's last page may be partial; entries past the warp's range count -1
+  // once when a chunk arrives: the sequence's last page may be partial; entries past the warp's range count -1.
+  // An invalid block id counts no live token, and its tokens score -inf.  Who stores that is a matter of registers: behind
+  // the round (the entry then counts -1 less its tokens, and fetches nothing) 4 x 65536 x 64 heads takes 62.0 us, from
+  // here 63.9 (62.7 without either); an fp16 query of a wide group spills there, 8 falling lengths up to 32761 33.35 us,
+  // from here 32.3 (32.8).
+  constexpr bool kStoreHere = kQTerms == 2;
   auto bt_entry = [&](int64_t blk64, int e) -> int2 {
     const int pg = pg_first + e;
     const bool bad = blk64 < 0 || blk64 >= n_blocks_phys;
-    const int valid = e >= my_n ? -1 : bad ? 0 : (pg == last_pg ? len - pg * 16 : 16);
+    const int tokens = pg == last_pg ? len - pg * 16 : 16, valid = e >= my_n ? -1 : !bad ? tokens : kStoreHere ? 0 : -1 - tokens;
+    if (kDoK && kStoreHere && valid == 0) {
+      float* row = p.scores + (static_cast<int64_t>(b) * p.H_q + hkv * p.G) * p.max_S + pg * 16;
+#pragma unroll 1
+      for (int h = 0; h < p.G; ++h, row += p.max_S)
+#pragma unroll 1
+        for (int i = 0; i < tokens; ++i) row[i] = -INFINITY;
+    }
     return make_int2(static_cast<int>(head_page0 + (bad ? 0u : static_cast<uint32_t>(blk64))), valid);
   };
   // The copies of a slot's one or two pages, 16 bytes a lane: each half of the warp fetches a page
@@ -572,9 +583,22 @@ scan_k3v2_kernel(const ScanParams p) {
     const int4 ent = ent_s[(it >> 1) & (kBtChunk - 1)];   // the round's parked entries are still resident
     if (ent.y + ent.w == 32)
       k3v2_round<kQTerms, false, kParts, kNarrow, kSplitQ>(st, sb, off, g, 16, 16, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store, lane);
-    else
+    else {
       k3v2_round<kQTerms, true, kParts, kNarrow, kSplitQ>(st, sb, off, g, ent.y, ent.w, attn, row0, row1, at, st0, st1, pm_row, pm_at, pm_store,
                                         lane);
+      if (kDoK && !kStoreHere && min(ent.y, ent.w) < -1) {
+        const int na = -1 - ent.y, nb = -1 - ent.w;
+        float* const s0 = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(row0) + at);
+        for (int h = 0; h < 2; ++h) {
+          float* const s = s0 + (h ? p.max_S : 0);
+          if (!(h ? st1 : st0)) continue;
+          if (g < na) s[0] = -INFINITY;
+          if (g + 8 < na) s[8] = -INFINITY;
+          if (g < nb) s[16] = -INFINITY;
+          if (g + 8 < nb) s[24] = -INFINITY;
+        }
+      }
+    }
     at += 128u;
     pm_at += 4u;
     __syncwarp();

@@ -151,6 +151,8 @@ struct K4State {
   uint32_t s_off;             // byte offset of this lane's scale entries
 };
 
+constexpr int kNoBlock = 1 << 24;   // in a tile's mask: page A has no block (page B: the bit above)
+
 // One tile: two 16-token pages (the second may be absent) processed together, written out so
 // that the two pages' instruction streams interleave (the asm statements keep their program
 // order): all shared-memory loads first, the integer MMAs of both pages alternating, one
@@ -161,8 +163,8 @@ struct K4State {
 // `sbA / sbB` = shared-memory addresses of the pages' K tiles (V tiles follow at kVOff),
 // `ssA / ssB` = of their K scales (V scales follow at kVsOff).
 // kMasked: `mask` holds, per page, the range [lo, hi) of its 16 tokens that belong to this tile
-//   (the last page of a sequence, a page whose block id was invalid, a page cut by a boundary of
-//   the reference's splits, an absent second page); tokens outside score -inf and weigh nothing.
+//   (the last page of a sequence, a page cut by a boundary of the reference's splits, an absent
+//   second page), and whether the page has a block; tokens outside and tokens without a block score -inf and weigh nothing.
 // kInt8P: the weights follow the reference's batch > 1 Stage B for this mode
 //   (jetfire_vllm/csrc/int8tc_softmax_v_fused.cu:1203-1235): per tile of 32 tokens and query
 //   head, pv = p * v_scale is rounded to 127 levels of the tile's largest pv before it meets V.
@@ -177,12 +179,14 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
                                           int mask, int t0, float attn, float* spA0, float* spA1, bool st0, bool st1,
                                           bool want_pm, float* pm, int lane) {
   constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
-  bool aLo = true, aHi = true, bLo = true, bHi = true;   // is this lane's token of page A / B (rows g, g + 8) in the tile
+  bool inA0 = true, inA8 = true, inB0 = true, inB8 = true;   // is this lane's token of page A / B (rows g, g + 8) in the tile
   if (kMasked) {
     const int loA = mask & 31, hiA = (mask >> 5) & 31, loB = (mask >> 10) & 31, hiB = (mask >> 15) & 31;
-    aLo = t0 >= loA && t0 < hiA;  aHi = t0 + 8 >= loA && t0 + 8 < hiA;
-    bLo = t0 >= loB && t0 < hiB;  bHi = t0 + 8 >= loB && t0 + 8 < hiB;
+    inA0 = t0 >= loA && t0 < hiA;  inA8 = t0 + 8 >= loA && t0 + 8 < hiA;
+    inB0 = t0 >= loB && t0 < hiB;  inB8 = t0 + 8 >= loB && t0 + 8 < hiB;
   }
+  const bool hasA = !kMasked || !(mask & kNoBlock), hasB = !kMasked || !(mask & (kNoBlock << 1));
+  const bool aLo = inA0 && hasA, aHi = inA8 && hasA, bLo = inB0 && hasB, bHi = inB8 && hasB;   // ... and has it a cache row
   float* spB0 = spA0 + 16;
   float* spB1 = spA1 + 16;
   float sA[4] = {0.f, 0.f, 0.f, 0.f}, sB[4] = {0.f, 0.f, 0.f, 0.f};
@@ -256,14 +260,14 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
   }
   if (kDoK) {
     if (kMasked) {
-      if (st0 && aLo) spA0[0] = sA[0];
-      if (st0 && aHi) spA0[8] = sA[2];
-      if (st0 && bLo) spB0[0] = sB[0];
-      if (st0 && bHi) spB0[8] = sB[2];
-      if (st1 && aLo) spA1[0] = sA[1];
-      if (st1 && aHi) spA1[8] = sA[3];
-      if (st1 && bLo) spB1[0] = sB[1];
-      if (st1 && bHi) spB1[8] = sB[3];
+      if (st0 && inA0) spA0[0] = sA[0];
+      if (st0 && inA8) spA0[8] = sA[2];
+      if (st0 && inB0) spB0[0] = sB[0];
+      if (st0 && inB8) spB0[8] = sB[2];
+      if (st1 && inA0) spA1[0] = sA[1];
+      if (st1 && inA8) spA1[8] = sA[3];
+      if (st1 && inB0) spB1[0] = sB[1];
+      if (st1 && inB8) spB1[8] = sB[3];
     } else {
       if (st0) { spA0[0] = sA[0]; spA0[8] = sA[2]; spB0[0] = sB[0]; spB0[8] = sB[2]; }
       if (st1) { spA1[0] = sA[1]; spA1[8] = sA[3]; spB1[0] = sB[1]; spB1[8] = sB[3]; }
@@ -381,12 +385,13 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
                                                  float* sp1, bool st0, bool st1, bool want_pm, float* pm, int lane) {
   constexpr bool kDoK = kParts != 2, kDoV = kParts != 1;
   const int page = (lane >> 1) & 1;
-  bool lo = true, hi = true;   // are this lane's tokens (rows g, g + 8) in the tile
+  bool in0 = true, in8 = true;   // are this lane's tokens (rows g, g + 8) in the tile
   if (kMasked) {
     const int range = mask >> (10 * page), first = range & 31, end = (range >> 5) & 31;
-    lo = t0 >= first && t0 < end;
-    hi = t0 + 8 >= first && t0 + 8 < end;
+    in0 = t0 >= first && t0 < end;
+    in8 = t0 + 8 >= first && t0 + 8 < end;
   }
+  const bool has = !kMasked || !(mask & (kNoBlock << page)), lo = in0 && has, hi = in8 && has;   // ... and have they cache rows
   constexpr int kB = T4::kPageBytes;   // page B's tiles, from page A's
   const uint32_t sa = ss + st.s_off;
   float sc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -440,8 +445,8 @@ __device__ __forceinline__ void k4v4_tile_narrow(K4State& st, uint32_t sb, uint3
     if (!hi) { sc[2] = sc[3] = -INFINITY; vs1 = 0.f; }
   }
   if (kDoK) {
-    if (st0) { if (lo) sp0[0] = sc[0]; if (hi) sp0[8] = sc[2]; }
-    if (st1) { if (lo) sp1[0] = sc[1]; if (hi) sp1[8] = sc[3]; }
+    if (st0) { if (in0) sp0[0] = sc[0]; if (in8) sp0[8] = sc[2]; }
+    if (st1) { if (in0) sp1[0] = sc[1]; if (in8) sp1[8] = sc[3]; }
   }
   float mx0 = fmaxf(sc[0], sc[2]), mx1 = fmaxf(sc[1], sc[3]);
   if (kDoK && want_pm) {
@@ -570,7 +575,7 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
   const int head_row0 = static_cast<int>(static_cast<int64_t>(hkv >> p.kv_shift) * p.num_slots);  // first cache row of this KV head
 
   // Tile T of the warp (tile t_first + T of the row): its first page and the token ranges of its
-  // pages, packed as lo_A | hi_A << 5 | lo_B << 10 | hi_B << 15 | pages << 20 | cut flags << 22; 0 = no such tile
+  // pages, packed as lo_A | hi_A << 5 | lo_B << 10 | hi_B << 15 | pages << 20 | cut flags << 22 (| kNoBlock); 0 = no such tile
   // (past the warp's range or past the sequence; such tiles are a suffix of the range).
   auto tile_geom = [&](int T, int& pageA) -> int {
     const int gT = t_first + T;
@@ -616,12 +621,12 @@ scan_k4v4_kernel(const ScanParams p, const __grid_constant__ CUtensorMap k_map,
     }
     return r;
   };
-  // an invalid block id reads block 0 and counts no live token
+  // an invalid block id reads block 0 and its tokens score -inf
   auto desc_make = [&](const Pending& r) -> int4 {
     int mask = r.mask;
     const bool badA = r.ba < 0 || r.ba >= n_blocks_phys, badB = r.bb < 0 || r.bb >= n_blocks_phys;
-    if (badA) mask &= ~0x3FF;
-    if (badB) mask &= ~(0x3FF << 10);
+    if (mask && badA) mask |= kNoBlock;
+    if (((mask >> 20) & 3) == 2 && badB) mask |= kNoBlock << 1;
     const int rowA = head_row0 + static_cast<int>(badA ? 0 : r.ba) * 16;
     const int rowB = ((mask >> 20) & 3) == 2 ? head_row0 + static_cast<int>(badB ? 0 : r.bb) * 16 : -1;
     return make_int4(rowA, rowB, mask, r.pageA);
