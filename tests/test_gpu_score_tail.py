@@ -51,3 +51,23 @@ def test_row_statistics(max_S):
             # exp's bound of 2 + |x| units in fp32 and a sum of positive terms: 2e-5 for scores within 15 of the maximum's
             want = 1.0 / torch.exp(row - row.max()).sum()
             assert abs(float(inv[b, h]) - float(want)) <= 2e-5 * float(want)
+
+
+@pytest.mark.parametrize("mode", ["k3v2", "k4v4"])
+@pytest.mark.parametrize("B,H_q,H_kv,max_S", [(4, 8, 2, 97), (3, 8, 2, 1022), (3, 16, 2, 4003),
+                                              (64, 16, 2, 131071)])   # more than 512 MB of scores: a kernel of its own
+def test_tails_at_every_alignment(mode, B, H_q, H_kv, max_S):
+    from jetfire_b200 import ops
+    g = torch.Generator().manual_seed(B)
+    lens = [max(0, n) for n in (max_S - 1, 0, 1, max_S - 5, 7, max_S // 2 + 1, max_S, 18)][:min(B, 8)]
+    lens = torch.tensor((lens * B)[:B], dtype=torch.int32)
+    table = torch.randint(0, 256, (B, (max_S + 15) // 16), generator=g)
+    row = {"k3v2": (48, 2), "k4v4": (64, 1)}[mode]
+    kd = torch.randint(0, 256, (H_kv, 4096, row[0]), dtype=torch.uint8, generator=g)
+    ks = torch.rand(H_kv, 4096, row[1], generator=g).bfloat16()
+    q = torch.randn(B, H_q, 128, generator=g).bfloat16()
+    stage_a = ops.int3_qk_scores_topk if mode == "k3v2" else ops.int8tc_qk_scores_topk_stats
+    scores = stage_a(q.cuda(), kd.cuda(), ks.cuda(), table.cuda(), lens.cuda(), max_S, H_q, H_kv, 16, 0.1, 8)[0]
+    past = torch.arange(max_S, device="cuda") >= lens.cuda()[:, None]
+    for b in range(B):
+        assert torch.isneginf(scores[b][:, past[b]]).all() and torch.isfinite(scores[b][:, ~past[b]]).all()
