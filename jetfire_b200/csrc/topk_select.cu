@@ -29,7 +29,9 @@
 // Run-time loops are not unrolled: they go round once or twice, by four with their remainders the kernel was
 // 153 KB of code, more than the instruction cache (111 KB now; a fused call of 32 rows of 2048: 16.3 -> 15.7 us,
 // K4V4 14.6 -> 13.6, 128 rows of 8192: 24.95 -> 24.6, 512 of 16384: 90.9 -> 89.5, steps of them 0.6-3 us less).
-// A third of the stalls of a row on its own multiprocessor still wait for instructions.
+// A third of the stalls of a row on its own multiprocessor still wait for instructions.  The one exception counts the better
+// candidates of a bin: rows of ties have hundreds in one (not unrolled / unrolled, K4V4 32 rows of 32768 of 64 keys, top-k
+// 512: 92.4 / 62.0 us; 256 of 4096 of eight keys 56.7 / 44.2; other rows the same).
 #include <algorithm>
 
 #include "finish_tail.cuh"
@@ -1199,7 +1201,6 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
             }
             left[k] &= lo < K;   // a rank past the last one is as good as any other
           } else {
-#pragma unroll 1
             for (int m = lo; m < hi2; ++m) above += (keys[bucket[m]] > mine[k]) ? 1 : 0;
           }
           if (left[k]) late.close[atomicAdd(&sm.nlist, 1)] = static_cast<uint16_t>(c);
