@@ -44,7 +44,7 @@ decode_finish_kernel(const FinishParams p, const TailParams tp) {
   const int n = min(p.seq_lens[b], tp.max_S);
   const float M = block_max_of_splits<kFinishThreads>(tp.part_m, pbase, hi, n_splits, sm_m);
   merge_splits(tp, splits, pbase, n_splits, hi, M);
-  finish_tail<MODE, kFinishThreads, false>(tp, tsm, TailPrefetch{}, splits, M, n, b, h,
+  finish_tail<MODE, kFinishThreads, false, tail_rounds(MODE, true)>(tp, tsm, TailPrefetch{}, splits, M, n, b, h,
                                         p.block_table + static_cast<int64_t>(b) * p.max_blocks, [&](int kk, int& pos, int& cidx) {
                                           const int64_t v = kk == first ? first_sel : sel[kk];
                                           if (v < 0 || v >= n) return false;

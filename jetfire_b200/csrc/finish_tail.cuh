@@ -100,9 +100,14 @@ struct TailPrefetch {
 
 __device__ __forceinline__ uint32_t f16_bits_sat(float x) { return pack_f16x2_sat(x, 0.f) & 0xFFFFu; }
 
+// Rounds in flight where a warp may have many and reads them from global memory (`many`: the stand-alone kernel, and the block of
+// top-k above 512).  K4V4 gains by it, K3V2, with twice the arithmetic an entry, loses.  Four / one, us: the finish of 256 rows, top-k
+// 2048, 40.3 / 47.2 (K3V2 51.8 / 43.1), of 512 12.9 / 14.1 (16.2 / 14.7); scan + select of 256 rows of 32768, top-k 4096, 344 / 354 (386 / 383).
+__host__ __device__ constexpr int tail_rounds(int mode, bool many) { return mode == JF_MODE_K4V4 && many ? 4 : 1; }
+
 // PPW channel ranges (part0 ...) of the selected set's weighted V sum, by one warp: groups of sixteen
 // entries g0, g0 + step, ... of `top_k`.  `row(e)` = address of entry e's packed V row.
-template <int MODE, int PPW, typename RowFn>
+template <int MODE, int PPW, int kRounds, typename RowFn>
 __device__ __forceinline__ void tail_part(const TailSmem<MODE>& sm, float* red, int part0, int g0, int step, int top_k, RowFn row) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
   constexpr int NT_ = (MODE == JF_MODE_K3V2) ? 4 : 2;   // output tiles per part, and one for the sum of weights
@@ -115,7 +120,7 @@ __device__ __forceinline__ void tail_part(const TailSmem<MODE>& sm, float* red, 
   const int e_a = (MODE == JF_MODE_K3V2) ? tig : ((2 * tig >> 2) & 1) | (((2 * tig >> 1) & 1) << 2) | ((2 * tig & 1) << 1);
   const int e_b = (MODE == JF_MODE_K3V2) ? tig + 4
                                          : (((2 * tig + 1) >> 2) & 1) | ((((2 * tig + 1) >> 1) & 1) << 2) | (((2 * tig + 1) & 1) << 1);
-#pragma unroll 1
+#pragma unroll kRounds
   for (int grp = g0; 16 * grp < top_k; grp += step) {
     const int e0 = 16 * grp;   // entries past top_k have a place in the arrays and weigh nothing
     const uint8_t *ra = row(e0 + e_a), *rb = row(e0 + e_b), *rc = row(e0 + e_a + 8), *rd = row(e0 + e_b + 8);
@@ -193,7 +198,7 @@ __device__ __forceinline__ void tail_part(const TailSmem<MODE>& sm, float* red, 
 // index in the prefetched arrays; false if there is no such entry.  PRE: the prefetched arrays are there.
 // M = max over the splits of the scan's reference points.  n = sequence length.  `splits` = the merged
 // partials, written before the block's last barrier or by the same threads as here.
-template <int MODE, int NT, bool PRE, typename Src>
+template <int MODE, int NT, bool PRE, int kRounds, typename Src>
 __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>& sm, const TailPrefetch& pf,
                                             const SplitSums& splits, float M, int n, int b, int h, const int64_t* bt, Src src) {
   constexpr int VW = TailSmem<MODE>::VW, kRows = TailSmem<MODE>::kRows;
@@ -207,7 +212,7 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
   const float* srow = p.scores + bh * p.max_S;
 
   // ---- selected set: weights from the scan's scores, 32 entries per warp and step ----
-#pragma unroll 1
+#pragma unroll kRounds
   for (int k0 = 32 * warp; k0 < p.top_k; k0 += NT) {
     const int kk = k0 + lane;
     int ref = 0;
@@ -255,10 +260,10 @@ __device__ __forceinline__ void finish_tail(const TailParams& p, TailSmem<MODE>&
     const int r = warp % kRows, part0 = (warp / kRows) * PPW;
     if (r < groups) {
       if (PRE)
-        tail_part<MODE, PPW>(sm, sm.red[r], part0, r, kRows, p.top_k,
+        tail_part<MODE, PPW, kRounds>(sm, sm.red[r], part0, r, kRows, p.top_k,
                              [&](int e) { return reinterpret_cast<const uint8_t*>(pf.vrows + sm.ref[e] * VW); });
       else
-        tail_part<MODE, PPW>(sm, sm.red[r], part0, r, kRows, p.top_k,
+        tail_part<MODE, PPW, kRounds>(sm, sm.red[r], part0, r, kRows, p.top_k,
                              [&](int e) { return v_rows + static_cast<int64_t>(sm.ref[e]) * (4 * VW); });
     }
   }

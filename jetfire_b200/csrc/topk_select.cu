@@ -1294,9 +1294,9 @@ topk_select_kernel(const TopkParams p, const TailParams tp) {
     };
     if (prefetch) {
       const TailPrefetch pf{late.cand_slot, cand_score, late.vsc, late.vrows};
-      finish_tail<MODE, NT, true>(tp, late.tail, pf, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
+      finish_tail<MODE, NT, true, 1>(tp, late.tail, pf, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
     } else {
-      finish_tail<MODE, NT, false>(tp, late.tail, TailPrefetch{}, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
+      finish_tail<MODE, NT, false, tail_rounds(MODE, NT == kSelThreads)>(tp, late.tail, TailPrefetch{}, sm.splits, row_max, n_seq, b, h, ctx.bt, entry);
     }
   }
 }
