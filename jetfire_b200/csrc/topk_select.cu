@@ -42,8 +42,7 @@ namespace {
 
 constexpr int kBins = 2048;
 constexpr float kBinsPerUnit = 64.0f;
-constexpr int kCloseTopK = 256;   // see launch_select_block
-constexpr int64_t kL2Bytes = 126ll << 20, kK3RowBytes = 88;   // packed K and V of a position and KV head
+constexpr int kCloseTopK = 256, kCutTopK = 384;   // see launch_select_block
 
 struct TopkParams {
   const float* scores;
@@ -1352,13 +1351,14 @@ jf_status_t launch_select_block(const jf_decode_args* a, TopkParams& sp, const T
   if constexpr (MODE == JF_MODE_K3V2 && NT == 512 && VEC == 8) {
     if (static_cast<int>(grid.x * grid.y) > num_sms()) {
       if (a->top_k <= kCloseTopK) return launch_select_variant<MODE, LEAN, NT, VEC, kClose>(sp, tp, grid, smem, stream, fused);
-      // A wider top-k of a cache that does not stay in L2: candidates are cut down before their rows are fetched from DRAM.
-      // Scan + select, us, 512 of 65536 x 256 rows (185 MB) 98.2 / 96.3, of 50000 x 512 (282 MB) 180.3 / 180.3; of 32761
-      // falling x 256 (92 MB) 65.1 / 65.7.  (Not worth it at 256, where the rest is half as much: 84.3 / 85.4; nor for staged rows: 4096 x
-      // 512 62.5 / 64.9.)
+      // Of a wide top-k the candidates are cut down before their rows are fetched.  A step, us, without / with, at a top-k of
+      //   512: 256 rows of 65536 102.2 / 100.5, 512 189.2 / 186.6, 6 falling lengths x 32 rows 112.2 / 104.4, 256 of 131072 158.7 / 157.8
+      //   448: 256 of 57344 134.7 / 133.2;  400: of 65536 96.4 / 96.3, falling from 51200 102.8 / 100.5;  384: falling from 65536 118.5 / 116.9
+      //   320: 256 of 65536 92.3 / 92.4, fp16 100.5 / 100.9;  257: 90.3 / 91.1, 200 of 33008 76.0 / 77.0
+      // The fewer entries, the less there is to leave out; a pass over the candidates costs the same.  (Where the cache stays in L2
+      // there is next to nothing in it either way: 160 rows of 65536, 512, 115 MB 78.2 / 78.0, 58 MB 73.8 / 73.8.)
       if constexpr (LEAN) {
-        if (static_cast<int64_t>(a->B) * a->H_kv * a->max_S * kK3RowBytes > kL2Bytes)
-          return launch_select_variant<MODE, LEAN, NT, VEC, kCut>(sp, tp, grid, smem, stream, fused);
+        if (a->top_k >= kCutTopK) return launch_select_variant<MODE, LEAN, NT, VEC, kCut>(sp, tp, grid, smem, stream, fused);
       }
     }
   }

@@ -27,7 +27,7 @@ CASES = [
     ("k3v2", "fp32", 2, 16, 2, 2001, 64, torch.float16),
     ("k3v2", "fp32", 1, 8, 2, 40000, 64, torch.bfloat16),      # from page maxima
     ("k3v2", "fp32", 5, 32, 2, 1600, 64, torch.float16),       # rows share a multiprocessor: close candidates re-scored
-    ("k3v2", "fp32", 6, 32, 8, 33008, 257, torch.bfloat16),    # and a cache beyond L2: candidates cut down first
+    ("k3v2", "fp32", 6, 32, 8, 33008, 257, torch.bfloat16),    # from page maxima, every candidate re-scored
     ("k4v4", "fp32", 1, 8, 2, 2001, 64, torch.bfloat16),
     ("k4v4", "int8p", 3, 8, 2, 6007, 64, torch.bfloat16),
     ("k4v4", "int8p", 2, 16, 2, 6007, 64, torch.bfloat16),
