@@ -36,8 +36,10 @@ __host__ __device__ inline HeadGeom head_geom(int H_q, int H_kv) {
   return HeadGeom{H_kv << shift, G >> shift, shift};
 }
 
-// Query heads of a KV head up to which the K3V2 scan repeats them on its unused columns (scan_k3v2_kernel, kNarrow).
+// Query heads of a KV head up to which both scans use the other four of the eight columns too (kNarrow: scan_k3v2_kernel
+// repeats the heads there, scan_k4v4_kernel has a tile's second page there).
 constexpr int kNarrowGroup = 4;
+static_assert(kNarrowGroup <= kHeadsPad / 2, "columns 4-7 are free");
 // Resident scan CTAs per SM (set by registers / shared memory of the kernel variant); G: query heads per (virtual) KV head.
 __host__ __device__ inline int scan_ctas_per_sm(int mode, int q_dtype, int G) {
   return (mode == JF_MODE_K3V2 && q_dtype == JF_DTYPE_FP16 && G > kNarrowGroup) ? 3 : 4;
