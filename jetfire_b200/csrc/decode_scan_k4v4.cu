@@ -375,7 +375,9 @@ __device__ __forceinline__ void k4v4_tile(K4State& st, uint32_t sbA, uint32_t sb
 // P.V and the softmax sums add in the order of k4v4_tile, to the same bits: page A meets the weights as they lie, page B the
 // same turned round by four columns, both in columns 0-3 (4-7 hold what nobody reads).  (Sums kept apart by page until the end
 // of the loop saved two MMAs' turns, and nothing in time: 16 x 131072 the scan alone 462 / 465 us, 4 x 32768 30.5 / 30.3; but where
-// sum(P * code) and 8 * sum(P) nearly cancel, outputs of few and of many heads to a group differed by 4e-4.)
+// sum(P * code) and 8 * sum(P) nearly cancel, outputs of few and of many heads to a group differed by 4e-4.  Against 64 bits
+// o_hat of 131072 positions is then off by 5e-4 of itself, wide groups and this by 1e-3; of 32768 by 2.1e-4 either way.)
+// 253 warp instructions a page, 275 with the columns half empty.
 // 32 / 8 heads, with the columns half empty / like this, scan + select, us: 4 x 32768 42.9 / 42.2, 16 x 131072 506 / 500, 1 x 2048 13.4 /
 // 13.3 (the scan of 16 x 131072 alone 473 / 465: instruction issue counts where many tiles follow one another, its chain
 // elsewhere).  Trading the two heads' maxima instead of reducing both: the same.  Groups of five to eight heads have no empty columns.

@@ -27,7 +27,7 @@
 // 32768 positions 30.9 k -> 24.7 k; 256 rows of 65536 (top-k 512): 60.0 k -> 54.2 k, bound by the
 // scattered reads of the candidates' rows (0.7 M accesses of 64 bytes a layer).
 // Run-time loops are not unrolled: they go round once or twice, by four with their remainders the kernel was
-// 153 KB of code, more than the instruction cache (111 KB now; a fused call of 32 rows of 2048: 16.3 -> 15.7 us,
+// 153 KB of code, more than the instruction cache (111 KB without, before the kinds of rows; a fused call of 32 rows of 2048: 16.3 -> 15.7 us,
 // K4V4 14.6 -> 13.6, 128 rows of 8192: 24.95 -> 24.6, 512 of 16384: 90.9 -> 89.5, steps of them 0.6-3 us less).
 // A third of the stalls of a row on its own multiprocessor still wait for instructions.  The one exception counts the better
 // candidates of a bin: rows of ties have hundreds in one (not unrolled / unrolled, K4V4 32 rows of 32768 of 64 keys, top-k
